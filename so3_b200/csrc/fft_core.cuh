@@ -17,6 +17,28 @@ namespace so3g {
 
 constexpr int kMaxPasses = 16;
 
+// Plan of the tensor-core DFTs (dft_mm.cuh).
+struct MmLevel {       // one matrix DFT of length p
+  int p, H;            // H = p / 2 pairs (reduction entries)
+  int KS, QT;          // 4-entry reduction steps, 8-row output tiles (rows q0..H)
+  int q0;              // 1: X_0 is summed apart (H a multiple of 8)
+  int MT, QG;          // row tiles per warp task, tasks per column tile
+  const double2* tab;  // fragments [QT][KS][lane]: (cos, sin)(2 pi q r / p), q = 8 t + lane / 4 + q0, r = 4 s + lane % 4 + 1
+};
+struct MmPlan {
+  int n;               // transform length (0: no plan)
+  int kind;            // 1: one level, 2: two levels a * b, 3: cyclic convolution of length m = a * b
+  int m, rader;        // kind 3: Rader (m = n - 1) or Bluestein (m >= 2n - 1)
+  int a, b, lda, ldb;  // split and row pitches (complex slots, 2 or 6 mod 8)
+  unsigned mdiv_a, mdiv_b;
+  int ts;              // slots of one sequence in a buffer
+  MmLevel la, lb;
+  const double2* tw;     // e^{-2 pi i n2 k1 / m}, [n2 < b][k1 < a]
+  const double2* chirp;  // e^{-i pi k^2 / n}, k < n (Bluestein)
+  const double2* kern;   // DFT_m of the convolution kernel / m
+  const int* perm;       // Rader: g^j mod n, then g^{-j} mod n (j < m)
+};
+
 struct FftPlan {
   int n;                     // transform length
   int npass;                 // Stockham passes for length n (0 if Bluestein)
@@ -35,6 +57,8 @@ struct FftPlan {
   const double2* rroots;     // e^{-2 pi i k/(n-1)}, k < n-1
   const double2* rkern;      // FFT_{n-1}(e^{-2 pi i 3^{-m}/n}) / (n-1)
   const int* rperm;          // [0, n-1): 3^a mod n (gather); [n-1, 2n-2): 3^{-b} mod n (scatter)
+  MmPlan mm;                 // tensor-core plan of the same length (n = 0: none)
+  MmLevel l1;                // one-level tables of length n (p = 0: none), the gamma stages
   int ld() const { return blue ? m : n; }
   // any radix above 8 (needs the large-radix kernel instances)
   bool big() const {

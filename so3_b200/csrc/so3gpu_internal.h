@@ -92,6 +92,9 @@ struct DevPlan {
   FftPlan plan{};
   double2* mem = nullptr;  // owns roots/mroots/chirp/kern/half/rroots/rkern
   int* imem = nullptr;     // owns rperm
+  double2* mm_mem = nullptr;  // own the tensor-core plan's tables
+  int* mm_imem = nullptr;
+  size_t mm_bytes = 0;
 };
 
 // Resident int8 digits of the split-precision contractions' Delta products
@@ -165,6 +168,9 @@ Device* device_state(int device);  // lazily created per CUDA device
 
 int ensure_dl(Device* D, int L, int method, cudaStream_t s, const double** out);
 int ensure_fft(Device* D, int n, FftPlan* out);
+// Tensor-core plan of length n into F->mm and F->l1 (dft_plan.cpp); the caller
+// owns *mem and *imem (device memory, *bytes in total).
+int build_mm_plan(int n, FftPlan* F, double2** mem, int** imem, size_t* bytes);
 int ensure_conv_kernel(Device* D, const Geometry& g, const double2** out);
 int ensure_bases(Device* D, const so3_parameters_t& p, int real, const long long** out);
 int ensure_ws(Workspace* W, size_t bytes, void** out);
@@ -211,6 +217,17 @@ int launch_fwd_gamma(const Geometry& g, const FftPlan& pg, const void* f, double
 int launch_fwd_alpha(const Geometry& g, const FftPlan& pP, double2* W, cudaStream_t s);
 int launch_fwd_beta_conv(const Geometry& g, const FftPlan& pP, const FftPlan& pc, const double2* wr,
                          double2* W, cudaStream_t s);
+
+// The same stages on the FP64 tensor cores (stages_mm.cu), for plans that
+// build_mm_plan covered.
+bool mm_gamma_ok(const Geometry& g, const FftPlan& p);
+bool mm_ok(const FftPlan& p);
+int launch_mm_inv_gamma(const Geometry& g, const FftPlan& p, const double2* W, void* f, cudaStream_t s, int row_lo,
+                        int row_hi);
+int launch_mm_fwd_gamma(const Geometry& g, const FftPlan& p, const void* f, double2* W, cudaStream_t s, int row_lo,
+                        int row_hi);
+int launch_mm_alpha(const Geometry& g, const FftPlan& p, double2* W, bool inverse, cudaStream_t s);
+int launch_mm_inv_beta(const Geometry& g, const FftPlan& p, double2* W, cudaStream_t s);
 
 // Beta stages of the adjoint transforms (MW, complex; stages.cu).  Inverse
 // adjoint: per column of the row-major part, zero-extend the nb beta samples

@@ -1,0 +1,534 @@
+// DFT stages of the transforms on the FP64 tensor cores (dft_mm.cuh): the
+// same stages as stages.cu, any length the planner covers.
+//
+// Measured against the scalar engines of stages.cu (us, one transform):
+//   gamma    L=512 N=64 (127)    769 -> 744 inverse, 800 -> 705 forward
+//            L=512 N=16 (31)    1125 -> 135, 1182 -> 127
+//            L=256 N=32 real     156 -> 59,   179 -> 92
+//   alpha    L=128 N=16 (255)     43 -> 23;  L=256 N=16 (511) 339 -> 78
+//            L=300 N=16 (599)    737 -> 190; L=1024 N=8 (2047) 3774 -> 525
+//   inv beta L=256 N=16 320 -> 103; L=300 N=16 791 -> 227; L=1024 N=8 3635 -> 758
+// What bounds them now: gamma at N = 64 the tensor pipe (0.47 ms of products),
+// at small N the memory system; alpha and beta instruction issue and latency
+// (ncu at 1023: 43 % of issue slots, 40 % of the FP64 pipe, 21 warps per SM).
+#include <algorithm>
+
+#include "dft_mm.cuh"
+#include "so3gpu_internal.h"
+
+namespace so3g {
+
+namespace {
+
+constexpr int kGT = 128;               // threads of the gamma kernels
+constexpr size_t kSmemMax = 200 * 1024;
+constexpr int kMaxThr = 256, kMinB = 3;  // alpha / beta kernels: 80 registers a thread, 24 warps per SM
+constexpr int kMaxT = 16;              // sequences per CTA
+
+template <typename K>
+int set_smem(K kernel, size_t bytes) {
+  SO3G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  return kOk;
+}
+
+int launched() {
+  SO3G_LAUNCHED();
+  SO3G_CUDA(cudaGetLastError());
+  return kOk;
+}
+
+__device__ __forceinline__ long long row_off(const Geometry& g, int row) {
+  return (long long)(row / g.nb) * g.PS + (long long)(row % g.nb) * g.RS;
+}
+
+// ------------------------------------------------------------------ gamma
+// One matrix level over the planes: a CTA holds TA consecutive alpha samples
+// of one beta row of every plane, row pitch TA + 2 slots (2 mod 8).
+//
+struct InvGammaOut {
+  double2* dst;
+  long long plane_sz;
+  int nf;
+  __device__ __forceinline__ double2* col(int j) const { return dst + j; }
+  __device__ __forceinline__ void put(double2* d, int q, double2 v) const {
+    if (q < nf) d[q * plane_sz] = v;
+  }
+};
+struct FwdGammaOut {
+  double2* dst;
+  long long PS;
+  double scale;
+  int N, ng, plane0, steer;
+  __device__ __forceinline__ double2* col(int j) const { return dst + j; }
+  __device__ __forceinline__ void put(double2* d, int k, double2 v) const {
+    const int n = k < N ? k : k - ng;
+    if (n + plane0 < 0) return;  // k = N of the 2N-point circle: no plane
+    const bool keep = !steer || ((n - (N - 1)) & 1) == 0;
+    d[(n + plane0) * PS] = keep ? cscale(v, scale) : make_double2(0.0, 0.0);
+  }
+};
+
+// Complex inverse: circle entry r holds plane n = r (r < N) or r - ng; the
+// 2N-point circle of a steerable signal has no plane n = N and keeps N samples.
+__global__ void __launch_bounds__(kGT, 4) inv_gamma_mm_kernel(Geometry g, MmLevel lv, const double2* __restrict__ W,
+                                                         double2* __restrict__ f, int tash, int row0) {
+  extern __shared__ __align__(16) double2 sm[];
+  const int TA = 1 << tash, rp = TA + 2;
+  const int row = row0 + blockIdx.y, a0 = blockIdx.x << tash, ng = g.ng, nc = min(TA, g.na - a0);
+  const double2* src = W + (long long)row * g.RS + a0;
+  for (int i = threadIdx.x; i < g.nplanes << tash; i += kGT) {
+    const int p = i >> tash, c = i & (TA - 1);
+    int r = p - g.plane0;
+    if (r < 0) r += ng;
+    if (c < nc) mm::cp16(sm + r * rp + c, src + (long long)p * g.PS + c);
+  }
+  if (g.steer)
+    for (int c = threadIdx.x; c < TA; c += kGT) sm[g.N * rp + c] = make_double2(0.0, 0.0);
+  mm::cp_wait_all();
+  __syncthreads();
+  const long long plane_sz = (long long)g.nb * g.na;
+  double2* dst = f + (long long)row * g.na + a0;
+  mm::level<4, true>(sm, rp, lv, nc, [](int j) { return j; }, InvGammaOut{dst, plane_sz, g.nf});
+}
+
+// Complex forward; steerable: samples N..2N-1 of the circle are zero and only
+// n = N-1 (mod 2) is analysed (so3_core.c:309-328).
+__global__ void __launch_bounds__(kGT, 4) fwd_gamma_mm_kernel(Geometry g, MmLevel lv, const double2* __restrict__ f,
+                                                         double2* __restrict__ W, int tash, int row0) {
+  extern __shared__ __align__(16) double2 sm[];
+  const int TA = 1 << tash, rp = TA + 2;
+  const int row = row0 + blockIdx.y, a0 = blockIdx.x << tash, ng = g.ng, nc = min(TA, g.na - a0);
+  const long long plane_sz = (long long)g.nb * g.na;
+  const double2* src = f + (long long)row * g.na + a0;
+  for (int i = threadIdx.x; i < ng << tash; i += kGT) {
+    const int r = i >> tash, c = i & (TA - 1);
+    if (r >= g.nf)
+      sm[r * rp + c] = make_double2(0.0, 0.0);
+    else if (c < nc)
+      mm::cp16(sm + r * rp + c, src + (long long)r * plane_sz + c);
+  }
+  mm::cp_wait_all();
+  __syncthreads();
+  const double scale = 2.0 * 3.141592653589793238462643383279502884 / g.nf;
+  double2* dst = W + (long long)row * g.RS + a0;
+  mm::level<4, false>(sm, rp, lv, nc, [](int j) { return j; },
+            FwdGammaOut{dst, g.PS, scale, g.N, ng, g.plane0, g.steer});
+}
+
+// Real inverse (c2r): y(q) = Re x_0 + sum_r 2 Re x_r cos - 2 Im x_r sin over
+// the planes n = r >= 0; 8 real columns (alpha) per tile, so lane (g, c) of an
+// accumulator holds output q = g of columns 2c, 2c + 1.
+template <int MT>
+__device__ __forceinline__ void c2r_task(const double2* __restrict__ src, int rp, const MmLevel& lv, int qt0, int j0,
+                                         int nc, double* __restrict__ dst, long long plane_sz) {
+  constexpr int NT = 2;
+  const int lane = threadIdx.x & 31, kk = lane & 3, gr = lane >> 2, H = lv.H;
+  double a[MT][NT][2], b[MT][NT][2];
+  const double2* bp[NT];
+#pragma unroll
+  for (int t = 0; t < NT; t++) {
+    bp[t] = src + min(j0 + 8 * t + gr, nc - 1);
+    const int c0 = j0 + 8 * t + 2 * kk;
+#pragma unroll
+    for (int i = 0; i < MT; i++) {
+      a[i][t][0] = src[min(c0, nc - 1)].x;
+      a[i][t][1] = src[min(c0 + 1, nc - 1)].x;
+      b[i][t][0] = b[i][t][1] = 0.0;
+    }
+  }
+  const double2* tab = lv.tab + (size_t)qt0 * lv.KS * 32 + lane;
+#pragma unroll 2
+  for (int ks = 0; ks < lv.KS; ks++) {
+    const int r = min(4 * ks + kk + 1, H);
+    double2 x[NT];
+#pragma unroll
+    for (int t = 0; t < NT; t++) x[t] = cscale(bp[t][r * rp], 2.0);
+#pragma unroll
+    for (int i = 0; i < MT; i++) {
+      const double2 w = __ldg(tab + (i * lv.KS + ks) * 32);
+#pragma unroll
+      for (int t = 0; t < NT; t++) {
+        mm::dmma(a[i][t], w.x, x[t].x);
+        mm::dmma(b[i][t], w.y, x[t].y);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < MT; i++) {
+    const int q = 8 * (qt0 + i) + gr;
+    if (q > H) continue;
+#pragma unroll
+    for (int t = 0; t < NT; t++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int j = j0 + 8 * t + 2 * kk + e;
+        if (j >= nc) continue;
+        dst[(long long)q * plane_sz + j] = a[i][t][e] - b[i][t][e];
+        if (q) dst[(long long)(lv.p - q) * plane_sz + j] = a[i][t][e] + b[i][t][e];
+      }
+  }
+}
+
+__global__ void __launch_bounds__(kGT, 4) inv_gamma_real_mm_kernel(Geometry g, MmLevel lv,
+                                                              const double2* __restrict__ W, double* __restrict__ f,
+                                                              int tash, int row0) {
+  extern __shared__ __align__(16) double2 sm[];
+  const int TA = 1 << tash, rp = TA + 2;
+  const int row = row0 + blockIdx.y, a0 = blockIdx.x << tash, nc = min(TA, g.na - a0);
+  const double2* src = W + (long long)row * g.RS + a0;
+  for (int i = threadIdx.x; i < g.nplanes << tash; i += kGT) {
+    const int p = i >> tash, c = i & (TA - 1);
+    if (c < nc) mm::cp16(sm + p * rp + c, src + (long long)p * g.PS + c);
+  }
+  mm::cp_wait_all();
+  __syncthreads();
+  const long long plane_sz = (long long)g.nb * g.na;
+  double* dst = f + (long long)row * g.na + a0;
+  const int ng = lv.QG, tasks = (nc + 15) / 16 * ng;
+  for (int w = threadIdx.x >> 5; w < tasks; w += kGT / 32) {
+    const int qt0 = (w % ng) * lv.MT, j0 = (w / ng) * 16;
+    switch (min(lv.MT, lv.QT - qt0)) {
+      case 1: c2r_task<1>(sm, rp, lv, qt0, j0, nc, dst, plane_sz); break;
+      case 2: c2r_task<2>(sm, rp, lv, qt0, j0, nc, dst, plane_sz); break;
+      case 3: c2r_task<3>(sm, rp, lv, qt0, j0, nc, dst, plane_sz); break;
+      default: c2r_task<4>(sm, rp, lv, qt0, j0, nc, dst, plane_sz); break;
+    }
+  }
+}
+
+// Real forward (r2c): planes n = q = 0 .. N-1 of the samples, (a_q, -b_q).
+template <int MT>
+__device__ __forceinline__ void r2c_task(const double* __restrict__ src, int rp, const MmLevel& lv, int qt0, int j0,
+                                         int nc, double2* __restrict__ dst, long long PS, double scale) {
+  constexpr int NT = 2;
+  const int lane = threadIdx.x & 31, kk = lane & 3, gr = lane >> 2, H = lv.H;
+  double a[MT][NT][2], b[MT][NT][2];
+  const double* bp[NT];
+#pragma unroll
+  for (int t = 0; t < NT; t++) {
+    bp[t] = src + min(j0 + 8 * t + gr, nc - 1);
+    const int c0 = j0 + 8 * t + 2 * kk;
+#pragma unroll
+    for (int i = 0; i < MT; i++) {
+      a[i][t][0] = src[min(c0, nc - 1)];
+      a[i][t][1] = src[min(c0 + 1, nc - 1)];
+      b[i][t][0] = b[i][t][1] = 0.0;
+    }
+  }
+  const double2* tab = lv.tab + (size_t)qt0 * lv.KS * 32 + lane;
+#pragma unroll 2
+  for (int ks = 0; ks < lv.KS; ks++) {
+    const int r = min(4 * ks + kk + 1, H);
+    double s[NT], d[NT];
+#pragma unroll
+    for (int t = 0; t < NT; t++) {
+      const double xp = bp[t][r * rp], xn = bp[t][(lv.p - r) * rp];
+      s[t] = xp + xn;
+      d[t] = xp - xn;
+    }
+#pragma unroll
+    for (int i = 0; i < MT; i++) {
+      const double2 w = __ldg(tab + (i * lv.KS + ks) * 32);
+#pragma unroll
+      for (int t = 0; t < NT; t++) {
+        mm::dmma(a[i][t], w.x, s[t]);
+        mm::dmma(b[i][t], w.y, d[t]);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < MT; i++) {
+    const int q = 8 * (qt0 + i) + gr;
+    if (q > H) continue;
+#pragma unroll
+    for (int t = 0; t < NT; t++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int j = j0 + 8 * t + 2 * kk + e;
+        if (j < nc) dst[(long long)q * PS + j] = make_double2(a[i][t][e] * scale, -b[i][t][e] * scale);
+      }
+  }
+}
+
+// Sample rows of TA + 4 doubles (4 mod 16): 4 rows x 4 columns per half warp
+// in distinct banks.
+__global__ void __launch_bounds__(kGT, 4) fwd_gamma_real_mm_kernel(Geometry g, MmLevel lv,
+                                                              const double* __restrict__ f, double2* __restrict__ W,
+                                                              int tash, int row0) {
+  extern __shared__ __align__(16) double smd[];
+  const int TA = 1 << tash, rp = TA + 4;
+  const int row = row0 + blockIdx.y, a0 = blockIdx.x << tash, nc = min(TA, g.na - a0);
+  const long long plane_sz = (long long)g.nb * g.na;
+  const double* src = f + (long long)row * g.na + a0;
+  for (int i = threadIdx.x; i < g.ng << tash; i += kGT) {
+    const int r = i >> tash, c = i & (TA - 1);
+    if (c < nc) smd[r * rp + c] = __ldg(src + (long long)r * plane_sz + c);
+  }
+  __syncthreads();
+  const double scale = 2.0 * 3.141592653589793238462643383279502884 / g.nf;
+  double2* dst = W + (long long)row * g.RS + a0;
+  const int ng = lv.QG, tasks = (nc + 15) / 16 * ng;
+  for (int w = threadIdx.x >> 5; w < tasks; w += kGT / 32) {
+    const int qt0 = (w % ng) * lv.MT, j0 = (w / ng) * 16;
+    switch (min(lv.MT, lv.QT - qt0)) {
+      case 1: r2c_task<1>(smd, rp, lv, qt0, j0, nc, dst, g.PS, scale); break;
+      case 2: r2c_task<2>(smd, rp, lv, qt0, j0, nc, dst, g.PS, scale); break;
+      case 3: r2c_task<3>(smd, rp, lv, qt0, j0, nc, dst, g.PS, scale); break;
+      default: r2c_task<4>(smd, rp, lv, qt0, j0, nc, dst, g.PS, scale); break;
+    }
+  }
+}
+
+// ------------------------------------------------------------------ alpha
+// T consecutive rows (plane-major over the beta rows) per CTA, two buffers of
+// T sequences.  Inverse: column m + L - 1 of the row is entry m mod P (the
+// MWSS Nyquist entry is zero); forward: the other way round, over 1/P.
+template <bool INV>
+struct AlphaOut {
+  double2* const* rows;
+  double inv;
+  int L, P;
+  typedef double2* Seq;
+  __device__ __forceinline__ Seq seq(int t) const { return rows[t]; }
+  __device__ __forceinline__ void put(Seq d, int k, double2 v) const {
+    if (INV) {
+      d[k] = v;
+    } else {
+      const int c = k < L ? k + L - 1 : k - P + L - 1;
+      if (c >= 0) d[c] = cscale(v, inv);
+    }
+  }
+};
+
+template <bool INV>
+__global__ void __launch_bounds__(kMaxThr, kMinB) alpha_mm_kernel(Geometry g, MmPlan P, double2* __restrict__ W, int T) {
+  extern __shared__ __align__(16) double2 sm[];
+  __shared__ double2 x0[2 * kMaxT];
+  __shared__ double2* rows[kMaxT];
+  double2* A = sm;
+  double2* Z = sm + (size_t)T * P.ts;
+  const int L = g.L, Pn = g.P, nrows = g.nplanes * g.nb, r0 = blockIdx.x * T, Ta = min(T, nrows - r0);
+  if (threadIdx.x < Ta) rows[threadIdx.x] = W + row_off(g, r0 + threadIdx.x);
+  // column of entry k; -1: the MWSS Nyquist entry k = L, which has no column
+  auto col = [&](int k) { return k <= L - 1 ? k + L - 1 : k - Pn + L - 1; };
+  for (int t = 0; t < Ta; t++) {
+    const double2* src = W + row_off(g, r0 + t);
+    if (P.kind == 3) {
+      mm::stage_conv<INV>(P, A + t * P.ts, x0 + 2 * t, [&](int k) {
+        const int c = INV ? col(k) : k;
+        return c >= 0 ? src[c] : make_double2(0.0, 0.0);
+      });
+    } else {
+      for (int k = threadIdx.x; k < Pn; k += blockDim.x) {
+        const int c = INV ? col(k) : k;
+        double2* d = A + t * P.ts + mm::pos(P, k);
+        if (c >= 0)
+          mm::cp16(d, src + c);
+        else
+          *d = make_double2(0.0, 0.0);
+      }
+    }
+  }
+  mm::cp_wait_all();
+  __syncthreads();
+  mm::run<INV>(P, A, Z, Ta, x0, AlphaOut<INV>{rows, 1.0 / Pn, L, Pn});
+}
+
+// ------------------------------------------------------------------ inverse beta
+// Two columns per DFT as in stages.cu (inv_beta_kernel): T adjacent column
+// pairs per CTA; the synthesis of a pair lands in shared memory, where each
+// row meets its mirror.
+struct SmemOut {
+  double2* X;
+  int ts;
+  typedef double2* Seq;
+  __device__ __forceinline__ Seq seq(int t) const { return X + t * ts; }
+  __device__ __forceinline__ void put(Seq d, int k, double2 v) const { d[k] = v; }
+};
+
+__global__ void __launch_bounds__(kMaxThr, kMinB) inv_beta_mm_kernel(Geometry g, MmPlan P,
+                                                                     const double2* __restrict__ half,
+                                                                     double2* __restrict__ W, int T) {
+  extern __shared__ __align__(16) double2 sm[];
+  __shared__ double2 x0[2 * kMaxT], b0s[kMaxT];
+  double2* A = sm;
+  double2* Z = sm + (size_t)T * P.ts;
+  const int plane = blockIdx.y, n = plane - g.plane0, L = g.L, Pn = g.P, ncols = 2 * L - 1;
+  const int q0 = blockIdx.x * T, Ta = min(T, L - q0);
+  double2* base = W + (long long)plane * g.PS;
+  const double2* cbase = W + g.QOFF + (long long)plane * g.QS;
+  const bool first_is_a = ((L - 1 + n) & 1) == 0;  // column 2q has m + n even
+  // both columns of each pair into Z first (L + L <= ts entries), all copies in flight at once
+  for (int t = 0; t < Ta; t++) {
+    const int c = 2 * (q0 + t);
+    const double2* src = cbase + (long long)c * g.CS;
+    double2* z = Z + t * P.ts;
+    for (int mp = threadIdx.x; mp < L; mp += blockDim.x) {
+      mm::cp16(z + mp, src + mp);
+      if (c + 1 < ncols)
+        mm::cp16(z + L + mp, src + g.CS + mp);
+      else
+        z[L + mp] = make_double2(0.0, 0.0);
+    }
+  }
+  mm::cp_wait_all();
+  __syncthreads();
+  // z at +m' and -m'
+  auto pair = [&](int t, int mp, double2& zp, double2& zn) {
+    const double2 v0 = Z[t * P.ts + mp], v1 = Z[t * P.ts + L + mp];
+    const double2 av = first_is_a ? v0 : v1, bv = first_is_a ? v1 : v0;
+    zp = cadd(av, bv);
+    if (mp == 0) {
+      b0s[t] = bv;
+      zn = zp;
+      return;
+    }
+    zn = csub(av, bv);
+    if (g.mw) {
+      const double2 e = __ldg(half + mp);  // e^{-i pi m'/(2L-1)}
+      zp = cmul(zp, cconj(e));
+      zn = cmul(zn, e);
+    }
+  };
+  for (int t = 0; t < Ta; t++) {
+    double2* s = A + t * P.ts;
+    if (P.kind == 3) {
+      mm::stage_conv<true>(P, s, x0 + 2 * t, [&](int k) {
+        double2 zp, zn;
+        const int mp = k <= L - 1 ? k : Pn - k;
+        if (mp >= L) return make_double2(0.0, 0.0);  // MWSS Nyquist entry
+        pair(t, mp, zp, zn);
+        return k <= L - 1 ? zp : zn;
+      });
+    } else {
+      for (int mp = threadIdx.x; mp < L; mp += blockDim.x) {
+        double2 zp, zn;
+        pair(t, mp, zp, zn);
+        s[mm::pos(P, mp)] = zp;
+        if (mp) s[mm::pos(P, Pn - mp)] = zn;
+      }
+      if (!g.mw && threadIdx.x == 0) s[mm::pos(P, L)] = make_double2(0.0, 0.0);
+    }
+  }
+  __syncthreads();
+  double2* X = P.kind == 1 ? Z : A;
+  const int ts = P.ts;
+  mm::run<true>(P, A, Z, Ta, x0, SmemOut{X, ts});
+  __syncthreads();
+  // rows k < nb of both columns
+  const int rows = blockDim.x / T, t = threadIdx.x % T;
+  if (t >= Ta || threadIdx.x >= rows * T) return;
+  for (int row = threadIdx.x / T; row < g.nb; row += rows) {
+    const int c = 2 * (q0 + t);
+    int mrow = g.mw ? Pn - 1 - row : Pn - row;
+    if (mrow >= Pn) mrow -= Pn;
+    const double2 y0 = X[t * ts + row], y1 = X[t * ts + mrow], B0 = b0s[t];
+    const double2 yA = make_double2(0.5 * (y0.x + y1.x) - B0.x, 0.5 * (y0.y + y1.y) - B0.y);
+    const double2 yB = make_double2(0.5 * (y0.x - y1.x) + B0.x, 0.5 * (y0.y - y1.y) + B0.y);
+    double2* dst = base + (long long)row * g.RS + c;
+    dst[0] = first_is_a ? yA : yB;
+    if (c + 1 < ncols) dst[1] = first_is_a ? yB : yA;
+  }
+}
+
+size_t seq_smem(const MmPlan& P, int T, int bufs) { return bufs * sizeof(double2) * (size_t)T * P.ts; }
+
+// Launch shape of a stage over `nseq` sequences: sequences per CTA, warps, and
+// row tiles per warp task of each level (in the returned plan).
+//
+// About 800 points per CTA at 220 per warp: measured over 1-16 sequences x 2-8
+// warps at lengths 31 to 2047, the best shapes hold 150-260 points per warp
+// and 600-1000 per CTA (255: 3 x 4 warps, 511: 2 x 5, 1023: 1 x 4, 2047: 1 x
+// 8); larger CTAs wait longer at their barriers (1023: 4 sequences on 8 warps
+// takes 1.4x the time), smaller ones leave column tiles half empty.  One-level
+// plans take 8 columns, a full task.  Fewer sequences where the device would
+// not fill; one row tile per task where two would leave warps idle.
+struct Shape {
+  int T, warps;
+  size_t smem;
+  MmPlan P;
+};
+Shape shape_for(const MmPlan& P0, int nseq, int bufs) {
+  Shape z{1, 2, 0, P0};
+  z.T = P0.kind == 1 ? 8 : std::max(1, std::min(8, (800 + P0.n / 2) / P0.n));
+  while (z.T > 1 && (nseq + z.T - 1) / z.T < 148) z.T >>= 1;
+  z.warps = std::max(2, std::min(kMaxThr / 32, (z.T * P0.n + 110) / 220));
+  if (P0.kind == 1) z.warps = std::max(z.warps, std::min(kMaxThr / 32, (P0.la.QT + 1) / 2));
+  for (int l = 0; l < (P0.kind == 1 ? 1 : 2); l++) {
+    MmLevel& v = l ? z.P.lb : z.P.la;
+    const int cols = P0.kind == 1 ? z.T : z.T * (l ? P0.a : P0.b), nc = (cols + 4 * mm::kNT - 1) / (4 * mm::kNT);
+    v.MT = std::min(v.QT, nc * ((v.QT + 1) / 2) < z.warps ? 1 : 2);
+    v.QG = (v.QT + v.MT - 1) / v.MT;
+  }
+  z.smem = seq_smem(P0, z.T, bufs);
+  return z;
+}
+
+// alpha samples per CTA of a gamma kernel: four warp tasks where the row
+// tiles allow, 64 at most
+int gamma_shift(const MmLevel& lv, int cols) {
+  int sh = 4;
+  while (sh < 6 && (1 << (sh + 1)) * lv.QG <= 4 * 8 * (cols / 8)) sh++;
+  return sh;
+}
+
+}  // namespace
+
+bool mm_gamma_ok(const Geometry& g, const FftPlan& p) {
+  return p.l1.p == g.ng && (size_t)g.ng * 18 * sizeof(double2) <= kSmemMax;
+}
+bool mm_ok(const FftPlan& p) { return p.mm.n == p.n && seq_smem(p.mm, 1, 2) <= kSmemMax; }
+
+int launch_mm_inv_gamma(const Geometry& g, const FftPlan& p, const double2* W, void* f, cudaStream_t s, int row_lo,
+                        int row_hi) {
+  int sh = gamma_shift(p.l1, g.real ? 16 : 8);
+  const int rows = g.real ? g.nplanes : g.ng;
+  while (sh > 4 && (size_t)rows * ((1 << sh) + 2) * sizeof(double2) > kSmemMax / 4) sh--;
+  const size_t smem = (size_t)rows * ((1 << sh) + 2) * sizeof(double2);
+  const dim3 grid((g.na + (1 << sh) - 1) >> sh, row_hi - row_lo);
+  if (g.real) {
+    if (int rc = set_smem(inv_gamma_real_mm_kernel, smem)) return rc;
+    inv_gamma_real_mm_kernel<<<grid, kGT, smem, s>>>(g, p.l1, W, static_cast<double*>(f), sh, row_lo);
+  } else {
+    if (int rc = set_smem(inv_gamma_mm_kernel, smem)) return rc;
+    inv_gamma_mm_kernel<<<grid, kGT, smem, s>>>(g, p.l1, W, static_cast<double2*>(f), sh, row_lo);
+  }
+  return launched();
+}
+
+int launch_mm_fwd_gamma(const Geometry& g, const FftPlan& p, const void* f, double2* W, cudaStream_t s, int row_lo,
+                        int row_hi) {
+  int sh = gamma_shift(p.l1, g.real ? 16 : 8);
+  while (sh > 4 && (size_t)g.ng * ((1 << sh) + 4) * (g.real ? 8 : 16) > kSmemMax / 4) sh--;
+  const size_t smem = (size_t)g.ng * (g.real ? ((1 << sh) + 4) * 8 : ((1 << sh) + 2) * 16);
+  const dim3 grid((g.na + (1 << sh) - 1) >> sh, row_hi - row_lo);
+  if (g.real) {
+    if (int rc = set_smem(fwd_gamma_real_mm_kernel, smem)) return rc;
+    fwd_gamma_real_mm_kernel<<<grid, kGT, smem, s>>>(g, p.l1, static_cast<const double*>(f), W, sh, row_lo);
+  } else {
+    if (int rc = set_smem(fwd_gamma_mm_kernel, smem)) return rc;
+    fwd_gamma_mm_kernel<<<grid, kGT, smem, s>>>(g, p.l1, static_cast<const double2*>(f), W, sh, row_lo);
+  }
+  return launched();
+}
+
+int launch_mm_alpha(const Geometry& g, const FftPlan& p, double2* W, bool inverse, cudaStream_t s) {
+  const int nrows = g.nplanes * g.nb;
+  const Shape z = shape_for(p.mm, nrows, p.mm.kind == 1 ? 1 : 2);
+  auto go = [&](auto kernel) -> int {
+    if (int rc = set_smem(kernel, z.smem)) return rc;
+    kernel<<<(nrows + z.T - 1) / z.T, 32 * z.warps, z.smem, s>>>(g, z.P, W, z.T);
+    return launched();
+  };
+  return inverse ? go(alpha_mm_kernel<true>) : go(alpha_mm_kernel<false>);
+}
+
+int launch_mm_inv_beta(const Geometry& g, const FftPlan& p, double2* W, cudaStream_t s) {
+  const Shape z = shape_for(p.mm, g.L * g.nplanes, 2);
+  const dim3 grid((g.L + z.T - 1) / z.T, g.nplanes);
+  if (int rc = set_smem(inv_beta_mm_kernel, z.smem)) return rc;
+  inv_beta_mm_kernel<<<grid, 32 * z.warps, z.smem, s>>>(g, z.P, p.half, W, z.T);
+  return launched();
+}
+
+}  // namespace so3g

@@ -123,7 +123,7 @@ size_t resident_bytes(Device* D) {
   for (const auto& t : D->digit_tables) b += t->bytes + (size_t)t->L * t->N * sizeof(long long);
   for (const auto& t : D->beta_tables) b += t->bytes;
   for (const auto& kv : D->conv_kernels) b += (size_t)(16 * (kv.first / 2) + 2 * (kv.first / 2)) * sizeof(double2);  // 2 Pc <= 16L, plus 2L
-  for (const auto& kv : D->ffts) b += (size_t)4 * (kv.first + 256) * sizeof(double2);
+  for (const auto& kv : D->ffts) b += (size_t)4 * (kv.first + 256) * sizeof(double2) + kv.second->mm_bytes;
   for (const auto& kv : D->bases) b += 4096 * sizeof(long long);
   return b;
 }
@@ -390,6 +390,7 @@ int ensure_fft(Device* D, int n, FftPlan* out) {
     P.chirp = dp->mem + P.m;
     P.kern = dp->mem + P.m + n;
   }
+  if (int rc = build_mm_plan(n, &P, &dp->mm_mem, &dp->mm_imem, &dp->mm_bytes)) return rc;
   *out = P;
   D->ffts[key] = std::move(dp);
   return kOk;
