@@ -27,7 +27,13 @@ static int acquire(Device* D, const so3_parameters_t& p, int real, cudaStream_t 
   if (int rc = ensure_fft(D, r->g.P, &r->pP)) return rc;
   if (int rc = ensure_fft(D, r->g.ng, &r->pg)) return rc;
   if (int rc = ensure_bases(D, p, real, &r->bases)) return rc;
-  if (conv) {
+  // the inverse's matrix also for forward calls: either may be followed by a
+  // captured inverse of the same parameters
+  if (beta_matrix_pays(r->g, kBetaInverse))
+    if (int rc = ensure_beta_matrix(D, r->g, kBetaInverse, r->pP, s, &r->g.beta_mat[kBetaInverse])) return rc;
+  if (conv && beta_matrix_pays(r->g, kBetaForward)) {
+    if (int rc = ensure_beta_matrix(D, r->g, kBetaForward, r->pP, s, &r->g.beta_mat[kBetaForward])) return rc;
+  } else if (conv) {
     if (int rc = ensure_fft(D, r->g.Pc, &r->pc)) return rc;
     if (int rc = ensure_conv_kernel(D, r->g, &r->wr)) return rc;
   }
@@ -66,7 +72,7 @@ static int ensure_tuned(Device* D, const so3_parameters_t& p, int real, Resource
   if (!(env && env[0] == '0')) {
     FftPlan pc{};
     const double2* wr = nullptr;
-    {
+    if (!beta_matrix_pays(g, kBetaForward)) {
       std::lock_guard<std::mutex> lk(D->mu);
       if (int rc = ensure_fft(D, g.Pc, &pc)) return rc;
       if (int rc = ensure_conv_kernel(D, g, &wr)) return rc;
@@ -765,12 +771,18 @@ static int adjoint_check(const so3_parameters_t& p) {
   return kOk;
 }
 
+static int acquire_adjoint(Device* D, int kind, cudaStream_t s, Resources* r) {
+  std::lock_guard<std::mutex> lk(D->mu);
+  return ensure_beta_matrix(D, r->g, kind, r->pP, s, &r->g.beta_mat[kind]);
+}
+
 int run_adjoint_inverse(Device* D, Workspace* wk, const so3_parameters_t& p, const void* f_d, void* flmn_d,
                         cudaStream_t s) {
   if (int rc = adjoint_check(p)) return rc;
   const int real = p.reality ? 1 : 0;
   Resources r;
   if (int rc = acquire(D, p, real, s, &r, false)) return rc;
+  if (int rc = acquire_adjoint(D, kBetaAdjInverse, s, &r)) return rc;
   void* ws = nullptr;
   if (int rc = ensure_ws(wk, workspace_bytes(p, real), &ws)) return rc;
   double2* W = static_cast<double2*>(ws);
@@ -780,7 +792,7 @@ int run_adjoint_inverse(Device* D, Workspace* wk, const so3_parameters_t& p, con
   int rc;
   if ((rc = launch_fwd_gamma(r.g, r.pg, f_d, W, s))) return rc;
   if ((rc = launch_fwd_alpha(r.g, r.pP, W, s))) return rc;
-  if ((rc = launch_adj_inv_beta(r.g, r.pP, W, s))) return rc;
+  if ((rc = launch_beta_matrix(r.g, kBetaAdjInverse, r.g.beta_mat[kBetaAdjInverse], W, s))) return rc;
   const double kPi = 3.141592653589793238462643383279502884;
   const double lw = (double)(2 * p.N - 1) * (2 * p.L - 1) / (16.0 * kPi * kPi * kPi);  // (2l+1)/(8pi^2) (2N-1)(2L-1)/(2pi)
   return launch_forward_contract(r.g, p.n_mode, W, r.bases, r.dl, static_cast<double2*>(flmn_d),
@@ -792,7 +804,8 @@ int run_adjoint_forward(Device* D, Workspace* wk, const so3_parameters_t& p, con
   if (int rc = adjoint_check(p)) return rc;
   const int real = p.reality ? 1 : 0;
   Resources r;
-  if (int rc = acquire(D, p, real, s, &r, true)) return rc;
+  if (int rc = acquire(D, p, real, s, &r, false)) return rc;
+  if (int rc = acquire_adjoint(D, kBetaAdjForward, s, &r)) return rc;
   void* ws = nullptr;
   if (int rc = ensure_ws(wk, workspace_bytes(p, real), &ws)) return rc;
   double2* W = static_cast<double2*>(ws);
@@ -802,7 +815,7 @@ int run_adjoint_forward(Device* D, Workspace* wk, const so3_parameters_t& p, con
   if ((rc = launch_inverse_contract(r.g, p.n_mode, static_cast<const double2*>(flmn_d), r.bases, r.dl, W, 0, s, 0,
                                     -1, wconst)))
     return rc;
-  if ((rc = launch_adj_fwd_beta(r.g, r.pP, r.pc, r.wr, W, s))) return rc;
+  if ((rc = launch_beta_matrix(r.g, kBetaAdjForward, r.g.beta_mat[kBetaAdjForward], W, s))) return rc;
   if ((rc = launch_inv_alpha(r.g, r.pP, W, s))) return rc;
   return launch_inv_gamma(r.g, r.pg, W, f_d, s);
 }

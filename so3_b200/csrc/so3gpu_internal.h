@@ -68,6 +68,8 @@ struct Geometry {
   // Kernel variant of each DFT stage (index = Stage below; 0 = default),
   // chosen by the autotuner for this geometry.
   signed char var[8];
+  // Matrices of the beta stages (beta_mm.cu) by BetaKind; null: through DFTs.
+  const double* beta_mat[4];
 };
 Geometry make_geometry(const so3_parameters_t& p, int real);
 
@@ -90,8 +92,7 @@ __host__ __device__ inline long long dl_plane_offset(int l) {
 
 struct DevPlan {
   FftPlan plan{};
-  double2* mem = nullptr;  // owns roots/mroots/chirp/kern/half/rroots/rkern
-  int* imem = nullptr;     // owns rperm
+  double2* mem = nullptr;     // owns roots/mroots/chirp/kern/half
   double2* mm_mem = nullptr;  // own the tensor-core plan's tables
   int* mm_imem = nullptr;
   size_t mm_bytes = 0;
@@ -122,6 +123,7 @@ struct Device {
   DlTable dl[2];                                 // per dl_method
   std::map<int, std::unique_ptr<DevPlan>> ffts;  // by length
   std::map<int, double2*> conv_kernels;          // forward-beta weight tables by 2L + (MW)
+  std::map<int, double*> beta_matrices;          // by (2L + (MW)) * kBetaKinds + kind
   std::map<std::string, long long*> bases;       // block bases by parameter key
   std::vector<std::unique_ptr<DigitTable>> digit_tables;
   std::map<long long, int> digit_uses;  // split-precision calls per (L, N, recursion) without a table
@@ -172,6 +174,7 @@ int ensure_fft(Device* D, int n, FftPlan* out);
 // owns *mem and *imem (device memory, *bytes in total).
 int build_mm_plan(int n, FftPlan* F, double2** mem, int** imem, size_t* bytes);
 int ensure_conv_kernel(Device* D, const Geometry& g, const double2** out);
+int ensure_beta_matrix(Device* D, const Geometry& g, int kind, const FftPlan& pP, cudaStream_t s, const double** out);
 int ensure_bases(Device* D, const so3_parameters_t& p, int real, const long long** out);
 int ensure_ws(Workspace* W, size_t bytes, void** out);
 size_t workspace_bytes(const so3_parameters_t& p, int real);
@@ -229,17 +232,13 @@ int launch_mm_fwd_gamma(const Geometry& g, const FftPlan& p, const void* f, doub
 int launch_mm_alpha(const Geometry& g, const FftPlan& p, double2* W, bool inverse, cudaStream_t s);
 int launch_mm_inv_beta(const Geometry& g, const FftPlan& p, double2* W, cudaStream_t s);
 
-// Beta stages of the adjoint transforms (MW, complex; stages.cu).  Inverse
-// adjoint: per column of the row-major part, zero-extend the nb beta samples
-// onto the 2L-1 circle, DFT, phase e^{-i m' pi/(2L-1)}, fold F(m') +
-// (-1)^{m+n} F(-m') onto m' >= 0 into the column-major part.  Forward
-// adjoint: per column of the column-major part, extend G(-m') = (-1)^{m+n}
-// G(m'), convolve with 4 pi^2 w (table wr), phase e^{+i m'' pi/(2L-1)},
-// inverse DFT / (2L-1), fold the periodic extension back onto the L beta
-// samples into the row-major part.
-int launch_adj_inv_beta(const Geometry& g, const FftPlan& pP, double2* W, cudaStream_t s);
-int launch_adj_fwd_beta(const Geometry& g, const FftPlan& pP, const FftPlan& pc, const double2* wr, double2* W,
-                        cudaStream_t s);
+// Beta stages as products with one real matrix per parity (beta_mm.cu).
+enum BetaKind : int { kBetaInverse = 0, kBetaForward, kBetaAdjInverse, kBetaAdjForward, kBetaKinds };
+bool beta_matrix_pays(const Geometry& g, int kind);
+size_t beta_matrix_bytes(const Geometry& g, int kind);
+int launch_beta_matrix_table(const Geometry& g, int kind, const FftPlan& pP, double* tab, cudaStream_t s);
+int launch_beta_matrix(const Geometry& g, int kind, const double* tab, double2* W, cudaStream_t s);
+
 int launch_s2toso3(const so3_parameters_t& hp, const long long* bases, const double2* flm, const double2* glm,
                    double2* hlmn, cudaStream_t s);
 int launch_harmonic_convolution(const so3_parameters_t& hp, const so3_parameters_t& fp,

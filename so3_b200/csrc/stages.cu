@@ -62,9 +62,7 @@ template <bool BIG>
 struct Gen {
   static constexpr bool fixed = false;
   static constexpr int NT = kThreads, MINB = BIG ? 1 : 2, T = 0, LD = 0, nP = 0;
-  static constexpr bool io = false, has_out = false;
-  template <class In, class Out>
-  static __device__ __forceinline__ void runIO(const In&, const Out&, double2*, double2*, const FftPlan&) {}
+  static constexpr bool has_out = false;
   template <class Out>
   static __device__ __forceinline__ void runPOut(double2*, double2*, const FftPlan&, const Out&) {}
   static __device__ __forceinline__ int at(int k) { return k; }
@@ -83,13 +81,6 @@ struct Fix {
   static constexpr int NT = NT_, MINB = MINB_, T = T_;
   static constexpr int ldP = PP<1, 1, 1>::ld, ldC = PC<1, 1, 1>::ld;
   static constexpr int nP = PP<1, 1, 1>::n;  // runP length
-  // the runP plan reads its input and writes its output through callables
-  static constexpr bool io = PP<1, 1, 1>::io;
-  template <class In, class Out>
-  static __device__ __forceinline__ void runIO(const In& in, const Out& out, double2* a, double2* b,
-                                               const FftPlan& P) {
-    PP<T_, LD, NT_>::run_io(in, out, a, b, P);
-  }
   // the runP plan's last pass can store through a callable (1023 = 31*11*3)
   static constexpr bool has_out = nP == 1023;
   template <class Out>
@@ -114,19 +105,13 @@ struct Fix {
 };
 
 // Variants the autotuner chooses from (sequences per CTA, CTA size, minimum
-// CTAs per SM): alpha / extended-beta length 1023 (L = 512), gamma length 127
-// (N = 64), and the forward beta pair 1023 / 2048.  Variant 0 is the default.
+// CTAs per SM): alpha / extended-beta length 1023 (L = 512) and the forward
+// beta pair 1023 / 2048.  Variant 0 is the default.
 using E1023a = Fix<fx::P1023, fx::P1023, 1, 128, 4>;
 using E1023b = Fix<fx::P1023, fx::P1023, 1, 64, 8>;
 using E1023c = Fix<fx::P1023, fx::P1023, 2, 128, 3>;
 using E1023p = Fix<fx::P1023, fx::P1023, 1, 128, 3>;  // persistent inverse alpha (prefetch registers)
 using E1023c2 = Fix<fx::P1023n2, fx::P1023n2, 2, 128, 3>;  // radix-31 butterflies in two output groups
-using E127a = Fix<fx::P127, fx::P127, 4, 128, 4>;
-using E127b = Fix<fx::P127, fx::P127, 8, 128, 3>;
-using E127c = Fix<fx::P127, fx::P127, 2, 64, 8>;
-using E127ra = Fix<fx::P127R, fx::P127R, 8, 128, 4>;
-using E127rb = Fix<fx::P127R, fx::P127R, 16, 256, 2>;
-using E127rc = Fix<fx::P127R, fx::P127R, 4, 64, 8>;
 using EConv1023a = Fix<fx::P1023, fx::P2048, 1, 128, 3>;
 using EConv1023b = Fix<fx::P1023, fx::P2048, 1, 256, 2>;
 
@@ -302,24 +287,6 @@ __global__ void __launch_bounds__(E::NT, E::MINB) inv_gamma_kernel(Geometry g, F
   double2* a = sm;
   double2* b = sm + (size_t)T * ld;
   const int row = row0 + blockIdx.y, a0 = blockIdx.x * T, ng = g.ng;
-  if constexpr (!REAL && E::io) {
-    // the plan reads plane (k + plane0) mod ng and writes gamma sample k
-    // straight from / to global memory (complex: nplanes == ng)
-    const long long plane_sz = (long long)g.nb * g.na;
-    double2* f = static_cast<double2*>(fout);
-    auto in = [&](int t, int k) {
-      const int al = a0 + t;
-      int p = k + g.plane0;
-      if (p >= ng) p -= ng;
-      return al < g.na ? cconj(W[(long long)p * g.PS + (long long)row * g.RS + al]) : make_double2(0.0, 0.0);
-    };
-    auto out = [&](int t, int k, double2 y) {
-      const int al = a0 + t;
-      if (al < g.na) f[(long long)k * plane_sz + (long long)row * g.na + al] = cconj(y);
-    };
-    E::runIO(in, out, a, b, P);
-    return;
-  }
   if (!REAL && g.steer)  // the 2N-point circle of a steerable signal has no plane n = N
     for (int t = threadIdx.x; t < T; t += E::NT) a[t * ld + E::at(g.N)] = make_double2(0.0, 0.0);
   for (int idx = threadIdx.x; idx < g.nplanes * T; idx += E::NT) {
@@ -405,23 +372,6 @@ __global__ void __launch_bounds__(E::NT, E::MINB) fwd_gamma_kernel(Geometry g, F
   const long long plane_sz = (long long)g.nb * g.na;
   // 2 pi / (2N-1); steerable (so3_core.c:309-328): 2 pi / N over the N samples
   const double scale = 2.0 * 3.141592653589793238462643383279502884 / g.nf;
-  if constexpr (!REAL && E::io) {
-    // the plan reads gamma sample k and writes plane (k + plane0) mod ng
-    // straight from / to global memory (complex: nplanes == ng)
-    const double2* f = static_cast<const double2*>(fin);
-    auto in = [&](int t, int k) {
-      const int al = a0 + t;
-      return al < g.na ? f[(long long)k * plane_sz + (long long)row * g.na + al] : make_double2(0.0, 0.0);
-    };
-    auto out = [&](int t, int k, double2 y) {
-      const int al = a0 + t;
-      int p = k + g.plane0;
-      if (p >= ng) p -= ng;
-      if (al < g.na) W[(long long)p * g.PS + (long long)row * g.RS + al] = cscale(y, scale);
-    };
-    E::runIO(in, out, a, b, P);
-    return;
-  }
   for (int idx = threadIdx.x; idx < ng * T; idx += E::NT) {
     const int t = idx % T, gi = idx / T, al = a0 + t;
     double2 v = make_double2(0.0, 0.0);
@@ -655,117 +605,12 @@ __global__ void __launch_bounds__(E::NT, E::MINB) fwd_beta_conv_kernel(Geometry 
   }
 }
 
-// ------------------------------------------------------------------ adjoint
-// Beta stages of the adjoint transforms (reference src/c/so3_adjoint.c, MW;
-// complex planes n = -(N-1)..N-1 or real planes n >= 0).  Generic engines
-// only (any length); one column (plane n, order m, s = (-1)^{m+n}) per
-// sequence.
-//
-// Inverse adjoint (so3_adjoint.c:190-231): the nb beta samples zero-extended
-// onto the 2L-1 circle, forward DFT, phase e^{-i m' pi/(2L-1)}, folded
-// F(m') + s F(-m') onto m' >= 0 (the contraction's sum over -l <= m' <= l).
-template <class E>
-__global__ void __launch_bounds__(E::NT, E::MINB) adj_inv_beta_kernel(Geometry g, FftPlan P, double2* __restrict__ W,
-                                                                 int T_, int ld_) {
-  static_assert(!E::fixed, "generic engines");
-  extern __shared__ double2 sm[];
-  const int T = T_, ld = ld_;
-  double2* a = sm;
-  double2* b = sm + (size_t)T * ld;
-  const int plane = blockIdx.y, n = plane - g.plane0;
-  const int c0 = blockIdx.x * T, L = g.L, ncols = 2 * L - 1, Pn = g.P;
-  const double2* base = W + (long long)plane * g.PS;
-  for (int idx = threadIdx.x; idx < Pn * T; idx += E::NT) {
-    const int t = idx % T, row = idx / T, c = c0 + t;  // columns fastest: rows read contiguously
-    a[t * ld + row] = (row < g.nb && c < ncols) ? base[(long long)row * g.RS + c] : make_double2(0.0, 0.0);
-  }
-  __syncthreads();
-  const double2* r = E::runP(a, b, T, ld, P);
-  double2* cbase = W + g.QOFF + (long long)plane * g.QS;
-  for (int idx = threadIdx.x; idx < L * T; idx += E::NT) {
-    const int mp = idx % L, t = idx / L, c = c0 + t;
-    if (c >= ncols) continue;
-    const int m = c - (L - 1);
-    const double sg = ((m + n) & 1) ? -1.0 : 1.0;
-    const double2 e = __ldg(P.half + mp);  // e^{-i pi m'/(2L-1)}
-    double2 v = cmul(r[t * ld + mp], e);
-    if (mp > 0) v = cadd(v, cscale(cmul(r[t * ld + Pn - mp], cconj(e)), sg));
-    cbase[(long long)c * g.CS + mp] = v;
-  }
-}
-
-// Forward adjoint (so3_adjoint.c:718-896): G(-m') = s G(m') extended from
-// the contraction's m' >= 0, convolved with the quadrature weights (F(m'') =
-// 4 pi^2 sum_{m'} G(m') w(m'' - m'), through the Pc-point product with the
-// table's full-weight spectrum), phase e^{+i m'' pi/(2L-1)}, inverse DFT over
-// the 2L-1 circle divided by 2L-1, and the adjoint of the periodic
-// extension: out(b) = y(b) + s y(2L-2-b) for b < L-1, out(L-1) = y(L-1).
-template <class E>
-__global__ void __launch_bounds__(E::NT, E::MINB) adj_fwd_beta_kernel(Geometry g, FftPlan P, FftPlan Pc,
-                                                                 const double2* __restrict__ wr,
-                                                                 double2* __restrict__ W, int T_, int ld_) {
-  static_assert(!E::fixed, "generic engines");
-  extern __shared__ double2 sm[];
-  const int T = T_, ld = ld_;
-  double2* a = sm;
-  double2* b = sm + (size_t)T * ld;
-  const int plane = blockIdx.y, n = plane - g.plane0;
-  const int c0 = blockIdx.x * T, L = g.L, ncols = 2 * L - 1, Pn = g.P, pc = g.Pc;
-  const double2* cbase = W + g.QOFF + (long long)plane * g.QS;
-  for (int idx = threadIdx.x; idx < pc * T; idx += E::NT) {
-    const int k = idx % pc, t = idx / pc, c = c0 + t;  // m' fastest: columns read contiguously
-    double2 v = make_double2(0.0, 0.0);
-    if (c < ncols) {
-      const int m = c - (L - 1);
-      const double sg = ((m + n) & 1) ? -1.0 : 1.0;
-      if (k < L) v = cbase[(long long)c * g.CS + k];
-      else if (k > pc - L) v = cscale(cbase[(long long)c * g.CS + (pc - k)], sg);
-    }
-    a[t * ld + k] = v;
-  }
-  __syncthreads();
-  double2* y = E::runC(a, b, T, ld, Pc);  // forward DFT
-  const double2* wf = wr + 2 * (size_t)L + pc;
-  for (int idx = threadIdx.x; idx < pc * T; idx += E::NT) {
-    const int k = idx % pc, t = idx / pc;
-    y[t * ld + k] = cconj(cmul(y[t * ld + k], __ldg(wf + k)));
-  }
-  __syncthreads();
-  double2* o = (y == a) ? b : a;
-  double2* cv = E::runC(y, o, T, ld, Pc);  // conj: 4 pi^2 (G * w)
-  double2* d = (cv == a) ? b : a;
-  for (int idx = threadIdx.x; idx < Pn * T; idx += E::NT) {
-    const int k = idx % Pn, t = idx / Pn;
-    const int mpp = k <= L - 1 ? k : k - Pn;  // m'' in [-(L-1), L-1]
-    const double2 F = cconj(cv[t * ld + (mpp < 0 ? mpp + pc : mpp)]);
-    const double2 e = __ldg(P.half + (mpp < 0 ? -mpp : mpp));  // e^{-i pi |m''|/(2L-1)}
-    const double2 ph = mpp < 0 ? e : cconj(e);                   // e^{+i pi m''/(2L-1)}
-    d[t * ld + k] = cconj(cmul(F, ph));
-  }
-  __syncthreads();
-  double2* other = (d == a) ? b : a;
-  const double2* yb = E::runP(d, other, T, ld, P);  // conj: (2L-1) y(b)
-  const double invP = 1.0 / Pn;
-  double2* base = W + (long long)plane * g.PS;
-  for (int idx = threadIdx.x; idx < g.nb * T; idx += E::NT) {
-    const int t = idx % T, row = idx / T, c = c0 + t;  // columns fastest: rows written contiguously
-    if (c >= ncols) continue;
-    const int m = c - (L - 1);
-    const double sg = ((m + n) & 1) ? -1.0 : 1.0;
-    double2 v = cscale(cconj(yb[t * ld + row]), invP);
-    if (row < L - 1) v = cadd(v, cscale(cconj(yb[t * ld + (Pn - 1 - row)]), sg * invP));
-    base[(long long)row * g.RS + c] = v;
-  }
-}
-
 // ------------------------------------------------------------------ launchers
 namespace {
 
-enum class Eng { kGenSmall, kGenBig, k1023, k127, k127r };
+enum class Eng { kGenSmall, kGenBig, k1023 };
 Eng pick(const FftPlan& p) {
   if (!p.blue && p.n == 1023) return Eng::k1023;
-  if (p.blue && p.n == 127 && p.rkern) return Eng::k127r;
-  if (p.blue && p.n == 127 && p.m == 256) return Eng::k127;
   return p.big() ? Eng::kGenBig : Eng::kGenSmall;
 }
 
@@ -869,15 +714,14 @@ int launched() {
 
 }  // namespace
 
-// Where the tensor-core DFT replaces the scalar engines below (us per 31-plane
-// transform, inverse beta / inverse alpha): every length but the 1023 of the
-// compile-time plan (L = 512: mm 276 / 191, fixed 217 / 168), and for the
-// inverse beta stage the 127 of the Rader plan (L = 64: mm 7.2, fixed 5.6).
-static bool mm_alpha(const FftPlan& p) { return mm_ok(p) && pick(p) != Eng::k1023; }
-static bool mm_beta(const FftPlan& p) { return mm_alpha(p) && pick(p) != Eng::k127r; }
+// Where the tensor-core DFT replaces the scalar engines below: every length
+// but the 1023 of the compile-time plan (us per 31-plane transform at L = 512,
+// inverse beta / inverse alpha: 276 / 191 against 225 / 175).
+static bool mm_pays(const FftPlan& p) { return mm_ok(p) && pick(p) != Eng::k1023; }
 
 int launch_inv_beta(const Geometry& g, const FftPlan& p, double2* W, cudaStream_t s) {
-  if (mm_beta(p)) return launch_mm_inv_beta(g, p, W, s);
+  if (g.beta_mat[kBetaInverse]) return launch_beta_matrix(g, kBetaInverse, g.beta_mat[kBetaInverse], W, s);
+  if (mm_pays(p)) return launch_mm_inv_beta(g, p, W, s);
   int rc;
   const int v = g.var[kStInvBeta];
   switch (pick(p)) {
@@ -887,12 +731,6 @@ int launch_inv_beta(const Geometry& g, const FftPlan& p, double2* W, cudaStream_
            : v == 3 ? inv_beta<E1023c2>(g, p, W, s)
                     : inv_beta<E1023a>(g, p, W, s);
       break;
-    case Eng::k127:
-      rc = v == 1 ? inv_beta<E127b>(g, p, W, s) : v == 2 ? inv_beta<E127c>(g, p, W, s) : inv_beta<E127a>(g, p, W, s);
-      break;
-    case Eng::k127r:
-      rc = v == 1 ? inv_beta<E127rb>(g, p, W, s) : v == 2 ? inv_beta<E127rc>(g, p, W, s) : inv_beta<E127ra>(g, p, W, s);
-      break;
     case Eng::kGenBig: rc = inv_beta<Gen<true>>(g, p, W, s); break;
     default: rc = inv_beta<Gen<false>>(g, p, W, s); break;
   }
@@ -900,7 +738,7 @@ int launch_inv_beta(const Geometry& g, const FftPlan& p, double2* W, cudaStream_
 }
 
 int launch_inv_alpha(const Geometry& g, const FftPlan& p, double2* W, cudaStream_t s) {
-  if (mm_alpha(p)) return launch_mm_alpha(g, p, W, true, s);
+  if (mm_pays(p)) return launch_mm_alpha(g, p, W, true, s);
   int rc;
   const int v = g.var[kStInvAlpha];
   switch (pick(p)) {
@@ -909,13 +747,6 @@ int launch_inv_alpha(const Geometry& g, const FftPlan& p, double2* W, cudaStream
            : v == 2 ? inv_alpha<E1023c>(g, p, W, s)
            : v == 3 ? inv_alpha_pf<E1023p>(g, p, W, s)
                     : inv_alpha<E1023a>(g, p, W, s);
-      break;
-    case Eng::k127:
-      rc = v == 1 ? inv_alpha<E127b>(g, p, W, s) : v == 2 ? inv_alpha<E127c>(g, p, W, s) : inv_alpha<E127a>(g, p, W, s);
-      break;
-    case Eng::k127r:
-      rc = v == 1 ? inv_alpha<E127rb>(g, p, W, s) : v == 2 ? inv_alpha<E127rc>(g, p, W, s)
-                                                             : inv_alpha<E127ra>(g, p, W, s);
       break;
     case Eng::kGenBig: rc = inv_alpha<Gen<true>>(g, p, W, s); break;
     default: rc = inv_alpha<Gen<false>>(g, p, W, s); break;
@@ -930,18 +761,9 @@ int launch_inv_gamma(const Geometry& g, const FftPlan& p, const double2* W, void
   if (mm_gamma_ok(g, p)) return launch_mm_inv_gamma(g, p, W, f, s, row_lo, row_hi);
   int rc;
   const Eng e = pick(p);
-  const int v = g.var[kStInvGamma];
   if (g.real) {
     rc = e == Eng::kGenBig ? inv_gamma<true, Gen<true>>(g, p, W, f, s, row_lo, row_hi)
                            : inv_gamma<true, Gen<false>>(g, p, W, f, s, row_lo, row_hi);
-  } else if (e == Eng::k127) {
-    rc = v == 1   ? inv_gamma<false, E127b>(g, p, W, f, s, row_lo, row_hi)
-         : v == 2 ? inv_gamma<false, E127c>(g, p, W, f, s, row_lo, row_hi)
-                  : inv_gamma<false, E127a>(g, p, W, f, s, row_lo, row_hi);
-  } else if (e == Eng::k127r) {
-    rc = v == 1   ? inv_gamma<false, E127rb>(g, p, W, f, s, row_lo, row_hi)
-         : v == 2 ? inv_gamma<false, E127rc>(g, p, W, f, s, row_lo, row_hi)
-                  : inv_gamma<false, E127ra>(g, p, W, f, s, row_lo, row_hi);
   } else {
     rc = e == Eng::kGenBig ? inv_gamma<false, Gen<true>>(g, p, W, f, s, row_lo, row_hi)
                            : inv_gamma<false, Gen<false>>(g, p, W, f, s, row_lo, row_hi);
@@ -956,18 +778,9 @@ int launch_fwd_gamma(const Geometry& g, const FftPlan& p, const void* f, double2
   if (mm_gamma_ok(g, p)) return launch_mm_fwd_gamma(g, p, f, W, s, row_lo, row_hi);
   int rc;
   const Eng e = pick(p);
-  const int v = g.var[kStFwdGamma];
   if (g.real) {
     rc = e == Eng::kGenBig ? fwd_gamma<true, Gen<true>>(g, p, f, W, s, row_lo, row_hi)
                            : fwd_gamma<true, Gen<false>>(g, p, f, W, s, row_lo, row_hi);
-  } else if (e == Eng::k127) {
-    rc = v == 1   ? fwd_gamma<false, E127b>(g, p, f, W, s, row_lo, row_hi)
-         : v == 2 ? fwd_gamma<false, E127c>(g, p, f, W, s, row_lo, row_hi)
-                  : fwd_gamma<false, E127a>(g, p, f, W, s, row_lo, row_hi);
-  } else if (e == Eng::k127r) {
-    rc = v == 1   ? fwd_gamma<false, E127rb>(g, p, f, W, s, row_lo, row_hi)
-         : v == 2 ? fwd_gamma<false, E127rc>(g, p, f, W, s, row_lo, row_hi)
-                  : fwd_gamma<false, E127ra>(g, p, f, W, s, row_lo, row_hi);
   } else {
     rc = e == Eng::kGenBig ? fwd_gamma<false, Gen<true>>(g, p, f, W, s, row_lo, row_hi)
                            : fwd_gamma<false, Gen<false>>(g, p, f, W, s, row_lo, row_hi);
@@ -976,7 +789,7 @@ int launch_fwd_gamma(const Geometry& g, const FftPlan& p, const void* f, double2
 }
 
 int launch_fwd_alpha(const Geometry& g, const FftPlan& p, double2* W, cudaStream_t s) {
-  if (mm_alpha(p)) return launch_mm_alpha(g, p, W, false, s);
+  if (mm_pays(p)) return launch_mm_alpha(g, p, W, false, s);
   int rc;
   const int v = g.var[kStFwdAlpha];
   switch (pick(p)) {
@@ -985,13 +798,6 @@ int launch_fwd_alpha(const Geometry& g, const FftPlan& p, double2* W, cudaStream
            : v == 2 ? fwd_alpha<E1023c>(g, p, W, s)
            : v == 3 ? fwd_alpha_pf<E1023a>(g, p, W, s)
                     : fwd_alpha<E1023a>(g, p, W, s);
-      break;
-    case Eng::k127:
-      rc = v == 1 ? fwd_alpha<E127b>(g, p, W, s) : v == 2 ? fwd_alpha<E127c>(g, p, W, s) : fwd_alpha<E127a>(g, p, W, s);
-      break;
-    case Eng::k127r:
-      rc = v == 1 ? fwd_alpha<E127rb>(g, p, W, s) : v == 2 ? fwd_alpha<E127rc>(g, p, W, s)
-                                                             : fwd_alpha<E127ra>(g, p, W, s);
       break;
     case Eng::kGenBig: rc = fwd_alpha<Gen<true>>(g, p, W, s); break;
     default: rc = fwd_alpha<Gen<false>>(g, p, W, s); break;
@@ -1005,49 +811,13 @@ bool conv_fixed(const FftPlan& p, const FftPlan& pc) { return pick(p) == Eng::k1
 
 int launch_fwd_beta_conv(const Geometry& g, const FftPlan& p, const FftPlan& pc, const double2* wr, double2* W,
                          cudaStream_t s) {
+  if (g.beta_mat[kBetaForward]) return launch_beta_matrix(g, kBetaForward, g.beta_mat[kBetaForward], W, s);
   int rc;
   if (conv_fixed(p, pc))
     rc = g.var[kStFwdBetaConv] == 1 ? fwd_beta_conv<EConv1023b>(g, p, pc, wr, W, s)
                                     : fwd_beta_conv<EConv1023a>(g, p, pc, wr, W, s);
-  else if (p.big() || pc.big())
-    rc = fwd_beta_conv<Gen<true>>(g, p, pc, wr, W, s);
   else
-    rc = fwd_beta_conv<Gen<false>>(g, p, pc, wr, W, s);
-  return rc ? rc : launched();
-}
-
-namespace {
-template <class E>
-int adj_inv_beta(const Geometry& g, const FftPlan& p, double2* W, cudaStream_t s) {
-  const Sizing z = sizing<E>(p.ld(), 16);
-  dim3 grid((2 * g.L - 1 + z.T - 1) / z.T, g.nplanes);
-  if (int rc = set_smem(adj_inv_beta_kernel<E>, z.smem)) return rc;
-  adj_inv_beta_kernel<E><<<grid, E::NT, z.smem, s>>>(g, p, W, z.T, p.ld());
-  return kOk;
-}
-template <class E>
-int adj_fwd_beta(const Geometry& g, const FftPlan& p, const FftPlan& pc, const double2* wr, double2* W,
-                 cudaStream_t s) {
-  const int ld = p.ld() > pc.ld() ? p.ld() : pc.ld();
-  const Sizing z = sizing<E>(ld, 8);
-  dim3 grid((2 * g.L - 1 + z.T - 1) / z.T, g.nplanes);
-  if (int rc = set_smem(adj_fwd_beta_kernel<E>, z.smem)) return rc;
-  adj_fwd_beta_kernel<E><<<grid, E::NT, z.smem, s>>>(g, p, pc, wr, W, z.T, ld);
-  return kOk;
-}
-}  // namespace
-
-int launch_adj_inv_beta(const Geometry& g, const FftPlan& p, double2* W, cudaStream_t s) {
-  if (!g.mw) return fail(kUnsupported, "adjoint transforms: MW sampling only");
-  const int rc = p.big() ? adj_inv_beta<Gen<true>>(g, p, W, s) : adj_inv_beta<Gen<false>>(g, p, W, s);
-  return rc ? rc : launched();
-}
-
-int launch_adj_fwd_beta(const Geometry& g, const FftPlan& p, const FftPlan& pc, const double2* wr, double2* W,
-                        cudaStream_t s) {
-  if (!g.mw) return fail(kUnsupported, "adjoint transforms: MW sampling only");
-  const int rc = (p.big() || pc.big()) ? adj_fwd_beta<Gen<true>>(g, p, pc, wr, W, s)
-                                       : adj_fwd_beta<Gen<false>>(g, p, pc, wr, W, s);
+    return fail(kUnsupported, "forward beta stage: no plan for this length");
   return rc ? rc : launched();
 }
 
@@ -1057,9 +827,7 @@ int stage_variants(const Geometry& g, const FftPlan& pP, const FftPlan& pg, cons
     case kStInvBeta:
     case kStInvAlpha:
     case kStFwdAlpha:
-      return pick(pP) == Eng::k1023 ? 4 : (pick(pP) == Eng::k127 || pick(pP) == Eng::k127r) ? 3 : 1;
-    case kStInvGamma:
-    case kStFwdGamma: return (!g.real && (pick(pg) == Eng::k127 || pick(pg) == Eng::k127r)) ? 3 : 1;
+      return pick(pP) == Eng::k1023 ? 4 : 1;
     case kStFwdBetaConv: return conv_fixed(pP, pc) ? 2 : 1;
     default: return 1;
   }

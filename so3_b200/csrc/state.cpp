@@ -122,7 +122,14 @@ size_t resident_bytes(Device* D) {
     if (t.d) b += (size_t)dl_plane_offset(t.Lcap) * sizeof(double);
   for (const auto& t : D->digit_tables) b += t->bytes + (size_t)t->L * t->N * sizeof(long long);
   for (const auto& t : D->beta_tables) b += t->bytes;
-  for (const auto& kv : D->conv_kernels) b += (size_t)(16 * (kv.first / 2) + 2 * (kv.first / 2)) * sizeof(double2);  // 2 Pc <= 16L, plus 2L
+  for (const auto& kv : D->conv_kernels) b += (size_t)(8 * (kv.first / 2) + 2 * (kv.first / 2)) * sizeof(double2);  // Pc <= 8L, plus 2L
+  for (const auto& kv : D->beta_matrices) {
+    Geometry g{};
+    g.L = kv.first / kBetaKinds / 2;
+    g.mw = kv.first / kBetaKinds % 2;
+    g.nb = g.mw ? g.L : g.L + 1;
+    b += beta_matrix_bytes(g, kv.first % kBetaKinds);
+  }
   for (const auto& kv : D->ffts) b += (size_t)4 * (kv.first + 256) * sizeof(double2) + kv.second->mm_bytes;
   for (const auto& kv : D->bases) b += 4096 * sizeof(long long);
   return b;
@@ -338,51 +345,11 @@ int ensure_fft(Device* D, int n, FftPlan* out) {
     cld r = root_l(k, 2LL * n);  // e^{-i pi k/n}
     host[half_at + k] = make_double2((double)r.real(), (double)r.imag());
   }
-  // Rader's algorithm for the prime 127 (gamma length at N = 64): X[3^{-b}] =
-  // x[0] + sum_a x[3^a] w^{3^{a-b}}, a cyclic convolution of length 126
-  const bool rader = n == 127;
-  size_t rader_at = host.size();
-  std::vector<int> perm;
-  if (rader) {
-    const int q = n - 1;
-    host.resize(rader_at + 2 * (size_t)q);
-    for (int k = 0; k < q; k++) {
-      cld r = root_l(k, q);
-      host[rader_at + k] = make_double2((double)r.real(), (double)r.imag());
-    }
-    perm.resize(2 * (size_t)q);
-    std::vector<int> pw(q);  // 3^a mod n
-    long long v = 1;
-    for (int a = 0; a < q; a++) {
-      pw[a] = (int)v;
-      v = v * 3 % n;
-    }
-    for (int a = 0; a < q; a++) {
-      perm[a] = pw[a];
-      perm[q + a] = pw[(q - a) % q];  // 3^{-a} = 3^{q-a}
-    }
-    // kernel: FFT_q of v[m] = w^{3^{-m}}, divided by q (direct long-double DFT)
-    for (int k = 0; k < q; k++) {
-      cld acc(0, 0);
-      for (int m = 0; m < q; m++) acc += root_l(perm[q + m], n) * root_l((long long)m * k % q, q);
-      acc /= (long double)q;
-      host[rader_at + q + k] = make_double2((double)acc.real(), (double)acc.imag());
-    }
-  }
   cudaError_t e = cudaMalloc(&dp->mem, host.size() * sizeof(double2));
   if (e != cudaSuccess) return fail(kOutOfMemory, "FFT table allocation failed");
   e = cudaMemcpy(dp->mem, host.data(), host.size() * sizeof(double2), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return fail(kCudaError, std::string("FFT table upload: ") + cudaGetErrorString(e));
   P.half = dp->mem + half_at;
-  if (rader) {
-    P.rroots = dp->mem + rader_at;
-    P.rkern = dp->mem + rader_at + (n - 1);
-    e = cudaMalloc(&dp->imem, perm.size() * sizeof(int));
-    if (e != cudaSuccess) return fail(kOutOfMemory, "FFT table allocation failed");
-    e = cudaMemcpy(dp->imem, perm.data(), perm.size() * sizeof(int), cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) return fail(kCudaError, std::string("FFT table upload: ") + cudaGetErrorString(e));
-    P.rperm = dp->imem;
-  }
   if (!P.blue) {
     P.roots = dp->mem;
   } else {
@@ -408,9 +375,7 @@ int ensure_fft(Device* D, int n, FftPlan* out) {
 //                 a unit sample at its first self-mirror beta row (MW: row
 //                 L-1 at beta = pi; MWSS: row 0 at beta = 0), with the full
 //                 weights w (so3_sampling.c:32-51);
-//  [Pc + L, Pc + 2L) h_1(m'): the same for MWSS row L (beta = pi); zero for MW;
-//  [Pc + 2L, 2 Pc + 2L) 4 pi^2 / Pc * DFT(w) of the full weights (the
-//                 convolution of the adjoint forward transform).
+//  [Pc + L, Pc + 2L) h_1(m'): the same for MWSS row L (beta = pi); zero for MW.
 // h(m') = G(m') - G(-m') (m' >= 1), G(0), with G = 2 pi v * w and v(m'') =
 // e^{-i m'' beta} / P, m'' in [-(L-1), L-1].
 int ensure_conv_kernel(Device* D, const Geometry& g, const double2** out) {
@@ -431,16 +396,7 @@ int ensure_conv_kernel(Device* D, const Geometry& g, const double2** out) {
   std::vector<cld> w(Pc, cld(0, 0));
   for (int p = -2 * (L - 1); p <= 2 * (L - 1); p += 2) w[((p % Pc) + Pc) % Pc] += weight(p);
   fft_ld(w, +1);
-  std::vector<double2> host(2 * (size_t)Pc + 2 * (size_t)L, make_double2(0.0, 0.0));
-  {
-    std::vector<cld> wf(Pc, cld(0, 0));
-    for (int p = -2 * (L - 1); p <= 2 * (L - 1); p++) wf[((p % Pc) + Pc) % Pc] += weight(p);
-    fft_ld(wf, -1);  // forward DFT
-    for (int r = 0; r < Pc; r++) {
-      const cld v = wf[r] * (4.0L * kPiL * kPiL / (long double)Pc);
-      host[(size_t)Pc + 2 * (size_t)L + r] = make_double2((double)v.real(), (double)v.imag());
-    }
-  }
+  std::vector<double2> host((size_t)Pc + 2 * (size_t)L, make_double2(0.0, 0.0));
   for (int r = 0; r < Pc; r++) {
     // w_e is real and even: its spectrum is real
     const long double v = w[r].real() * (2.0L * kPiL / (long double)Pc);
@@ -468,6 +424,27 @@ int ensure_conv_kernel(Device* D, const Geometry& g, const double2** out) {
     return fail(kOutOfMemory, "beta-stage weight table allocation failed");
   SO3G_CUDA(cudaMemcpy(d, host.data(), host.size() * sizeof(double2), cudaMemcpyHostToDevice));
   D->conv_kernels[key] = d;
+  *out = d;
+  return kOk;
+}
+
+int ensure_beta_matrix(Device* D, const Geometry& g, int kind, const FftPlan& pP, cudaStream_t s, const double** out) {
+  const int key = (2 * g.L + (g.mw ? 1 : 0)) * kBetaKinds + kind;
+  auto it = D->beta_matrices.find(key);
+  if (it != D->beta_matrices.end()) {
+    *out = it->second;
+    return kOk;
+  }
+  double* d = nullptr;
+  if (cudaMalloc(&d, beta_matrix_bytes(g, kind)) != cudaSuccess)
+    return fail(kOutOfMemory, "beta-stage matrix allocation failed");
+  int rc = launch_beta_matrix_table(g, kind, pP, d, s);
+  if (rc == kOk && cudaStreamSynchronize(s) != cudaSuccess) rc = fail(kCudaError, "beta-stage matrix build failed");
+  if (rc != kOk) {
+    cudaFree(d);
+    return rc;
+  }
+  D->beta_matrices[key] = d;
   *out = d;
   return kOk;
 }
