@@ -26,8 +26,11 @@
 //  * Grid order |n|-pair fastest, then rows, then |m|: CTAs resident at the
 //    same time share one Delta tile column and one coefficient slice in L2.
 #include <cstdlib>
+#include <type_traits>
 
+#include "dft_mm.cuh"
 #include "so3gpu_internal.h"
+#include "tc_sm100.cuh"
 
 namespace so3g {
 
@@ -110,10 +113,9 @@ __device__ __forceinline__ void mac_chunk(const Slab& S, int lc, int warp, int l
 }
 }  // namespace
 
-// FP64 contraction engine for complex signals: the FP64 tensor cores
-// (mma.sync f64; measured 1.3-1.6x faster at L=512, N=64), unless the
-// environment sets SO3GPU_FP64_MMA=0 (the FP64 FMA kernels, which real
-// signals always use).
+// FP64 contraction engine: the FP64 tensor cores, unless the environment sets
+// SO3GPU_FP64_MMA=0 (the FP64 FMA kernels, an independent implementation that
+// the tests compare with).
 static bool fp64_tensor_cores() {
   const char* e = getenv("SO3GPU_FP64_MMA");
   return !(e && e[0] == '0');
@@ -167,14 +169,14 @@ __global__ void __launch_bounds__(kThreads, 1) inverse_contract_kernel(InvArgs a
       const int lc = idx / (kRows * kCols), rem = idx - lc * kRows * kCols, r = rem / kCols, col = rem - r * kCols;
       const int l = lbase + lc;
       const bool ok = l < L && mp0 + r <= l && mu0 + col <= l;
-      const double* src = ok ? a.dl + dl_plane_offset(l) + (long long)(mp0 + r) * (l + 1) + mu0 + col : a.dl;
+      const double* src = ok ? a.dl + dl_index(l, mp0 + r, mu0 + col) : a.dl;
       cp_async8(&S.B[lc][r][col], src, ok);
     }
     for (int idx = tid; idx < kChunk * kRows * kNG; idx += kThreads) {
       const int lc = idx / (kRows * kNG), rem = idx - lc * kRows * kNG, r = rem / kNG, j = rem - r * kNG;
       const int l = lbase + lc, nu = nu0 + j;
       const bool ok = l < L && act[j] && mp0 + r <= l && nu <= l;
-      const double* src = ok ? a.dl + dl_plane_offset(l) + (long long)(mp0 + r) * (l + 1) + nu : a.dl;
+      const double* src = ok ? a.dl + dl_index(l, mp0 + r, nu) : a.dl;
       cp_async8(&S.A[lc][r][j], src, ok);
     }
     for (int idx = tid; idx < kChunk * kCols * kNG * NSIGN; idx += kThreads) {
@@ -241,205 +243,6 @@ __global__ void __launch_bounds__(kThreads, 1) inverse_contract_kernel(InvArgs a
   }
 }
 
-// ------------------------------------------------------------------ inverse, FP64 tensor cores
-// The same contraction as inverse_contract_kernel on the FP64 tensor cores
-// (mma.sync.aligned.m8n8k4 f64): for a pair (mu, nu) = (|m|, |n|) it is the
-// product Y[m', c] = sum_l W[m', l] X[l, c] with W[m', l] = Delta^l_{m' mu}
-// Delta^l_{m' nu} and one column c = 2 s + part per sign combination s
-// (bit 0: m = -mu, bit 1: n = -nu) and real / imaginary part; X carries
-// (2l+1)/(8 pi^2), and (-1)^l on combinations with one negative index (the
-// output carries the (-1)^{m'} of those).  One MMA: 8 rows m' x 8 columns x
-// 4 reduction steps l (256 multiply-adds).  CTA tile: 32 m' x 16 mu x 2 nu;
-// warp w: rows 8 (w & 3) .. +7, mu block 8 (w >> 2) .. +7, both nu: 16 MMAs
-// (32 accumulators per lane) per 4-step chunk.  Delta tiles staged with
-// cp.async (double buffered); X built from the coefficients with the weights
-// applied while staging (its loads are issued one chunk ahead).
-namespace {
-constexpr int kDT = 256;       // threads
-constexpr int kDR = 32;        // m' per CTA
-constexpr int kDM = 16;        // mu per CTA
-constexpr int kDN = 2;         // nu per CTA
-constexpr int kDK = 4;         // l per chunk (MMA K)
-constexpr int kBP = 17;        // Bm pitch (doubles): lanes (g, q) hit distinct bank pairs
-constexpr int kAP = 3;         // An pitch
-// X block of one (mu, nu): 8 columns c x 4 steps l, element c * 4 + l.  Block
-// pitches 36 (nu) and 81 (mu) doubles put the staging stores of a warp on 16
-// distinct bank pairs (inverse lanes: sign, nu, 4 mu; forward lanes: l, sign,
-// nu); a fragment read is 32 consecutive doubles either way.
-constexpr int kXJ = 36, kXM = 81;
-struct DSlab {
-  double Bm[kDR][kDK][kBP];           // Delta^l_{m', mu0 + j}
-  double An[kDR][kDK][kAP];           // Delta^l_{m', nu0 + j}
-  double X[kDM * kXM];                // [mu][nu][c][l], weighted and sign-folded
-};
-__device__ __forceinline__ double& xat(DSlab& S, int jm, int j, int c, int l) {
-  return S.X[jm * kXM + j * kXJ + c * kDK + l];
-}
-
-__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-               : "+d"(c[0]), "+d"(c[1])
-               : "d"(a), "d"(b));
-}
-}  // namespace
-
-template <int NSIGN>
-__global__ void __launch_bounds__(kDT, 2) inverse_contract_dmma_kernel(InvArgs a) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  DSlab* st = reinterpret_cast<DSlab*>(smraw);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
-  const int nu0 = a.nu_lo + blockIdx.x * kDN, mp0 = blockIdx.y * kDR, mu0 = blockIdx.z * kDM;
-  const int L = a.L;
-  bool act[kDN];
-#pragma unroll
-  for (int j = 0; j < kDN; j++) act[j] = (nu0 + j < a.nu_hi) && !plane_skipped(a.n_mode, a.N, nu0 + j);
-  const int mb = warp & 3, jm0 = 8 * (warp >> 2);  // rows 8 mb .., mu block jm0 ..
-  double acc[8][kDN][2];
-#pragma unroll
-  for (int i = 0; i < 8; i++)
-#pragma unroll
-    for (int j = 0; j < kDN; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
-
-  // reduction range, aligned to the chunk: l in [l_lo, L), l_lo = 4 floor(max(...)/4)
-  const int lstart = max(max(a.L0, nu0), max(mp0, mu0));
-  const int l_lo = lstart & ~(kDK - 1);
-  const int nchunk = l_lo < L ? (L - l_lo + kDK - 1) / kDK : 0;
-  long long bsel[kDN][2];
-#pragma unroll
-  for (int j = 0; j < kDN; j++) {
-    const int nu = min(nu0 + j, a.N - 1);
-    bsel[j][0] = a.base[a.plane0 + nu];
-    bsel[j][1] = NSIGN == 4 ? a.base[a.plane0 - nu] : 0;
-  }
-
-  auto stage_delta = [&](int c, DSlab& S) {
-    const int lb = l_lo + c * kDK;
-    for (int idx = tid; idx < kDR * kDK * kDM; idx += kDT) {  // mu fastest: a row segment of a plane
-      const int j = idx % kDM, rest = idx / kDM, lc = rest % kDK, r = rest / kDK;
-      const int l = lb + lc, mp = mp0 + r, mu = mu0 + j;
-      const bool ok = l < L && l >= lstart && mp <= l && mu <= l;
-      const double* src = ok ? a.dl + dl_plane_offset(l) + (long long)mp * (l + 1) + mu : a.dl;
-      cp_async8(&S.Bm[r][lc][j], src, ok);
-    }
-    for (int idx = tid; idx < kDR * kDK * kDN; idx += kDT) {
-      const int j = idx % kDN, rest = idx / kDN, lc = rest % kDK, r = rest / kDK;
-      const int l = lb + lc, mp = mp0 + r, nu = nu0 + j;
-      const bool ok = l < L && l >= lstart && act[j] && mp <= l && nu <= l;
-      const double* src = ok ? a.dl + dl_plane_offset(l) + (long long)mp * (l + 1) + nu : a.dl;
-      cp_async8(&S.An[r][lc][j], src, ok);
-    }
-  };
-  // coefficient loads of a chunk: 4 l x 16 mu x 2 nu x NSIGN complex values, 2 per thread
-  constexpr int kXN = kDK * kDM * kDN * 4;  // 512 (NSIGN 4) slots, 2 per thread
-  double2 xv[2];
-  auto load_x = [&](int c) {
-    const int lb = l_lo + c * kDK;
-#pragma unroll
-    for (int u = 0; u < 2; u++) {
-      const int idx = tid + u * kDT;  // sg fastest, then nu, mu, l
-      const int sg = idx & 3, j = (idx >> 2) & 1, jm = (idx >> 3) & 15, lc = idx >> 7;
-      const int l = lb + lc, mu = mu0 + jm, nu = nu0 + j;
-      const bool ok = sg < NSIGN && l < L && l >= lstart && act[j] && mu <= l && nu <= l &&
-                      !((sg & 1) && mu == 0) && !((sg & 2) && nu == 0);
-      const int m = (sg & 1) ? -mu : mu;
-      xv[u] = ok ? __ldg(a.flmn + bsel[j][sg >> 1] + (long long)l * l + l + m) : make_double2(0.0, 0.0);
-    }
-  };
-  auto store_x = [&](int c, DSlab& S) {
-    const int lb = l_lo + c * kDK;
-#pragma unroll
-    for (int u = 0; u < 2; u++) {
-      const int idx = tid + u * kDT;
-      const int sg = idx & 3, j = (idx >> 2) & 1, jm = (idx >> 3) & 15, lc = idx >> 7;
-      const int l = lb + lc;
-      double w = a.wconst > 0.0 ? a.wconst : (2.0 * l + 1.0) * kInv8Pi2;
-      if ((sg == 1 || sg == 2) && (l & 1)) w = -w;  // one negative index: (-1)^l here
-      xat(S, jm, j, 2 * sg, lc) = xv[u].x * w;
-      xat(S, jm, j, 2 * sg + 1, lc) = xv[u].y * w;
-    }
-  };
-  static_assert(kXN == 2 * kDT, "two coefficient slots per thread");
-
-  if (nchunk > 0) {
-    stage_delta(0, st[0]);
-    cp_commit();
-    load_x(0);
-    for (int c = 0; c < nchunk; c++) {
-      DSlab& S = st[c & 1];
-      store_x(c, S);
-      if (c + 1 < nchunk) {
-        stage_delta(c + 1, st[(c + 1) & 1]);
-        cp_commit();
-        load_x(c + 1);
-        cp_wait<1>();
-      } else {
-        cp_wait<0>();
-      }
-      __syncthreads();
-      // fragments: A (W) row g = m' 8 mb + g, column q = l; B (X) row q = l, column g = c
-      const double an0 = S.An[8 * mb + g][q][0], an1 = S.An[8 * mb + g][q][1];
-#pragma unroll
-      for (int i = 0; i < 8; i++) {
-        const double bm = S.Bm[8 * mb + g][q][jm0 + i];
-        dmma(acc[i][0], bm * an0, xat(S, jm0 + i, 0, g, q));
-        dmma(acc[i][1], bm * an1, xat(S, jm0 + i, 1, g, q));
-      }
-      __syncthreads();
-    }
-  }
-
-  // accumulator (row g, columns 2q, 2q+1) = sign combination q, real / imaginary part
-  const int mp = mp0 + 8 * mb + g;
-  const int s = q;
-  if (mp >= L || s >= NSIGN) return;
-  const int ms = (s & 1) ? -1 : 1, ns = (s & 2) ? -1 : 1;
-  const double odd_mp = (mp & 1) ? -1.0 : 1.0;
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    const int mu = mu0 + jm0 + i;
-    if (mu >= L || (ms < 0 && mu == 0)) continue;
-#pragma unroll
-    for (int j = 0; j < kDN; j++) {
-      const int nu = nu0 + j;
-      if (nu >= a.nu_hi || (ns < 0 && nu == 0)) continue;
-      const int m = ms * mu, n = ns * nu;
-      double2 v = make_double2(acc[i][j][0], acc[i][j][1]);
-      if (ms * ns < 0) v = sc(v, odd_mp);
-      v = ipow_mul(v, n - m + 4 * L);
-      a.W[(long long)(a.plane0 + n) * a.QS + (long long)(m + L - 1) * a.CS + mp] = v;
-    }
-  }
-}
-
-int launch_inverse_contract(const Geometry& g, int n_mode, const double2* flmn, const long long* bases,
-                            const double* dl, double2* W, int sym_n0, cudaStream_t s, int nu_lo, int nu_hi,
-                            double wconst) {
-  if (nu_hi < 0 || nu_hi > g.N) nu_hi = g.N;
-  if (nu_lo >= nu_hi) return kOk;
-  InvArgs a{flmn, bases, dl, W + g.QOFF, g.L, g.N, g.L0, g.plane0, n_mode, g.real, sym_n0, nu_lo, nu_hi, g.CS, g.QS,
-            wconst};
-  if (!g.real && !sym_n0 && fp64_tensor_cores()) {
-    dim3 gd((nu_hi - nu_lo + kDN - 1) / kDN, (g.L + kDR - 1) / kDR, (g.L + kDM - 1) / kDM);
-    const int smem = (int)(2 * sizeof(DSlab));
-    SO3G_CUDA(cudaFuncSetAttribute(inverse_contract_dmma_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    inverse_contract_dmma_kernel<4><<<gd, kDT, smem, s>>>(a);
-    SO3G_LAUNCHED();
-    SO3G_CUDA(cudaGetLastError());
-    return kOk;
-  }
-  dim3 grid((nu_hi - nu_lo + kNG - 1) / kNG, (g.L + kRows - 1) / kRows, (g.L + kCols - 1) / kCols);
-  if (g.real) {
-    SO3G_CUDA(cudaFuncSetAttribute(inverse_contract_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
-    inverse_contract_kernel<2><<<grid, kThreads, kSmem, s>>>(a);
-  } else {
-    SO3G_CUDA(cudaFuncSetAttribute(inverse_contract_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
-    inverse_contract_kernel<4><<<grid, kThreads, kSmem, s>>>(a);
-  }
-  SO3G_LAUNCHED();
-  SO3G_CUDA(cudaGetLastError());
-  return kOk;
-}
-
 // ------------------------------------------------------------------ forward
 struct FwdArgs {
   const double2* W;
@@ -482,14 +285,14 @@ __global__ void __launch_bounds__(kThreads, 1) forward_contract_kernel(FwdArgs a
       const int mc = idx / (kRows * kCols), rem = idx - mc * kRows * kCols, r = rem / kCols, col = rem - r * kCols;
       const int mp = mbase + mc, l = l0 + r;
       const bool ok = l < L && mp <= l && mu0 + col <= l;
-      const double* src = ok ? a.dl + dl_plane_offset(l) + (long long)mp * (l + 1) + mu0 + col : a.dl;
+      const double* src = ok ? a.dl + dl_index(l, mp, mu0 + col) : a.dl;
       cp_async8(&S.B[mc][r][col], src, ok);
     }
     for (int idx = tid; idx < kChunk * kRows * kNG; idx += kThreads) {
       const int mc = idx / (kRows * kNG), rem = idx - mc * kRows * kNG, r = rem / kNG, j = rem - r * kNG;
       const int mp = mbase + mc, l = l0 + r, nu = nu0 + j;
       const bool ok = l < L && act[j] && mp <= l && nu <= l;
-      const double* src = ok ? a.dl + dl_plane_offset(l) + (long long)mp * (l + 1) + nu : a.dl;
+      const double* src = ok ? a.dl + dl_index(l, mp, nu) : a.dl;
       cp_async8(&S.A[mc][r][j], src, ok);
     }
     for (int idx = tid; idx < kChunk * kCols * kNG * NSIGN; idx += kThreads) {
@@ -555,130 +358,345 @@ __global__ void __launch_bounds__(kThreads, 1) forward_contract_kernel(FwdArgs a
   }
 }
 
-// ------------------------------------------------------------------ forward, FP64 tensor cores
-// The forward contraction on the FP64 tensor cores: for a pair (mu, nu),
-// Y[l, c] = sum_{m'} W[l, m'] X[m', c] with W[l, m'] = Delta^l_{m' mu}
-// Delta^l_{m' nu} (m' <= l) and X the spectra G(n, m, m') of the column-major
-// scratch, (-1)^{m'} folded in for combinations with one negative index (the
-// output carries their (-1)^l).  CTA tile 32 l x 16 mu x 2 nu, warps and
-// staging as in inverse_contract_dmma_kernel.
-template <int NSIGN>
-__global__ void __launch_bounds__(kDT, 2) forward_contract_dmma_kernel(FwdArgs a) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  DSlab* st = reinterpret_cast<DSlab*>(smraw);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
-  const int nu0 = a.nu_lo + blockIdx.x * kDN, l0 = blockIdx.y * kDR, mu0 = blockIdx.z * kDM;
-  const int L = a.L;
-  bool act[kDN];
-#pragma unroll
-  for (int j = 0; j < kDN; j++) act[j] = (nu0 + j < a.nu_hi) && !plane_skipped(a.n_mode, a.N, nu0 + j);
-  if (!act[0] && !act[1]) return;  // caller-zeroed blocks stay untouched
-  const int mb = warp & 3, jm0 = 8 * (warp >> 2);
-  double acc[8][kDN][2];
-#pragma unroll
-  for (int i = 0; i < 8; i++)
-#pragma unroll
-    for (int j = 0; j < kDN; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
+// ------------------------------------------------------------------ FP64 tensor cores
+// Both contractions on the FP64 tensor cores (mma.sync m8n8k4 f64).  For a pair
+// (mu, nu) = (|m|, |n|) they are products with W = Delta_{m' mu} Delta_{m' nu}:
+//   inverse  Y[m', c] = sum_l  W[m', l] X[l, c]
+//   forward  Y[l, c]  = sum_m' W[m', l] X[m', c]
+// with 8 columns c = 2 s + part: sign combination s (bit 0: m = -mu, bit 1:
+// n = -nu) and real / imaginary part.  One MMA: 8 rows x 8 columns x 4
+// reduction steps (256 multiply-adds), its row operand formed in registers by
+// one multiplication.  (2l+1)/(8 pi^2) rides on the nu factor, the sign
+// (-1)^(reduction index) of combinations with one negative index is flipped in
+// the column operand, the one of the row index in the result.
+//
+// CTA tile: 32 rows x 8 mu x 2 nu, two CTAs per SM; 8 reduction entries (two
+// MMA steps) per stage of a three-stage ring.  Eight warps multiply (16 rows x 4
+// mu x 1 nu each: 14 fragment reads per 8 MMAs), a ninth copies and runs ahead:
+// the Delta blocks as they are stored (dl_index) by bulk copies, 512 bytes per mu
+// and row tile, the coefficients from the caller's layout or the spectra from the
+// column-major scratch by cp.async, all counted on mbarriers.  Row tiles that a
+// degree does not reach (m' > l) are neither copied nor multiplied.
+//
+// Bound by shared-memory reads (3.5 of 4 wavefronts per MMA) and by the
+// multiplications that form W on the same pipe.  Measured at L = 512, N = 64
+// (ms, inverse / forward): 2.60 / 2.44, against 4.97 / 5.92 for staging by all
+// warps with 8-byte copies from row-major planes; 3.09 / 2.89 without the copying
+// warp (a barrier per chunk aligned the warps' bursts).  64 rows x 4 nu (one CTA
+// of 16 warps) gives 2.57 / 2.42 there but 39 / 37 us against 23 / 30 at L = 128,
+// N = 16; m16n8k8 MMAs change nothing.
+namespace {
+constexpr int kCRt = 4, kCMu = 8, kCNu = 2;  // row tiles, mu, nu of a CTA
+constexpr int kCMt = 2, kCNw = 1;            // row tiles and nu of a warp (4 mu)
+constexpr int kCStages = 3;
+constexpr int kCThreads = 32 * (kCRt / kCMt) * 2 * (kCNu / kCNw) + 32;
+constexpr int kXB = 33;  // slots of an X block of one (mu, nu): 8 entries x 4 combinations, and one of padding
 
-  const int ltop = min(L - 1, l0 + kDR - 1);
-  const bool any = ltop >= max(max(a.L0, nu0), mu0);
-  const int nchunk = any ? (ltop + 1 + kDK - 1) / kDK : 0;  // m' = 0 .. ltop
+struct ContractArgs {
+  const double2* flmn_in;  // inverse: coefficients
+  double2* flmn_out;       // forward: coefficients
+  const long long* base;   // per plane
+  const double* dl;
+  double2* W;              // column-major scratch part
+  int L, N, L0, plane0, n_mode, nsign, sym_n0, compact;
+  int nu_lo, nu_hi, nu0;   // |n| range of this launch; first nu of the grid (a multiple of the tile)
+  long long CS, QS;
+  double wconst;           // inverse, > 0: this weight for every l
+  double lw;               // forward, > 0: outputs times lw (2l+1)
+};
 
-  auto stage_delta = [&](int c, DSlab& S) {
-    const int mb0 = c * kDK;
-    for (int idx = tid; idx < kDR * kDK * kDM; idx += kDT) {
-      const int j = idx % kDM, rest = idx / kDM, mc = rest % kDK, r = rest / kDK;
-      const int mp = mb0 + mc, l = l0 + r, mu = mu0 + j;
-      const bool ok = l < L && mp <= l && mu <= l;
-      const double* src = ok ? a.dl + dl_plane_offset(l) + (long long)mp * (l + 1) + mu : a.dl;
-      cp_async8(&S.Bm[r][mc][j], src, ok);
-    }
-    for (int idx = tid; idx < kDR * kDK * kDN; idx += kDT) {
-      const int j = idx % kDN, rest = idx / kDN, mc = rest % kDK, r = rest / kDK;
-      const int mp = mb0 + mc, l = l0 + r, nu = nu0 + j;
-      const bool ok = l < L && act[j] && mp <= l && nu <= l;
-      const double* src = ok ? a.dl + dl_plane_offset(l) + (long long)mp * (l + 1) + nu : a.dl;
-      cp_async8(&S.An[r][mc][j], src, ok);
-    }
-  };
-  double2 xv[2];
-  auto load_x = [&](int c) {
-    const int mb0 = c * kDK;
-#pragma unroll
-    for (int u = 0; u < 2; u++) {
-      const int idx = tid + u * kDT;  // m' fastest (contiguous in a column), then sign, nu, mu
-      const int mc = idx & 3, sg = (idx >> 2) & 3, j = (idx >> 4) & 1, jm = idx >> 5;
-      const int mp = mb0 + mc, mu = mu0 + jm, nu = nu0 + j;
-      const bool ok = sg < NSIGN && mp < L && act[j] && mu < L && !((sg & 1) && mu == 0) && !((sg & 2) && nu == 0);
-      const int n = (sg & 2) ? -nu : nu, m = (sg & 1) ? -mu : mu;
-      xv[u] = ok ? __ldg(a.W + (long long)(a.plane0 + n) * a.QS + (long long)(L - 1 + m) * a.CS + mp)
-                 : make_double2(0.0, 0.0);
-    }
-  };
-  auto store_x = [&](int c, DSlab& S) {
-    const int mb0 = c * kDK;
-#pragma unroll
-    for (int u = 0; u < 2; u++) {
-      const int idx = tid + u * kDT;
-      const int mc = idx & 3, sg = (idx >> 2) & 3, j = (idx >> 4) & 1, jm = idx >> 5;
-      const double w = ((sg == 1 || sg == 2) && ((mb0 + mc) & 1)) ? -1.0 : 1.0;  // (-1)^{m'}
-      xat(S, jm, j, 2 * sg, mc) = xv[u].x * w;
-      xat(S, jm, j, 2 * sg + 1, mc) = xv[u].y * w;
-    }
-  };
+__device__ int g_contract_error;  // bit 2: a wait for a copy gave up (see tc::mbar_wait)
 
-  if (nchunk > 0) {
-    stage_delta(0, st[0]);
-    cp_commit();
-    load_x(0);
-    for (int c = 0; c < nchunk; c++) {
-      DSlab& S = st[c & 1];
-      store_x(c, S);
-      if (c + 1 < nchunk) {
-        stage_delta(c + 1, st[(c + 1) & 1]);
-        cp_commit();
-        load_x(c + 1);
-        cp_wait<1>();
+__device__ __forceinline__ void cp16_to(uint32_t dst, const void* src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0));
+}
+
+constexpr int kCStage = kCRt * kCMu * 64 + kCRt * kCNu * 64 + 2 * kCMu * kCNu * kXB;  // doubles
+}  // namespace
+
+template <bool FWD>
+__global__ void __launch_bounds__(kCThreads, 2) contract_mma_kernel(ContractArgs a) {
+  constexpr int RT = kCRt, NU = kCNu, MT = kCMt, NW = kCNw, ST = kCStages;
+  constexpr int WR = RT / MT, NWARP = kCThreads / 32 - 1;  // product warps; one more copies
+  constexpr int BSZ = RT * kCMu * 64, ASZ = RT * NU * 64, STAGE = kCStage;
+  extern __shared__ __align__(16) double smc[];
+  __shared__ long long bsel[NU][2];
+  __shared__ __align__(8) unsigned long long full[ST], empty[ST];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
+  const int wr = warp % WR, wm = warp / WR % 2, wn = warp / (2 * WR);
+  const int nu0 = a.nu0 + blockIdx.x * NU, rt0 = blockIdx.y * RT, mu0 = blockIdx.z * kCMu;
+  const int L = a.L, LC = (L + 7) >> 3;
+  unsigned act = 0;  // bit j: nu0 + j is computed by this launch
+#pragma unroll
+  for (int j = 0; j < NU; j++)
+    if (nu0 + j >= a.nu_lo && nu0 + j < a.nu_hi && !plane_skipped(a.n_mode, a.N, nu0 + j)) act |= 1u << j;
+  if (FWD && !act) return;  // caller-zeroed blocks stay untouched
+  if (tid < NU) {
+    const int nu = min(nu0 + tid, a.N - 1);
+    bsel[tid][0] = a.base[a.plane0 + nu];
+    bsel[tid][1] = a.nsign == 4 ? a.base[a.plane0 - nu] : 0;
+  }
+  __syncthreads();
+
+  // chunks of 8 reduction entries: inverse l >= max(L0, mu, nu, m'), forward m' <= l
+  const int lmin = max(max(a.L0, nu0), mu0);
+  int ch0, ch1;
+  if (FWD) {
+    ch0 = 0;
+    ch1 = 8 * (rt0 + RT) > lmin ? min(rt0 + RT, LC) : 0;
+  } else {
+    ch0 = max(lmin >> 3, rt0);
+    ch1 = act ? LC : 0;
+  }
+
+  const uint32_t full0 = tc::smem_u32(full), empty0 = tc::smem_u32(empty);
+  if (tid == 0) {
+    for (int st = 0; st < ST; st++) {
+      tc::mbar_init(full0 + 8 * st, 33);  // the copying lanes' loads of X and the expected bytes
+      tc::mbar_init(empty0 + 8 * st, NWARP);
+    }
+    tc::mbar_fence_init();
+  }
+  __syncthreads();
+
+  if (warp == NWARP) {
+    // ------------------------------------------------ copies
+    // The Delta blocks of a row tile are one run per operand (8 mu, NU nu): 2 RT
+    // lanes bring them with one bulk copy each.  X by 16-byte copies, forward
+    // with m' fastest (128 bytes of a column), inverse with mu fastest (runs of
+    // a coefficient row).
+    static_assert(2 * RT <= 32, "one lane per bulk copy");
+    const uint32_t sm0 = tc::smem_u32(smc), xs0 = sm0 + (BSZ + ASZ) * 8;
+    const int trt = rt0 + lane % RT;
+    const bool tmu = lane < RT;
+    const uint32_t tdst = sm0 + (tmu ? (trt - rt0) * (kCMu * 512) : BSZ * 8 + (trt - rt0) * (NU * 512));
+    const long long toff = (tmu ? mu0 : nu0) * 64;
+    // forward: lane = (entry, combination); inverse: lane = (mu, entry & 3)
+    const int xe = FWD ? lane & 7 : lane >> 3, xm = lane & 7, xc = lane >> 3;
+    const double2* px[FWD ? NU : 4 * NU];
+    int xlo[NU];
+#pragma unroll
+    for (int j = 0; j < NU; j++) {
+      const int nu = nu0 + j, mu = mu0 + xm;
+      if (FWD) {
+        px[j] = a.W + (long long)(a.plane0 + ((xc & 2) ? -nu : nu)) * a.QS + (long long)(L - 1 + ((xc & 1) ? -mu0 : mu0)) * a.CS;
+        xlo[j] = xc < a.nsign && (act >> j & 1) ? 0 : L;
       } else {
-        cp_wait<0>();
-      }
-      __syncthreads();
-      const double an0 = S.An[8 * mb + g][q][0], an1 = S.An[8 * mb + g][q][1];
 #pragma unroll
-      for (int i = 0; i < 8; i++) {
-        const double bm = S.Bm[8 * mb + g][q][jm0 + i];
-        dmma(acc[i][0], bm * an0, xat(S, jm0 + i, 0, g, q));
-        dmma(acc[i][1], bm * an1, xat(S, jm0 + i, 1, g, q));
+        for (int c = 0; c < 4; c++) px[4 * j + c] = a.flmn_in + bsel[j][c >> 1] + ((c & 1) ? -mu : mu);
+        xlo[j] = mu < L && (act >> j & 1) ? max(max(a.L0, mu), nu) : L;
       }
-      __syncthreads();
     }
+    const long long cstep = (xc & 1) ? -a.CS : a.CS;
+    int st = 0;
+    uint32_t phase = 1;  // of the ring slot's previous use
+    for (int ch = ch0; ch < ch1; ch++) {
+      if (ch - ch0 >= ST) tc::mbar_wait(empty0 + 8 * st, phase, &g_contract_error, 4);
+      const uint32_t at = (uint32_t)(st * STAGE * 8), bar = full0 + 8 * st;
+      const int lc = FWD ? trt : ch, mt = FWD ? ch : trt;
+      const bool v = lane < 2 * RT && mt <= lc && lc < LC && (tmu ? mu0 <= 8 * lc : nu0 < 8 * (lc + 1));
+      const unsigned got = __ballot_sync(0xffffffffu, v);
+      if (lane == 0)
+        tc::mbar_arrive_expect_tx(bar, __popc(got & ((1u << RT) - 1)) * (kCMu * 512) + __popc(got >> RT) * (NU * 512));
+      __syncwarp();
+      if (v)
+        tc::bulk_g2s(tdst + at, a.dl + dl_base(lc) + (long long)mt * (512 * (lc + 1)) + toff, (tmu ? kCMu : NU) * 512, bar);
+#pragma unroll
+      for (int j = 0; j < NU; j++) {
+        if (FWD) {
+          const int e = 8 * ch + xe;
+          const double2* src = px[j] + e;
+#pragma unroll
+          for (int m = 0; m < kCMu; m++, src += cstep) {
+            const bool ok = e >= xlo[j] && e < L && mu0 + m < L;
+            cp16_to(xs0 + at + 16 * ((j * kCMu + m) * kXB + xc * 8 + (xe ^ (4 * (xc & 1)))), ok ? src : a.W, ok);
+          }
+        } else {
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            const int e = 8 * ch + 4 * h + xe, off = e * e + e;
+            const bool in = e >= xlo[j] && e < L;
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+              const bool ok = in && c < a.nsign;
+              cp16_to(xs0 + at + 16 * ((j * kCMu + xm) * kXB + 4 * (4 * h + xe) + (c ^ (xe & 2))), ok ? px[4 * j + c] + off : a.flmn_in,
+                      ok);
+            }
+          }
+        }
+      }
+      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(bar) : "memory");
+      if (++st == ST) st = 0;
+      if (st == 0) phase ^= 1;
+    }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    return;
   }
 
-  const int l = l0 + 8 * mb + g;
-  const int s = q;
-  if (l >= L || s >= NSIGN) return;
-  const int ms = (s & 1) ? -1 : 1, ns = (s & 2) ? -1 : 1;
-  const double odd_l = (l & 1) ? -1.0 : 1.0;
+  // -------------------------------------------------- products
+  double acc[MT][4][NW][2];
 #pragma unroll
-  for (int i = 0; i < 8; i++) {
-    const int mu = mu0 + jm0 + i;
-    if (mu >= L || mu > l || (ms < 0 && mu == 0)) continue;
+  for (int i = 0; i < MT; i++)
 #pragma unroll
-    for (int j = 0; j < kDN; j++) {
-      const int nu = nu0 + j;
-      if (!act[j] || (ns < 0 && nu == 0)) continue;
-      if (a.compact && l < nu) continue;  // not stored
-      const int m = ms * mu, n = ns * nu;
-      double2 v = make_double2(0.0, 0.0);
-      if (l >= max(a.L0, nu)) {
-        v = make_double2(acc[i][j][0], acc[i][j][1]);
-        if (ms * ns < 0) v = sc(v, odd_l);
-        v = ipow_mul(v, m - n + 4 * L);
-        if (a.lw > 0.0) v = sc(v, a.lw * (2.0 * l + 1.0));
+    for (int m = 0; m < 4; m++)
+#pragma unroll
+      for (int n = 0; n < NW; n++) acc[i][m][n][0] = acc[i][m][n][1] = 0.0;
+
+  const int s = g >> 1, part = g & 1;
+  // real signals with N = 1: the -m coefficient is (-1)^m conj of the +m one
+  const bool sym = !FWD && a.sym_n0 && s == 1;
+  const int xs = sym ? 0 : s;
+  // sign of this lane's column entries, for even and odd mu: the parity of the
+  // reduction index (entry 4 ks + q) of combinations with one negative index
+  const int flip = (s == 1 || s == 2) && (q & 1) ? 0x80000000 : 0;
+  const int flip0 = flip ^ (sym && part ? 0x80000000 : 0), flip1 = flip ^ (sym && !part ? 0x80000000 : 0);
+  const int slot0 = FWD ? q * 8 + (g ^ ((q >> 1) * 4)) : g * 8 + (q ^ (((g >> 1) & 1) * 4));
+  const int x0 = FWD ? 2 * (s * 8 + (q ^ (4 * (s & 1)))) + part : 2 * (4 * q + (xs ^ (q & 2))) + part;
+  // weight (2l+1)/(8 pi^2), or the constant one: fma(2l+1, wmul, wadd) is exact in its product
+  const double wmul = a.wconst > 0.0 ? 0.0 : kInv8Pi2, wadd = a.wconst > 0.0 ? a.wconst : 0.0;
+  double l21 = 2.0 * (8 * ch0 + q) + 1.0;
+  const int rt_lo = rt0 + wr * MT;
+  // one chunk; ALL: every row tile of the warp has entries with m' <= l
+  auto products = [&](int ch, int st, auto all) {
+    constexpr bool ALL = decltype(all)::value;
+    const double* Bs = smc + st * STAGE + (wr * MT * kCMu + wm * 4) * 64;
+    const double* As = smc + st * STAGE + BSZ + (wr * MT * NU + wn * NW) * 64;
+    const double* Xs = smc + st * STAGE + BSZ + ASZ + 2 * (wn * NW * kCMu + wm * 4) * kXB + x0;
+#pragma unroll
+    for (int ks = 0; ks < 2; ks++) {
+      // entry 4 + q: forward the lower half block (its row pairs swap alike), inverse the other l half
+      const int slot = FWD ? slot0 + 32 * ks : slot0 ^ (4 * ks);
+      const int dx = FWD ? 8 * ks * (1 - 2 * (s & 1)) : 32 * ks;
+      const double w = fma(l21 + 8.0 * ks, wmul, wadd);
+      double an[MT][NW];
+#pragma unroll
+      for (int i = 0; i < MT; i++)
+#pragma unroll
+        for (int n = 0; n < NW; n++) {
+          an[i][n] = As[(i * NU + n) * 64 + slot];
+          if (!FWD) an[i][n] *= w;
+        }
+#pragma unroll
+      for (int m = 0; m < 4; m++) {
+        double x[NW], wp[MT][NW];
+#pragma unroll
+        for (int n = 0; n < NW; n++) {
+          const double v = Xs[2 * (n * kCMu + m) * kXB + dx];
+          x[n] = __hiloint2double(__double2hiint(v) ^ ((m & 1) ? flip1 : flip0), __double2loint(v));
+        }
+#pragma unroll
+        for (int i = 0; i < MT; i++) {
+          const double bm = Bs[(i * kCMu + m) * 64 + slot];
+#pragma unroll
+          for (int n = 0; n < NW; n++) wp[i][n] = bm * an[i][n];
+        }
+#pragma unroll
+        for (int i = 0; i < MT; i++) {
+          if (!ALL && (FWD ? ch > rt_lo + i || rt_lo + i >= LC : rt_lo + i > ch)) continue;  // m' > l throughout
+#pragma unroll
+          for (int n = 0; n < NW; n++) mm::dmma(acc[i][m][n], wp[i][n], x[n]);
+        }
       }
-      a.flmn[a.base[a.plane0 + n] + (long long)l * l + l + m] = v;
+    }
+  };
+  const int rt_hi = rt_lo + MT - 1;
+  int st = 0;
+  uint32_t phase = 0;
+  for (int ch = ch0; ch < ch1; ch++) {
+    tc::mbar_wait(full0 + 8 * st, phase, &g_contract_error, 4);
+    if (FWD ? (ch <= rt_lo && rt_hi < LC) : rt_hi <= ch)
+      products(ch, st, std::true_type{});
+    else
+      products(ch, st, std::false_type{});
+    l21 += 16.0;
+    __syncwarp();
+    if (lane == 0) tc::mbar_arrive(empty0 + 8 * st);
+    if (++st == ST) st = 0, phase ^= 1;
+  }
+
+  // accumulator (row g, columns 2q, 2q+1) = combination q, real / imaginary part
+  const int ms = (q & 1) ? -1 : 1, ns = (q & 2) ? -1 : 1;
+  if (q >= a.nsign) return;
+#pragma unroll
+  for (int i = 0; i < MT; i++) {
+    const int row = 8 * (rt0 + wr * MT + i) + g;
+    if (row >= L) break;
+    const double odd_row = (row & 1) ? -1.0 : 1.0;
+#pragma unroll
+    for (int n = 0; n < NW; n++) {
+      const int nu = nu0 + wn * NW + n;
+      if (nu < a.nu_lo || nu >= a.nu_hi || (ns < 0 && nu == 0)) continue;
+      const bool on = act >> (wn * NW + n) & 1;
+      if (FWD && (!on || (a.compact && row < nu))) continue;  // untouched, or not stored
+#pragma unroll
+      for (int m = 0; m < 4; m++) {
+        const int mu = mu0 + wm * 4 + m;
+        if (mu >= L || (ms < 0 && mu == 0) || (FWD && mu > row)) continue;
+        double2 v = make_double2(acc[i][m][n][0], acc[i][m][n][1]);
+        if (ms * ns < 0) v = sc(v, odd_row);
+        if (FWD) {
+          if (row >= max(a.L0, nu)) {
+            v = ipow_mul(v, ms * mu - ns * nu + 4 * L);
+            if (a.lw > 0.0) v = sc(v, a.lw * (2.0 * row + 1.0));
+          } else {
+            v = make_double2(0.0, 0.0);
+          }
+          a.flmn_out[bsel[wn * NW + n][q >> 1] + (long long)row * row + row + ms * mu] = v;
+        } else {
+          v = ipow_mul(v, ns * nu - ms * mu + 4 * L);
+          a.W[(long long)(a.plane0 + ns * nu) * a.QS + (long long)(ms * mu + L - 1) * a.CS + row] = v;
+        }
+      }
     }
   }
+}
+
+namespace {
+template <bool FWD>
+int contract(ContractArgs a, cudaStream_t s) {
+  constexpr size_t smem = kCStages * kCStage * sizeof(double);
+  SO3G_CUDA(cudaFuncSetAttribute(contract_mma_kernel<FWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  a.nu0 = a.nu_lo / kCNu * kCNu;  // tiles stay aligned: a block of 8 degrees holds whole groups of nu
+  const dim3 grid((a.nu_hi - a.nu0 + kCNu - 1) / kCNu, (a.L + 8 * kCRt - 1) / (8 * kCRt), (a.L + kCMu - 1) / kCMu);
+  contract_mma_kernel<FWD><<<grid, kCThreads, smem, s>>>(a);
+  SO3G_LAUNCHED();
+  SO3G_CUDA(cudaGetLastError());
+  return kOk;
+}
+}  // namespace
+
+int contract_take_error() {
+  int v = 0, zero = 0;
+  if (cudaMemcpyFromSymbol(&v, g_contract_error, sizeof(int)) != cudaSuccess) return -1;
+  if (v) cudaMemcpyToSymbol(g_contract_error, &zero, sizeof(int));
+  return v;
+}
+
+int launch_inverse_contract(const Geometry& g, int n_mode, const double2* flmn, const long long* bases,
+                            const double* dl, double2* W, int sym_n0, cudaStream_t s, int nu_lo, int nu_hi,
+                            double wconst) {
+  if (nu_hi < 0 || nu_hi > g.N) nu_hi = g.N;
+  if (nu_lo >= nu_hi) return kOk;
+  InvArgs a{flmn, bases, dl, W + g.QOFF, g.L, g.N, g.L0, g.plane0, n_mode, g.real, sym_n0, nu_lo, nu_hi, g.CS, g.QS,
+            wconst};
+  if (fp64_tensor_cores()) {
+    ContractArgs c{};
+    c.flmn_in = flmn, c.base = bases, c.dl = dl, c.W = W + g.QOFF;
+    c.L = g.L, c.N = g.N, c.L0 = g.L0, c.plane0 = g.plane0, c.n_mode = n_mode, c.nsign = g.real ? 2 : 4;
+    c.sym_n0 = sym_n0, c.nu_lo = nu_lo, c.nu_hi = nu_hi, c.CS = g.CS, c.QS = g.QS, c.wconst = wconst;
+    return contract<false>(c, s);
+  }
+  dim3 grid((nu_hi - nu_lo + kNG - 1) / kNG, (g.L + kRows - 1) / kRows, (g.L + kCols - 1) / kCols);
+  if (g.real) {
+    SO3G_CUDA(cudaFuncSetAttribute(inverse_contract_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
+    inverse_contract_kernel<2><<<grid, kThreads, kSmem, s>>>(a);
+  } else {
+    SO3G_CUDA(cudaFuncSetAttribute(inverse_contract_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
+    inverse_contract_kernel<4><<<grid, kThreads, kSmem, s>>>(a);
+  }
+  SO3G_LAUNCHED();
+  SO3G_CUDA(cudaGetLastError());
+  return kOk;
 }
 
 int launch_forward_contract(const Geometry& g, int n_mode, const double2* W, const long long* bases,
@@ -688,14 +706,12 @@ int launch_forward_contract(const Geometry& g, int n_mode, const double2* W, con
   if (nu_lo >= nu_hi) return kOk;
   FwdArgs a{W + g.QOFF, bases, dl, flmn, g.L, g.N, g.L0, g.plane0, n_mode, g.real, storage_compact, nu_lo, nu_hi,
             g.CS, g.QS, lw};
-  if (!g.real && fp64_tensor_cores()) {
-    dim3 gd((nu_hi - nu_lo + kDN - 1) / kDN, (g.L + kDR - 1) / kDR, (g.L + kDM - 1) / kDM);
-    const int smem = (int)(2 * sizeof(DSlab));
-    SO3G_CUDA(cudaFuncSetAttribute(forward_contract_dmma_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    forward_contract_dmma_kernel<4><<<gd, kDT, smem, s>>>(a);
-    SO3G_LAUNCHED();
-    SO3G_CUDA(cudaGetLastError());
-    return kOk;
+  if (fp64_tensor_cores()) {
+    ContractArgs c{};
+    c.flmn_out = flmn, c.base = bases, c.dl = dl, c.W = const_cast<double2*>(W) + g.QOFF;
+    c.L = g.L, c.N = g.N, c.L0 = g.L0, c.plane0 = g.plane0, c.n_mode = n_mode, c.nsign = g.real ? 2 : 4;
+    c.compact = storage_compact, c.nu_lo = nu_lo, c.nu_hi = nu_hi, c.CS = g.CS, c.QS = g.QS, c.lw = lw;
+    return contract<true>(c, s);
   }
   dim3 grid((nu_hi - nu_lo + kNG - 1) / kNG, (g.L + kRows - 1) / kRows, (g.L + kCols - 1) / kCols);
   if (g.real) {

@@ -1,5 +1,5 @@
 // Resident Wigner Delta(pi/2) table: quarter planes 0 <= m', m <= l for every
-// degree l < Lcap, plane l at dl_plane_offset(l), row-major (m' rows).
+// degree l < Lcap, in the blocked layout of so3gpu_internal.h (dl_index).
 //
 // Replaces the per-call, per-n recomputation inside SSHT (called from the
 // reference's src/c/so3_core.c:204, :408) and the in-tree recursions at
@@ -27,15 +27,13 @@ __global__ void dl_trapani_top_rows(double* __restrict__ T, int Lcap) {
   if (threadIdx.x == 0) T[0] = 1.0;
   __syncthreads();
   for (int l = 1; l < Lcap; l++) {
-    const double* prev = T + dl_plane_offset(l - 1) + (long long)(l - 1) * l;  // row l-1 of plane l-1
-    double* row = T + dl_plane_offset(l) + (long long)l * (l + 1);            // row l of plane l
     for (int m = threadIdx.x; m <= l; m += blockDim.x) {
       double v;
       if (m == 0)
-        v = -sqrt((2.0 * l - 1.0) / (2.0 * l)) * prev[0];
+        v = -sqrt((2.0 * l - 1.0) / (2.0 * l)) * T[dl_index(l - 1, l - 1, 0)];
       else
-        v = sqrt((double)l * (2.0 * l - 1.0) / (2.0 * (l + m) * (l + m - 1.0))) * prev[m - 1];
-      row[m] = v;
+        v = sqrt((double)l * (2.0 * l - 1.0) / (2.0 * (l + m) * (l + m - 1.0))) * T[dl_index(l - 1, l - 1, m - 1)];
+      T[dl_index(l, l, m)] = v;
     }
     __syncthreads();
   }
@@ -45,15 +43,13 @@ __global__ void dl_trapani_top_rows(double* __restrict__ T, int Lcap) {
 // sqrt((l-m')(l+m'+1)) D_{m'} = 2m D_{m'+1} - sqrt((l-m'-1)(l+m'+2)) D_{m'+2}.
 __global__ void dl_trapani_columns(double* __restrict__ T) {
   const int l = blockIdx.x;
-  double* P = T + dl_plane_offset(l);
-  const int ld = l + 1;
   for (int m = threadIdx.x; m <= l; m += blockDim.x) {
-    double d1 = P[(long long)l * ld + m], d2 = 0.0;  // D_{m'+1}, D_{m'+2}
+    double d1 = T[dl_index(l, l, m)], d2 = 0.0;  // D_{m'+1}, D_{m'+2}
     for (int mp = l - 1; mp >= m; mp--) {
       const double t1 = sqrt((double)(l - mp) * (double)(l + mp + 1));
       const double t2 = (mp + 2 <= l) ? sqrt((double)(l - mp - 1) * (double)(l + mp + 2)) : 0.0;
       const double d0 = (2.0 * m * d1 - t2 * d2) / t1;
-      P[(long long)mp * ld + m] = d0;
+      T[dl_index(l, mp, m)] = d0;
       d2 = d1;
       d1 = d0;
     }
@@ -62,16 +58,16 @@ __global__ void dl_trapani_columns(double* __restrict__ T) {
 
 __global__ void dl_fill_upper(double* __restrict__ T) {
   const int l = blockIdx.x;
-  double* P = T + dl_plane_offset(l);
   const int ld = l + 1;
   for (int i = threadIdx.x; i < ld * ld; i += blockDim.x) {
-    const int mp = i / ld, m = i - mp * ld;
-    if (mp < m) P[i] = sgn(m - mp) * P[(long long)m * ld + mp];
+    const int m = i / ld, mp = i - m * ld;
+    if (mp < m) T[dl_index(l, mp, m)] = sgn(m - mp) * T[dl_index(l, m, mp)];
   }
 }
 
 int launch_build_dl_trapani(double* table, int L0cap, int Lcap, cudaStream_t s) {
   (void)L0cap;
+  SO3G_CUDA(cudaMemsetAsync(table, 0, (size_t)dl_entries(Lcap) * sizeof(double), s));
   dl_trapani_top_rows<<<1, 1024, 0, s>>>(table, Lcap);
   SO3G_LAUNCHED();
   dl_trapani_columns<<<Lcap, 256, 0, s>>>(table);
@@ -155,11 +151,10 @@ __global__ void __launch_bounds__(1024) dl_risbo_sweep(double* __restrict__ T, i
     __syncthreads();
     // quarter plane el into the table
     {
-      double* P = T + dl_plane_offset(el);
       const int ld = el + 1;
       for (int i = tid; i < ld * ld; i += nt) {
         const int u = i / ld, v = i - u * ld;
-        P[i] = v <= u ? RA(u, v) : sgn(v - u) * RA(v, u);
+        T[dl_index(el, u, v)] = v <= u ? RA(u, v) : sgn(v - u) * RA(v, u);
       }
     }
     __syncthreads();
@@ -169,6 +164,7 @@ __global__ void __launch_bounds__(1024) dl_risbo_sweep(double* __restrict__ T, i
 }
 
 int launch_build_dl_risbo(double* table, int Lcap, double* work, cudaStream_t s) {
+  SO3G_CUDA(cudaMemsetAsync(table, 0, (size_t)dl_entries(Lcap) * sizeof(double), s));
   dl_risbo_sweep<<<1, 1024, 0, s>>>(table, Lcap, work);
   SO3G_LAUNCHED();
   SO3G_CUDA(cudaGetLastError());

@@ -172,12 +172,13 @@ __host__ __device__ inline long long digit_block(int t, int kc, int q, int nc) {
 // rho; the 32 lanes of a warp store 32 distinct banks.
 //   inverse: row = m' (r0 + rho), reduction = l;  A^T[l, m'] = Delta_{mu m'} Delta_{nu m'} (l >= m', l >= lmin)
 //   forward: row = l  (r0 + rho), reduction = m'; same product
-// Delta_{mu m'} is read as row mu of the quarter plane (the transpose
-// symmetry's sign (-1)^{mu+nu} is applied in the epilogue).
+// The digits are those of Delta_{mu m'} Delta_{nu m'} = (-1)^{mu+nu}
+// Delta_{m' mu} Delta_{m' nu}; the epilogue applies that sign again.
 template <bool FWD>
 __device__ __forceinline__ void gen_load(const MixArgs& a, int mu, int nu, int lmin, int r0, int k0, int gw, int lane,
                                          double (&x)[4][4]) {
   const int rho = 8 * gw + (lane & 7);
+  const double half = ((mu + nu) & 1) ? -0.5 : 0.5;  // A scale 2
 #pragma unroll
   for (int it = 0; it < 4; it++) {
     const int q = 4 * it + (lane >> 3);
@@ -194,10 +195,10 @@ __device__ __forceinline__ void gen_load(const MixArgs& a, int mu, int nu, int l
       }
       double v = 0.0;
       if (l < a.L && l >= lmin && mp <= l) {
-        const double* P = a.dl + dl_plane_offset(l);
-        v = P[(long long)mu * (l + 1) + mp] * P[(long long)nu * (l + 1) + mp];
+        const double* P = a.dl + dl_index(l, mp, 0);
+        v = P[64 * mu] * P[64 * nu];
       }
-      x[it][e] = 0.5 * v;  // A scale 2
+      x[it][e] = half * v;
     }
   }
 }

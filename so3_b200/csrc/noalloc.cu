@@ -6,8 +6,8 @@
 // cudaMalloc, cudaFree or any allocating routine: the transform scratch, the
 // Wigner Delta(pi/2) tables, the FFT tables and the block-offset table live
 // in the file-scope device arrays below, which every GPU that loads the
-// library holds until the process exits: kStaticBytes = 35,089,464 bytes
-// (33.5 MiB), of which 32 MiB are scratch.
+// library holds until the process exits: kStaticBytes = 35,329,592 bytes
+// (33.7 MiB), of which 32 MiB are scratch.
 //
 // Limits: complex, non-steerable signals only (reality != 0 or steerable !=
 // 0: status 3, before any device work -- a real signal's buffers are sized
@@ -49,7 +49,7 @@ namespace {
 constexpr size_t kScratchBytes = 32u << 20;
 constexpr int kMaxL = 64;
 constexpr int kMaxN = 64;
-constexpr int kDlEntries = kMaxL * (kMaxL + 1) * (2 * kMaxL + 1) / 6;
+constexpr int kDlEntries = 512 * (kMaxL / 8) * (kMaxL / 8 + 1) * (2 * (kMaxL / 8) + 1) / 6;  // dl_entries(kMaxL)
 constexpr int kRisboWork = 2 * (kMaxL + 6) * (kMaxL + 6);
 constexpr int kFftSlot = 2 * 256 + 2 * 128;  // Bluestein m + n + m, then n half-step roots, for n <= 128
 constexpr int kMaxPlanes = 2 * kMaxN - 1;
@@ -61,7 +61,7 @@ static __device__ __align__(256) double2 g_fft[2][kFftSlot];
 static __device__ __align__(256) long long g_bases[kMaxPlanes];
 constexpr size_t kStaticBytes = kScratchBytes + sizeof(double) * (2 * (size_t)kDlEntries + kRisboWork) +
                                 sizeof(double2) * 2 * kFftSlot + sizeof(long long) * kMaxPlanes;
-static_assert(kStaticBytes == 35089464, "the documented size of the static arrays");
+static_assert(kStaticBytes == 35329592, "the documented size of the static arrays");
 
 struct NoAllocDevice {
   bool ready = false;

@@ -144,7 +144,7 @@ class Server {
       int cap = 1;
       while (cap < max_L_) cap <<= 1;
       if (cap < 64) cap = 64;
-      dl_charge_ = 2 * (size_t)dl_plane_offset(cap) * sizeof(double);
+      dl_charge_ = 2 * (size_t)dl_entries(cap) * sizeof(double);
     }
     worker_ = std::thread([this] {
       set_thread_autotune(false);  // never stall admission on tuning a new geometry

@@ -79,16 +79,32 @@ Geometry make_geometry(const so3_parameters_t& p, int real);
 std::vector<long long> block_bases(const so3_parameters_t& p, int real);
 
 // ---------------------------------------------------------------- tables
-// Quarter Delta(pi/2) planes of every degree l < Lcap, plane l at offset
-// l(l+1)(2l+1)/6, row-major (m' rows, m columns, both 0..l).  Planes do not
-// depend on the band limit, so one table serves every L <= Lcap.
+// Quarter Delta(pi/2) planes of every degree l < Lcap (0 <= m', mu <= l).
+// Planes do not depend on the band limit, so one table serves every L <= Lcap
+// (a multiple of 8).  Stored in blocks of 8 degrees x 8 rows m' per column mu:
+// block (l / 8, m' / 8) of the rows that degree reaches, then mu = 0 .. 8
+// (l / 8) + 7, then the 64 values, [m' % 8][l % 8] with the l halves swapped in
+// every other row pair; entries with m' > l or mu > l are zero.  A block is the
+// operand of one FP64 MMA step pair in either direction -- rows m' against l
+// (inverse) or rows l against m' (forward) -- and the swap puts both fragment
+// reads on distinct shared-memory banks, so the contractions copy runs of
+// blocks (512 bytes per mu) straight to shared memory.
 struct DlTable {
   int Lcap = 0;
   double* d = nullptr;
 };
-__host__ __device__ inline long long dl_plane_offset(int l) {
-  return (long long)l * (l + 1) * (2 * l + 1) / 6;
+// Entries before degree 8 lc: 512 sum_{k <= lc} k^2.
+__host__ __device__ inline long long dl_base(int lc) {
+  return 512LL * lc * (lc + 1) * (2 * lc + 1) / 6;
 }
+// Place of (m' % 8, l % 8) in a block.
+__host__ __device__ inline int dl_slot(int mp, int l) { return (mp & 7) * 8 + ((l & 7) ^ (((mp >> 1) & 1) * 4)); }
+__host__ __device__ inline long long dl_index(int l, int mp, int mu) {
+  const int lc = l >> 3;
+  return dl_base(lc) + ((long long)(mp >> 3) * (8 * (lc + 1)) + mu) * 64 + dl_slot(mp, l);
+}
+// Entries of a table of capacity Lcap.
+__host__ __device__ inline long long dl_entries(int Lcap) { return dl_base((Lcap + 7) / 8); }
 
 struct DevPlan {
   FftPlan plan{};
@@ -306,6 +322,7 @@ const DigitTable* covering_digit_table(Device* D, int L, int N, int method, cons
 // Reads and clears the flag the tensor-core kernels set when a bounded wait
 // gave up (0: none; synchronous).
 int mixed_take_error();
+int contract_take_error();  // the same of the FP64 contractions' copies
 
 // ---------------------------------------------------------------- drivers
 // Per-thread switch of the stage autotuner (default on).

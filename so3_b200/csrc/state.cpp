@@ -119,7 +119,7 @@ size_t resident_bytes(Device* D) {
   std::lock_guard<std::mutex> lk(D->mu);
   size_t b = 0;
   for (const DlTable& t : D->dl)
-    if (t.d) b += (size_t)dl_plane_offset(t.Lcap) * sizeof(double);
+    if (t.d) b += (size_t)dl_entries(t.Lcap) * sizeof(double);
   for (const auto& t : D->digit_tables) b += t->bytes + (size_t)t->L * t->N * sizeof(long long);
   for (const auto& t : D->beta_tables) b += t->bytes;
   for (const auto& kv : D->conv_kernels) b += (size_t)(8 * (kv.first / 2) + 2 * (kv.first / 2)) * sizeof(double2);  // Pc <= 8L, plus 2L
@@ -213,7 +213,7 @@ int ensure_dl(Device* D, int L, int method, cudaStream_t s, const double** out) 
   int Lcap = 1;
   while (Lcap < L) Lcap <<= 1;  // power-of-two capacity: a few rebuilds at most
   if (Lcap < 64) Lcap = 64;
-  size_t bytes = (size_t)dl_plane_offset(Lcap) * sizeof(double);
+  size_t bytes = (size_t)dl_entries(Lcap) * sizeof(double);
   double* d = nullptr;
   cudaError_t e = cudaMalloc(&d, bytes);
   if (e != cudaSuccess) return fail(kOutOfMemory, std::string("Delta table allocation failed: ") + cudaGetErrorString(e));
