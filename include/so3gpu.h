@@ -52,7 +52,10 @@ int so3gpu_forward_real(so3gpu_context *ctx, void *flmn, const double *f,
  * the Wigner contractions of all signals run as int8 tensor-core products
  * (7-slice Ozaki split, exact int32 accumulation, FP64 recombination) while
  * Delta, the quadrature weights and every DFT stay FP64; normwise relative
- * error against the FP64 path below 1e-10 (about 1e-12 measured).  Real
+ * error against the FP64 path below 1e-10 (about 1e-12 measured).  The products
+ * run 16 signals to an operand; the last signals of a batch that would leave
+ * most of one empty (fewer than 8 inverse, 12 forward) take the FP64
+ * contractions, which are then faster.  Real
  * signals (parameters->reality) take the split contractions over their planes
  * n >= 0 and the FP64 forward beta stage; real signals with N = 1 use the
  * FP64 path.  The batch workspace holds `count` scratch plane sets (2.13 GB
@@ -71,8 +74,8 @@ int so3gpu_forward_batch(so3gpu_context *ctx, void *const *flmn, const void *con
  * Wigner contractions of all complex signals run in one int8 tensor-core
  * launch per Delta recursion -- signals sorted by (L, N) share 16-signal
  * operand tiles at the tile's largest L and N -- while every DFT stage runs
- * per signal in FP64; real signals, and precision FP64, take the FP64 path
- * per signal.  Same error contract as so3gpu_inverse_batch. */
+ * per signal in FP64; tiles whose padding would cost more than the products
+ * save, real signals, and precision FP64 take the FP64 path per signal.  Same error contract as so3gpu_inverse_batch. */
 int so3gpu_inverse_ragged(so3gpu_context *ctx, void *const *f, const void *const *flmn,
                           const so3_parameters_t *parameters, int count, int precision);
 int so3gpu_forward_ragged(so3gpu_context *ctx, void *const *flmn, const void *const *f,

@@ -43,6 +43,7 @@ struct BetaMmArgs {
   double2* W;              // scratch of the transform
   int M, K, RT, KS;        // rows, reduction entries; row tiles and steps of the table (zero padded)
   double isign;            // s = -1: times isign * i
+  long long wstride;       // blockIdx.z = plane + nplanes * signal
 };
 
 // SPEC_IN: reduction over the spectra m' (column-major part -> row-major
@@ -59,10 +60,12 @@ __global__ void __launch_bounds__(32 * WR * WC, WR * WC == 8 ? 2 : 4) beta_mm_ke
   extern __shared__ __align__(16) double smd[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wr = warp % WR, wc = warp / WR;
   const int kk = lane & 3, gr = lane >> 2;
-  const int ncols = 2 * g.L - 1, c0 = blockIdx.x * COLS, plane = blockIdx.z, rt0 = blockIdx.y * RT;
+  const int ncols = 2 * g.L - 1, c0 = blockIdx.x * COLS, rt0 = blockIdx.y * RT;
+  const int sig = blockIdx.z / g.nplanes, plane = blockIdx.z - sig * g.nplanes;
+  double2* const W = a.W + sig * a.wstride;
   const int first_is_a = ((g.L - 1 + plane - g.plane0) & 1) == 0;  // even columns have s = +1
-  const double2* in = SPEC_IN ? a.W + g.QOFF + (long long)plane * g.QS + (long long)c0 * g.CS
-                              : a.W + (long long)plane * g.PS + c0;
+  const double2* in = SPEC_IN ? W + g.QOFF + (long long)plane * g.QS + (long long)c0 * g.CS
+                              : W + (long long)plane * g.PS + c0;
   const int nch = (a.K + kK - 1) / kK;
 
   auto stage = [&](int ch) {
@@ -78,7 +81,7 @@ __global__ void __launch_bounds__(32 * WR * WC, WR * WC == 8 ? 2 : 4) beta_mm_ke
       const bool ok = ch * kK + k < a.K && c0 + c < ncols;
       const double2* src = SPEC_IN ? in + (long long)c * g.CS + ch * kK + k : in + (long long)(ch * kK + k) * g.RS + c;
       const int h = (c & 1) * HC + (c >> 1);
-      cp16z(Bs + (SPEC_IN ? h * CP + k : k * KP + h), ok ? src : a.W, ok);
+      cp16z(Bs + (SPEC_IN ? h * CP + k : k * KP + h), ok ? src : W, ok);
     }
   };
 
@@ -137,9 +140,9 @@ __global__ void __launch_bounds__(32 * WR * WC, WR * WC == 8 ? 2 : 4) beta_mm_ke
         const double2 y = p == 1 - first_is_a ? make_double2(v[0], v[1])
                                               : make_double2(-a.isign * v[1], a.isign * v[0]);
         if (SPEC_IN)
-          a.W[(long long)plane * g.PS + (long long)row * g.RS + c] = y;
+          W[(long long)plane * g.PS + (long long)row * g.RS + c] = y;
         else
-          a.W[g.QOFF + (long long)plane * g.QS + (long long)c * g.CS + row] = y;
+          W[g.QOFF + (long long)plane * g.QS + (long long)c * g.CS + row] = y;
       }
   }
 }
@@ -208,13 +211,13 @@ void table_shape(const Geometry& g, int kind, int* M, int* K, int* RT, int* KS) 
 }
 
 template <bool SPEC_IN, int MT, int WR, int NP, int WC>
-int go(const Geometry& g, const BetaMmArgs& a, cudaStream_t s) {
+int go(const Geometry& g, const BetaMmArgs& a, int nsig, cudaStream_t s) {
   constexpr int COLS = 8 * NP * WC, ROWS = 8 * MT * WR;
   constexpr int BSZ = SPEC_IN ? COLS * (kK + 4) : kK * (COLS + 2);
   constexpr size_t smem = kStages * (2 * MT * WR * 128 + 2 * BSZ) * sizeof(double);
   auto kernel = beta_mm_kernel<SPEC_IN, MT, WR, NP, WC>;
   SO3G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const dim3 grid((2 * g.L - 1 + COLS - 1) / COLS, (a.M + ROWS - 1) / ROWS, g.nplanes);
+  const dim3 grid((2 * g.L - 1 + COLS - 1) / COLS, (a.M + ROWS - 1) / ROWS, g.nplanes * nsig);
   kernel<<<grid, 32 * WR * WC, smem, s>>>(g, a);
   SO3G_LAUNCHED();
   SO3G_CUDA(cudaGetLastError());
@@ -253,22 +256,24 @@ int launch_beta_matrix_table(const Geometry& g, int kind, const FftPlan& pP, dou
   return kOk;
 }
 
-int launch_beta_matrix(const Geometry& g, int kind, const double* tab, double2* W, cudaStream_t s) {
+int launch_beta_matrix(const Geometry& g, int kind, const double* tab, double2* W, cudaStream_t s, const Batch& bt) {
+  const int nsig = bt.n ? bt.n : 1;
   BetaMmArgs a{};
   a.tab = tab;
   a.W = W;
+  a.wstride = bt.wstride;
   table_shape(g, kind, &a.M, &a.K, &a.RT, &a.KS);
   a.isign = kind == kBetaInverse || kind == kBetaForward ? 1.0 : -1.0;
   const bool spec_in = kind == kBetaInverse || kind == kBetaAdjForward;
   // 64 x 64 tiles (two CTAs per SM), 32 x 32 (four per SM; 5-7 % slower per
   // product) where their waves over 148 SMs and the padding of the rows cost
   // less, 16 x 32 where those would not fill half the device.
-  const long long big = (long long)((2 * g.L + 62) / 64) * ((a.M + 63) / 64) * g.nplanes;
-  const long long mid = (long long)((2 * g.L + 30) / 32) * ((a.M + 31) / 32) * g.nplanes;
+  const long long big = (long long)((2 * g.L + 62) / 64) * ((a.M + 63) / 64) * g.nplanes * nsig;
+  const long long mid = (long long)((2 * g.L + 30) / 32) * ((a.M + 31) / 32) * g.nplanes * nsig;
   if (mid >= 296 && 1.9 * ((big + 295) / 296) <= (mid + 591) / 592)
-    return spec_in ? go<true, 4, 2, 2, 4>(g, a, s) : go<false, 4, 2, 2, 4>(g, a, s);
-  if (mid >= 296) return spec_in ? go<true, 4, 1, 1, 4>(g, a, s) : go<false, 4, 1, 1, 4>(g, a, s);
-  return spec_in ? go<true, 2, 1, 1, 4>(g, a, s) : go<false, 2, 1, 1, 4>(g, a, s);
+    return spec_in ? go<true, 4, 2, 2, 4>(g, a, nsig, s) : go<false, 4, 2, 2, 4>(g, a, nsig, s);
+  if (mid >= 296) return spec_in ? go<true, 4, 1, 1, 4>(g, a, nsig, s) : go<false, 4, 1, 1, 4>(g, a, nsig, s);
+  return spec_in ? go<true, 2, 1, 1, 4>(g, a, nsig, s) : go<false, 2, 1, 1, 4>(g, a, nsig, s);
 }
 
 }  // namespace so3g

@@ -393,8 +393,8 @@ constexpr int kCThreads = 32 * (kCRt / kCMt) * 2 * (kCNu / kCNw) + 32;
 constexpr int kXB = 33;  // slots of an X block of one (mu, nu): 8 entries x 4 combinations, and one of padding
 
 struct ContractArgs {
-  const double2* flmn_in;  // inverse: coefficients
-  double2* flmn_out;       // forward: coefficients
+  void* flmn[kMaxBatch];   // coefficients of each signal (blockIdx.z = mu tile + tiles * signal)
+  long long wstride;       // scratch of signal b at W + b * wstride
   const long long* base;   // per plane
   const double* dl;
   double2* W;              // column-major scratch part
@@ -415,7 +415,7 @@ constexpr int kCStage = kCRt * kCMu * 64 + kCRt * kCNu * 64 + 2 * kCMu * kCNu * 
 }  // namespace
 
 template <bool FWD>
-__global__ void __launch_bounds__(kCThreads, 2) contract_mma_kernel(ContractArgs a) {
+__global__ void __launch_bounds__(kCThreads, 2) contract_mma_kernel(const __grid_constant__ ContractArgs a) {
   constexpr int RT = kCRt, NU = kCNu, MT = kCMt, NW = kCNw, ST = kCStages;
   constexpr int WR = RT / MT, NWARP = kCThreads / 32 - 1;  // product warps; one more copies
   constexpr int BSZ = RT * kCMu * 64, ASZ = RT * NU * 64, STAGE = kCStage;
@@ -424,7 +424,10 @@ __global__ void __launch_bounds__(kCThreads, 2) contract_mma_kernel(ContractArgs
   __shared__ __align__(8) unsigned long long full[ST], empty[ST];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
   const int wr = warp % WR, wm = warp / WR % 2, wn = warp / (2 * WR);
-  const int nu0 = a.nu0 + blockIdx.x * NU, rt0 = blockIdx.y * RT, mu0 = blockIdx.z * kCMu;
+  const int nu0 = a.nu0 + blockIdx.x * NU, rt0 = blockIdx.y * RT;
+  const int mts = (a.L + kCMu - 1) / kCMu, sig = blockIdx.z / mts, mu0 = (blockIdx.z - sig * mts) * kCMu;
+  double2* const flmn = static_cast<double2*>(a.flmn[sig]);
+  double2* const W = a.W + sig * a.wstride;
   const int L = a.L, LC = (L + 7) >> 3;
   unsigned act = 0;  // bit j: nu0 + j is computed by this launch
 #pragma unroll
@@ -479,11 +482,11 @@ __global__ void __launch_bounds__(kCThreads, 2) contract_mma_kernel(ContractArgs
     for (int j = 0; j < NU; j++) {
       const int nu = nu0 + j, mu = mu0 + xm;
       if (FWD) {
-        px[j] = a.W + (long long)(a.plane0 + ((xc & 2) ? -nu : nu)) * a.QS + (long long)(L - 1 + ((xc & 1) ? -mu0 : mu0)) * a.CS;
+        px[j] = W + (long long)(a.plane0 + ((xc & 2) ? -nu : nu)) * a.QS + (long long)(L - 1 + ((xc & 1) ? -mu0 : mu0)) * a.CS;
         xlo[j] = xc < a.nsign && (act >> j & 1) ? 0 : L;
       } else {
 #pragma unroll
-        for (int c = 0; c < 4; c++) px[4 * j + c] = a.flmn_in + bsel[j][c >> 1] + ((c & 1) ? -mu : mu);
+        for (int c = 0; c < 4; c++) px[4 * j + c] = flmn + bsel[j][c >> 1] + ((c & 1) ? -mu : mu);
         xlo[j] = mu < L && (act >> j & 1) ? max(max(a.L0, mu), nu) : L;
       }
     }
@@ -509,7 +512,7 @@ __global__ void __launch_bounds__(kCThreads, 2) contract_mma_kernel(ContractArgs
 #pragma unroll
           for (int m = 0; m < kCMu; m++, src += cstep) {
             const bool ok = e >= xlo[j] && e < L && mu0 + m < L;
-            cp16_to(xs0 + at + 16 * ((j * kCMu + m) * kXB + xc * 8 + (xe ^ (4 * (xc & 1)))), ok ? src : a.W, ok);
+            cp16_to(xs0 + at + 16 * ((j * kCMu + m) * kXB + xc * 8 + (xe ^ (4 * (xc & 1)))), ok ? src : W, ok);
           }
         } else {
 #pragma unroll
@@ -519,7 +522,7 @@ __global__ void __launch_bounds__(kCThreads, 2) contract_mma_kernel(ContractArgs
 #pragma unroll
             for (int c = 0; c < 4; c++) {
               const bool ok = in && c < a.nsign;
-              cp16_to(xs0 + at + 16 * ((j * kCMu + xm) * kXB + 4 * (4 * h + xe) + (c ^ (xe & 2))), ok ? px[4 * j + c] + off : a.flmn_in,
+              cp16_to(xs0 + at + 16 * ((j * kCMu + xm) * kXB + 4 * (4 * h + xe) + (c ^ (xe & 2))), ok ? px[4 * j + c] + off : flmn,
                       ok);
             }
           }
@@ -641,10 +644,10 @@ __global__ void __launch_bounds__(kCThreads, 2) contract_mma_kernel(ContractArgs
           } else {
             v = make_double2(0.0, 0.0);
           }
-          a.flmn_out[bsel[wn * NW + n][q >> 1] + (long long)row * row + row + ms * mu] = v;
+          flmn[bsel[wn * NW + n][q >> 1] + (long long)row * row + row + ms * mu] = v;
         } else {
           v = ipow_mul(v, ns * nu - ms * mu + 4 * L);
-          a.W[(long long)(a.plane0 + ns * nu) * a.QS + (long long)(ms * mu + L - 1) * a.CS + row] = v;
+          W[(long long)(a.plane0 + ns * nu) * a.QS + (long long)(ms * mu + L - 1) * a.CS + row] = v;
         }
       }
     }
@@ -653,11 +656,14 @@ __global__ void __launch_bounds__(kCThreads, 2) contract_mma_kernel(ContractArgs
 
 namespace {
 template <bool FWD>
-int contract(ContractArgs a, cudaStream_t s) {
+int contract(ContractArgs a, const void* flmn, const Batch& bt, cudaStream_t s) {
+  for (int b = 0; b < bt.n; b++) a.flmn[b] = bt.io[b];
+  if (!bt.n) a.flmn[0] = const_cast<void*>(flmn);
+  a.wstride = bt.wstride;
   constexpr size_t smem = kCStages * kCStage * sizeof(double);
   SO3G_CUDA(cudaFuncSetAttribute(contract_mma_kernel<FWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   a.nu0 = a.nu_lo / kCNu * kCNu;  // tiles stay aligned: a block of 8 degrees holds whole groups of nu
-  const dim3 grid((a.nu_hi - a.nu0 + kCNu - 1) / kCNu, (a.L + 8 * kCRt - 1) / (8 * kCRt), (a.L + kCMu - 1) / kCMu);
+  const dim3 grid((a.nu_hi - a.nu0 + kCNu - 1) / kCNu, (a.L + 8 * kCRt - 1) / (8 * kCRt), (a.L + kCMu - 1) / kCMu * (bt.n ? bt.n : 1));
   contract_mma_kernel<FWD><<<grid, kCThreads, smem, s>>>(a);
   SO3G_LAUNCHED();
   SO3G_CUDA(cudaGetLastError());
@@ -674,18 +680,25 @@ int contract_take_error() {
 
 int launch_inverse_contract(const Geometry& g, int n_mode, const double2* flmn, const long long* bases,
                             const double* dl, double2* W, int sym_n0, cudaStream_t s, int nu_lo, int nu_hi,
-                            double wconst) {
+                            double wconst, const Batch& bt) {
   if (nu_hi < 0 || nu_hi > g.N) nu_hi = g.N;
   if (nu_lo >= nu_hi) return kOk;
-  InvArgs a{flmn, bases, dl, W + g.QOFF, g.L, g.N, g.L0, g.plane0, n_mode, g.real, sym_n0, nu_lo, nu_hi, g.CS, g.QS,
-            wconst};
   if (fp64_tensor_cores()) {
     ContractArgs c{};
-    c.flmn_in = flmn, c.base = bases, c.dl = dl, c.W = W + g.QOFF;
+    c.base = bases, c.dl = dl, c.W = W + g.QOFF;
     c.L = g.L, c.N = g.N, c.L0 = g.L0, c.plane0 = g.plane0, c.n_mode = n_mode, c.nsign = g.real ? 2 : 4;
     c.sym_n0 = sym_n0, c.nu_lo = nu_lo, c.nu_hi = nu_hi, c.CS = g.CS, c.QS = g.QS, c.wconst = wconst;
-    return contract<false>(c, s);
+    return contract<false>(c, flmn, bt, s);
   }
+  if (bt.n) {  // the FMA engine runs signal by signal
+    for (int b = 0; b < bt.n; b++)
+      if (int rc = launch_inverse_contract(g, n_mode, static_cast<const double2*>(bt.io[b]), bases, dl,
+                                           W + b * bt.wstride, sym_n0, s, nu_lo, nu_hi, wconst))
+        return rc;
+    return kOk;
+  }
+  InvArgs a{flmn, bases, dl, W + g.QOFF, g.L, g.N, g.L0, g.plane0, n_mode, g.real, sym_n0, nu_lo, nu_hi, g.CS, g.QS,
+            wconst};
   dim3 grid((nu_hi - nu_lo + kNG - 1) / kNG, (g.L + kRows - 1) / kRows, (g.L + kCols - 1) / kCols);
   if (g.real) {
     SO3G_CUDA(cudaFuncSetAttribute(inverse_contract_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
@@ -701,18 +714,25 @@ int launch_inverse_contract(const Geometry& g, int n_mode, const double2* flmn, 
 
 int launch_forward_contract(const Geometry& g, int n_mode, const double2* W, const long long* bases,
                             const double* dl, double2* flmn, int storage_compact, cudaStream_t s, int nu_lo,
-                            int nu_hi, double lw) {
+                            int nu_hi, double lw, const Batch& bt) {
   if (nu_hi < 0 || nu_hi > g.N) nu_hi = g.N;
   if (nu_lo >= nu_hi) return kOk;
-  FwdArgs a{W + g.QOFF, bases, dl, flmn, g.L, g.N, g.L0, g.plane0, n_mode, g.real, storage_compact, nu_lo, nu_hi,
-            g.CS, g.QS, lw};
   if (fp64_tensor_cores()) {
     ContractArgs c{};
-    c.flmn_out = flmn, c.base = bases, c.dl = dl, c.W = const_cast<double2*>(W) + g.QOFF;
+    c.base = bases, c.dl = dl, c.W = const_cast<double2*>(W) + g.QOFF;
     c.L = g.L, c.N = g.N, c.L0 = g.L0, c.plane0 = g.plane0, c.n_mode = n_mode, c.nsign = g.real ? 2 : 4;
     c.compact = storage_compact, c.nu_lo = nu_lo, c.nu_hi = nu_hi, c.CS = g.CS, c.QS = g.QS, c.lw = lw;
-    return contract<true>(c, s);
+    return contract<true>(c, flmn, bt, s);
   }
+  if (bt.n) {
+    for (int b = 0; b < bt.n; b++)
+      if (int rc = launch_forward_contract(g, n_mode, W + b * bt.wstride, bases, dl, static_cast<double2*>(bt.io[b]),
+                                           storage_compact, s, nu_lo, nu_hi, lw))
+        return rc;
+    return kOk;
+  }
+  FwdArgs a{W + g.QOFF, bases, dl, flmn, g.L, g.N, g.L0, g.plane0, n_mode, g.real, storage_compact, nu_lo, nu_hi,
+            g.CS, g.QS, lw};
   dim3 grid((nu_hi - nu_lo + kNG - 1) / kNG, (g.L + kRows - 1) / kRows, (g.L + kCols - 1) / kCols);
   if (g.real) {
     SO3G_CUDA(cudaFuncSetAttribute(forward_contract_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));

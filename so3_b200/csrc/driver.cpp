@@ -394,16 +394,145 @@ size_t batch_workspace_bytes(const so3_parameters_t& p, int real, int nsig, int 
   return batch_layout(make_geometry(p, real), p, real, nsig).total;
 }
 
+// Signals of one geometry whose DFT stages (and FP64 contractions) share
+// launches: up to 192 MB of row-major scratch.  A small signal does not fill the
+// device and pays a launch gap per stage; inverse + forward of 64 signals, FP64,
+// one launch per signal against chunks of 48 / 192 / 400 MB (us a signal):
+// L = 32, N = 16: 53 / 6.7 / 6.8 / 6.8; L = 128, N = 16: 188 / 140 / 120 / 116;
+// L = 256, N = 32 (alone in a chunk up to 256 MB): 1500 / 1500 / 1500 / 1430.
+static int batch_chunk(const Geometry& g, int nsig) {
+  const size_t rows = (size_t)g.nplanes * g.PS * sizeof(double2);
+  const int fit = (int)std::min<size_t>(kMaxBatch, (size_t(192) << 20) / std::max<size_t>(rows, 1));
+  return std::max(1, std::min({nsig, fit, 65535 / g.nplanes}));
+}
+
+// Signals [b0, b0 + n) of a batch; io: their coefficient or sample arrays.
+static Batch batch_of(long long wstride, void* const* io, int b0, int n) {
+  Batch bt;
+  bt.n = n;
+  bt.wstride = wstride;
+  for (int b = 0; b < n && io; b++) bt.io[b] = io[b0 + b];
+  return bt;
+}
+
+// Inverse DFT stages of signals in chunks (W: scratch of the first).
+static int inverse_stages(const Resources& r, StageTimer* T, double2* W, long long wstride, int nsig, void* const* f_d,
+                          cudaStream_t s) {
+  const int step = batch_chunk(r.g, nsig);
+  cudaEvent_t ev;
+  int rc;
+  for (int b0 = 0; b0 < nsig; b0 += step) {
+    const Batch bt = batch_of(wstride, f_d, b0, std::min(step, nsig - b0));
+    double2* Wb = W + (size_t)b0 * wstride;
+    timer_begin(T, s, &ev);
+    if ((rc = launch_inv_beta(r.g, r.pP, Wb, s, bt))) return rc;
+    timer_end(T, s, kStInvBeta, ev, bt.n);
+    timer_begin(T, s, &ev);
+    if ((rc = launch_inv_alpha(r.g, r.pP, Wb, s, bt))) return rc;
+    timer_end(T, s, kStInvAlpha, ev, bt.n);
+    timer_begin(T, s, &ev);
+    if ((rc = launch_inv_gamma(r.g, r.pg, Wb, nullptr, s, 0, -1, bt))) return rc;
+    timer_end(T, s, kStInvGamma, ev, bt.n);
+  }
+  return kOk;
+}
+
+// Forward gamma, alpha and (unless the caller has its own) FP64 beta stages.
+static int forward_stages(const Resources& r, StageTimer* T, double2* W, long long wstride, int nsig,
+                          const void* const* f_d, bool beta, cudaStream_t s) {
+  const int step = batch_chunk(r.g, nsig);
+  cudaEvent_t ev;
+  int rc;
+  for (int b0 = 0; b0 < nsig; b0 += step) {
+    const Batch bt = batch_of(wstride, const_cast<void* const*>(f_d), b0, std::min(step, nsig - b0));
+    double2* Wb = W + (size_t)b0 * wstride;
+    timer_begin(T, s, &ev);
+    if ((rc = launch_fwd_gamma(r.g, r.pg, nullptr, Wb, s, 0, -1, bt))) return rc;
+    timer_end(T, s, kStFwdGamma, ev, bt.n);
+    timer_begin(T, s, &ev);
+    if ((rc = launch_fwd_alpha(r.g, r.pP, Wb, s, bt))) return rc;
+    timer_end(T, s, kStFwdAlpha, ev, bt.n);
+    if (!beta) continue;
+    timer_begin(T, s, &ev);
+    if ((rc = launch_fwd_beta_conv(r.g, r.pP, r.pc, r.wr, Wb, s, bt))) return rc;
+    timer_end(T, s, kStFwdBetaConv, ev, bt.n);
+  }
+  return kOk;
+}
+
+// FP64 contractions of signals in chunks of a launch.
+static int fp64_contractions(const Resources& r, const so3_parameters_t& p, int real, bool fwd, StageTimer* T, double2* W,
+                             long long wstride, int nsig, void* const* flmn_d, cudaStream_t s) {
+  cudaEvent_t ev;
+  timer_begin(T, s, &ev);
+  for (int b0 = 0; b0 < nsig; b0 += kMaxBatch) {
+    const Batch bt = batch_of(wstride, flmn_d, b0, std::min(kMaxBatch, nsig - b0));
+    double2* Wb = W + (size_t)b0 * wstride;
+    const int rc = fwd ? launch_forward_contract(r.g, p.n_mode, Wb, r.bases, r.dl, nullptr,
+                                                 p.storage == SO3_STORAGE_COMPACT, s, 0, -1, 0.0, bt)
+                       : launch_inverse_contract(r.g, p.n_mode, nullptr, r.bases, r.dl, Wb, real && p.N == 1, s, 0, -1,
+                                                 0.0, bt);
+    if (rc) return rc;
+  }
+  timer_end(T, s, fwd ? kStFwdContract : kStInvContract, ev, nsig);
+  return kOk;
+}
+
+// FP64 batch: chunks that share launches, on a workspace of one chunk (of one
+// signal where the caller's workspace holds no more).
+static int run_fp64_batch(Device* D, Workspace* wk, const so3_parameters_t& p, int real, bool fwd, int nsig,
+                          const void* const* in, void* const* out, cudaStream_t s) {
+  if (nsig == 0) return kOk;
+  Resources r;
+  if (int rc = acquire(D, p, real, s, &r, fwd)) return rc;
+  const size_t wb = (workspace_bytes(p, real) + 255) & ~size_t(255);
+  int step = batch_chunk(r.g, nsig);
+  if (wk->borrowed) step = (int)std::min<size_t>(step, std::max<size_t>(1, wk->ws_bytes / wb));
+  void* ws = nullptr;
+  if (int rc = ensure_ws(wk, step > 1 ? wb * step : workspace_bytes(p, real), &ws)) return rc;
+  double2* W = static_cast<double2*>(ws);
+  if (int rc = ensure_tuned(D, p, real, &r, W, s)) return rc;
+  const long long wstride = (long long)(wb / sizeof(double2));
+  for (int b0 = 0; b0 < nsig; b0 += step) {
+    const int n = std::min(step, nsig - b0);
+    int rc;
+    if (fwd) {
+      if ((rc = forward_stages(r, &wk->timer, W, wstride, n, in + b0, true, s))) return rc;
+      rc = fp64_contractions(r, p, real, true, &wk->timer, W, wstride, n, out + b0, s);
+    } else {
+      rc = fp64_contractions(r, p, real, false, &wk->timer, W, wstride, n, const_cast<void* const*>(in + b0), s);
+      if (rc) return rc;
+      rc = inverse_stages(r, &wk->timer, W, wstride, n, out + b0, s);
+    }
+    if (rc) return rc;
+  }
+  return kOk;
+}
+
+// Split contractions run 16 signals to an operand at the largest band limits
+// among them, FP64 contractions signal by signal: per 16-signal tile against
+// one FP64 signal of the tile's size they take 7.9 times as long inverse and
+// 11.6 times forward (L = 512, N = 64: 20.6 / 2.60 ms and 28.3 / 2.44 ms; L =
+// 128, N = 16: 0.27 / 0.023 and 0.34 / 0.030).  So a tile whose signals add up
+// to less (work N L^3 against the largest L and N) runs FP64, which is closer
+// to the FP64 path it is held to.  SO3GPU_DIGIT_TABLE, which pins the split
+// path's operand source, pins the path too.
+static bool split_pays(bool fwd, double work, double largest) {
+  const char* e = getenv("SO3GPU_DIGIT_TABLE");
+  return (e && *e) || work >= (fwd ? 12.0 : 8.0) * largest;
+}
+// Signals of a uniform batch that the split contractions take.
+static int split_count(bool fwd, int nsig) {
+  const int rest = nsig % 16;
+  return rest == 0 || split_pays(fwd, rest, 1.0) ? nsig : nsig - rest;
+}
+
 int run_inverse_batch(Device* D, Workspace* wk, const so3_parameters_t& p, int real, int nsig,
                       const void* const* flmn_d, void* const* f_d, int precision, cudaStream_t s) {
   if (nsig < 0) return fail(kInvalidParameter, "negative batch size");
   if (precision != kPrecFp64 && precision != kPrecMixedInt8) return fail(kInvalidParameter, "unknown precision");
-  if (precision == kPrecFp64 || !split_real_ok(p, real)) {
-    for (int b = 0; b < nsig; b++)
-      if (int rc = run_inverse(D, wk, p, flmn_d[b], f_d[b], real, s)) return rc;
-    return kOk;
-  }
-  if (nsig == 0) return kOk;
+  const int nsplit = precision == kPrecFp64 || !split_real_ok(p, real) ? 0 : split_count(false, nsig);
+  if (nsplit == 0) return run_fp64_batch(D, wk, p, real, false, nsig, flmn_d, f_d, s);
   Resources r;
   if (int rc = acquire(D, p, real, s, &r, false)) return rc;
   const BatchLayout bl = batch_layout(r.g, p, real, nsig);
@@ -412,7 +541,7 @@ int run_inverse_batch(Device* D, Workspace* wk, const so3_parameters_t& p, int r
   char* base = static_cast<char*>(ws);
   double2* W = reinterpret_cast<double2*>(base);
   if (int rc = ensure_tuned(D, p, real, &r, W, s)) return rc;
-  if (int rc = upload_table(base + bl.table_off, flmn_d, nsig, s)) return rc;
+  if (int rc = upload_table(base + bl.table_off, flmn_d, nsplit, s)) return rc;
   StageTimer* T = &wk->timer;
   cudaEvent_t ev;
   int rc;
@@ -420,34 +549,25 @@ int run_inverse_batch(Device* D, Workspace* wk, const so3_parameters_t& p, int r
   const DigitTable* tab = nullptr;
   if ((rc = ensure_digit_table(D, r.g, p.dl_method, r.dl, s, &tab))) return rc;
   timer_begin(T, s, &ev);
-  rc = launch_mixed_inverse(r.g, p.n_mode, reinterpret_cast<const double2* const*>(base + bl.table_off), nsig, r.bases,
+  rc = launch_mixed_inverse(r.g, p.n_mode, reinterpret_cast<const double2* const*>(base + bl.table_off), nsplit, r.bases,
                             r.dl, tab, W, wstride, base + bl.scratch_off, s);
   if (rc) return rc;
   timer_end(T, s, kStMixInv, ev);
-  for (int b = 0; b < nsig; b++) {
-    double2* Wb = W + (size_t)b * wstride;
-    timer_begin(T, s, &ev);
-    if ((rc = launch_inv_beta(r.g, r.pP, Wb, s))) return rc;
-    timer_end(T, s, kStInvBeta, ev);
-    timer_begin(T, s, &ev);
-    if ((rc = launch_inv_alpha(r.g, r.pP, Wb, s))) return rc;
-    timer_end(T, s, kStInvAlpha, ev);
-    timer_begin(T, s, &ev);
-    if ((rc = launch_inv_gamma(r.g, r.pg, Wb, f_d[b], s))) return rc;
-    timer_end(T, s, kStInvGamma, ev);
-  }
-  return kOk;
+  if (nsplit < nsig)
+    if ((rc = fp64_contractions(r, p, real, false, T, W + (size_t)nsplit * wstride, wstride, nsig - nsplit,
+                                const_cast<void* const*>(flmn_d + nsplit), s)))
+      return rc;
+  return inverse_stages(r, T, W, wstride, nsig, f_d, s);
 }
 
 int run_forward_batch(Device* D, Workspace* wk, const so3_parameters_t& p, int real, int nsig, const void* const* f_d,
                       void* const* flmn_d, int precision, cudaStream_t s) {
   if (nsig < 0) return fail(kInvalidParameter, "negative batch size");
   if (precision != kPrecFp64 && precision != kPrecMixedInt8) return fail(kInvalidParameter, "unknown precision");
-  if (precision == kPrecFp64 || !split_real_ok(p, real)) {
-    for (int b = 0; b < nsig; b++)
-      if (int rc = run_forward(D, wk, p, f_d[b], flmn_d[b], real, s)) return rc;
-    return kOk;
-  }
+  // the split beta stage needs no full tile of signals; it stays with the split contractions
+  const int nsplit = precision == kPrecFp64 || !split_real_ok(p, real) ? 0 : split_count(true, nsig);
+  if (nsplit == 0 && (precision == kPrecFp64 || !split_real_ok(p, real) || !mixed_beta_supported(make_geometry(p, real))))
+    return run_fp64_batch(D, wk, p, real, true, nsig, f_d, flmn_d, s);
   if (nsig == 0) return kOk;
   Resources r;
   if (int rc = acquire(D, p, real, s, &r, true)) return rc;
@@ -457,38 +577,32 @@ int run_forward_batch(Device* D, Workspace* wk, const so3_parameters_t& p, int r
   char* base = static_cast<char*>(ws);
   double2* W = reinterpret_cast<double2*>(base);
   if (int rc = ensure_tuned(D, p, real, &r, W, s)) return rc;
-  if (int rc = upload_table(base + bl.table_off, flmn_d, nsig, s)) return rc;
+  if (nsplit)
+    if (int rc = upload_table(base + bl.table_off, flmn_d, nsplit, s)) return rc;
   StageTimer* T = &wk->timer;
   cudaEvent_t ev;
   int rc;
   const long long wstride = (long long)(bl.wbytes / sizeof(double2));
   // forward beta stage: one tensor-core product over the whole batch where
   // supported (complex MW) and its matrix table is resident, else the FP64
-  // DFT + weight convolution per signal
+  // stage per signal
   const BetaTable* bt = nullptr;
   if (mixed_beta_supported(r.g) && (rc = ensure_beta_table(D, r.g, s, &bt))) return rc;
-  for (int b = 0; b < nsig; b++) {
-    double2* Wb = W + (size_t)b * wstride;
-    timer_begin(T, s, &ev);
-    if ((rc = launch_fwd_gamma(r.g, r.pg, f_d[b], Wb, s))) return rc;
-    timer_end(T, s, kStFwdGamma, ev);
-    timer_begin(T, s, &ev);
-    if ((rc = launch_fwd_alpha(r.g, r.pP, Wb, s))) return rc;
-    timer_end(T, s, kStFwdAlpha, ev);
-    if (bt) continue;
-    timer_begin(T, s, &ev);
-    if ((rc = launch_fwd_beta_conv(r.g, r.pP, r.pc, r.wr, Wb, s))) return rc;
-    timer_end(T, s, kStFwdBetaConv, ev);
-  }
+  if ((rc = forward_stages(r, T, W, wstride, nsig, f_d, bt == nullptr, s))) return rc;
   if (bt) {
     timer_begin(T, s, &ev);
     if ((rc = launch_mixed_fwd_beta(r.g, W, wstride, nsig, bt, base + bl.scratch_off, s))) return rc;
     timer_end(T, s, kStMixFwdBeta, ev);
   }
+  if (nsplit < nsig)
+    if ((rc = fp64_contractions(r, p, real, true, T, W + (size_t)nsplit * wstride, wstride, nsig - nsplit,
+                                flmn_d + nsplit, s)))
+      return rc;
+  if (nsplit == 0) return kOk;
   const DigitTable* tab = nullptr;
   if ((rc = ensure_digit_table(D, r.g, p.dl_method, r.dl, s, &tab))) return rc;
   timer_begin(T, s, &ev);
-  rc = launch_mixed_forward(r.g, p.n_mode, W, wstride, nsig, r.bases, r.dl, tab,
+  rc = launch_mixed_forward(r.g, p.n_mode, W, wstride, nsplit, r.bases, r.dl, tab,
                             reinterpret_cast<double2* const*>(base + bl.table_off), p.storage == SO3_STORAGE_COMPACT,
                             base + bl.scratch_off, s);
   if (rc) return rc;
@@ -505,17 +619,28 @@ int run_conv_inverse_batch(Device* D, Workspace* wk, const so3_parameters_t& p, 
   Resources r;
   if (int rc = acquire(D, p, 0, s, &r, false)) return rc;
   int rc;
-  if (precision == kPrecFp64) {
-    // hlmn of each kernel after the transform's scratch; run_inverse keeps the (larger) workspace
+  if (precision == kPrecFp64 || split_count(false, nsig) == 0) {
+    // scratch of a chunk of signals, then hlmn of each
     const size_t wb = (workspace_bytes(p, 0) + 255) & ~size_t(255);
+    const size_t hb = ((size_t)so3_sampling_flmn_size(&p) * sizeof(double2) + 255) & ~size_t(255);
+    int step = batch_chunk(r.g, nsig);
+    if (wk->borrowed) step = (int)std::min<size_t>(step, std::max<size_t>(1, wk->ws_bytes / (wb + hb)));
     void* ws = nullptr;
-    if ((rc = ensure_ws(wk, wb + (size_t)so3_sampling_flmn_size(&p) * sizeof(double2), &ws))) return rc;
-    double2* h = reinterpret_cast<double2*>(static_cast<char*>(ws) + wb);
-    for (int b = 0; b < nsig; b++) {
-      if ((rc = launch_s2toso3(p, r.bases, static_cast<const double2*>(flm_d), static_cast<const double2*>(glm_d[b]),
-                               h, s)))
-        return rc;
-      if ((rc = run_inverse(D, wk, p, h, f_d[b], 0, s))) return rc;
+    if ((rc = ensure_ws(wk, (wb + hb) * step, &ws))) return rc;
+    double2* W = static_cast<double2*>(ws);
+    if ((rc = ensure_tuned(D, p, 0, &r, W, s))) return rc;
+    const long long wstride = (long long)(wb / sizeof(double2));
+    for (int b0 = 0; b0 < nsig; b0 += step) {
+      const int n = std::min(step, nsig - b0);
+      void* h[kMaxBatch];
+      for (int b = 0; b < n; b++) {
+        h[b] = static_cast<char*>(ws) + wb * step + hb * b;
+        if ((rc = launch_s2toso3(p, r.bases, static_cast<const double2*>(flm_d),
+                                 static_cast<const double2*>(glm_d[b0 + b]), static_cast<double2*>(h[b]), s)))
+          return rc;
+      }
+      if ((rc = fp64_contractions(r, p, 0, false, &wk->timer, W, wstride, n, h, s))) return rc;
+      if ((rc = inverse_stages(r, &wk->timer, W, wstride, n, f_d + b0, s))) return rc;
     }
     return kOk;
   }
@@ -537,19 +662,7 @@ int run_conv_inverse_batch(Device* D, Workspace* wk, const so3_parameters_t& p, 
                             reinterpret_cast<const double2* const*>(base + bl.table_off));
   if (rc) return rc;
   timer_end(T, s, kStMixInv, ev);
-  for (int b = 0; b < nsig; b++) {
-    double2* Wb = W + (size_t)b * wstride;
-    timer_begin(T, s, &ev);
-    if ((rc = launch_inv_beta(r.g, r.pP, Wb, s))) return rc;
-    timer_end(T, s, kStInvBeta, ev);
-    timer_begin(T, s, &ev);
-    if ((rc = launch_inv_alpha(r.g, r.pP, Wb, s))) return rc;
-    timer_end(T, s, kStInvAlpha, ev);
-    timer_begin(T, s, &ev);
-    if ((rc = launch_inv_gamma(r.g, r.pg, Wb, f_d[b], s))) return rc;
-    timer_end(T, s, kStInvGamma, ev);
-  }
-  return kOk;
+  return inverse_stages(r, T, W, wstride, nsig, f_d, s);
 }
 
 // ------------------------------------------------------------ ragged batches
@@ -562,8 +675,37 @@ struct RagItem {
   size_t ws_off;
 };
 
-// Signals of a ragged split-precision batch: complex ones go to the
-// tensor-core contraction (per Delta recursion), real ones to the FP64 path.
+// Signals of a ragged split-precision batch that take the FP64 path: real
+// ones, and those of tiles (16 signals, similar sizes together, per Delta
+// recursion as ragged_plan cuts them) whose padding costs more than the split
+// products save.
+std::vector<char> ragged_fp64(const so3_parameters_t* ps, int nsig, bool fwd) {
+  std::vector<char> f(nsig, 0);
+  for (int m = 0; m < 2; m++) {
+    std::vector<int> order;
+    for (int i = 0; i < nsig; i++) {
+      if (ps[i].reality) f[i] = 1;
+      else if (ps[i].dl_method == m) order.push_back(i);
+    }
+    std::stable_sort(order.begin(), order.end(),
+                     [&](int x, int y) { return ps[x].L != ps[y].L ? ps[x].L > ps[y].L : ps[x].N > ps[y].N; });
+    for (size_t t = 0; t < order.size(); t += 16) {
+      const size_t e = std::min(order.size(), t + 16);
+      double work = 0.0, Lg = 0.0, Ng = 0.0;
+      for (size_t i = t; i < e; i++) {
+        const so3_parameters_t& p = ps[order[i]];
+        work += (double)p.N * p.L * p.L * p.L;
+        Lg = std::max(Lg, (double)p.L), Ng = std::max(Ng, (double)p.N);
+      }
+      if (!split_pays(fwd, work, Ng * Lg * Lg * Lg))
+        for (size_t i = t; i < e; i++) f[order[i]] = 1;
+    }
+  }
+  return f;
+}
+
+// Signals of a ragged split-precision batch for the tensor-core contraction
+// (per Delta recursion), and those for the FP64 path.
 int ragged_prepare(Device* D, const so3_parameters_t* ps, int nsig, bool conv_tables, cudaStream_t s,
                    std::vector<RagItem>* items, std::vector<int>* fp64) {
   int Lmax[2] = {0, 0};
@@ -580,8 +722,9 @@ int ragged_prepare(Device* D, const so3_parameters_t* ps, int nsig, bool conv_ta
         if (int rc = ensure_dl(D, Lmax[m], m, s, &t)) return rc;
   }
   size_t off = 0;
+  const std::vector<char> to_fp64 = ragged_fp64(ps, nsig, conv_tables);
   for (int i = 0; i < nsig; i++) {
-    if (ps[i].reality) {
+    if (to_fp64[i]) {
       fp64->push_back(i);
       continue;
     }
@@ -626,8 +769,8 @@ int run_inverse_ragged(Device* D, Workspace* wk, const so3_parameters_t* ps, int
   std::vector<RagItem> items;
   std::vector<int> fp64;
   if (int rc = ragged_prepare(D, ps, nsig, false, s, &items, &fp64)) return rc;
-  for (int i : fp64)  // real signals: the FP64 path, before the batch workspace is laid out
-    if (int rc = run_inverse(D, wk, ps[i], flmn_d[i], f_d[i], 1, s)) return rc;
+  for (int i : fp64)  // the FP64 path, before the batch workspace is laid out
+    if (int rc = run_inverse(D, wk, ps[i], flmn_d[i], f_d[i], ps[i].reality != 0, s)) return rc;
   if (items.empty()) return kOk;
   const size_t sig_end = ragged_ws_end(items, ps);
   std::vector<RaggedSig> rs[2];
@@ -699,7 +842,7 @@ int run_forward_ragged(Device* D, Workspace* wk, const so3_parameters_t* ps, int
   std::vector<int> fp64;
   if (int rc = ragged_prepare(D, ps, nsig, true, s, &items, &fp64)) return rc;
   for (int i : fp64)
-    if (int rc = run_forward(D, wk, ps[i], f_d[i], flmn_d[i], 1, s)) return rc;
+    if (int rc = run_forward(D, wk, ps[i], f_d[i], flmn_d[i], ps[i].reality != 0, s)) return rc;
   if (items.empty()) return kOk;
   const size_t sig_end = ragged_ws_end(items, ps);
   std::vector<RaggedSig> rs[2];

@@ -171,7 +171,7 @@ struct StageTimer {
 };
 // Marks the start of `stage` on stream s; call mark_end after the launch.
 void timer_begin(StageTimer* t, cudaStream_t s, cudaEvent_t* ev);
-void timer_end(StageTimer* t, cudaStream_t s, int stage, cudaEvent_t start);
+void timer_end(StageTimer* t, cudaStream_t s, int stage, cudaEvent_t start, int signals = 1);  // counts signals
 int timer_collect(StageTimer* t);  // synchronises on the recorded events
 
 // Grow-only device scratch owned by one caller context (never shared between
@@ -218,42 +218,52 @@ __host__ __device__ inline bool plane_skipped(int mode, int N, int n) {
 // wconst > 0 replaces the inverse's per-degree weight (2l+1)/(8 pi^2) by a
 // constant; lw > 0 multiplies the forward's outputs by lw (2l+1) (the
 // adjoint transforms).
+// bt: n signals of one geometry in one launch, scratch of signal b at W + b *
+// wstride, their coefficient (or sample) arrays in bt.io; n = 0: one signal,
+// the array given.
+constexpr int kMaxBatch = 32;
+struct Batch {
+  int n = 0;
+  long long wstride = 0;
+  void* io[kMaxBatch] = {};
+};
 int launch_inverse_contract(const Geometry& g, int n_mode, const double2* flmn, const long long* bases,
                             const double* dl, double2* W, int sym_n0, cudaStream_t s, int nu_lo = 0,
-                            int nu_hi = -1, double wconst = 0.0);
+                            int nu_hi = -1, double wconst = 0.0, const Batch& bt = Batch());
 int launch_forward_contract(const Geometry& g, int n_mode, const double2* W, const long long* bases,
                             const double* dl, double2* flmn, int storage_compact, cudaStream_t s, int nu_lo = 0,
-                            int nu_hi = -1, double lw = 0.0);
+                            int nu_hi = -1, double lw = 0.0, const Batch& bt = Batch());
 
-int launch_inv_beta(const Geometry& g, const FftPlan& pP, double2* W, cudaStream_t s);
-int launch_inv_alpha(const Geometry& g, const FftPlan& pP, double2* W, cudaStream_t s);
+int launch_inv_beta(const Geometry& g, const FftPlan& pP, double2* W, cudaStream_t s, const Batch& bt = Batch());
+int launch_inv_alpha(const Geometry& g, const FftPlan& pP, double2* W, cudaStream_t s, const Batch& bt = Batch());
 // row_lo/row_hi restrict the gamma stages to the beta rows [row_lo, row_hi)
 // (row_hi < 0: up to nb).
 int launch_inv_gamma(const Geometry& g, const FftPlan& pg, const double2* W, void* f, cudaStream_t s,
-                     int row_lo = 0, int row_hi = -1);
+                     int row_lo = 0, int row_hi = -1, const Batch& bt = Batch());
 int launch_fwd_gamma(const Geometry& g, const FftPlan& pg, const void* f, double2* W, cudaStream_t s,
-                     int row_lo = 0, int row_hi = -1);
-int launch_fwd_alpha(const Geometry& g, const FftPlan& pP, double2* W, cudaStream_t s);
+                     int row_lo = 0, int row_hi = -1, const Batch& bt = Batch());
+int launch_fwd_alpha(const Geometry& g, const FftPlan& pP, double2* W, cudaStream_t s, const Batch& bt = Batch());
 int launch_fwd_beta_conv(const Geometry& g, const FftPlan& pP, const FftPlan& pc, const double2* wr,
-                         double2* W, cudaStream_t s);
+                         double2* W, cudaStream_t s, const Batch& bt = Batch());
 
 // The same stages on the FP64 tensor cores (stages_mm.cu), for plans that
 // build_mm_plan covered.
 bool mm_gamma_ok(const Geometry& g, const FftPlan& p);
 bool mm_ok(const FftPlan& p);
 int launch_mm_inv_gamma(const Geometry& g, const FftPlan& p, const double2* W, void* f, cudaStream_t s, int row_lo,
-                        int row_hi);
+                        int row_hi, const Batch& bt);
 int launch_mm_fwd_gamma(const Geometry& g, const FftPlan& p, const void* f, double2* W, cudaStream_t s, int row_lo,
-                        int row_hi);
-int launch_mm_alpha(const Geometry& g, const FftPlan& p, double2* W, bool inverse, cudaStream_t s);
-int launch_mm_inv_beta(const Geometry& g, const FftPlan& p, double2* W, cudaStream_t s);
+                        int row_hi, const Batch& bt);
+int launch_mm_alpha(const Geometry& g, const FftPlan& p, double2* W, bool inverse, cudaStream_t s, const Batch& bt);
+int launch_mm_inv_beta(const Geometry& g, const FftPlan& p, double2* W, cudaStream_t s, const Batch& bt);
 
 // Beta stages as products with one real matrix per parity (beta_mm.cu).
 enum BetaKind : int { kBetaInverse = 0, kBetaForward, kBetaAdjInverse, kBetaAdjForward, kBetaKinds };
 bool beta_matrix_pays(const Geometry& g, int kind);
 size_t beta_matrix_bytes(const Geometry& g, int kind);
 int launch_beta_matrix_table(const Geometry& g, int kind, const FftPlan& pP, double* tab, cudaStream_t s);
-int launch_beta_matrix(const Geometry& g, int kind, const double* tab, double2* W, cudaStream_t s);
+int launch_beta_matrix(const Geometry& g, int kind, const double* tab, double2* W, cudaStream_t s,
+                       const Batch& bt = Batch());
 
 int launch_s2toso3(const so3_parameters_t& hp, const long long* bases, const double2* flm, const double2* glm,
                    double2* hlmn, cudaStream_t s);

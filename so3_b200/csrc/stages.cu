@@ -714,14 +714,23 @@ int launched() {
 
 }  // namespace
 
+// Stages without a batched kernel run signal by signal.
+template <class F>
+static int each(const Batch& bt, const F& run) {
+  for (int b = 0; b < bt.n; b++)
+    if (int rc = run(b)) return rc;
+  return kOk;
+}
+
 // Where the tensor-core DFT replaces the scalar engines below: every length
 // but the 1023 of the compile-time plan (us per 31-plane transform at L = 512,
 // inverse beta / inverse alpha: 276 / 191 against 225 / 175).
 static bool mm_pays(const FftPlan& p) { return mm_ok(p) && pick(p) != Eng::k1023; }
 
-int launch_inv_beta(const Geometry& g, const FftPlan& p, double2* W, cudaStream_t s) {
-  if (g.beta_mat[kBetaInverse]) return launch_beta_matrix(g, kBetaInverse, g.beta_mat[kBetaInverse], W, s);
-  if (mm_pays(p)) return launch_mm_inv_beta(g, p, W, s);
+int launch_inv_beta(const Geometry& g, const FftPlan& p, double2* W, cudaStream_t s, const Batch& bt) {
+  if (g.beta_mat[kBetaInverse]) return launch_beta_matrix(g, kBetaInverse, g.beta_mat[kBetaInverse], W, s, bt);
+  if (mm_pays(p)) return launch_mm_inv_beta(g, p, W, s, bt);
+  if (bt.n) return each(bt, [&](int b) { return launch_inv_beta(g, p, W + b * bt.wstride, s); });
   int rc;
   const int v = g.var[kStInvBeta];
   switch (pick(p)) {
@@ -737,8 +746,9 @@ int launch_inv_beta(const Geometry& g, const FftPlan& p, double2* W, cudaStream_
   return rc ? rc : launched();
 }
 
-int launch_inv_alpha(const Geometry& g, const FftPlan& p, double2* W, cudaStream_t s) {
-  if (mm_pays(p)) return launch_mm_alpha(g, p, W, true, s);
+int launch_inv_alpha(const Geometry& g, const FftPlan& p, double2* W, cudaStream_t s, const Batch& bt) {
+  if (mm_pays(p)) return launch_mm_alpha(g, p, W, true, s, bt);
+  if (bt.n) return each(bt, [&](int b) { return launch_inv_alpha(g, p, W + b * bt.wstride, s); });
   int rc;
   const int v = g.var[kStInvAlpha];
   switch (pick(p)) {
@@ -755,10 +765,12 @@ int launch_inv_alpha(const Geometry& g, const FftPlan& p, double2* W, cudaStream
 }
 
 int launch_inv_gamma(const Geometry& g, const FftPlan& p, const double2* W, void* f, cudaStream_t s, int row_lo,
-                     int row_hi) {
+                     int row_hi, const Batch& bt) {
   if (row_hi < 0 || row_hi > g.nb) row_hi = g.nb;
   if (row_lo >= row_hi) return kOk;
-  if (mm_gamma_ok(g, p)) return launch_mm_inv_gamma(g, p, W, f, s, row_lo, row_hi);
+  if (mm_gamma_ok(g, p)) return launch_mm_inv_gamma(g, p, W, f, s, row_lo, row_hi, bt);
+  if (bt.n)
+    return each(bt, [&](int b) { return launch_inv_gamma(g, p, W + b * bt.wstride, bt.io[b], s, row_lo, row_hi); });
   int rc;
   const Eng e = pick(p);
   if (g.real) {
@@ -772,10 +784,12 @@ int launch_inv_gamma(const Geometry& g, const FftPlan& p, const double2* W, void
 }
 
 int launch_fwd_gamma(const Geometry& g, const FftPlan& p, const void* f, double2* W, cudaStream_t s, int row_lo,
-                     int row_hi) {
+                     int row_hi, const Batch& bt) {
   if (row_hi < 0 || row_hi > g.nb) row_hi = g.nb;
   if (row_lo >= row_hi) return kOk;
-  if (mm_gamma_ok(g, p)) return launch_mm_fwd_gamma(g, p, f, W, s, row_lo, row_hi);
+  if (mm_gamma_ok(g, p)) return launch_mm_fwd_gamma(g, p, f, W, s, row_lo, row_hi, bt);
+  if (bt.n)
+    return each(bt, [&](int b) { return launch_fwd_gamma(g, p, bt.io[b], W + b * bt.wstride, s, row_lo, row_hi); });
   int rc;
   const Eng e = pick(p);
   if (g.real) {
@@ -788,8 +802,9 @@ int launch_fwd_gamma(const Geometry& g, const FftPlan& p, const void* f, double2
   return rc ? rc : launched();
 }
 
-int launch_fwd_alpha(const Geometry& g, const FftPlan& p, double2* W, cudaStream_t s) {
-  if (mm_pays(p)) return launch_mm_alpha(g, p, W, false, s);
+int launch_fwd_alpha(const Geometry& g, const FftPlan& p, double2* W, cudaStream_t s, const Batch& bt) {
+  if (mm_pays(p)) return launch_mm_alpha(g, p, W, false, s, bt);
+  if (bt.n) return each(bt, [&](int b) { return launch_fwd_alpha(g, p, W + b * bt.wstride, s); });
   int rc;
   const int v = g.var[kStFwdAlpha];
   switch (pick(p)) {
@@ -810,8 +825,9 @@ bool conv_fixed(const FftPlan& p, const FftPlan& pc) { return pick(p) == Eng::k1
 }  // namespace
 
 int launch_fwd_beta_conv(const Geometry& g, const FftPlan& p, const FftPlan& pc, const double2* wr, double2* W,
-                         cudaStream_t s) {
-  if (g.beta_mat[kBetaForward]) return launch_beta_matrix(g, kBetaForward, g.beta_mat[kBetaForward], W, s);
+                         cudaStream_t s, const Batch& bt) {
+  if (g.beta_mat[kBetaForward]) return launch_beta_matrix(g, kBetaForward, g.beta_mat[kBetaForward], W, s, bt);
+  if (bt.n) return each(bt, [&](int b) { return launch_fwd_beta_conv(g, p, pc, wr, W + b * bt.wstride, s); });
   int rc;
   if (conv_fixed(p, pc))
     rc = g.var[kStFwdBetaConv] == 1 ? fwd_beta_conv<EConv1023b>(g, p, pc, wr, W, s)

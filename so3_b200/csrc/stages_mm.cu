@@ -37,8 +37,26 @@ int launched() {
   return kOk;
 }
 
-__device__ __forceinline__ long long row_off(const Geometry& g, int row) {
-  return (long long)(row / g.nb) * g.PS + (long long)(row % g.nb) * g.RS;
+// Signals of a batch (blockIdx.z of the gamma kernels): their samples, and
+// their scratch at W + z * wstride.
+struct SigIo {
+  long long wstride;
+  void* f[kMaxBatch];
+};
+SigIo sig_io(const Batch& bt, const void* f) {
+  SigIo io{};
+  io.wstride = bt.wstride;
+  for (int b = 0; b < bt.n; b++) io.f[b] = bt.io[b];
+  if (!bt.n) io.f[0] = const_cast<void*>(f);
+  return io;
+}
+int count(const Batch& bt) { return bt.n ? bt.n : 1; }
+
+// Rows of all signals, plane-major over the nb beta rows of each.
+__device__ __forceinline__ long long row_off(const Geometry& g, int row, long long wstride) {
+  const int per = g.nplanes * g.nb, sig = row / per;
+  row -= sig * per;
+  return sig * wstride + (long long)(row / g.nb) * g.PS + (long long)(row % g.nb) * g.RS;
 }
 
 // ------------------------------------------------------------------ gamma
@@ -71,8 +89,10 @@ struct FwdGammaOut {
 // Complex inverse: circle entry r holds plane n = r (r < N) or r - ng; the
 // 2N-point circle of a steerable signal has no plane n = N and keeps N samples.
 __global__ void __launch_bounds__(kGT, 4) inv_gamma_mm_kernel(Geometry g, MmLevel lv, const double2* __restrict__ W,
-                                                         double2* __restrict__ f, int tash, int row0) {
+                                                         const __grid_constant__ SigIo io, int tash, int row0) {
   extern __shared__ __align__(16) double2 sm[];
+  W += blockIdx.z * io.wstride;
+  double2* f = static_cast<double2*>(io.f[blockIdx.z]);
   const int TA = 1 << tash, rp = TA + 2;
   const int row = row0 + blockIdx.y, a0 = blockIdx.x << tash, ng = g.ng, nc = min(TA, g.na - a0);
   const double2* src = W + (long long)row * g.RS + a0;
@@ -93,9 +113,11 @@ __global__ void __launch_bounds__(kGT, 4) inv_gamma_mm_kernel(Geometry g, MmLeve
 
 // Complex forward; steerable: samples N..2N-1 of the circle are zero and only
 // n = N-1 (mod 2) is analysed (so3_core.c:309-328).
-__global__ void __launch_bounds__(kGT, 4) fwd_gamma_mm_kernel(Geometry g, MmLevel lv, const double2* __restrict__ f,
+__global__ void __launch_bounds__(kGT, 4) fwd_gamma_mm_kernel(Geometry g, MmLevel lv, const __grid_constant__ SigIo io,
                                                          double2* __restrict__ W, int tash, int row0) {
   extern __shared__ __align__(16) double2 sm[];
+  W += blockIdx.z * io.wstride;
+  const double2* f = static_cast<const double2*>(io.f[blockIdx.z]);
   const int TA = 1 << tash, rp = TA + 2;
   const int row = row0 + blockIdx.y, a0 = blockIdx.x << tash, ng = g.ng, nc = min(TA, g.na - a0);
   const long long plane_sz = (long long)g.nb * g.na;
@@ -170,9 +192,11 @@ __device__ __forceinline__ void c2r_task(const double2* __restrict__ src, int rp
 }
 
 __global__ void __launch_bounds__(kGT, 4) inv_gamma_real_mm_kernel(Geometry g, MmLevel lv,
-                                                              const double2* __restrict__ W, double* __restrict__ f,
+                                                              const double2* __restrict__ W, const __grid_constant__ SigIo io,
                                                               int tash, int row0) {
   extern __shared__ __align__(16) double2 sm[];
+  W += blockIdx.z * io.wstride;
+  double* f = static_cast<double*>(io.f[blockIdx.z]);
   const int TA = 1 << tash, rp = TA + 2;
   const int row = row0 + blockIdx.y, a0 = blockIdx.x << tash, nc = min(TA, g.na - a0);
   const double2* src = W + (long long)row * g.RS + a0;
@@ -253,9 +277,11 @@ __device__ __forceinline__ void r2c_task(const double* __restrict__ src, int rp,
 // Sample rows of TA + 4 doubles (4 mod 16): 4 rows x 4 columns per half warp
 // in distinct banks.
 __global__ void __launch_bounds__(kGT, 4) fwd_gamma_real_mm_kernel(Geometry g, MmLevel lv,
-                                                              const double* __restrict__ f, double2* __restrict__ W,
+                                                              const __grid_constant__ SigIo io, double2* __restrict__ W,
                                                               int tash, int row0) {
   extern __shared__ __align__(16) double smd[];
+  W += blockIdx.z * io.wstride;
+  const double* f = static_cast<const double*>(io.f[blockIdx.z]);
   const int TA = 1 << tash, rp = TA + 4;
   const int row = row0 + blockIdx.y, a0 = blockIdx.x << tash, nc = min(TA, g.na - a0);
   const long long plane_sz = (long long)g.nb * g.na;
@@ -301,18 +327,19 @@ struct AlphaOut {
 };
 
 template <bool INV>
-__global__ void __launch_bounds__(kMaxThr, kMinB) alpha_mm_kernel(Geometry g, MmPlan P, double2* __restrict__ W, int T) {
+__global__ void __launch_bounds__(kMaxThr, kMinB) alpha_mm_kernel(Geometry g, MmPlan P, double2* __restrict__ W, int T,
+                                                              int nrows, long long wstride) {
   extern __shared__ __align__(16) double2 sm[];
   __shared__ double2 x0[2 * kMaxT];
   __shared__ double2* rows[kMaxT];
   double2* A = sm;
   double2* Z = sm + (size_t)T * P.ts;
-  const int L = g.L, Pn = g.P, nrows = g.nplanes * g.nb, r0 = blockIdx.x * T, Ta = min(T, nrows - r0);
-  if (threadIdx.x < Ta) rows[threadIdx.x] = W + row_off(g, r0 + threadIdx.x);
+  const int L = g.L, Pn = g.P, r0 = blockIdx.x * T, Ta = min(T, nrows - r0);
+  if (threadIdx.x < Ta) rows[threadIdx.x] = W + row_off(g, r0 + threadIdx.x, wstride);
   // column of entry k; -1: the MWSS Nyquist entry k = L, which has no column
   auto col = [&](int k) { return k <= L - 1 ? k + L - 1 : k - Pn + L - 1; };
   for (int t = 0; t < Ta; t++) {
-    const double2* src = W + row_off(g, r0 + t);
+    const double2* src = W + row_off(g, r0 + t, wstride);
     if (P.kind == 3) {
       mm::stage_conv<INV>(P, A + t * P.ts, x0 + 2 * t, [&](int k) {
         const int c = INV ? col(k) : k;
@@ -348,12 +375,14 @@ struct SmemOut {
 
 __global__ void __launch_bounds__(kMaxThr, kMinB) inv_beta_mm_kernel(Geometry g, MmPlan P,
                                                                      const double2* __restrict__ half,
-                                                                     double2* __restrict__ W, int T) {
+                                                                     double2* __restrict__ W, int T, long long wstride) {
   extern __shared__ __align__(16) double2 sm[];
   __shared__ double2 x0[2 * kMaxT], b0s[kMaxT];
   double2* A = sm;
   double2* Z = sm + (size_t)T * P.ts;
-  const int plane = blockIdx.y, n = plane - g.plane0, L = g.L, Pn = g.P, ncols = 2 * L - 1;
+  const int sig = blockIdx.y / g.nplanes, plane = blockIdx.y - sig * g.nplanes;
+  const int n = plane - g.plane0, L = g.L, Pn = g.P, ncols = 2 * L - 1;
+  W += sig * wstride;
   const int q0 = blockIdx.x * T, Ta = min(T, L - q0);
   double2* base = W + (long long)plane * g.PS;
   const double2* cbase = W + g.QOFF + (long long)plane * g.QS;
@@ -480,54 +509,56 @@ bool mm_gamma_ok(const Geometry& g, const FftPlan& p) {
 bool mm_ok(const FftPlan& p) { return p.mm.n == p.n && seq_smem(p.mm, 1, 2) <= kSmemMax; }
 
 int launch_mm_inv_gamma(const Geometry& g, const FftPlan& p, const double2* W, void* f, cudaStream_t s, int row_lo,
-                        int row_hi) {
+                        int row_hi, const Batch& bt) {
   int sh = gamma_shift(p.l1, g.real ? 16 : 8);
   const int rows = g.real ? g.nplanes : g.ng;
   while (sh > 4 && (size_t)rows * ((1 << sh) + 2) * sizeof(double2) > kSmemMax / 4) sh--;
   const size_t smem = (size_t)rows * ((1 << sh) + 2) * sizeof(double2);
-  const dim3 grid((g.na + (1 << sh) - 1) >> sh, row_hi - row_lo);
+  const dim3 grid((g.na + (1 << sh) - 1) >> sh, row_hi - row_lo, count(bt));
+  const SigIo io = sig_io(bt, f);
   if (g.real) {
     if (int rc = set_smem(inv_gamma_real_mm_kernel, smem)) return rc;
-    inv_gamma_real_mm_kernel<<<grid, kGT, smem, s>>>(g, p.l1, W, static_cast<double*>(f), sh, row_lo);
+    inv_gamma_real_mm_kernel<<<grid, kGT, smem, s>>>(g, p.l1, W, io, sh, row_lo);
   } else {
     if (int rc = set_smem(inv_gamma_mm_kernel, smem)) return rc;
-    inv_gamma_mm_kernel<<<grid, kGT, smem, s>>>(g, p.l1, W, static_cast<double2*>(f), sh, row_lo);
+    inv_gamma_mm_kernel<<<grid, kGT, smem, s>>>(g, p.l1, W, io, sh, row_lo);
   }
   return launched();
 }
 
 int launch_mm_fwd_gamma(const Geometry& g, const FftPlan& p, const void* f, double2* W, cudaStream_t s, int row_lo,
-                        int row_hi) {
+                        int row_hi, const Batch& bt) {
   int sh = gamma_shift(p.l1, g.real ? 16 : 8);
   while (sh > 4 && (size_t)g.ng * ((1 << sh) + 4) * (g.real ? 8 : 16) > kSmemMax / 4) sh--;
   const size_t smem = (size_t)g.ng * (g.real ? ((1 << sh) + 4) * 8 : ((1 << sh) + 2) * 16);
-  const dim3 grid((g.na + (1 << sh) - 1) >> sh, row_hi - row_lo);
+  const dim3 grid((g.na + (1 << sh) - 1) >> sh, row_hi - row_lo, count(bt));
+  const SigIo io = sig_io(bt, f);
   if (g.real) {
     if (int rc = set_smem(fwd_gamma_real_mm_kernel, smem)) return rc;
-    fwd_gamma_real_mm_kernel<<<grid, kGT, smem, s>>>(g, p.l1, static_cast<const double*>(f), W, sh, row_lo);
+    fwd_gamma_real_mm_kernel<<<grid, kGT, smem, s>>>(g, p.l1, io, W, sh, row_lo);
   } else {
     if (int rc = set_smem(fwd_gamma_mm_kernel, smem)) return rc;
-    fwd_gamma_mm_kernel<<<grid, kGT, smem, s>>>(g, p.l1, static_cast<const double2*>(f), W, sh, row_lo);
+    fwd_gamma_mm_kernel<<<grid, kGT, smem, s>>>(g, p.l1, io, W, sh, row_lo);
   }
   return launched();
 }
 
-int launch_mm_alpha(const Geometry& g, const FftPlan& p, double2* W, bool inverse, cudaStream_t s) {
-  const int nrows = g.nplanes * g.nb;
+int launch_mm_alpha(const Geometry& g, const FftPlan& p, double2* W, bool inverse, cudaStream_t s, const Batch& bt) {
+  const int nrows = g.nplanes * g.nb * count(bt);
   const Shape z = shape_for(p.mm, nrows, p.mm.kind == 1 ? 1 : 2);
   auto go = [&](auto kernel) -> int {
     if (int rc = set_smem(kernel, z.smem)) return rc;
-    kernel<<<(nrows + z.T - 1) / z.T, 32 * z.warps, z.smem, s>>>(g, z.P, W, z.T);
+    kernel<<<(nrows + z.T - 1) / z.T, 32 * z.warps, z.smem, s>>>(g, z.P, W, z.T, nrows, bt.wstride);
     return launched();
   };
   return inverse ? go(alpha_mm_kernel<true>) : go(alpha_mm_kernel<false>);
 }
 
-int launch_mm_inv_beta(const Geometry& g, const FftPlan& p, double2* W, cudaStream_t s) {
-  const Shape z = shape_for(p.mm, g.L * g.nplanes, 2);
-  const dim3 grid((g.L + z.T - 1) / z.T, g.nplanes);
+int launch_mm_inv_beta(const Geometry& g, const FftPlan& p, double2* W, cudaStream_t s, const Batch& bt) {
+  const Shape z = shape_for(p.mm, g.L * g.nplanes * count(bt), 2);
+  const dim3 grid((g.L + z.T - 1) / z.T, g.nplanes * count(bt));
   if (int rc = set_smem(inv_beta_mm_kernel, z.smem)) return rc;
-  inv_beta_mm_kernel<<<grid, 32 * z.warps, z.smem, s>>>(g, z.P, p.half, W, z.T);
+  inv_beta_mm_kernel<<<grid, 32 * z.warps, z.smem, s>>>(g, z.P, p.half, W, z.T, bt.wstride);
   return launched();
 }
 

@@ -167,8 +167,9 @@ void timer_begin(StageTimer* t, cudaStream_t s, cudaEvent_t* ev) {
   cudaEventRecord(*ev, s);
 }
 
-void timer_end(StageTimer* t, cudaStream_t s, int stage, cudaEvent_t start) {
+void timer_end(StageTimer* t, cudaStream_t s, int stage, cudaEvent_t start, int signals) {
   if (!t || !t->on || !start) return;
+  t->count[stage] += signals - 1;
   cudaEvent_t e = take_event(t);
   cudaEventRecord(e, s);
   t->pending.push_back({stage, {start, e}});
