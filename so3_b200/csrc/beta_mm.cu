@@ -24,6 +24,7 @@
 #include <algorithm>
 
 #include "dft_mm.cuh"
+#include "launch.cuh"
 #include "so3gpu_internal.h"
 
 namespace so3g {
@@ -68,14 +69,16 @@ __global__ void __launch_bounds__(32 * WR * WC, WR * WC == 8 ? 2 : 4) beta_mm_ke
                               : W + (long long)plane * g.PS + c0;
   const int nch = (a.K + kK - 1) / kK;
 
-  auto stage = [&](int ch) {
+  auto stage_matrix = [&](int ch) {
     double* As = smd + (ch % kStages) * STAGE;
-    double2* Bs = reinterpret_cast<double2*>(As + ASZ);
     for (int i = tid; i < ASZ / 2; i += NTHR) {  // 16-byte pieces: [parity][row tile][64 of 4 steps]
       const int p = i / (RT * 64), rt = i / 64 % RT, o = i % 64;
       const int par = first_is_a ? p : 1 - p;
       mm::cp16(As + 2 * i, a.tab + (((size_t)par * a.RT + rt0 + rt) * a.KS + 4 * ch) * 32 + 2 * o);
     }
+  };
+  auto stage_columns = [&](int ch) {
+    double2* Bs = reinterpret_cast<double2*>(smd + (ch % kStages) * STAGE + ASZ);
     for (int i = tid; i < COLS * kK; i += NTHR) {
       const int k = SPEC_IN ? i % kK : i / COLS, c = SPEC_IN ? i / kK : i % COLS;
       const bool ok = ch * kK + k < a.K && c0 + c < ncols;
@@ -94,14 +97,21 @@ __global__ void __launch_bounds__(32 * WR * WC, WR * WC == 8 ? 2 : 4) beta_mm_ke
       for (int t = 0; t < NP; t++) acc[p][i][t][0] = acc[p][i][t][1] = 0.0;
 
 #pragma unroll
+  for (int s = 0; s < kStages - 1; s++)
+    if (s < nch) stage_matrix(s);
+  dep_wait();  // the columns are the stage before's
+#pragma unroll
   for (int s = 0; s < kStages - 1; s++) {
-    if (s < nch) stage(s);
+    if (s < nch) stage_columns(s);
     asm volatile("cp.async.commit_group;\n" ::);
   }
   for (int ch = 0; ch < nch; ch++) {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(kStages - 2) : "memory");
     __syncthreads();
-    if (ch + kStages - 1 < nch) stage(ch + kStages - 1);
+    if (ch + kStages - 1 < nch) {
+      stage_matrix(ch + kStages - 1);
+      stage_columns(ch + kStages - 1);
+    }
     asm volatile("cp.async.commit_group;\n" ::);
     const double* As = smd + (ch % kStages) * STAGE + wr * MT * 128 + lane;
     const double* Bs = smd + (ch % kStages) * STAGE + ASZ + (gr & 1);
@@ -125,6 +135,7 @@ __global__ void __launch_bounds__(32 * WR * WC, WR * WC == 8 ? 2 : 4) beta_mm_ke
     }
   }
 
+  dep_launch();
   // lane (gr, kk): row gr of a tile, columns 2c and 2c + 1 (c = 4 (wc NP + t) + kk)
 #pragma unroll
   for (int i = 0; i < MT; i++) {
@@ -215,13 +226,8 @@ int go(const Geometry& g, const BetaMmArgs& a, int nsig, cudaStream_t s) {
   constexpr int COLS = 8 * NP * WC, ROWS = 8 * MT * WR;
   constexpr int BSZ = SPEC_IN ? COLS * (kK + 4) : kK * (COLS + 2);
   constexpr size_t smem = kStages * (2 * MT * WR * 128 + 2 * BSZ) * sizeof(double);
-  auto kernel = beta_mm_kernel<SPEC_IN, MT, WR, NP, WC>;
-  SO3G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const dim3 grid((2 * g.L - 1 + COLS - 1) / COLS, (a.M + ROWS - 1) / ROWS, g.nplanes * nsig);
-  kernel<<<grid, 32 * WR * WC, smem, s>>>(g, a);
-  SO3G_LAUNCHED();
-  SO3G_CUDA(cudaGetLastError());
-  return kOk;
+  return launch_after(beta_mm_kernel<SPEC_IN, MT, WR, NP, WC>, grid, 32 * WR * WC, smem, s, g, a);
 }
 
 }  // namespace

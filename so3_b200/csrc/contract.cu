@@ -29,6 +29,7 @@
 #include <type_traits>
 
 #include "dft_mm.cuh"
+#include "launch.cuh"
 #include "so3gpu_internal.h"
 #include "tc_sm100.cuh"
 
@@ -491,19 +492,27 @@ __global__ void __launch_bounds__(kCThreads, 2) contract_mma_kernel(const __grid
       }
     }
     const long long cstep = (xc & 1) ? -a.CS : a.CS;
-    int st = 0;
-    uint32_t phase = 1;  // of the ring slot's previous use
-    for (int ch = ch0; ch < ch1; ch++) {
-      if (ch - ch0 >= ST) tc::mbar_wait(empty0 + 8 * st, phase, &g_contract_error, 4);
-      const uint32_t at = (uint32_t)(st * STAGE * 8), bar = full0 + 8 * st;
+    auto blocks = [&](int ch, int st) {
       const int lc = FWD ? trt : ch, mt = FWD ? ch : trt;
       const bool v = lane < 2 * RT && mt <= lc && lc < LC && (tmu ? mu0 <= 8 * lc : nu0 < 8 * (lc + 1));
       const unsigned got = __ballot_sync(0xffffffffu, v);
       if (lane == 0)
-        tc::mbar_arrive_expect_tx(bar, __popc(got & ((1u << RT) - 1)) * (kCMu * 512) + __popc(got >> RT) * (NU * 512));
+        tc::mbar_arrive_expect_tx(full0 + 8 * st, __popc(got & ((1u << RT) - 1)) * (kCMu * 512) +
+                                                      __popc(got >> RT) * (NU * 512));
       __syncwarp();
       if (v)
-        tc::bulk_g2s(tdst + at, a.dl + dl_base(lc) + (long long)mt * (512 * (lc + 1)) + toff, (tmu ? kCMu : NU) * 512, bar);
+        tc::bulk_g2s(tdst + (uint32_t)(st * STAGE * 8), a.dl + dl_base(lc) + (long long)mt * (512 * (lc + 1)) + toff,
+                     (tmu ? kCMu : NU) * 512, full0 + 8 * st);
+    };
+    // the first Delta blocks come while the kernel before finishes; X is its output
+    if (ch0 < ch1) blocks(ch0, 0);
+    dep_wait();
+    int st = 0;
+    uint32_t phase = 1;  // of the ring slot's previous use
+    for (int ch = ch0; ch < ch1; ch++) {
+      if (ch - ch0 >= ST) tc::mbar_wait(empty0 + 8 * st, phase, &g_contract_error, 4);
+      if (ch > ch0) blocks(ch, st);
+      const uint32_t at = (uint32_t)(st * STAGE * 8), bar = full0 + 8 * st;
 #pragma unroll
       for (int j = 0; j < NU; j++) {
         if (FWD) {
@@ -537,6 +546,7 @@ __global__ void __launch_bounds__(kCThreads, 2) contract_mma_kernel(const __grid
   }
 
   // -------------------------------------------------- products
+  dep_wait();
   double acc[MT][4][NW][2];
 #pragma unroll
   for (int i = 0; i < MT; i++)
@@ -617,6 +627,7 @@ __global__ void __launch_bounds__(kCThreads, 2) contract_mma_kernel(const __grid
     if (++st == ST) st = 0, phase ^= 1;
   }
 
+  dep_launch();
   // accumulator (row g, columns 2q, 2q+1) = combination q, real / imaginary part
   const int ms = (q & 1) ? -1 : 1, ns = (q & 2) ? -1 : 1;
   if (q >= a.nsign) return;
@@ -661,13 +672,9 @@ int contract(ContractArgs a, const void* flmn, const Batch& bt, cudaStream_t s) 
   if (!bt.n) a.flmn[0] = const_cast<void*>(flmn);
   a.wstride = bt.wstride;
   constexpr size_t smem = kCStages * kCStage * sizeof(double);
-  SO3G_CUDA(cudaFuncSetAttribute(contract_mma_kernel<FWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   a.nu0 = a.nu_lo / kCNu * kCNu;  // tiles stay aligned: a block of 8 degrees holds whole groups of nu
   const dim3 grid((a.nu_hi - a.nu0 + kCNu - 1) / kCNu, (a.L + 8 * kCRt - 1) / (8 * kCRt), (a.L + kCMu - 1) / kCMu * (bt.n ? bt.n : 1));
-  contract_mma_kernel<FWD><<<grid, kCThreads, smem, s>>>(a);
-  SO3G_LAUNCHED();
-  SO3G_CUDA(cudaGetLastError());
-  return kOk;
+  return launch_after(contract_mma_kernel<FWD>, grid, kCThreads, smem, s, a);
 }
 }  // namespace
 

@@ -14,6 +14,7 @@
 #include <algorithm>
 
 #include "dft_mm.cuh"
+#include "launch.cuh"
 #include "so3gpu_internal.h"
 
 namespace so3g {
@@ -24,18 +25,6 @@ constexpr int kGT = 128;               // threads of the gamma kernels
 constexpr size_t kSmemMax = 200 * 1024;
 constexpr int kMaxThr = 256, kMinB = 3;  // alpha / beta kernels: 80 registers a thread, 24 warps per SM
 constexpr int kMaxT = 16;              // sequences per CTA
-
-template <typename K>
-int set_smem(K kernel, size_t bytes) {
-  SO3G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  return kOk;
-}
-
-int launched() {
-  SO3G_LAUNCHED();
-  SO3G_CUDA(cudaGetLastError());
-  return kOk;
-}
 
 // Signals of a batch (blockIdx.z of the gamma kernels): their samples, and
 // their scratch at W + z * wstride.
@@ -91,6 +80,7 @@ struct FwdGammaOut {
 __global__ void __launch_bounds__(kGT, 4) inv_gamma_mm_kernel(Geometry g, MmLevel lv, const double2* __restrict__ W,
                                                          const __grid_constant__ SigIo io, int tash, int row0) {
   extern __shared__ __align__(16) double2 sm[];
+  dep_wait();
   W += blockIdx.z * io.wstride;
   double2* f = static_cast<double2*>(io.f[blockIdx.z]);
   const int TA = 1 << tash, rp = TA + 2;
@@ -106,6 +96,7 @@ __global__ void __launch_bounds__(kGT, 4) inv_gamma_mm_kernel(Geometry g, MmLeve
     for (int c = threadIdx.x; c < TA; c += kGT) sm[g.N * rp + c] = make_double2(0.0, 0.0);
   mm::cp_wait_all();
   __syncthreads();
+  dep_launch();
   const long long plane_sz = (long long)g.nb * g.na;
   double2* dst = f + (long long)row * g.na + a0;
   mm::level<4, true>(sm, rp, lv, nc, [](int j) { return j; }, InvGammaOut{dst, plane_sz, g.nf});
@@ -116,6 +107,7 @@ __global__ void __launch_bounds__(kGT, 4) inv_gamma_mm_kernel(Geometry g, MmLeve
 __global__ void __launch_bounds__(kGT, 4) fwd_gamma_mm_kernel(Geometry g, MmLevel lv, const __grid_constant__ SigIo io,
                                                          double2* __restrict__ W, int tash, int row0) {
   extern __shared__ __align__(16) double2 sm[];
+  dep_wait();
   W += blockIdx.z * io.wstride;
   const double2* f = static_cast<const double2*>(io.f[blockIdx.z]);
   const int TA = 1 << tash, rp = TA + 2;
@@ -131,6 +123,7 @@ __global__ void __launch_bounds__(kGT, 4) fwd_gamma_mm_kernel(Geometry g, MmLeve
   }
   mm::cp_wait_all();
   __syncthreads();
+  dep_launch();
   const double scale = 2.0 * 3.141592653589793238462643383279502884 / g.nf;
   double2* dst = W + (long long)row * g.RS + a0;
   mm::level<4, false>(sm, rp, lv, nc, [](int j) { return j; },
@@ -195,6 +188,7 @@ __global__ void __launch_bounds__(kGT, 4) inv_gamma_real_mm_kernel(Geometry g, M
                                                               const double2* __restrict__ W, const __grid_constant__ SigIo io,
                                                               int tash, int row0) {
   extern __shared__ __align__(16) double2 sm[];
+  dep_wait();
   W += blockIdx.z * io.wstride;
   double* f = static_cast<double*>(io.f[blockIdx.z]);
   const int TA = 1 << tash, rp = TA + 2;
@@ -206,6 +200,7 @@ __global__ void __launch_bounds__(kGT, 4) inv_gamma_real_mm_kernel(Geometry g, M
   }
   mm::cp_wait_all();
   __syncthreads();
+  dep_launch();
   const long long plane_sz = (long long)g.nb * g.na;
   double* dst = f + (long long)row * g.na + a0;
   const int ng = lv.QG, tasks = (nc + 15) / 16 * ng;
@@ -280,6 +275,7 @@ __global__ void __launch_bounds__(kGT, 4) fwd_gamma_real_mm_kernel(Geometry g, M
                                                               const __grid_constant__ SigIo io, double2* __restrict__ W,
                                                               int tash, int row0) {
   extern __shared__ __align__(16) double smd[];
+  dep_wait();
   W += blockIdx.z * io.wstride;
   const double* f = static_cast<const double*>(io.f[blockIdx.z]);
   const int TA = 1 << tash, rp = TA + 4;
@@ -291,6 +287,7 @@ __global__ void __launch_bounds__(kGT, 4) fwd_gamma_real_mm_kernel(Geometry g, M
     if (c < nc) smd[r * rp + c] = __ldg(src + (long long)r * plane_sz + c);
   }
   __syncthreads();
+  dep_launch();
   const double scale = 2.0 * 3.141592653589793238462643383279502884 / g.nf;
   double2* dst = W + (long long)row * g.RS + a0;
   const int ng = lv.QG, tasks = (nc + 15) / 16 * ng;
@@ -330,6 +327,7 @@ template <bool INV>
 __global__ void __launch_bounds__(kMaxThr, kMinB) alpha_mm_kernel(Geometry g, MmPlan P, double2* __restrict__ W, int T,
                                                               int nrows, long long wstride) {
   extern __shared__ __align__(16) double2 sm[];
+  dep_wait();
   __shared__ double2 x0[2 * kMaxT];
   __shared__ double2* rows[kMaxT];
   double2* A = sm;
@@ -358,6 +356,7 @@ __global__ void __launch_bounds__(kMaxThr, kMinB) alpha_mm_kernel(Geometry g, Mm
   }
   mm::cp_wait_all();
   __syncthreads();
+  dep_launch();
   mm::run<INV>(P, A, Z, Ta, x0, AlphaOut<INV>{rows, 1.0 / Pn, L, Pn});
 }
 
@@ -377,6 +376,7 @@ __global__ void __launch_bounds__(kMaxThr, kMinB) inv_beta_mm_kernel(Geometry g,
                                                                      const double2* __restrict__ half,
                                                                      double2* __restrict__ W, int T, long long wstride) {
   extern __shared__ __align__(16) double2 sm[];
+  dep_wait();
   __shared__ double2 x0[2 * kMaxT], b0s[kMaxT];
   double2* A = sm;
   double2* Z = sm + (size_t)T * P.ts;
@@ -402,6 +402,7 @@ __global__ void __launch_bounds__(kMaxThr, kMinB) inv_beta_mm_kernel(Geometry g,
   }
   mm::cp_wait_all();
   __syncthreads();
+  dep_launch();
   // z at +m' and -m'
   auto pair = [&](int t, int mp, double2& zp, double2& zn) {
     const double2 v0 = Z[t * P.ts + mp], v1 = Z[t * P.ts + L + mp];
@@ -517,13 +518,9 @@ int launch_mm_inv_gamma(const Geometry& g, const FftPlan& p, const double2* W, v
   const dim3 grid((g.na + (1 << sh) - 1) >> sh, row_hi - row_lo, count(bt));
   const SigIo io = sig_io(bt, f);
   if (g.real) {
-    if (int rc = set_smem(inv_gamma_real_mm_kernel, smem)) return rc;
-    inv_gamma_real_mm_kernel<<<grid, kGT, smem, s>>>(g, p.l1, W, io, sh, row_lo);
-  } else {
-    if (int rc = set_smem(inv_gamma_mm_kernel, smem)) return rc;
-    inv_gamma_mm_kernel<<<grid, kGT, smem, s>>>(g, p.l1, W, io, sh, row_lo);
+    return launch_after(inv_gamma_real_mm_kernel, grid, kGT, smem, s, g, p.l1, W, io, sh, row_lo);
   }
-  return launched();
+  return launch_after(inv_gamma_mm_kernel, grid, kGT, smem, s, g, p.l1, W, io, sh, row_lo);
 }
 
 int launch_mm_fwd_gamma(const Geometry& g, const FftPlan& p, const void* f, double2* W, cudaStream_t s, int row_lo,
@@ -534,32 +531,22 @@ int launch_mm_fwd_gamma(const Geometry& g, const FftPlan& p, const void* f, doub
   const dim3 grid((g.na + (1 << sh) - 1) >> sh, row_hi - row_lo, count(bt));
   const SigIo io = sig_io(bt, f);
   if (g.real) {
-    if (int rc = set_smem(fwd_gamma_real_mm_kernel, smem)) return rc;
-    fwd_gamma_real_mm_kernel<<<grid, kGT, smem, s>>>(g, p.l1, io, W, sh, row_lo);
-  } else {
-    if (int rc = set_smem(fwd_gamma_mm_kernel, smem)) return rc;
-    fwd_gamma_mm_kernel<<<grid, kGT, smem, s>>>(g, p.l1, io, W, sh, row_lo);
+    return launch_after(fwd_gamma_real_mm_kernel, grid, kGT, smem, s, g, p.l1, io, W, sh, row_lo);
   }
-  return launched();
+  return launch_after(fwd_gamma_mm_kernel, grid, kGT, smem, s, g, p.l1, io, W, sh, row_lo);
 }
 
 int launch_mm_alpha(const Geometry& g, const FftPlan& p, double2* W, bool inverse, cudaStream_t s, const Batch& bt) {
   const int nrows = g.nplanes * g.nb * count(bt);
   const Shape z = shape_for(p.mm, nrows, p.mm.kind == 1 ? 1 : 2);
-  auto go = [&](auto kernel) -> int {
-    if (int rc = set_smem(kernel, z.smem)) return rc;
-    kernel<<<(nrows + z.T - 1) / z.T, 32 * z.warps, z.smem, s>>>(g, z.P, W, z.T, nrows, bt.wstride);
-    return launched();
-  };
-  return inverse ? go(alpha_mm_kernel<true>) : go(alpha_mm_kernel<false>);
+  return launch_after(inverse ? alpha_mm_kernel<true> : alpha_mm_kernel<false>, dim3((nrows + z.T - 1) / z.T),
+                      32 * z.warps, z.smem, s, g, z.P, W, z.T, nrows, bt.wstride);
 }
 
 int launch_mm_inv_beta(const Geometry& g, const FftPlan& p, double2* W, cudaStream_t s, const Batch& bt) {
   const Shape z = shape_for(p.mm, g.L * g.nplanes * count(bt), 2);
   const dim3 grid((g.L + z.T - 1) / z.T, g.nplanes * count(bt));
-  if (int rc = set_smem(inv_beta_mm_kernel, z.smem)) return rc;
-  inv_beta_mm_kernel<<<grid, 32 * z.warps, z.smem, s>>>(g, z.P, p.half, W, z.T, bt.wstride);
-  return launched();
+  return launch_after(inv_beta_mm_kernel, grid, 32 * z.warps, z.smem, s, g, z.P, p.half, W, z.T, bt.wstride);
 }
 
 }  // namespace so3g
