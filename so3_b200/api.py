@@ -166,16 +166,19 @@ def is_elmn_non_zero(el, m, n, p) -> bool:
 
 
 # ------------------------------------------------------------ transforms (host)
+# Outputs that the call writes whole are left uninitialised: clearing 8 MB that
+# the copy back overwrites costs as much again as the copy (0.24 ms of zeroing,
+# then the pages are faulted in by the copy; 1.08 against 0.44 ms together).
 def inverse(flmn: np.ndarray, p) -> np.ndarray:
     """bindings.pyx:315-336: flmn -> samples (complex, or real when p.reality)."""
     q = _checked(p)
     lib = _lib.load()
     flmn = np.ascontiguousarray(flmn, dtype=np.complex128)
     if q.reality:
-        f = np.zeros(f_size(q), np.float64)
+        f = np.empty(f_size(q), np.float64)
         lib.so3_core_inverse_via_ssht_real(_ptr(f), _ptr(flmn), ctypes.byref(q))
     else:
-        f = np.zeros(f_size(q), np.complex128)
+        f = np.empty(f_size(q), np.complex128)
         lib.so3_core_inverse_via_ssht(_ptr(f), _ptr(flmn), ctypes.byref(q))
     _lib.check("inverse")
     return f
@@ -185,7 +188,9 @@ def forward(f: np.ndarray, p) -> np.ndarray:
     """bindings.pyx:338-357: samples -> flmn; a real array needs p.reality."""
     q = _checked(p)
     lib = _lib.load()
-    flmn = np.zeros(flmn_size(q), np.complex128)
+    # every coefficient is written unless the n-mode skips planes
+    alloc = np.empty if q.n_mode in (SO3_N_MODE_ALL, SO3_N_MODE_L) else np.zeros
+    flmn = alloc(flmn_size(q), np.complex128)
     if np.isrealobj(f):
         if not q.reality:
             raise ValueError("f has a real data type but reality flag not set")
@@ -203,7 +208,7 @@ def adjoint_inverse(f: np.ndarray, p) -> np.ndarray:
     (so3_adjoint_inverse_direct, reference src/c/so3_adjoint.c:34; with
     p.reality, so3_adjoint_inverse_direct_real, :939, on real samples)."""
     q = _checked(p)
-    flmn = np.zeros(flmn_size(q), np.complex128)
+    flmn = np.empty(flmn_size(q), np.complex128)
     lib = _lib.load()
     if q.reality:
         f = np.ascontiguousarray(f, dtype=np.float64)
@@ -223,10 +228,10 @@ def adjoint_forward(flmn: np.ndarray, p) -> np.ndarray:
     lib = _lib.load()
     flmn = np.ascontiguousarray(flmn, dtype=np.complex128)
     if q.reality:
-        f = np.zeros(f_size(q), np.float64)
+        f = np.empty(f_size(q), np.float64)
         lib.so3_adjoint_forward_direct_real(_ptr(f), _ptr(flmn), ctypes.byref(q))
     else:
-        f = np.zeros(f_size(q), np.complex128)
+        f = np.empty(f_size(q), np.complex128)
         lib.so3_adjoint_forward_direct(_ptr(f), _ptr(flmn), ctypes.byref(q))
     _lib.check("adjoint_forward")
     return f
