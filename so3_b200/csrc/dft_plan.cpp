@@ -222,7 +222,11 @@ int build_mm_plan(int n, FftPlan* F, double2** mem, int** imem, size_t* bytes) {
       for (const cld& x : dft_host(v, a, b)) host.push_back(to_d2(x / (long double)P.m));
     }
   }
-  if (host.empty()) return kOk;
+  if (host.empty()) {  // length 1: no entries to multiply
+    F->mm = P;
+    F->l1 = one;
+    return kOk;
+  }
   *bytes = host.size() * sizeof(double2) + perm.size() * sizeof(int);
   cudaError_t e = cudaMalloc(mem, host.size() * sizeof(double2));
   if (e == cudaSuccess && !perm.empty()) e = cudaMalloc(imem, perm.size() * sizeof(int));

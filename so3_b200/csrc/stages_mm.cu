@@ -2,9 +2,9 @@
 // same stages as stages.cu, any length the planner covers.
 //
 // Measured against the scalar engines of stages.cu (us, one transform):
-//   gamma    L=512 N=64 (127)    769 -> 744 inverse, 800 -> 705 forward
-//            L=512 N=16 (31)    1125 -> 135, 1182 -> 127
-//            L=256 N=32 real     156 -> 59,   179 -> 92
+//   gamma    L=512 N=64 (127)    769 -> 697 inverse, 800 -> 721 forward
+//            L=512 N=16 (31)    1125 -> 113, 1182 -> 107
+//            L=256 N=32 real     156 -> 44,   179 -> 44
 //   alpha    L=128 N=16 (255)     43 -> 23;  L=256 N=16 (511) 339 -> 78
 //            L=300 N=16 (599)    737 -> 190; L=1024 N=8 (2047) 3774 -> 525
 //   inv beta L=256 N=16 320 -> 103; L=300 N=16 791 -> 227; L=1024 N=8 3635 -> 758
@@ -77,7 +77,7 @@ struct FwdGammaOut {
 
 // Complex inverse: circle entry r holds plane n = r (r < N) or r - ng; the
 // 2N-point circle of a steerable signal has no plane n = N and keeps N samples.
-__global__ void __launch_bounds__(kGT, 4) inv_gamma_mm_kernel(Geometry g, MmLevel lv, const double2* __restrict__ W,
+__global__ void __launch_bounds__(kGT, 6) inv_gamma_mm_kernel(Geometry g, MmLevel lv, const double2* __restrict__ W,
                                                          const __grid_constant__ SigIo io, int tash, int row0) {
   extern __shared__ __align__(16) double2 sm[];
   dep_wait();
@@ -99,12 +99,12 @@ __global__ void __launch_bounds__(kGT, 4) inv_gamma_mm_kernel(Geometry g, MmLeve
   dep_launch();
   const long long plane_sz = (long long)g.nb * g.na;
   double2* dst = f + (long long)row * g.na + a0;
-  mm::level<4, true>(sm, rp, lv, nc, [](int j) { return j; }, InvGammaOut{dst, plane_sz, g.nf});
+  mm::level<2, true>(sm, rp, lv, nc, [](int j) { return j; }, InvGammaOut{dst, plane_sz, g.nf});
 }
 
 // Complex forward; steerable: samples N..2N-1 of the circle are zero and only
 // n = N-1 (mod 2) is analysed (so3_core.c:309-328).
-__global__ void __launch_bounds__(kGT, 4) fwd_gamma_mm_kernel(Geometry g, MmLevel lv, const __grid_constant__ SigIo io,
+__global__ void __launch_bounds__(kGT, 6) fwd_gamma_mm_kernel(Geometry g, MmLevel lv, const __grid_constant__ SigIo io,
                                                          double2* __restrict__ W, int tash, int row0) {
   extern __shared__ __align__(16) double2 sm[];
   dep_wait();
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(kGT, 4) fwd_gamma_mm_kernel(Geometry g, MmLeve
   dep_launch();
   const double scale = 2.0 * 3.141592653589793238462643383279502884 / g.nf;
   double2* dst = W + (long long)row * g.RS + a0;
-  mm::level<4, false>(sm, rp, lv, nc, [](int j) { return j; },
+  mm::level<2, false>(sm, rp, lv, nc, [](int j) { return j; },
             FwdGammaOut{dst, g.PS, scale, g.N, ng, g.plane0, g.steer});
 }
 
@@ -184,7 +184,7 @@ __device__ __forceinline__ void c2r_task(const double2* __restrict__ src, int rp
   }
 }
 
-__global__ void __launch_bounds__(kGT, 4) inv_gamma_real_mm_kernel(Geometry g, MmLevel lv,
+__global__ void __launch_bounds__(kGT, 6) inv_gamma_real_mm_kernel(Geometry g, MmLevel lv,
                                                               const double2* __restrict__ W, const __grid_constant__ SigIo io,
                                                               int tash, int row0) {
   extern __shared__ __align__(16) double2 sm[];
@@ -203,15 +203,13 @@ __global__ void __launch_bounds__(kGT, 4) inv_gamma_real_mm_kernel(Geometry g, M
   dep_launch();
   const long long plane_sz = (long long)g.nb * g.na;
   double* dst = f + (long long)row * g.na + a0;
-  const int ng = lv.QG, tasks = (nc + 15) / 16 * ng;
+  const int ng = (lv.QT + 1) / 2, tasks = (nc + 15) / 16 * ng;
   for (int w = threadIdx.x >> 5; w < tasks; w += kGT / 32) {
-    const int qt0 = (w % ng) * lv.MT, j0 = (w / ng) * 16;
-    switch (min(lv.MT, lv.QT - qt0)) {
-      case 1: c2r_task<1>(sm, rp, lv, qt0, j0, nc, dst, plane_sz); break;
-      case 2: c2r_task<2>(sm, rp, lv, qt0, j0, nc, dst, plane_sz); break;
-      case 3: c2r_task<3>(sm, rp, lv, qt0, j0, nc, dst, plane_sz); break;
-      default: c2r_task<4>(sm, rp, lv, qt0, j0, nc, dst, plane_sz); break;
-    }
+    const int qt0 = (w % ng) * 2, j0 = (w / ng) * 16;
+    if (lv.QT - qt0 == 1)
+      c2r_task<1>(sm, rp, lv, qt0, j0, nc, dst, plane_sz);
+    else
+      c2r_task<2>(sm, rp, lv, qt0, j0, nc, dst, plane_sz);
   }
 }
 
@@ -271,7 +269,7 @@ __device__ __forceinline__ void r2c_task(const double* __restrict__ src, int rp,
 
 // Sample rows of TA + 4 doubles (4 mod 16): 4 rows x 4 columns per half warp
 // in distinct banks.
-__global__ void __launch_bounds__(kGT, 4) fwd_gamma_real_mm_kernel(Geometry g, MmLevel lv,
+__global__ void __launch_bounds__(kGT, 6) fwd_gamma_real_mm_kernel(Geometry g, MmLevel lv,
                                                               const __grid_constant__ SigIo io, double2* __restrict__ W,
                                                               int tash, int row0) {
   extern __shared__ __align__(16) double smd[];
@@ -284,21 +282,20 @@ __global__ void __launch_bounds__(kGT, 4) fwd_gamma_real_mm_kernel(Geometry g, M
   const double* src = f + (long long)row * g.na + a0;
   for (int i = threadIdx.x; i < g.ng << tash; i += kGT) {
     const int r = i >> tash, c = i & (TA - 1);
-    if (c < nc) smd[r * rp + c] = __ldg(src + (long long)r * plane_sz + c);
+    if (c < nc) mm::cp8(smd + r * rp + c, src + (long long)r * plane_sz + c);
   }
+  mm::cp_wait_all();
   __syncthreads();
   dep_launch();
   const double scale = 2.0 * 3.141592653589793238462643383279502884 / g.nf;
   double2* dst = W + (long long)row * g.RS + a0;
-  const int ng = lv.QG, tasks = (nc + 15) / 16 * ng;
+  const int ng = (lv.QT + 1) / 2, tasks = (nc + 15) / 16 * ng;
   for (int w = threadIdx.x >> 5; w < tasks; w += kGT / 32) {
-    const int qt0 = (w % ng) * lv.MT, j0 = (w / ng) * 16;
-    switch (min(lv.MT, lv.QT - qt0)) {
-      case 1: r2c_task<1>(smd, rp, lv, qt0, j0, nc, dst, g.PS, scale); break;
-      case 2: r2c_task<2>(smd, rp, lv, qt0, j0, nc, dst, g.PS, scale); break;
-      case 3: r2c_task<3>(smd, rp, lv, qt0, j0, nc, dst, g.PS, scale); break;
-      default: r2c_task<4>(smd, rp, lv, qt0, j0, nc, dst, g.PS, scale); break;
-    }
+    const int qt0 = (w % ng) * 2, j0 = (w / ng) * 16;
+    if (lv.QT - qt0 == 1)
+      r2c_task<1>(smd, rp, lv, qt0, j0, nc, dst, g.PS, scale);
+    else
+      r2c_task<2>(smd, rp, lv, qt0, j0, nc, dst, g.PS, scale);
   }
 }
 
@@ -494,11 +491,21 @@ Shape shape_for(const MmPlan& P0, int nseq, int bufs) {
   return z;
 }
 
-// alpha samples per CTA of a gamma kernel: four warp tasks where the row
-// tiles allow, 64 at most
-int gamma_shift(const MmLevel& lv, int cols) {
-  int sh = 4;
-  while (sh < 6 && (1 << (sh + 1)) * lv.QG <= 4 * 8 * (cols / 8)) sh++;
+// Gamma kernels: two row tiles per warp task (80 registers, 24 warps per SM;
+// four tiles at 128 registers and 16 warps: 766 against 697 us at L = 512, N = 64,
+// 277 / 241 at N = 32, 255 / 177 at L = 1024, N = 8).
+MmLevel gamma_level(const FftPlan& p) {
+  MmLevel lv = p.l1;
+  lv.MT = std::min(2, lv.QT);
+  lv.QG = (lv.QT + lv.MT - 1) / lv.MT;
+  return lv;
+}
+// log2 of the alpha samples per CTA: the planes of six CTAs fit in shared memory
+// and a CTA has four tasks or more (L = 1024, N = 2: 16 samples 224 us, 256: 78; N = 8:
+// 16: 292, 64: 177; L = 512, N = 32: 16: 241, 32: 253), fewer where the device would not fill.
+int gamma_shift(int ng, int na, int rows) {
+  int sh = ng <= 7 ? 8 : ng <= 11 ? 7 : ng <= 23 ? 6 : ng <= 47 ? 5 : 4;
+  while (sh > 4 && ((na + (1 << sh) - 1) >> sh) * rows < 296) sh--;
   return sh;
 }
 
@@ -511,29 +518,31 @@ bool mm_ok(const FftPlan& p) { return p.mm.n == p.n && seq_smem(p.mm, 1, 2) <= k
 
 int launch_mm_inv_gamma(const Geometry& g, const FftPlan& p, const double2* W, void* f, cudaStream_t s, int row_lo,
                         int row_hi, const Batch& bt) {
-  int sh = gamma_shift(p.l1, g.real ? 16 : 8);
+  int sh = gamma_shift(g.ng, g.na, (row_hi - row_lo) * count(bt));
+  const MmLevel lv = gamma_level(p);
   const int rows = g.real ? g.nplanes : g.ng;
   while (sh > 4 && (size_t)rows * ((1 << sh) + 2) * sizeof(double2) > kSmemMax / 4) sh--;
   const size_t smem = (size_t)rows * ((1 << sh) + 2) * sizeof(double2);
   const dim3 grid((g.na + (1 << sh) - 1) >> sh, row_hi - row_lo, count(bt));
   const SigIo io = sig_io(bt, f);
   if (g.real) {
-    return launch_after(inv_gamma_real_mm_kernel, grid, kGT, smem, s, g, p.l1, W, io, sh, row_lo);
+    return launch_after(inv_gamma_real_mm_kernel, grid, kGT, smem, s, g, lv, W, io, sh, row_lo);
   }
-  return launch_after(inv_gamma_mm_kernel, grid, kGT, smem, s, g, p.l1, W, io, sh, row_lo);
+  return launch_after(inv_gamma_mm_kernel, grid, kGT, smem, s, g, lv, W, io, sh, row_lo);
 }
 
 int launch_mm_fwd_gamma(const Geometry& g, const FftPlan& p, const void* f, double2* W, cudaStream_t s, int row_lo,
                         int row_hi, const Batch& bt) {
-  int sh = gamma_shift(p.l1, g.real ? 16 : 8);
+  int sh = gamma_shift(g.ng, g.na, (row_hi - row_lo) * count(bt));
+  const MmLevel lv = gamma_level(p);
   while (sh > 4 && (size_t)g.ng * ((1 << sh) + 4) * (g.real ? 8 : 16) > kSmemMax / 4) sh--;
   const size_t smem = (size_t)g.ng * (g.real ? ((1 << sh) + 4) * 8 : ((1 << sh) + 2) * 16);
   const dim3 grid((g.na + (1 << sh) - 1) >> sh, row_hi - row_lo, count(bt));
   const SigIo io = sig_io(bt, f);
   if (g.real) {
-    return launch_after(fwd_gamma_real_mm_kernel, grid, kGT, smem, s, g, p.l1, io, W, sh, row_lo);
+    return launch_after(fwd_gamma_real_mm_kernel, grid, kGT, smem, s, g, lv, io, W, sh, row_lo);
   }
-  return launch_after(fwd_gamma_mm_kernel, grid, kGT, smem, s, g, p.l1, io, W, sh, row_lo);
+  return launch_after(fwd_gamma_mm_kernel, grid, kGT, smem, s, g, lv, io, W, sh, row_lo);
 }
 
 int launch_mm_alpha(const Geometry& g, const FftPlan& p, double2* W, bool inverse, cudaStream_t s, const Batch& bt) {
