@@ -371,26 +371,35 @@ __global__ void __launch_bounds__(kThreads, 1) forward_contract_kernel(FwdArgs a
 // (-1)^(reduction index) of combinations with one negative index is flipped in
 // the column operand, the one of the row index in the result.
 //
-// CTA tile: 32 rows x 8 mu x 2 nu, two CTAs per SM; 8 reduction entries (two
-// MMA steps) per stage of a three-stage ring.  Eight warps multiply (16 rows x 4
-// mu x 1 nu each: 14 fragment reads per 8 MMAs), a ninth copies and runs ahead:
+// CTA tile: 32 rows x 8 mu x 2 nu; 8 reduction entries (two MMA steps) per stage
+// of a ring.  Eight warps multiply (16 rows x 4 mu x 1 nu each: 14 fragment reads
+// per 8 MMAs), one (forward) or two (inverse, a nu each) more copy and run ahead:
 // the Delta blocks as they are stored (dl_index) by bulk copies, 512 bytes per mu
 // and row tile, the coefficients from the caller's layout or the spectra from the
 // column-major scratch by cp.async, all counted on mbarriers.  Row tiles that a
 // degree does not reach (m' > l) are neither copied nor multiplied.
 //
-// Bound by shared-memory reads (3.5 of 4 wavefronts per MMA) and by the
-// multiplications that form W on the same pipe.  Measured at L = 512, N = 64
-// (ms, inverse / forward): 2.60 / 2.44, against 4.97 / 5.92 for staging by all
-// warps with 8-byte copies from row-major planes; 3.09 / 2.89 without the copying
-// warp (a barrier per chunk aligned the warps' bursts).  64 rows x 4 nu (one CTA
-// of 16 warps) gives 2.57 / 2.42 there but 39 / 37 us against 23 / 30 at L = 128,
-// N = 16; m16n8k8 MMAs change nothing.
+// Bound by the latency of the product warps' chains (wait, fragment read, product,
+// MMA): MMAs hold the FP64 pipe 49 % of the time and the multiplications that form W
+// 10 %, no other unit above 50 %.  Hence as many warps as fit: forward three CTAs
+// per SM at 72 registers and two ring slots, inverse (whose copies scatter and whose
+// weight takes registers) two at 96 and three slots; forward as inverse 2.48 ms at
+// L = 512, N = 64, inverse as forward 2.77.  Measured at L = 512, N = 64 (ms, inverse
+// / forward): 2.51 / 2.30, against 2.61 / 2.48 with one copying warp and two CTAs in
+// both; 4.97 / 5.92 for staging by all warps with 8-byte copies from row-major
+// planes; 3.09 / 2.89 without copying warps (a barrier per chunk aligned the warps'
+// bursts).  64 rows x 4 nu (one CTA of 16 warps) gives 2.57 / 2.42 there but 39 / 37
+// us against 23 / 30 at L = 128, N = 16.  Two signals per CTA share the Delta reads:
+// forward 2.02 ms a signal, inverse 2.51, and 12 % slower below L = 256.  X by
+// 128-byte bulk copies: 6.4 / 6.7 ms (64 per stage are too many).  m16n8k8 MMAs
+// change nothing.
 namespace {
 constexpr int kCRt = 4, kCMu = 8, kCNu = 2;  // row tiles, mu, nu of a CTA
-constexpr int kCMt = 2, kCNw = 1;            // row tiles and nu of a warp (4 mu)
-constexpr int kCStages = 3;
-constexpr int kCThreads = 32 * (kCRt / kCMt) * 2 * (kCNu / kCNw) + 32;
+constexpr int kCMt = 2;                      // row tiles of a warp (4 mu, 1 nu)
+constexpr int contract_slots(int ctas) { return ctas == 3 ? 2 : 3; }  // of the ring, by CTAs per SM
+constexpr int kCCopy[2] = {2, 1};    // copying warps
+constexpr int kCWarps = (kCRt / kCMt) * 2 * kCNu;  // product warps
+constexpr int contract_threads(bool fwd) { return 32 * (kCWarps + kCCopy[fwd]); }
 constexpr int kXB = 33;  // slots of an X block of one (mu, nu): 8 entries x 4 combinations, and one of padding
 
 struct ContractArgs {
@@ -415,10 +424,10 @@ __device__ __forceinline__ void cp16_to(uint32_t dst, const void* src, bool vali
 constexpr int kCStage = kCRt * kCMu * 64 + kCRt * kCNu * 64 + 2 * kCMu * kCNu * kXB;  // doubles
 }  // namespace
 
-template <bool FWD>
-__global__ void __launch_bounds__(kCThreads, 2) contract_mma_kernel(const __grid_constant__ ContractArgs a) {
-  constexpr int RT = kCRt, NU = kCNu, MT = kCMt, NW = kCNw, ST = kCStages;
-  constexpr int WR = RT / MT, NWARP = kCThreads / 32 - 1;  // product warps; one more copies
+template <bool FWD, int CTAS>
+__global__ void __launch_bounds__(contract_threads(FWD), CTAS) contract_mma_kernel(const __grid_constant__ ContractArgs a) {
+  constexpr int RT = kCRt, NU = kCNu, MT = kCMt, ST = contract_slots(CTAS);
+  constexpr int WR = RT / MT, NWARP = kCWarps, CW = kCCopy[FWD];
   constexpr int BSZ = RT * kCMu * 64, ASZ = RT * NU * 64, STAGE = kCStage;
   extern __shared__ __align__(16) double smc[];
   __shared__ long long bsel[NU][2];
@@ -427,7 +436,6 @@ __global__ void __launch_bounds__(kCThreads, 2) contract_mma_kernel(const __grid
   const int wr = warp % WR, wm = warp / WR % 2, wn = warp / (2 * WR);
   const int nu0 = a.nu0 + blockIdx.x * NU, rt0 = blockIdx.y * RT;
   const int mts = (a.L + kCMu - 1) / kCMu, sig = blockIdx.z / mts, mu0 = (blockIdx.z - sig * mts) * kCMu;
-  double2* const flmn = static_cast<double2*>(a.flmn[sig]);
   double2* const W = a.W + sig * a.wstride;
   const int L = a.L, LC = (L + 7) >> 3;
   unsigned act = 0;  // bit j: nu0 + j is computed by this launch
@@ -456,14 +464,14 @@ __global__ void __launch_bounds__(kCThreads, 2) contract_mma_kernel(const __grid
   const uint32_t full0 = tc::smem_u32(full), empty0 = tc::smem_u32(empty);
   if (tid == 0) {
     for (int st = 0; st < ST; st++) {
-      tc::mbar_init(full0 + 8 * st, 33);  // the copying lanes' loads of X and the expected bytes
+      tc::mbar_init(full0 + 8 * st, 32 * CW + 1);  // the copying lanes' loads of X and the expected bytes
       tc::mbar_init(empty0 + 8 * st, NWARP);
     }
     tc::mbar_fence_init();
   }
   __syncthreads();
 
-  if (warp == NWARP) {
+  if (warp >= NWARP) {
     // ------------------------------------------------ copies
     // The Delta blocks of a row tile are one run per operand (8 mu, NU nu): 2 RT
     // lanes bring them with one bulk copy each.  X by 16-byte copies, forward
@@ -477,18 +485,21 @@ __global__ void __launch_bounds__(kCThreads, 2) contract_mma_kernel(const __grid
     const long long toff = (tmu ? mu0 : nu0) * 64;
     // forward: lane = (entry, combination); inverse: lane = (mu, entry & 3)
     const int xe = FWD ? lane & 7 : lane >> 3, xm = lane & 7, xc = lane >> 3;
-    const double2* px[FWD ? NU : 4 * NU];
-    int xlo[NU];
+    constexpr int NJ = NU / CW;  // nu of a copying warp
+    const int j0 = (warp - NWARP) * NJ;
+    const double2* const flmn = static_cast<const double2*>(a.flmn[sig]);
+    const double2* px[FWD ? NJ : 1];
+    int poff[FWD ? 1 : 4 * NJ], xlo[NJ];  // coefficient counts fit an int (the C interface)
 #pragma unroll
-    for (int j = 0; j < NU; j++) {
-      const int nu = nu0 + j, mu = mu0 + xm;
+    for (int j = 0; j < NJ; j++) {
+      const int nu = nu0 + j0 + j, mu = mu0 + xm;
       if (FWD) {
         px[j] = W + (long long)(a.plane0 + ((xc & 2) ? -nu : nu)) * a.QS + (long long)(L - 1 + ((xc & 1) ? -mu0 : mu0)) * a.CS;
-        xlo[j] = xc < a.nsign && (act >> j & 1) ? 0 : L;
+        xlo[j] = xc < a.nsign && (act >> (j0 + j) & 1) ? 0 : L;
       } else {
 #pragma unroll
-        for (int c = 0; c < 4; c++) px[4 * j + c] = flmn + bsel[j][c >> 1] + ((c & 1) ? -mu : mu);
-        xlo[j] = mu < L && (act >> j & 1) ? max(max(a.L0, mu), nu) : L;
+        for (int c = 0; c < 4; c++) poff[4 * j + c] = (int)bsel[j0 + j][c >> 1] + ((c & 1) ? -mu : mu);
+        xlo[j] = mu < L && (act >> (j0 + j) & 1) ? max(max(a.L0, mu), nu) : L;
       }
     }
     const long long cstep = (xc & 1) ? -a.CS : a.CS;
@@ -505,23 +516,23 @@ __global__ void __launch_bounds__(kCThreads, 2) contract_mma_kernel(const __grid
                      (tmu ? kCMu : NU) * 512, full0 + 8 * st);
     };
     // the first Delta blocks come while the kernel before finishes; X is its output
-    if (ch0 < ch1) blocks(ch0, 0);
+    if (j0 == 0 && ch0 < ch1) blocks(ch0, 0);
     dep_wait();
     int st = 0;
     uint32_t phase = 1;  // of the ring slot's previous use
     for (int ch = ch0; ch < ch1; ch++) {
       if (ch - ch0 >= ST) tc::mbar_wait(empty0 + 8 * st, phase, &g_contract_error, 4);
-      if (ch > ch0) blocks(ch, st);
+      if (j0 == 0 && ch > ch0) blocks(ch, st);
       const uint32_t at = (uint32_t)(st * STAGE * 8), bar = full0 + 8 * st;
 #pragma unroll
-      for (int j = 0; j < NU; j++) {
+      for (int j = 0; j < NJ; j++) {
         if (FWD) {
           const int e = 8 * ch + xe;
           const double2* src = px[j] + e;
 #pragma unroll
           for (int m = 0; m < kCMu; m++, src += cstep) {
             const bool ok = e >= xlo[j] && e < L && mu0 + m < L;
-            cp16_to(xs0 + at + 16 * ((j * kCMu + m) * kXB + xc * 8 + (xe ^ (4 * (xc & 1)))), ok ? src : W, ok);
+            cp16_to(xs0 + at + 16 * (((j0 + j) * kCMu + m) * kXB + xc * 8 + (xe ^ (4 * (xc & 1)))), ok ? src : W, ok);
           }
         } else {
 #pragma unroll
@@ -531,8 +542,8 @@ __global__ void __launch_bounds__(kCThreads, 2) contract_mma_kernel(const __grid
 #pragma unroll
             for (int c = 0; c < 4; c++) {
               const bool ok = in && c < a.nsign;
-              cp16_to(xs0 + at + 16 * ((j * kCMu + xm) * kXB + 4 * (4 * h + xe) + (c ^ (xe & 2))), ok ? px[4 * j + c] + off : flmn,
-                      ok);
+              cp16_to(xs0 + at + 16 * (((j0 + j) * kCMu + xm) * kXB + 4 * (4 * h + xe) + (c ^ (xe & 2))),
+                      ok ? flmn + (poff[4 * j + c] + off) : flmn, ok);
             }
           }
         }
@@ -547,13 +558,11 @@ __global__ void __launch_bounds__(kCThreads, 2) contract_mma_kernel(const __grid
 
   // -------------------------------------------------- products
   dep_wait();
-  double acc[MT][4][NW][2];
+  double acc[MT][4][2];
 #pragma unroll
   for (int i = 0; i < MT; i++)
 #pragma unroll
-    for (int m = 0; m < 4; m++)
-#pragma unroll
-      for (int n = 0; n < NW; n++) acc[i][m][n][0] = acc[i][m][n][1] = 0.0;
+    for (int m = 0; m < 4; m++) acc[i][m][0] = acc[i][m][1] = 0.0;
 
   const int s = g >> 1, part = g & 1;
   // real signals with N = 1: the -m coefficient is (-1)^m conj of the +m one
@@ -573,41 +582,30 @@ __global__ void __launch_bounds__(kCThreads, 2) contract_mma_kernel(const __grid
   auto products = [&](int ch, int st, auto all) {
     constexpr bool ALL = decltype(all)::value;
     const double* Bs = smc + st * STAGE + (wr * MT * kCMu + wm * 4) * 64;
-    const double* As = smc + st * STAGE + BSZ + (wr * MT * NU + wn * NW) * 64;
-    const double* Xs = smc + st * STAGE + BSZ + ASZ + 2 * (wn * NW * kCMu + wm * 4) * kXB + x0;
+    const double* As = smc + st * STAGE + BSZ + (wr * MT * NU + wn) * 64;
+    const double* Xs = smc + st * STAGE + BSZ + ASZ + 2 * (wn * kCMu + wm * 4) * kXB + x0;
 #pragma unroll
     for (int ks = 0; ks < 2; ks++) {
       // entry 4 + q: forward the lower half block (its row pairs swap alike), inverse the other l half
       const int slot = FWD ? slot0 + 32 * ks : slot0 ^ (4 * ks);
       const int dx = FWD ? 8 * ks * (1 - 2 * (s & 1)) : 32 * ks;
       const double w = fma(l21 + 8.0 * ks, wmul, wadd);
-      double an[MT][NW];
+      double an[MT];
 #pragma unroll
-      for (int i = 0; i < MT; i++)
-#pragma unroll
-        for (int n = 0; n < NW; n++) {
-          an[i][n] = As[(i * NU + n) * 64 + slot];
-          if (!FWD) an[i][n] *= w;
-        }
+      for (int i = 0; i < MT; i++) {
+        an[i] = As[i * NU * 64 + slot];
+        if (!FWD) an[i] *= w;
+      }
 #pragma unroll
       for (int m = 0; m < 4; m++) {
-        double x[NW], wp[MT][NW];
+        double x = Xs[2 * m * kXB + dx], wp[MT];
+        x = __hiloint2double(__double2hiint(x) ^ ((m & 1) ? flip1 : flip0), __double2loint(x));
 #pragma unroll
-        for (int n = 0; n < NW; n++) {
-          const double v = Xs[2 * (n * kCMu + m) * kXB + dx];
-          x[n] = __hiloint2double(__double2hiint(v) ^ ((m & 1) ? flip1 : flip0), __double2loint(v));
-        }
-#pragma unroll
-        for (int i = 0; i < MT; i++) {
-          const double bm = Bs[(i * kCMu + m) * 64 + slot];
-#pragma unroll
-          for (int n = 0; n < NW; n++) wp[i][n] = bm * an[i][n];
-        }
+        for (int i = 0; i < MT; i++) wp[i] = Bs[(i * kCMu + m) * 64 + slot] * an[i];
 #pragma unroll
         for (int i = 0; i < MT; i++) {
           if (!ALL && (FWD ? ch > rt_lo + i || rt_lo + i >= LC : rt_lo + i > ch)) continue;  // m' > l throughout
-#pragma unroll
-          for (int n = 0; n < NW; n++) mm::dmma(acc[i][m][n], wp[i][n], x[n]);
+          mm::dmma(acc[i][m], wp[i], x);
         }
       }
     }
@@ -636,30 +634,27 @@ __global__ void __launch_bounds__(kCThreads, 2) contract_mma_kernel(const __grid
     const int row = 8 * (rt0 + wr * MT + i) + g;
     if (row >= L) break;
     const double odd_row = (row & 1) ? -1.0 : 1.0;
+    const int nu = nu0 + wn;
+    if (nu < a.nu_lo || nu >= a.nu_hi || (ns < 0 && nu == 0)) break;
+    const bool on = act >> wn & 1;
+    if (FWD && (!on || (a.compact && row < nu))) continue;  // untouched, or not stored
 #pragma unroll
-    for (int n = 0; n < NW; n++) {
-      const int nu = nu0 + wn * NW + n;
-      if (nu < a.nu_lo || nu >= a.nu_hi || (ns < 0 && nu == 0)) continue;
-      const bool on = act >> (wn * NW + n) & 1;
-      if (FWD && (!on || (a.compact && row < nu))) continue;  // untouched, or not stored
-#pragma unroll
-      for (int m = 0; m < 4; m++) {
-        const int mu = mu0 + wm * 4 + m;
-        if (mu >= L || (ms < 0 && mu == 0) || (FWD && mu > row)) continue;
-        double2 v = make_double2(acc[i][m][n][0], acc[i][m][n][1]);
-        if (ms * ns < 0) v = sc(v, odd_row);
-        if (FWD) {
-          if (row >= max(a.L0, nu)) {
-            v = ipow_mul(v, ms * mu - ns * nu + 4 * L);
-            if (a.lw > 0.0) v = sc(v, a.lw * (2.0 * row + 1.0));
-          } else {
-            v = make_double2(0.0, 0.0);
-          }
-          flmn[bsel[wn * NW + n][q >> 1] + (long long)row * row + row + ms * mu] = v;
+    for (int m = 0; m < 4; m++) {
+      const int mu = mu0 + wm * 4 + m;
+      if (mu >= L || (ms < 0 && mu == 0) || (FWD && mu > row)) continue;
+      double2 v = make_double2(acc[i][m][0], acc[i][m][1]);
+      if (ms * ns < 0) v = sc(v, odd_row);
+      if (FWD) {
+        if (row >= max(a.L0, nu)) {
+          v = ipow_mul(v, ms * mu - ns * nu + 4 * L);
+          if (a.lw > 0.0) v = sc(v, a.lw * (2.0 * row + 1.0));
         } else {
-          v = ipow_mul(v, ns * nu - ms * mu + 4 * L);
-          W[(long long)(a.plane0 + ns * nu) * a.QS + (long long)(ms * mu + L - 1) * a.CS + row] = v;
+          v = make_double2(0.0, 0.0);
         }
+        static_cast<double2*>(a.flmn[sig])[bsel[wn][q >> 1] + (long long)row * row + row + ms * mu] = v;
+      } else {
+        v = ipow_mul(v, ns * nu - ms * mu + 4 * L);
+        W[(long long)(a.plane0 + ns * nu) * a.QS + (long long)(ms * mu + L - 1) * a.CS + row] = v;
       }
     }
   }
@@ -671,10 +666,14 @@ int contract(ContractArgs a, const void* flmn, const Batch& bt, cudaStream_t s) 
   for (int b = 0; b < bt.n; b++) a.flmn[b] = bt.io[b];
   if (!bt.n) a.flmn[0] = const_cast<void*>(flmn);
   a.wstride = bt.wstride;
-  constexpr size_t smem = kCStages * kCStage * sizeof(double);
   a.nu0 = a.nu_lo / kCNu * kCNu;  // tiles stay aligned: a block of 8 degrees holds whole groups of nu
   const dim3 grid((a.nu_hi - a.nu0 + kCNu - 1) / kCNu, (a.L + 8 * kCRt - 1) / (8 * kCRt), (a.L + kCMu - 1) / kCMu * (bt.n ? bt.n : 1));
-  return launch_after(contract_mma_kernel<FWD>, grid, kCThreads, smem, s, a);
+  // Forward, three CTAs per SM where the grid fills them.  A grid that two per SM
+  // hold anyway keeps the registers: 9.4 against 10.5 us at L = 16, N = 4 and 10.7
+  // against 11.4 us at L = 32, N = 8 (8 signals each).
+  const bool three = FWD && (long long)grid.x * grid.y * grid.z > 2 * 148;
+  auto* const kernel = three ? contract_mma_kernel<FWD, FWD ? 3 : 2> : contract_mma_kernel<FWD, 2>;
+  return launch_after(kernel, grid, contract_threads(FWD), contract_slots(three ? 3 : 2) * kCStage * sizeof(double), s, a);
 }
 }  // namespace
 
