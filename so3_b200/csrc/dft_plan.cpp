@@ -189,6 +189,9 @@ int build_mm_plan(int n, FftPlan* F, double2** mem, int** imem, size_t* bytes) {
       P.lda = pitch(a);
       P.ldb = pitch(b);
       P.ts = a * P.ldb > b * P.lda ? a * P.ldb : b * P.lda;
+      // a sequence buffer also holds the n outputs, and the two columns (n + 1 entries) of
+      // an inverse beta pair; a Rader plan transforms only n - 1
+      if (P.ts < n + 1) P.ts = n + 1;
       at_a = host.size();
       level_table(P.la, &host);
       at_b = host.size();
@@ -235,9 +238,9 @@ int build_mm_plan(int n, FftPlan* F, double2** mem, int** imem, size_t* bytes) {
     *mem = nullptr;
     return fail(kOutOfMemory, "DFT table allocation failed");
   }
-  e = cudaMemcpy(*mem, host.data(), host.size() * sizeof(double2), cudaMemcpyHostToDevice);
+  e = upload(*mem, host.data(), host.size() * sizeof(double2));
   if (e == cudaSuccess && !perm.empty())
-    e = cudaMemcpy(*imem, perm.data(), perm.size() * sizeof(int), cudaMemcpyHostToDevice);
+    e = upload(*imem, perm.data(), perm.size() * sizeof(int));
   if (e != cudaSuccess) {
     cudaFree(*mem);
     cudaFree(*imem);
