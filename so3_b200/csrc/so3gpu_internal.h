@@ -16,6 +16,14 @@
 
 namespace so3g {
 
+// A table to the device, there when the call returns.  cudaMemcpy from pageable
+// memory may return while the last part is on its way; a kernel on a stream that
+// does not wait for the legacy one could then read it too early.
+inline cudaError_t upload(void* dst, const void* src, size_t bytes) {
+  const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+  return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
+}
+
 // ---------------------------------------------------------------- errors
 // Status codes returned by every internal entry point.
 enum Status : int {

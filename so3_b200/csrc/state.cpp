@@ -348,7 +348,7 @@ int ensure_fft(Device* D, int n, FftPlan* out) {
   }
   cudaError_t e = cudaMalloc(&dp->mem, host.size() * sizeof(double2));
   if (e != cudaSuccess) return fail(kOutOfMemory, "FFT table allocation failed");
-  e = cudaMemcpy(dp->mem, host.data(), host.size() * sizeof(double2), cudaMemcpyHostToDevice);
+  e = upload(dp->mem, host.data(), host.size() * sizeof(double2));
   if (e != cudaSuccess) return fail(kCudaError, std::string("FFT table upload: ") + cudaGetErrorString(e));
   P.half = dp->mem + half_at;
   if (!P.blue) {
@@ -423,7 +423,7 @@ int ensure_conv_kernel(Device* D, const Geometry& g, const double2** out) {
   double2* d = nullptr;
   if (cudaMalloc(&d, host.size() * sizeof(double2)) != cudaSuccess)
     return fail(kOutOfMemory, "beta-stage weight table allocation failed");
-  SO3G_CUDA(cudaMemcpy(d, host.data(), host.size() * sizeof(double2), cudaMemcpyHostToDevice));
+  SO3G_CUDA(upload(d, host.data(), host.size() * sizeof(double2)));
   D->conv_kernels[key] = d;
   *out = d;
   return kOk;
@@ -461,7 +461,7 @@ int ensure_bases(Device* D, const so3_parameters_t& p, int real, const long long
   std::vector<long long> b = block_bases(p, real);
   long long* d = nullptr;
   if (cudaMalloc(&d, b.size() * sizeof(long long)) != cudaSuccess) return fail(kOutOfMemory, "base table allocation failed");
-  SO3G_CUDA(cudaMemcpy(d, b.data(), b.size() * sizeof(long long), cudaMemcpyHostToDevice));
+  SO3G_CUDA(upload(d, b.data(), b.size() * sizeof(long long)));
   D->bases[key] = d;
   *out = d;
   return kOk;
