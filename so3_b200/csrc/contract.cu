@@ -442,7 +442,10 @@ __global__ void __launch_bounds__(contract_threads(FWD), CTAS) contract_mma_kern
 #pragma unroll
   for (int j = 0; j < NU; j++)
     if (nu0 + j >= a.nu_lo && nu0 + j < a.nu_hi && !plane_skipped(a.n_mode, a.N, nu0 + j)) act |= 1u << j;
-  if (FWD && !act) return;  // caller-zeroed blocks stay untouched
+  if (FWD && !act) {  // caller-zeroed blocks stay untouched
+    dep_wait();  // a launch of such blocks alone must not finish before the stage that the next launch reads
+    return;
+  }
   if (tid < NU) {
     const int nu = min(nu0 + tid, a.N - 1);
     bsel[tid][0] = a.base[a.plane0 + nu];
