@@ -772,13 +772,13 @@ int launch_inv_gamma(const Geometry& g, const FftPlan& p, const double2* W, void
   if (bt.n)
     return each(bt, [&](int b) { return launch_inv_gamma(g, p, W + b * bt.wstride, bt.io[b], s, row_lo, row_hi); });
   int rc;
-  const Eng e = pick(p);
+  const bool big = p.big();  // not pick(): the compile-time plan of 1023 points (N = 512) is no gamma engine
   if (g.real) {
-    rc = e == Eng::kGenBig ? inv_gamma<true, Gen<true>>(g, p, W, f, s, row_lo, row_hi)
-                           : inv_gamma<true, Gen<false>>(g, p, W, f, s, row_lo, row_hi);
+    rc = big ? inv_gamma<true, Gen<true>>(g, p, W, f, s, row_lo, row_hi)
+             : inv_gamma<true, Gen<false>>(g, p, W, f, s, row_lo, row_hi);
   } else {
-    rc = e == Eng::kGenBig ? inv_gamma<false, Gen<true>>(g, p, W, f, s, row_lo, row_hi)
-                           : inv_gamma<false, Gen<false>>(g, p, W, f, s, row_lo, row_hi);
+    rc = big ? inv_gamma<false, Gen<true>>(g, p, W, f, s, row_lo, row_hi)
+             : inv_gamma<false, Gen<false>>(g, p, W, f, s, row_lo, row_hi);
   }
   return rc ? rc : launched();
 }
@@ -791,13 +791,13 @@ int launch_fwd_gamma(const Geometry& g, const FftPlan& p, const void* f, double2
   if (bt.n)
     return each(bt, [&](int b) { return launch_fwd_gamma(g, p, bt.io[b], W + b * bt.wstride, s, row_lo, row_hi); });
   int rc;
-  const Eng e = pick(p);
+  const bool big = p.big();  // as in launch_inv_gamma
   if (g.real) {
-    rc = e == Eng::kGenBig ? fwd_gamma<true, Gen<true>>(g, p, f, W, s, row_lo, row_hi)
-                           : fwd_gamma<true, Gen<false>>(g, p, f, W, s, row_lo, row_hi);
+    rc = big ? fwd_gamma<true, Gen<true>>(g, p, f, W, s, row_lo, row_hi)
+             : fwd_gamma<true, Gen<false>>(g, p, f, W, s, row_lo, row_hi);
   } else {
-    rc = e == Eng::kGenBig ? fwd_gamma<false, Gen<true>>(g, p, f, W, s, row_lo, row_hi)
-                           : fwd_gamma<false, Gen<false>>(g, p, f, W, s, row_lo, row_hi);
+    rc = big ? fwd_gamma<false, Gen<true>>(g, p, f, W, s, row_lo, row_hi)
+             : fwd_gamma<false, Gen<false>>(g, p, f, W, s, row_lo, row_hi);
   }
   return rc ? rc : launched();
 }
