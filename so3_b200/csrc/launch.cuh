@@ -24,8 +24,7 @@ __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;"
 // Captured streams take plain launches.
 template <class... P, class... A>
 int launch_after(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... args) {
-  if (smem > 48 * 1024)
-    SO3G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (int rc = allow_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   const bool plain = cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
   cudaLaunchAttribute at{};

@@ -2177,7 +2177,7 @@ int launch_mixed_fwd_beta(const Geometry& g, double2* W, long long wstride, int 
   if (a.nchunk * kKC <= 512 && stream_slicing()) {
     // single read of the beta samples through shared memory
     const int bsmem = a.nchunk * kKC * kBsCols * (int)sizeof(double2) + (8 * 16 + 16) * (int)sizeof(double);
-    SO3G_CUDA(cudaFuncSetAttribute(beta_slice1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bsmem));
+    if (int rc = allow_smem(reinterpret_cast<const void*>(beta_slice1_kernel), bsmem)) return rc;
     beta_slice1_kernel<<<dim3((unsigned)(16 * ct * g.nplanes), (unsigned)nsig), 256, bsmem, s>>>(a, tiles);
   } else {
     beta_slice_kernel<<<dim3((unsigned)tiles, (unsigned)nsig), 256, 0, s>>>(a);

@@ -42,6 +42,9 @@ int fail(int code, const std::string& msg);  // records msg, returns code
       return ::so3g::fail(::so3g::kCudaError, std::string(#call) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
+// Lets a kernel be launched with `bytes` of dynamic shared memory.
+int allow_smem(const void* kernel, size_t bytes);
+
 // Counter of kernel launches issued by this library (all devices).
 extern std::atomic<long long> g_launches;
 #define SO3G_LAUNCHED() (::so3g::g_launches.fetch_add(1, std::memory_order_relaxed))

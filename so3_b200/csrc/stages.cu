@@ -46,8 +46,7 @@ Sizing size_for(bool big, int ld, int Tmax) {
 
 template <typename K>
 int set_smem(K kernel, size_t bytes) {
-  SO3G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  return kOk;
+  return allow_smem(reinterpret_cast<const void*>(kernel), bytes);
 }
 
 // DFT engines the stage kernels are instantiated with.  Gen<BIG> runs any

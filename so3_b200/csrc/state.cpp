@@ -21,6 +21,31 @@ int fail(int code, const std::string& msg) {
   return code;
 }
 
+// A block gets 48 KB unless the kernel opts in to more, static and dynamic
+// parts counted together (a few hundred bytes are static; the limit here leaves
+// them 8 KB).  The opt-in is a property of the kernel that all threads share: each
+// sets the same value, all that the static part leaves of a block's largest
+// size, so that no thread lowers it between another's opt-in and launch.
+int allow_smem(const void* kernel, size_t bytes) {
+  if (bytes <= 40 * 1024) return kOk;
+  static std::mutex mu;
+  static std::map<const void*, int> fixed;  // static part, as compiled
+  int st;
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = fixed.find(kernel);
+    if (it == fixed.end()) {
+      cudaFuncAttributes at;
+      SO3G_CUDA(cudaFuncGetAttributes(&at, kernel));
+      it = fixed.emplace(kernel, (int)at.sharedSizeBytes).first;
+    }
+    st = it->second;
+  }
+  constexpr int kBlockMax = 227 * 1024;
+  SO3G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBlockMax - st));
+  return kOk;
+}
+
 // ------------------------------------------------------------------ geometry
 Geometry make_geometry(const so3_parameters_t& p, int real) {
   Geometry g{};
