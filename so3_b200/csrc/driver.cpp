@@ -72,10 +72,15 @@ static int ensure_tuned(Device* D, const so3_parameters_t& p, int real, Resource
   if (!(env && env[0] == '0')) {
     FftPlan pc{};
     const double2* wr = nullptr;
-    if (!beta_matrix_pays(g, kBetaForward)) {
+    {  // the forward beta stage's tables, also for an inverse: a captured forward may follow it
       std::lock_guard<std::mutex> lk(D->mu);
-      if (int rc = ensure_fft(D, g.Pc, &pc)) return rc;
-      if (int rc = ensure_conv_kernel(D, g, &wr)) return rc;
+      const double* mat;
+      if (beta_matrix_pays(g, kBetaForward)) {
+        if (int rc = ensure_beta_matrix(D, g, kBetaForward, r->pP, s, &mat)) return rc;
+      } else {
+        if (int rc = ensure_fft(D, g.Pc, &pc)) return rc;
+        if (int rc = ensure_conv_kernel(D, g, &wr)) return rc;
+      }
     }
     if (int rc = autotune_stages(&g, r->pP, r->pg, pc, wr, W, s, 3)) return rc;
   }
