@@ -17,6 +17,9 @@ static thread_local std::string t_last_error;
 void set_error(const std::string& msg) { t_last_error = msg; }
 const std::string& last_error() { return t_last_error; }
 int fail(int code, const std::string& msg) {
+  // the runtime keeps a refused call's error until it is asked for, and the next
+  // call's launches would find it
+  if (code == kCudaError || code == kOutOfMemory) cudaGetLastError();
   set_error(msg);
   return code;
 }
