@@ -32,7 +32,10 @@ void so3gpu_context_destroy(so3gpu_context *ctx);
 int so3gpu_context_set_stream(so3gpu_context *ctx, void *stream);
 
 /* Builds the resident tables and plans the transform with these parameters
- * needs (blocking).  Call it before capturing transforms in a CUDA graph. */
+ * needs, and the context's scratch for one of them (blocking).  Call it before
+ * capturing transforms, or FP64 batches of them, in a CUDA graph.  A graph holds
+ * that scratch: it may be replayed until the context runs a call that needs
+ * more of it (a larger geometry, a split-precision batch, a convolution batch). */
 int so3gpu_prepare(so3gpu_context *ctx, const so3_parameters_t *parameters);
 /* Device scratch (bytes) one transform with these parameters uses. */
 size_t so3gpu_workspace_size(const so3_parameters_t *parameters);
@@ -47,8 +50,11 @@ int so3gpu_forward_real(so3gpu_context *ctx, void *flmn, const double *f,
 
 /* Batches of `count` signals sharing one parameter set (no counterpart in the
  * reference).  f and flmn are host arrays of `count` device pointers.
- * precision SO3GPU_PRECISION_FP64: the FP64 path signal by signal (results
- * identical to so3gpu_inverse / so3gpu_forward).  SO3GPU_PRECISION_MIXED_INT8:
+ * precision SO3GPU_PRECISION_FP64: the FP64 path, results identical to
+ * so3gpu_inverse / so3gpu_forward; up to 32 signals (192 MB of beta-row scratch,
+ * about 400 MB in all) share the launches, in scratch of their own that the
+ * context keeps, or run one by one in a capture and where there is no memory for
+ * more.  SO3GPU_PRECISION_MIXED_INT8:
  * the Wigner contractions of all signals run as int8 tensor-core products
  * (7-slice Ozaki split, exact int32 accumulation, FP64 recombination) while
  * Delta, the quadrature weights and every DFT stay FP64; normwise relative

@@ -425,6 +425,7 @@ void so3gpu_context_destroy(so3gpu_context* c) {
   cudaGetDevice(&prev);
   cudaSetDevice(c->device);
   if (c->wk.ws) cudaFree(c->wk.ws);
+  if (c->wk.chunk) cudaFree(c->wk.chunk);
   cudaSetDevice(prev);
   delete c;
 }

@@ -483,20 +483,20 @@ static int fp64_contractions(const Resources& r, const so3_parameters_t& p, int 
   return kOk;
 }
 
-// FP64 batch: chunks that share launches, on a workspace of one chunk (of one
-// signal where the caller's workspace holds no more).
+// FP64 batch: chunks that share launches, as many signals each as there is
+// scratch for (chunk_ws).
 static int run_fp64_batch(Device* D, Workspace* wk, const so3_parameters_t& p, int real, bool fwd, int nsig,
                           const void* const* in, void* const* out, cudaStream_t s) {
   if (nsig == 0) return kOk;
   Resources r;
   if (int rc = acquire(D, p, real, s, &r, fwd)) return rc;
   const size_t wb = (workspace_bytes(p, real) + 255) & ~size_t(255);
-  int step = batch_chunk(r.g, nsig);
-  if (wk->borrowed) step = (int)std::min<size_t>(step, std::max<size_t>(1, wk->ws_bytes / wb));
   void* ws = nullptr;
-  if (int rc = ensure_ws(wk, step > 1 ? wb * step : workspace_bytes(p, real), &ws)) return rc;
+  if (int rc = ensure_ws(wk, workspace_bytes(p, real), &ws)) return rc;
+  if (int rc = ensure_tuned(D, p, real, &r, static_cast<double2*>(ws), s)) return rc;
+  int step = batch_chunk(r.g, nsig);
+  chunk_ws(wk, wb, s, &step, &ws);
   double2* W = static_cast<double2*>(ws);
-  if (int rc = ensure_tuned(D, p, real, &r, W, s)) return rc;
   const long long wstride = (long long)(wb / sizeof(double2));
   for (int b0 = 0; b0 < nsig; b0 += step) {
     const int n = std::min(step, nsig - b0);
@@ -628,12 +628,12 @@ int run_conv_inverse_batch(Device* D, Workspace* wk, const so3_parameters_t& p, 
     // scratch of a chunk of signals, then hlmn of each
     const size_t wb = (workspace_bytes(p, 0) + 255) & ~size_t(255);
     const size_t hb = ((size_t)so3_sampling_flmn_size(&p) * sizeof(double2) + 255) & ~size_t(255);
-    int step = batch_chunk(r.g, nsig);
-    if (wk->borrowed) step = (int)std::min<size_t>(step, std::max<size_t>(1, wk->ws_bytes / (wb + hb)));
     void* ws = nullptr;
-    if ((rc = ensure_ws(wk, (wb + hb) * step, &ws))) return rc;
+    if ((rc = ensure_ws(wk, wb + (size_t)so3_sampling_flmn_size(&p) * sizeof(double2), &ws))) return rc;
+    if ((rc = ensure_tuned(D, p, 0, &r, static_cast<double2*>(ws), s))) return rc;
+    int step = batch_chunk(r.g, nsig);
+    chunk_ws(wk, wb + hb, s, &step, &ws);
     double2* W = static_cast<double2*>(ws);
-    if ((rc = ensure_tuned(D, p, 0, &r, W, s))) return rc;
     const long long wstride = (long long)(wb / sizeof(double2));
     for (int b0 = 0; b0 < nsig; b0 += step) {
       const int n = std::min(step, nsig - b0);

@@ -191,6 +191,10 @@ struct Workspace {
   void* ws = nullptr;
   size_t ws_bytes = 0;
   bool borrowed = false;  // ws is owned by the caller (never reallocated or freed here)
+  // Scratch of FP64 batches that share launches, beside ws: a captured transform
+  // holds pointers into ws, which a batch must not free.  Never used by a capture.
+  void* chunk = nullptr;
+  size_t chunk_bytes = 0;
   StageTimer timer;
 };
 Device* device_state(int device);  // lazily created per CUDA device
@@ -204,6 +208,9 @@ int ensure_conv_kernel(Device* D, const Geometry& g, const double2** out);
 int ensure_beta_matrix(Device* D, const Geometry& g, int kind, const FftPlan& pP, cudaStream_t s, const double** out);
 int ensure_bases(Device* D, const so3_parameters_t& p, int real, const long long** out);
 int ensure_ws(Workspace* W, size_t bytes, void** out);
+// Scratch of up to *n signals of `bytes` each (a multiple of 256), after an
+// ensure_ws for one: *n becomes the number that *out holds, one where no more can be had.
+void chunk_ws(Workspace* W, size_t bytes, cudaStream_t s, int* n, void** out);
 size_t workspace_bytes(const so3_parameters_t& p, int real);
 // Device bytes of the resident per-device tables (Delta tables, digit and
 // beta tables, weight tables, DFT plans, block bases).

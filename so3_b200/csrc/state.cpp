@@ -1,5 +1,6 @@
 // Per-device state of libso3gpu: error reporting, resident Wigner tables, FFT
 // plans, block-offset tables and grow-only scratch.  Host code only.
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <complex>
@@ -230,6 +231,38 @@ int ensure_ws(Workspace* W, size_t bytes, void** out) {
   }
   *out = W->ws;
   return kOk;
+}
+
+// A capture keeps to ws, which only a larger geometry replaces (prepare sizes
+// it), and neither frees nor allocates.  Where the memory for more signals is not
+// to be had, they run one by one as well.
+void chunk_ws(Workspace* W, size_t bytes, cudaStream_t s, int* n, void** out) {
+  const int want = *n, have = (int)std::min<size_t>(want, std::max<size_t>(1, W->ws_bytes / bytes));
+  *n = have;
+  *out = W->ws;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (have == want || W->borrowed || cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
+    return;
+  if (W->chunk_bytes < bytes * want) {
+    // another thread's capture may forbid unsafe calls to all threads; these touch nothing of it
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    void* d = nullptr;
+    cudaFree(W->chunk);
+    W->chunk = nullptr;
+    W->chunk_bytes = 0;
+    if (cudaMalloc(&d, bytes * want) == cudaSuccess) {
+      W->chunk = d;
+      W->chunk_bytes = bytes * want;
+    } else {
+      cudaGetLastError();
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+  }
+  if (W->chunk_bytes / bytes > (size_t)have) {
+    *n = (int)std::min<size_t>(want, W->chunk_bytes / bytes);
+    *out = W->chunk;
+  }
 }
 
 // ------------------------------------------------------------------ tables

@@ -36,3 +36,36 @@ def test_forward_captured_after_plain_inverse(sampling):
     ref = ctx.forward(f, p)
     torch.cuda.synchronize()
     assert back.abs().max() > 0.1 and torch.equal(torch.view_as_real(back), torch.view_as_real(ref))
+
+
+@pytest.mark.parametrize("prior", [0, 4])
+def test_batches_beside_captured_transforms(prior):
+    """After so3gpu_prepare single transforms and FP64 batches can be captured;
+    uncaptured batches of more signals, before or after, take none of the
+    scratch that the graphs hold."""
+    p = params(24, 4)
+    s = torch.cuda.Stream()
+    ctx = so3.Context(0, stream=s)
+    fls = [_coefficients(p, 10 + i) for i in range(33)]
+    one, three = _samples(p), [_samples(p) for _ in range(3)]
+    back = [torch.zeros_like(x) for x in fls[:3]]
+    torch.cuda.synchronize()
+    ctx.prepare(p)
+    if prior:
+        ctx.inverse_batch(fls[:prior], p, "fp64")
+        torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=s):
+        ctx.inverse(fls[0], p, out=one)
+        ctx.inverse_batch(fls[1:4], p, "fp64", outs=three)
+        ctx.forward_batch(three, p, "fp64", outs=back)
+    f = ctx.inverse_batch(fls, p, "fp64")
+    b = ctx.forward_batch(f, p, "fp64")
+    torch.cuda.synchronize()
+    for x in [one] + three + back:
+        x.fill_(float("nan"))
+    torch.cuda.synchronize()
+    graph.replay()
+    torch.cuda.synchronize()
+    for x, y in zip([one] + three + back, f[:4] + b[1:4]):
+        assert torch.equal(torch.view_as_real(x), torch.view_as_real(y))
