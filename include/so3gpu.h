@@ -188,10 +188,11 @@ const char *so3gpu_last_error(void);
 void so3gpu_set_error_mode(int mode);
 /* Number of kernels this library has launched since load (all devices). */
 long long so3gpu_launch_count(void);
-/* Reads and clears the current device's flag that the tensor-core kernels set
- * when one of their bounded waits gave up (0: none; a nonzero value means the
- * results of the split-precision calls since the last read are invalid).
- * Synchronous. */
+/* Reads and clears the current device's flag that kernels set when one of their
+ * bounded waits gave up (0: none).  Bit 1: the results of the split-precision
+ * calls since the last read are invalid.  Bit 2: an FP64 contraction lacked a
+ * copy; what depends on it is NaN.  The drop-in calls and the request server
+ * report the latter themselves, as status 2.  Synchronous. */
 int so3gpu_take_kernel_error(void);
 
 #ifdef __cplusplus

@@ -86,6 +86,7 @@ DropIn* dropin(int dev) {
     cudaStreamCreateWithFlags(&slot->cin, cudaStreamNonBlocking);
     cudaStreamCreateWithFlags(&slot->cout, cudaStreamNonBlocking);
     for (cudaEvent_t& e : slot->ev) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
+    so3g::open_fault(&slot->wk);
   }
   return slot.get();
 }
@@ -117,7 +118,7 @@ int device_view(DropIn* X, int slot, const void* host, size_t bytes, bool upload
 int download(DropIn* X, void* host, const void* dev, size_t bytes, bool staged) {
   if (staged && bytes) SO3G_CUDA(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, X->stream));
   SO3G_CUDA(cudaStreamSynchronize(X->stream));
-  return so3g::kOk;
+  return so3g::take_fault(&X->wk);
 }
 
 size_t f_bytes(const so3_parameters_t* p, int real) {
@@ -146,7 +147,8 @@ int drain(DropIn* X, int rc) {
   const cudaError_t a = cudaStreamSynchronize(X->cin);
   const cudaError_t b = cudaStreamSynchronize(X->stream);
   const cudaError_t c = cudaStreamSynchronize(X->cout);
-  if (rc) return rc;
+  const int fault = so3g::take_fault(&X->wk);
+  if (rc || fault) return rc ? rc : fault;
   const cudaError_t e = a != cudaSuccess ? a : (b != cudaSuccess ? b : c);
   if (e != cudaSuccess) return so3g::fail(so3g::kCudaError, std::string("staged transform: ") + cudaGetErrorString(e));
   return so3g::kOk;
@@ -233,6 +235,7 @@ int require_mw(const so3_parameters_t* p) {
 }  // namespace
 
 void so3g_record_status(int rc) { t_status = rc; }
+extern "C" int* so3g_dropin_fault_word(int device) { return dropin(device)->wk.fault; }
 
 struct so3gpu_context {
   int device = 0;

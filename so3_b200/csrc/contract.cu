@@ -385,8 +385,8 @@ __global__ void __launch_bounds__(kThreads, 1) forward_contract_kernel(FwdArgs a
 // per SM at 72 registers and two ring slots, inverse (whose copies scatter and whose
 // weight takes registers) two at 96 and three slots; forward as inverse 2.48 ms at
 // L = 512, N = 64, inverse as forward 2.77.  Measured at L = 512, N = 64 (ms, inverse
-// / forward): 2.51 / 2.30, against 2.61 / 2.48 with one copying warp and two CTAs in
-// both; 4.97 / 5.92 for staging by all warps with 8-byte copies from row-major
+// / forward): 2.54 / 2.36 (2.50 / 2.33 were no warp to look whether its wait gave up),
+// against 2.61 / 2.48 with one copying warp and two CTAs in both; 4.97 / 5.92 for staging by all warps with 8-byte copies from row-major
 // planes; 3.09 / 2.89 without copying warps (a barrier per chunk aligned the warps'
 // bursts).  64 rows x 4 nu (one CTA of 16 warps) gives 2.57 / 2.42 there but 39 / 37
 // us against 23 / 30 at L = 128, N = 16.  Two signals per CTA share the Delta reads:
@@ -413,12 +413,24 @@ struct ContractArgs {
   long long CS, QS;
   double wconst;           // inverse, > 0: this weight for every l
   double lw;               // forward, > 0: outputs times lw (2l+1)
+  int* fault;              // the caller's word (Workspace::fault) or null
 };
 
-__device__ int g_contract_error;  // bit 2: a wait for a copy gave up (see tc::mbar_wait)
+// Bit 2: a wait for a copy gave up (see tc::mbar_wait).  The results that lacked
+// the copy are NaN, and so is every sample that depends on them.
+__device__ int g_contract_error;
 
 __device__ __forceinline__ void cp16_to(uint32_t dst, const void* src, bool valid) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0));
+}
+
+// The end of a copying warp: no copy into the block's shared memory is in flight
+// any more, also where a product warp that would have waited for it gave up.  Bulk
+// copies by each slot's latest use: st is the slot that comes next, phase the parity
+// of its latest use.
+__device__ __forceinline__ void drain_copies(uint32_t full0, int slots, int st, uint32_t phase) {
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+  for (int i = 0; i < slots; i++) tc::mbar_wait(full0 + 8 * i, i < st ? phase ^ 1 : phase, &g_contract_error, 4);
 }
 
 constexpr int kCStage = kCRt * kCMu * 64 + kCRt * kCNu * 64 + 2 * kCMu * kCNu * kXB;  // doubles
@@ -432,6 +444,7 @@ __global__ void __launch_bounds__(contract_threads(FWD), CTAS) contract_mma_kern
   extern __shared__ __align__(16) double smc[];
   __shared__ long long bsel[NU][2];
   __shared__ __align__(8) unsigned long long full[ST], empty[ST];
+  __shared__ volatile int gave_up;  // a wait of this block did: its results are void
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
   const int wr = warp % WR, wm = warp / WR % 2, wn = warp / (2 * WR);
   const int nu0 = a.nu0 + blockIdx.x * NU, rt0 = blockIdx.y * RT;
@@ -466,6 +479,7 @@ __global__ void __launch_bounds__(contract_threads(FWD), CTAS) contract_mma_kern
 
   const uint32_t full0 = tc::smem_u32(full), empty0 = tc::smem_u32(empty);
   if (tid == 0) {
+    gave_up = 0;
     for (int st = 0; st < ST; st++) {
       tc::mbar_init(full0 + 8 * st, 32 * CW + 1);  // the copying lanes' loads of X and the expected bytes
       tc::mbar_init(empty0 + 8 * st, NWARP);
@@ -524,7 +538,12 @@ __global__ void __launch_bounds__(contract_threads(FWD), CTAS) contract_mma_kern
     int st = 0;
     uint32_t phase = 1;  // of the ring slot's previous use
     for (int ch = ch0; ch < ch1; ch++) {
-      if (ch - ch0 >= ST) tc::mbar_wait(empty0 + 8 * st, phase, &g_contract_error, 4);
+      if (ch - ch0 >= ST) {
+        if (!tc::mbar_wait(empty0 + 8 * st, phase, &g_contract_error, 4, &gave_up)) {
+          drain_copies(full0, ST, st, phase);  // the lanes that are left do not wait for one that has gone
+          return;
+        }
+      }
       if (j0 == 0 && ch > ch0) blocks(ch, st);
       const uint32_t at = (uint32_t)(st * STAGE * 8), bar = full0 + 8 * st;
 #pragma unroll
@@ -555,7 +574,7 @@ __global__ void __launch_bounds__(contract_threads(FWD), CTAS) contract_mma_kern
       if (++st == ST) st = 0;
       if (st == 0) phase ^= 1;
     }
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    drain_copies(full0, ST, st, phase);
     return;
   }
 
@@ -617,7 +636,7 @@ __global__ void __launch_bounds__(contract_threads(FWD), CTAS) contract_mma_kern
   int st = 0;
   uint32_t phase = 0;
   for (int ch = ch0; ch < ch1; ch++) {
-    tc::mbar_wait(full0 + 8 * st, phase, &g_contract_error, 4);
+    if (!__all_sync(0xffffffffu, tc::mbar_wait(full0 + 8 * st, phase, &g_contract_error, 4, &gave_up))) break;
     if (FWD ? (ch <= rt_lo && rt_hi < LC) : rt_hi <= ch)
       products(ch, st, std::true_type{});
     else
@@ -626,6 +645,13 @@ __global__ void __launch_bounds__(contract_threads(FWD), CTAS) contract_mma_kern
     __syncwarp();
     if (lane == 0) tc::mbar_arrive(empty0 + 8 * st);
     if (++st == ST) st = 0, phase ^= 1;
+  }
+  if (gave_up) {
+    if (a.fault) *static_cast<volatile int*>(a.fault) = 4;
+#pragma unroll
+    for (int i = 0; i < MT; i++)
+#pragma unroll
+      for (int m = 0; m < 4; m++) acc[i][m][0] = acc[i][m][1] = __longlong_as_double(0x7ff8000000000000ll);
   }
 
   dep_launch();
@@ -697,6 +723,7 @@ int launch_inverse_contract(const Geometry& g, int n_mode, const double2* flmn, 
     c.base = bases, c.dl = dl, c.W = W + g.QOFF;
     c.L = g.L, c.N = g.N, c.L0 = g.L0, c.plane0 = g.plane0, c.n_mode = n_mode, c.nsign = g.real ? 2 : 4;
     c.sym_n0 = sym_n0, c.nu_lo = nu_lo, c.nu_hi = nu_hi, c.CS = g.CS, c.QS = g.QS, c.wconst = wconst;
+    c.fault = g.fault;
     return contract<false>(c, flmn, bt, s);
   }
   if (bt.n) {  // the FMA engine runs signal by signal
@@ -731,6 +758,7 @@ int launch_forward_contract(const Geometry& g, int n_mode, const double2* W, con
     c.base = bases, c.dl = dl, c.W = const_cast<double2*>(W) + g.QOFF;
     c.L = g.L, c.N = g.N, c.L0 = g.L0, c.plane0 = g.plane0, c.n_mode = n_mode, c.nsign = g.real ? 2 : 4;
     c.compact = storage_compact, c.nu_lo = nu_lo, c.nu_hi = nu_hi, c.CS = g.CS, c.QS = g.QS, c.lw = lw;
+    c.fault = g.fault;
     return contract<true>(c, flmn, bt, s);
   }
   if (bt.n) {

@@ -19,9 +19,11 @@ struct Resources {
   const double2* wr = nullptr;
 };
 
-static int acquire(Device* D, const so3_parameters_t& p, int real, cudaStream_t s, Resources* r, bool conv) {
+static int acquire(Device* D, const Workspace* wk, const so3_parameters_t& p, int real, cudaStream_t s, Resources* r,
+                   bool conv) {
   if (int rc = validate(p, real)) return rc;
   r->g = make_geometry(p, real);
+  r->g.fault = wk ? wk->fault : nullptr;
   std::lock_guard<std::mutex> lk(D->mu);
   if (int rc = ensure_dl(D, p.L, p.dl_method, s, &r->dl)) return rc;
   if (int rc = ensure_fft(D, r->g.P, &r->pP)) return rc;
@@ -111,7 +113,7 @@ int set_stage_variants(Device* D, const so3_parameters_t& p, int real, const int
 
 int prepare(Device* D, const so3_parameters_t& p, int real, cudaStream_t s, Workspace* wk) {
   Resources r;
-  if (int rc = acquire(D, p, real, s, &r, true)) return rc;
+  if (int rc = acquire(D, wk, p, real, s, &r, true)) return rc;
   if (!wk) return kOk;
   void* ws = nullptr;
   if (int rc = ensure_ws(wk, workspace_bytes(p, real), &ws)) return rc;
@@ -121,7 +123,7 @@ int prepare(Device* D, const so3_parameters_t& p, int real, cudaStream_t s, Work
 int run_inverse(Device* D, Workspace* wk, const so3_parameters_t& p, const void* flmn_d, void* f_d, int real,
                 cudaStream_t s) {
   Resources r;
-  if (int rc = acquire(D, p, real, s, &r, false)) return rc;
+  if (int rc = acquire(D, wk, p, real, s, &r, false)) return rc;
   void* ws = nullptr;
   if (int rc = ensure_ws(wk, workspace_bytes(p, real), &ws)) return rc;
   double2* W = static_cast<double2*>(ws);
@@ -149,7 +151,7 @@ int run_inverse(Device* D, Workspace* wk, const so3_parameters_t& p, const void*
 int run_forward(Device* D, Workspace* wk, const so3_parameters_t& p, const void* f_d, void* flmn_d, int real,
                 cudaStream_t s) {
   Resources r;
-  if (int rc = acquire(D, p, real, s, &r, true)) return rc;
+  if (int rc = acquire(D, wk, p, real, s, &r, true)) return rc;
   void* ws = nullptr;
   if (int rc = ensure_ws(wk, workspace_bytes(p, real), &ws)) return rc;
   double2* W = static_cast<double2*>(ws);
@@ -250,7 +252,7 @@ int copy_rows(void* dst, const void* src, const Geometry& g, int r0, int r1, cud
 int run_inverse_staged(Device* D, Workspace* wk, const so3_parameters_t& p, int real, const StagedIo& io,
                        cudaStream_t s) {
   Resources r;
-  if (int rc = acquire(D, p, real, s, &r, false)) return rc;
+  if (int rc = acquire(D, wk, p, real, s, &r, false)) return rc;
   void* ws = nullptr;
   if (int rc = ensure_ws(wk, workspace_bytes(p, real), &ws)) return rc;
   double2* W = static_cast<double2*>(ws);
@@ -303,7 +305,7 @@ int run_inverse_staged(Device* D, Workspace* wk, const so3_parameters_t& p, int 
 int run_forward_staged(Device* D, Workspace* wk, const so3_parameters_t& p, int real, bool zero_first,
                        const StagedIo& io, cudaStream_t s) {
   Resources r;
-  if (int rc = acquire(D, p, real, s, &r, true)) return rc;
+  if (int rc = acquire(D, wk, p, real, s, &r, true)) return rc;
   void* ws = nullptr;
   if (int rc = ensure_ws(wk, workspace_bytes(p, real), &ws)) return rc;
   double2* W = static_cast<double2*>(ws);
@@ -489,7 +491,7 @@ static int run_fp64_batch(Device* D, Workspace* wk, const so3_parameters_t& p, i
                           const void* const* in, void* const* out, cudaStream_t s) {
   if (nsig == 0) return kOk;
   Resources r;
-  if (int rc = acquire(D, p, real, s, &r, fwd)) return rc;
+  if (int rc = acquire(D, wk, p, real, s, &r, fwd)) return rc;
   const size_t wb = (workspace_bytes(p, real) + 255) & ~size_t(255);
   void* ws = nullptr;
   if (int rc = ensure_ws(wk, workspace_bytes(p, real), &ws)) return rc;
@@ -539,7 +541,7 @@ int run_inverse_batch(Device* D, Workspace* wk, const so3_parameters_t& p, int r
   const int nsplit = precision == kPrecFp64 || !split_real_ok(p, real) ? 0 : split_count(false, nsig);
   if (nsplit == 0) return run_fp64_batch(D, wk, p, real, false, nsig, flmn_d, f_d, s);
   Resources r;
-  if (int rc = acquire(D, p, real, s, &r, false)) return rc;
+  if (int rc = acquire(D, wk, p, real, s, &r, false)) return rc;
   const BatchLayout bl = batch_layout(r.g, p, real, nsig);
   void* ws = nullptr;
   if (int rc = ensure_ws(wk, bl.total, &ws)) return rc;
@@ -575,7 +577,7 @@ int run_forward_batch(Device* D, Workspace* wk, const so3_parameters_t& p, int r
     return run_fp64_batch(D, wk, p, real, true, nsig, f_d, flmn_d, s);
   if (nsig == 0) return kOk;
   Resources r;
-  if (int rc = acquire(D, p, real, s, &r, true)) return rc;
+  if (int rc = acquire(D, wk, p, real, s, &r, true)) return rc;
   const BatchLayout bl = batch_layout(r.g, p, real, nsig);
   void* ws = nullptr;
   if (int rc = ensure_ws(wk, bl.total, &ws)) return rc;
@@ -622,7 +624,7 @@ int run_conv_inverse_batch(Device* D, Workspace* wk, const so3_parameters_t& p, 
   if (p.reality) return fail(kUnsupported, "directional convolutions produce complex signals");
   if (nsig == 0) return kOk;
   Resources r;
-  if (int rc = acquire(D, p, 0, s, &r, false)) return rc;
+  if (int rc = acquire(D, wk, p, 0, s, &r, false)) return rc;
   int rc;
   if (precision == kPrecFp64 || split_count(false, nsig) == 0) {
     // scratch of a chunk of signals, then hlmn of each
@@ -711,7 +713,7 @@ std::vector<char> ragged_fp64(const so3_parameters_t* ps, int nsig, bool fwd) {
 
 // Signals of a ragged split-precision batch for the tensor-core contraction
 // (per Delta recursion), and those for the FP64 path.
-int ragged_prepare(Device* D, const so3_parameters_t* ps, int nsig, bool conv_tables, cudaStream_t s,
+int ragged_prepare(Device* D, const Workspace* wk, const so3_parameters_t* ps, int nsig, bool conv_tables, cudaStream_t s,
                    std::vector<RagItem>* items, std::vector<int>* fp64) {
   int Lmax[2] = {0, 0};
   for (int i = 0; i < nsig; i++) {
@@ -735,7 +737,7 @@ int ragged_prepare(Device* D, const so3_parameters_t* ps, int nsig, bool conv_ta
     }
     RagItem it;
     it.idx = i;
-    if (int rc = acquire(D, ps[i], 0, s, &it.r, conv_tables)) return rc;
+    if (int rc = acquire(D, wk, ps[i], 0, s, &it.r, conv_tables)) return rc;
     it.ws_off = off;
     off += (workspace_bytes(ps[i], 0) + 255) & ~size_t(255);
     items->push_back(it);
@@ -773,7 +775,7 @@ int run_inverse_ragged(Device* D, Workspace* wk, const so3_parameters_t* ps, int
   }
   std::vector<RagItem> items;
   std::vector<int> fp64;
-  if (int rc = ragged_prepare(D, ps, nsig, false, s, &items, &fp64)) return rc;
+  if (int rc = ragged_prepare(D, wk, ps, nsig, false, s, &items, &fp64)) return rc;
   for (int i : fp64)  // the FP64 path, before the batch workspace is laid out
     if (int rc = run_inverse(D, wk, ps[i], flmn_d[i], f_d[i], ps[i].reality != 0, s)) return rc;
   if (items.empty()) return kOk;
@@ -845,7 +847,7 @@ int run_forward_ragged(Device* D, Workspace* wk, const so3_parameters_t* ps, int
   }
   std::vector<RagItem> items;
   std::vector<int> fp64;
-  if (int rc = ragged_prepare(D, ps, nsig, true, s, &items, &fp64)) return rc;
+  if (int rc = ragged_prepare(D, wk, ps, nsig, true, s, &items, &fp64)) return rc;
   for (int i : fp64)
     if (int rc = run_forward(D, wk, ps[i], f_d[i], flmn_d[i], ps[i].reality != 0, s)) return rc;
   if (items.empty()) return kOk;
@@ -929,7 +931,7 @@ int run_adjoint_inverse(Device* D, Workspace* wk, const so3_parameters_t& p, con
   if (int rc = adjoint_check(p)) return rc;
   const int real = p.reality ? 1 : 0;
   Resources r;
-  if (int rc = acquire(D, p, real, s, &r, false)) return rc;
+  if (int rc = acquire(D, wk, p, real, s, &r, false)) return rc;
   if (int rc = acquire_adjoint(D, kBetaAdjInverse, s, &r)) return rc;
   void* ws = nullptr;
   if (int rc = ensure_ws(wk, workspace_bytes(p, real), &ws)) return rc;
@@ -952,7 +954,7 @@ int run_adjoint_forward(Device* D, Workspace* wk, const so3_parameters_t& p, con
   if (int rc = adjoint_check(p)) return rc;
   const int real = p.reality ? 1 : 0;
   Resources r;
-  if (int rc = acquire(D, p, real, s, &r, false)) return rc;
+  if (int rc = acquire(D, wk, p, real, s, &r, false)) return rc;
   if (int rc = acquire_adjoint(D, kBetaAdjForward, s, &r)) return rc;
   void* ws = nullptr;
   if (int rc = ensure_ws(wk, workspace_bytes(p, real), &ws)) return rc;

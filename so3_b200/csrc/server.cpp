@@ -121,6 +121,7 @@ class Server {
       auto sl = std::make_unique<Slot>();
       SO3G_CUDA(cudaStreamCreateWithFlags(&sl->s, cudaStreamNonBlocking));
       sl->owner = this;
+      if (int rc = open_fault(&sl->wk)) return rc;
       slots_.push_back(std::move(sl));
     }
     // keep freed scratch in the pool up to the budget (no release to the OS
@@ -164,6 +165,7 @@ class Server {
       if (sl->s) {
         cudaStreamSynchronize(sl->s);
         cudaStreamDestroy(sl->s);
+        cudaFreeHost(sl->wk.fault);
       }
     for (auto& kv : reqs_) delete kv.second;
   }
@@ -365,6 +367,8 @@ class Server {
     for (auto& sl : slots_) {
       if (!sl->busy || !sl->finished.load()) continue;
       const double t = sl->t_finish.load();
+      const int fault = take_fault(&sl->wk);
+      if (sl->status == kOk) sl->status = fault;
       for (Req* r : sl->reqs) {
         r->t_done = t;
         r->status = sl->status;

@@ -81,6 +81,7 @@ struct Geometry {
   signed char var[8];
   // Matrices of the beta stages (beta_mm.cu) by BetaKind; null: through DFTs.
   const double* beta_mat[4];
+  int* fault;  // see Workspace::fault
 };
 Geometry make_geometry(const so3_parameters_t& p, int real);
 
@@ -195,6 +196,9 @@ struct Workspace {
   // holds pointers into ws, which a batch must not free.  Never used by a capture.
   void* chunk = nullptr;
   size_t chunk_bytes = 0;
+  // Host word that a kernel sets when one of its bounded waits gave up and its
+  // results are void, for owners that report the end of their calls (null: none).
+  int* fault = nullptr;
   StageTimer timer;
 };
 Device* device_state(int device);  // lazily created per CUDA device
@@ -208,6 +212,9 @@ int ensure_conv_kernel(Device* D, const Geometry& g, const double2** out);
 int ensure_beta_matrix(Device* D, const Geometry& g, int kind, const FftPlan& pP, cudaStream_t s, const double** out);
 int ensure_bases(Device* D, const so3_parameters_t& p, int real, const long long** out);
 int ensure_ws(Workspace* W, size_t bytes, void** out);
+int open_fault(Workspace* W);
+// kOk, or an error (and the word cleared) if a wait gave up; after the work has ended.
+int take_fault(Workspace* W);
 // Scratch of up to *n signals of `bytes` each (a multiple of 256), after an
 // ensure_ws for one: *n becomes the number that *out holds, one where no more can be had.
 void chunk_ws(Workspace* W, size_t bytes, cudaStream_t s, int* n, void** out);
@@ -434,3 +441,5 @@ int validate(const so3_parameters_t& p, int real);
 
 // Records the status of the calling thread's last call (so3gpu_last_status).
 void so3g_record_status(int rc);
+// The status word of the drop-in calls of a device (tests set it as a kernel would).
+extern "C" int* so3g_dropin_fault_word(int device);

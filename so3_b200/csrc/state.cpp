@@ -233,6 +233,18 @@ int ensure_ws(Workspace* W, size_t bytes, void** out) {
   return kOk;
 }
 
+int open_fault(Workspace* W) {
+  if (cudaHostAlloc(&W->fault, sizeof(int), cudaHostAllocMapped) != cudaSuccess)
+    return W->fault = nullptr, fail(kOutOfMemory, "status word allocation failed");
+  *W->fault = 0;
+  return kOk;
+}
+int take_fault(Workspace* W) {
+  if (!W->fault || *static_cast<volatile int*>(W->fault) == 0) return kOk;
+  *W->fault = 0;
+  return fail(kCudaError, "a kernel waited too long for a copy: the results are not valid");
+}
+
 // A capture keeps to ws, which only a larger geometry replaces (prepare sizes
 // it), and neither frees nor allocates.  Where the memory for more signals is not
 // to be had, they run one by one as well.

@@ -13,10 +13,14 @@
 namespace so3g {
 namespace tc {
 
-// Every wait in these kernels gives up after this many nanoseconds, records
-// the failure in a device flag the host can read, and lets the kernel run to
-// its end instead of hanging the GPU.
+// Every wait in these kernels gives up after this many nanoseconds of polling,
+// records the failure in a device flag the host can read, and lets the kernel
+// run to its end instead of hanging the GPU.  The clock runs on while the process
+// is switched out, when the awaited work stands still too: the time between
+// two readings (64 polls) counts as kWaitGapNs at most.
 constexpr unsigned long long kWaitLimitNs = 2000000000ull;  // 2 s
+constexpr unsigned long long kWaitGapNs = 10000000ull;      // 10 ms
+constexpr unsigned long long kWaitStopNs = 1000000ull;      // 1 ms
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -53,16 +57,25 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 }
 // Waits for the phase with the given parity to complete.  On timeout sets
 // *flag (global) and returns false; the caller carries on so that the kernel
-// always terminates.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* flag, int code) {
+// always terminates.  stop (shared, optional): set as well, and a block's other
+// waits then give up after kWaitStopNs.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* flag, int code,
+                                          volatile int* stop = nullptr) {
   if (mbar_try_wait(bar, parity)) return true;
-  const unsigned long long t0 = global_ns();
+  unsigned long long last = global_ns(), spent = 0;
   while (true) {
     for (int i = 0; i < 64; i++)
       if (mbar_try_wait(bar, parity)) return true;
-    if (global_ns() - t0 > kWaitLimitNs) {
-      atomicOr(flag, code);
-      return false;
+    const unsigned long long now = global_ns(), gap = now - last;
+    last = now;
+    spent += gap < kWaitGapNs ? gap : kWaitGapNs;
+    if (spent > kWaitStopNs) {
+      if (stop && *stop) return false;
+      if (spent > kWaitLimitNs) {
+        if (stop) *stop = 1;
+        atomicOr(flag, code);
+        return false;
+      }
     }
   }
 }
