@@ -81,7 +81,9 @@ int so3gpu_forward_batch(so3gpu_context *ctx, void *const *flmn, const void *con
  * launch per Delta recursion -- signals sorted by (L, N) share 16-signal
  * operand tiles at the tile's largest L and N -- while every DFT stage runs
  * per signal in FP64; tiles whose padding would cost more than the products
- * save, real signals, and precision FP64 take the FP64 path per signal.  Same error contract as so3gpu_inverse_batch. */
+ * save (useful work below 8 of 16 signals inverse, 12 forward), real signals, and
+ * precision FP64 take the FP64 path per signal.  Same error contract as
+ * so3gpu_inverse_batch. */
 int so3gpu_inverse_ragged(so3gpu_context *ctx, void *const *f, const void *const *flmn,
                           const so3_parameters_t *parameters, int count, int precision);
 int so3gpu_forward_ragged(so3gpu_context *ctx, void *const *flmn, const void *const *f,
@@ -151,8 +153,10 @@ int so3gpu_inverse_noalloc(void *f, const void *flmn, const so3_parameters_t *pa
  * batching.  Up to max_inflight units run at once on separate streams;
  * queued complex split-precision (SO3GPU_PRECISION_MIXED_INT8) requests of
  * one direction are admitted together, up to max_batch per unit, whatever
- * their parameters (companions chosen by geometry; the unit's contractions
- * share the ragged tensor-core launch of so3gpu_inverse_ragged).  The
+ * their parameters, where their split contractions would fill enough of the
+ * tiles (companions chosen by geometry; the unit's contractions share the ragged
+ * tensor-core launch of so3gpu_inverse_ragged); other requests run in FP64, one
+ * to a unit unless several of the same parameters can share launches.  The
  * memory_budget covers the device's resident tables, the scratch of the
  * units in flight and the callers' buffers of those units; a unit is
  * admitted when a slot and the budget allow, first come first served, and a

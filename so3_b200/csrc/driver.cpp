@@ -366,15 +366,17 @@ int run_forward_staged(Device* D, Workspace* wk, const so3_parameters_t& p, int 
 namespace {
 
 // Workspace layout of a split-precision batch: nsig scratch plane sets, the
-// sliced operand, and the table of per-signal coefficient pointers.
+// sliced operand of the nsplit signals that the split contractions take (and of
+// the forward beta stage, which takes all), and the table of per-signal
+// coefficient pointers.
 struct BatchLayout {
   size_t wbytes, scratch_off, table_off, total;
 };
-BatchLayout batch_layout(const Geometry& g, const so3_parameters_t& p, int real, int nsig) {
+BatchLayout batch_layout(const Geometry& g, const so3_parameters_t& p, int real, int nsig, int nsplit, bool fwd) {
   BatchLayout b;
   b.wbytes = (workspace_bytes(p, real) + 255) & ~size_t(255);
   b.scratch_off = b.wbytes * nsig;
-  b.table_off = b.scratch_off + ((mixed_scratch_bytes(g, nsig) + 255) & ~size_t(255));
+  b.table_off = b.scratch_off + ((mixed_scratch_bytes(g, nsplit, fwd ? nsig : 0) + 255) & ~size_t(255));
   b.total = b.table_off + sizeof(void*) * (size_t)nsig;
   return b;
 }
@@ -396,11 +398,6 @@ int upload_table(void* dst, const void* const* ptrs, int nsig, cudaStream_t s) {
 // transform for n = 0).
 static bool split_real_ok(const so3_parameters_t& p, int real) { return !real || p.N > 1; }
 
-size_t batch_workspace_bytes(const so3_parameters_t& p, int real, int nsig, int precision) {
-  if (precision == kPrecFp64 || !split_real_ok(p, real) || nsig <= 0) return workspace_bytes(p, real);
-  return batch_layout(make_geometry(p, real), p, real, nsig).total;
-}
-
 // Signals of one geometry whose DFT stages (and FP64 contractions) share
 // launches: up to 192 MB of row-major scratch.  A small signal does not fill the
 // device and pays a launch gap per stage; inverse + forward of 64 signals, FP64,
@@ -412,6 +409,8 @@ static int batch_chunk(const Geometry& g, int nsig) {
   const int fit = (int)std::min<size_t>(kMaxBatch, (size_t(192) << 20) / std::max<size_t>(rows, 1));
   return std::max(1, std::min({nsig, fit, 65535 / g.nplanes}));
 }
+
+bool batch_shares(const so3_parameters_t& p, int real) { return batch_chunk(make_geometry(p, real), 2) > 1; }
 
 // Signals [b0, b0 + n) of a batch; io: their coefficient or sample arrays.
 static Batch batch_of(long long wstride, void* const* io, int b0, int n) {
@@ -529,20 +528,36 @@ static bool split_pays(bool fwd, double work, double largest) {
   return (e && *e) || work >= (fwd ? 12.0 : 8.0) * largest;
 }
 // Signals of a uniform batch that the split contractions take.
-static int split_count(bool fwd, int nsig) {
+int split_count(bool fwd, int nsig) {
   const int rest = nsig % 16;
   return rest == 0 || split_pays(fwd, rest, 1.0) ? nsig : nsig - rest;
+}
+static int split_signals_of(const so3_parameters_t& p, int real, int nsig, int precision, bool fwd) {
+  return precision == kPrecFp64 || !split_real_ok(p, real) ? 0 : split_count(fwd, nsig);
+}
+// Whether a batch runs in the split path's layout: any split contraction, or
+// forward the split beta stage, which needs no full tile of signals.
+static bool split_batch(const so3_parameters_t& p, int real, int nsig, int precision, bool fwd) {
+  if (split_signals_of(p, real, nsig, precision, fwd) > 0) return true;
+  return fwd && precision != kPrecFp64 && split_real_ok(p, real) && mixed_beta_supported(make_geometry(p, real));
+}
+
+size_t batch_workspace_bytes(const so3_parameters_t& p, int real, int nsig, int precision, bool fwd) {
+  const Geometry g = make_geometry(p, real);
+  if (nsig <= 0 || !split_batch(p, real, nsig, precision, fwd))
+    return ((workspace_bytes(p, real) + 255) & ~size_t(255)) * std::max(1, batch_chunk(g, nsig));
+  return batch_layout(g, p, real, nsig, split_signals_of(p, real, nsig, precision, fwd), fwd).total;
 }
 
 int run_inverse_batch(Device* D, Workspace* wk, const so3_parameters_t& p, int real, int nsig,
                       const void* const* flmn_d, void* const* f_d, int precision, cudaStream_t s) {
   if (nsig < 0) return fail(kInvalidParameter, "negative batch size");
   if (precision != kPrecFp64 && precision != kPrecMixedInt8) return fail(kInvalidParameter, "unknown precision");
-  const int nsplit = precision == kPrecFp64 || !split_real_ok(p, real) ? 0 : split_count(false, nsig);
-  if (nsplit == 0) return run_fp64_batch(D, wk, p, real, false, nsig, flmn_d, f_d, s);
+  const int nsplit = split_signals_of(p, real, nsig, precision, false);
+  if (!split_batch(p, real, nsig, precision, false)) return run_fp64_batch(D, wk, p, real, false, nsig, flmn_d, f_d, s);
   Resources r;
   if (int rc = acquire(D, wk, p, real, s, &r, false)) return rc;
-  const BatchLayout bl = batch_layout(r.g, p, real, nsig);
+  const BatchLayout bl = batch_layout(r.g, p, real, nsig, nsplit, false);
   void* ws = nullptr;
   if (int rc = ensure_ws(wk, bl.total, &ws)) return rc;
   char* base = static_cast<char*>(ws);
@@ -571,14 +586,13 @@ int run_forward_batch(Device* D, Workspace* wk, const so3_parameters_t& p, int r
                       void* const* flmn_d, int precision, cudaStream_t s) {
   if (nsig < 0) return fail(kInvalidParameter, "negative batch size");
   if (precision != kPrecFp64 && precision != kPrecMixedInt8) return fail(kInvalidParameter, "unknown precision");
-  // the split beta stage needs no full tile of signals; it stays with the split contractions
-  const int nsplit = precision == kPrecFp64 || !split_real_ok(p, real) ? 0 : split_count(true, nsig);
-  if (nsplit == 0 && (precision == kPrecFp64 || !split_real_ok(p, real) || !mixed_beta_supported(make_geometry(p, real))))
+  const int nsplit = split_signals_of(p, real, nsig, precision, true);
+  if (!split_batch(p, real, nsig, precision, true))
     return run_fp64_batch(D, wk, p, real, true, nsig, f_d, flmn_d, s);
   if (nsig == 0) return kOk;
   Resources r;
   if (int rc = acquire(D, wk, p, real, s, &r, true)) return rc;
-  const BatchLayout bl = batch_layout(r.g, p, real, nsig);
+  const BatchLayout bl = batch_layout(r.g, p, real, nsig, nsplit, true);
   void* ws = nullptr;
   if (int rc = ensure_ws(wk, bl.total, &ws)) return rc;
   char* base = static_cast<char*>(ws);
@@ -651,7 +665,7 @@ int run_conv_inverse_batch(Device* D, Workspace* wk, const so3_parameters_t& p, 
     }
     return kOk;
   }
-  const BatchLayout bl = batch_layout(r.g, p, 0, nsig);
+  const BatchLayout bl = batch_layout(r.g, p, 0, nsig, nsig, false);
   void* ws = nullptr;
   if ((rc = ensure_ws(wk, bl.total, &ws))) return rc;
   char* base = static_cast<char*>(ws);
@@ -682,17 +696,18 @@ struct RagItem {
   size_t ws_off;
 };
 
-// Signals of a ragged split-precision batch that take the FP64 path: real
-// ones, and those of tiles (16 signals, similar sizes together, per Delta
-// recursion as ragged_plan cuts them) whose padding costs more than the split
-// products save.
-std::vector<char> ragged_fp64(const so3_parameters_t* ps, int nsig, bool fwd) {
-  std::vector<char> f(nsig, 0);
+}  // namespace
+
+// Signals of a ragged split-precision batch that the split products take: not
+// the real ones, nor those of tiles (16 signals, similar sizes together, per Delta
+// recursion as ragged_plan cuts them) whose padding costs more than the products
+// save.
+std::vector<char> split_signals(const so3_parameters_t* ps, int nsig, bool fwd) {
+  std::vector<char> split(nsig, 0);
   for (int m = 0; m < 2; m++) {
     std::vector<int> order;
     for (int i = 0; i < nsig; i++) {
-      if (ps[i].reality) f[i] = 1;
-      else if (ps[i].dl_method == m) order.push_back(i);
+      if (!ps[i].reality && ps[i].dl_method == m) order.push_back(i);
     }
     std::stable_sort(order.begin(), order.end(),
                      [&](int x, int y) { return ps[x].L != ps[y].L ? ps[x].L > ps[y].L : ps[x].N > ps[y].N; });
@@ -704,12 +719,14 @@ std::vector<char> ragged_fp64(const so3_parameters_t* ps, int nsig, bool fwd) {
         work += (double)p.N * p.L * p.L * p.L;
         Lg = std::max(Lg, (double)p.L), Ng = std::max(Ng, (double)p.N);
       }
-      if (!split_pays(fwd, work, Ng * Lg * Lg * Lg))
-        for (size_t i = t; i < e; i++) f[order[i]] = 1;
+      if (split_pays(fwd, work, Ng * Lg * Lg * Lg))
+        for (size_t i = t; i < e; i++) split[order[i]] = 1;
     }
   }
-  return f;
+  return split;
 }
+
+namespace {
 
 // Signals of a ragged split-precision batch for the tensor-core contraction
 // (per Delta recursion), and those for the FP64 path.
@@ -729,9 +746,9 @@ int ragged_prepare(Device* D, const Workspace* wk, const so3_parameters_t* ps, i
         if (int rc = ensure_dl(D, Lmax[m], m, s, &t)) return rc;
   }
   size_t off = 0;
-  const std::vector<char> to_fp64 = ragged_fp64(ps, nsig, conv_tables);
+  const std::vector<char> split = split_signals(ps, nsig, conv_tables);
   for (int i = 0; i < nsig; i++) {
-    if (to_fp64[i]) {
+    if (!split[i]) {
       fp64->push_back(i);
       continue;
     }
@@ -752,16 +769,20 @@ size_t ragged_ws_end(const std::vector<RagItem>& items, const so3_parameters_t* 
 }  // namespace
 
 size_t ragged_workspace_bytes(const so3_parameters_t* ps, int nsig, bool fwd) {
-  size_t sig = 0;
+  size_t sig = 0, alone = 0;
   std::vector<RaggedSig> rs[2];
+  const std::vector<char> split = split_signals(ps, nsig, fwd);
   for (int i = 0; i < nsig; i++) {
-    if (ps[i].reality) continue;
+    if (!split[i]) {
+      alone = std::max(alone, workspace_bytes(ps[i], ps[i].reality != 0));
+      continue;
+    }
     sig += (workspace_bytes(ps[i], 0) + 255) & ~size_t(255);
     RaggedSig r{};
     r.g = make_geometry(ps[i], 0);
     rs[ps[i].dl_method & 1].push_back(r);
   }
-  return sig + std::max(ragged_scratch_bytes(rs[0], fwd), ragged_scratch_bytes(rs[1], fwd));
+  return std::max(alone, sig + std::max(ragged_scratch_bytes(rs[0], fwd), ragged_scratch_bytes(rs[1], fwd)));
 }
 
 int run_inverse_ragged(Device* D, Workspace* wk, const so3_parameters_t* ps, int nsig, const void* const* flmn_d,

@@ -1874,11 +1874,11 @@ static size_t colscale_bytes(const Geometry& g, int nsig) {
   return (size_t)nsig * (g.real ? g.N : 2 * g.N - 1) * (2 * (size_t)g.L - 1) * 2 * sizeof(double);
 }
 
-size_t mixed_scratch_bytes(const Geometry& g, int nsig) {
+size_t mixed_scratch_bytes(const Geometry& g, int nsig, int nbeta) {
   const size_t groups = (nsig + kSig - 1) / kSig, pairs = (size_t)g.L * g.N;
   const size_t contr = ((groups * pairs * nchunks(g) * (size_t)kXStage + 255) & ~size_t(255)) +
                        ((groups * pairs * kM * sizeof(double) + 255) & ~size_t(255)) + colscale_bytes(g, nsig) + 256;
-  return mixed_beta_supported(g) ? std::max(contr, beta_scratch_bytes(g, nsig)) : contr;
+  return nbeta && mixed_beta_supported(g) ? std::max(contr, beta_scratch_bytes(g, nbeta)) : contr;
 }
 
 static int mixed_args(const Geometry& g, int n_mode, int nsig, void* scratch, MixArgs* m, SliceArgs* s) {

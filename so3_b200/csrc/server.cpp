@@ -19,9 +19,10 @@
 //    (L, N) share the operand tiles at the tiles' largest L and N (identical
 //    parameters take the uniform batch path and its resident digit tables).
 //    Companions are picked from the queue by geometry so that the padded
-//    work stays at least half useful.  A split-precision unit of fewer than 4
-//    signals runs on the FP64 path (the fallback: the tensor-core operands
-//    hold 16 signals, so small batches would waste most of the products).
+//    work stays at least half useful and the drivers take them to the split
+//    contractions (the tensor-core operands hold 16 signals; units that would
+//    waste most of the products run on the FP64 path, a request a unit unless
+//    several of the same parameters share launches).
 //    A result depends on its companions only through that choice: within a
 //    split-precision batch the split is per signal and the int32
 //    accumulation exact, and the FP64 path is within the split tolerance.
@@ -238,14 +239,21 @@ class Server {
     sv->cv_.notify_all();
   }
 
-  // Precision a unit runs in: split precision pays only for batches of at
-  // least kMinSplitBatch signals (the tensor-core operand holds 16 signals and
-  // its scratch is sized per group of 16); smaller split-precision units run
-  // on the FP64 path, the fallback (more accurate, so still within the split
-  // tolerance).
-  static constexpr int kMinSplitBatch = 4;
+  // Precision a unit runs in: split where the split contractions take it, by the
+  // drivers' own rule (pick_unit leaves requests they would not take out of
+  // ragged units); else the FP64 path, the fallback (more accurate, so still within
+  // the split tolerance).
   static int unit_precision(const std::vector<Req*>& b) {
-    return (b[0]->precision == kPrecMixedInt8 && (int)b.size() >= kMinSplitBatch) ? kPrecMixedInt8 : kPrecFp64;
+    if (b[0]->precision != kPrecMixedInt8) return kPrecFp64;
+    const bool fwd = b[0]->kind == 1;
+    if (!unit_ragged(b)) return split_count(fwd, (int)b.size()) > 0 ? kPrecMixedInt8 : kPrecFp64;
+    const std::vector<char> split = split_signals(params_of(b).data(), (int)b.size(), fwd);
+    return std::find(split.begin(), split.end(), 1) != split.end() ? kPrecMixedInt8 : kPrecFp64;
+  }
+  static std::vector<so3_parameters_t> params_of(const std::vector<Req*>& b) {
+    std::vector<so3_parameters_t> ps;
+    for (const Req* q : b) ps.push_back(q->p);
+    return ps;
   }
   // A unit whose requests differ in parameters: the ragged drivers, which run
   // each signal with its own parameters (in split precision, one shared
@@ -260,16 +268,10 @@ class Server {
     const Req& r = *b[0];
     const int real = r.p.reality != 0;
     size_t need;
-    if (unit_ragged(b) && unit_precision(b) == kPrecMixedInt8) {
-      std::vector<so3_parameters_t> ps;
-      for (const Req* q : b) ps.push_back(q->p);
-      need = ragged_workspace_bytes(ps.data(), (int)ps.size(), r.kind == 1);
-    } else if (unit_ragged(b)) {  // FP64, one signal at a time in one workspace
-      need = 0;
-      for (const Req* q : b) need = std::max(need, workspace_bytes(q->p, q->p.reality != 0));
-    } else {
-      need = batch_workspace_bytes(r.p, real, (int)b.size(), unit_precision(b));
-    }
+    if (unit_ragged(b))
+      need = ragged_workspace_bytes(params_of(b).data(), (int)b.size(), r.kind == 1);
+    else
+      need = batch_workspace_bytes(r.p, real, (int)b.size(), unit_precision(b), r.kind == 1);
     if (r.kind == 2) need = ((need + 255) & ~size_t(255)) + (size_t)so3_sampling_flmn_size(&r.p) * sizeof(double2);
     for (const Req* q : b) need += buffer_bytes(*q);  // the callers' buffers count against the budget
     return need;
@@ -278,7 +280,10 @@ class Server {
   // Companions of the oldest queued request r0 for a split-precision unit:
   // queued requests that may share its tiles, taken in order of geometric
   // closeness while the unit's useful work stays at least half of its padded
-  // work (sum of L^3 N over count * Lmax^3 Nmax).
+  // work (sum of L^3 N over count * Lmax^3 Nmax).  Requests that the split products
+  // would not take stay out (they run side by side in other slots); r0 itself then
+  // runs in FP64, with queued requests of the same parameters where those share
+  // its launches.
   std::vector<Req*> pick_unit() const {
     Req* r0 = queue_.front();
     std::vector<Req*> unit{r0};
@@ -302,7 +307,16 @@ class Server {
       sum += work_of(q);
       Lm = L2, Nm = N2;
     }
-    return unit;
+    const std::vector<char> split = split_signals(params_of(unit).data(), (int)unit.size(), r0->kind == 1);
+    std::vector<Req*> taken{r0};
+    if (split[0]) {
+      for (size_t i = 1; i < unit.size(); i++)
+        if (split[i]) taken.push_back(unit[i]);
+    } else if (batch_shares(r0->p, 0)) {
+      for (size_t i = 1; i < scan && (int)taken.size() < max_batch_; i++)
+        if (same_params(*queue_[i], *r0)) taken.push_back(queue_[i]);
+    }
+    return taken;
   }
 
   // Enqueues the unit's work, the release of its scratch and the completion
@@ -408,6 +422,7 @@ class Server {
         size_t need = unit_bytes(unit);
         while (need > room && unit.size() > 1) {  // shrink the batch to fit
           unit.pop_back();
+          if (unit_ragged(unit) && unit_precision(unit) == kPrecFp64) unit.resize(1);
           need = unit_bytes(unit);
         }
         if (need > room) {  // can never run beside the resident tables

@@ -310,8 +310,9 @@ int stage_variants(const Geometry& g, const FftPlan& pP, const FftPlan& pg, cons
 // Split-precision (int8 tensor-core) contractions of a batch of complex
 // signals sharing one parameter set.  flmn_dev / W: per-signal coefficient
 // pointers (a device array of nsig pointers) and scratch planes (signal b at
-// W + b * wstride); scratch: mixed_scratch_bytes(g, nsig) bytes.
-size_t mixed_scratch_bytes(const Geometry& g, int nsig);
+// W + b * wstride); scratch: mixed_scratch_bytes bytes.
+// nsig signals in the contractions, nbeta (forward batches) in the beta stage
+size_t mixed_scratch_bytes(const Geometry& g, int nsig, int nbeta);
 // force: build now instead of on the geometry's second call.
 int ensure_digit_table(Device* D, const Geometry& g, int method, const double* dl, cudaStream_t s,
                        const DigitTable** out, bool force = false);
@@ -378,8 +379,14 @@ int run_inverse(Device* D, Workspace* wk, const so3_parameters_t& p, const void*
                 cudaStream_t s);
 int run_forward(Device* D, Workspace* wk, const so3_parameters_t& p, const void* f_d, void* flmn_d, int real,
                 cudaStream_t s);
-// Workspace bytes a batch of nsig signals needs (run_*_batch).
-size_t batch_workspace_bytes(const so3_parameters_t& p, int real, int nsig, int precision);
+// Workspace bytes a batch of nsig signals uses (run_*_batch).
+size_t batch_workspace_bytes(const so3_parameters_t& p, int real, int nsig, int precision, bool fwd);
+// Signals of a uniform split-precision batch, and which of a ragged one, whose
+// contractions the split products take; the others run FP64.
+int split_count(bool fwd, int nsig);
+std::vector<char> split_signals(const so3_parameters_t* ps, int nsig, bool fwd);
+// Whether FP64 batches of these parameters share launches.
+bool batch_shares(const so3_parameters_t& p, int real);
 // Batches: f_d / flmn_d are host arrays of nsig device pointers.
 int run_inverse_batch(Device* D, Workspace* wk, const so3_parameters_t& p, int real, int nsig,
                       const void* const* flmn_d, void* const* f_d, int precision, cudaStream_t s);
@@ -400,7 +407,7 @@ int run_adjoint_inverse(Device* D, Workspace* wk, const so3_parameters_t& p, con
                         cudaStream_t s);
 int run_adjoint_forward(Device* D, Workspace* wk, const so3_parameters_t& p, const void* flmn_d, void* f_d,
                         cudaStream_t s);
-// Workspace bytes of a split-precision ragged call (complex signals).
+// Workspace bytes of a split-precision ragged call.
 size_t ragged_workspace_bytes(const so3_parameters_t* ps, int nsig, bool fwd);
 // Directional convolutions of one S^2 signal flm with nsig kernels glm_d[b]
 // (so3_conv_s2toso3_harmonic_convolution with h parameters p) followed by the

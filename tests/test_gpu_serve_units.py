@@ -1,0 +1,29 @@
+"""Units of the request server that the split contractions do not take: they run
+in FP64, and reserve what that uses."""
+import pytest
+
+torch = pytest.importorskip("torch")
+import so3_b200 as so3
+from so3_b200 import serve
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("kind", ["inverse", "forward"])
+def test_small_units_reserve_no_split_scratch(kind):
+    n, batch = 32, 4
+    p = so3.SO3Parameters(L=128, N=16)
+    size = {"inverse": (so3.flmn_size(p), so3.f_size(p)), "forward": (so3.f_size(p), so3.flmn_size(p))}[kind]
+    x = torch.randn(2 * size[0], dtype=torch.float64, device="cuda").view(-1, 2)
+    x = torch.view_as_complex(x)
+    outs = [torch.empty(size[1], dtype=torch.complex128, device="cuda") for _ in range(n)]
+    torch.cuda.synchronize()
+    with serve.Server(0, memory_budget=8 << 30, max_inflight=1, max_batch=batch, max_L=128) as sv:
+        ids = [sv.submit(kind, p, x, o, "mixed") for o in outs]
+        res = [sv.wait(i) for i in ids]
+        peak = sv.stats()["peak_bytes"]
+    torch.cuda.synchronize()
+    assert all(r.status == 0 for r in res) and max(r.batch for r in res) == batch
+    assert all(torch.equal(torch.view_as_real(o), torch.view_as_real(outs[0])) for o in outs)
+    scratch = so3.api.workspace_size(p)  # 33 MB; the split operand of a tile would be 235 MB
+    assert peak < batch * (scratch + 16 * (size[0] + size[1])) + (64 << 20)
