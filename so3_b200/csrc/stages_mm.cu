@@ -511,8 +511,25 @@ int gamma_shift(int ng, int na, int rows) {
 
 }  // namespace
 
+// One matrix level costs ng / 4 pairs of products per sample, the scalar engines a
+// few passes, so long circles go back to them; how long depends on their radices.
+// us a stage, matrix / scalar, inverse at L = 128:
+//   complex, radices to 8   135: 76 / 82, 175: 114 / 95, 243: 225 / 181, 399 (L = 64) 239 / 82
+//            larger ones    171: 114 / 162, 207: 171 / 179, 231: 214 / 189, 279: 370 / 238
+//            Bluestein      265: 279 / 1253, 359: 587 / 1286, 419: 1290 / 1342 (L = 64: 418 / 337;
+//                           from 390 on a block's 16 columns leave one block to an SM)
+//   real     radices to 8   315: 144 / 158, 343: 173 / 148
+//            larger ones    351: 174 / 242, 399: 252 / 236
+//            Bluestein      599: 587 / 2565
+// Where the device does not fill (L < 49), a warp's chain of products is what takes
+// the time: complex, L = 32, 81: 13 / 13, 105: 14 / 13, 175: 23 / 15.  The choice
+// depends on the geometry alone, not on the batch: batches equal single calls.
 bool mm_gamma_ok(const Geometry& g, const FftPlan& p) {
-  return p.l1.p == g.ng && (size_t)g.ng * 18 * sizeof(double2) <= kSmemMax;
+  if (p.l1.p != g.ng || (size_t)g.ng * 18 * sizeof(double2) > kSmemMax) return false;
+  const int blocks = (g.na + 15) / 16 * g.nb;
+  if (g.real) return p.blue || g.ng < (p.big() ? 390 : 340);
+  if (p.blue) return g.ng < 390;
+  return g.ng < (blocks < 2 * 148 ? 100 : p.big() ? 220 : 172);
 }
 bool mm_ok(const FftPlan& p) { return p.mm.n == p.n && seq_smem(p.mm, 1, 2) <= kSmemMax; }
 

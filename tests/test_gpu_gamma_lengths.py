@@ -29,3 +29,18 @@ def test_long_gamma_circles_against_oracle(O, N, kw):
     rng = np.random.default_rng(N)
     f = rng.normal(size=f_ref.size) + (0 if p.reality else 1j * rng.normal(size=f_ref.size))
     assert rel_err(so3.forward(f, p), O.forward(f, op)) < TOL
+
+
+# the choice of engine by length and radices, on both sides of each line
+CHOICE = [(49, n, {}) for n in (86, 88, 110, 113, 195, 199)] + [(49, n, dict(reality=1)) for n in (169, 172, 191, 200)] \
+    + [(20, n, {}) for n in (50, 53)] + [(49, 90, dict(steerable=1))]
+
+
+@pytest.mark.parametrize("L,N,kw", CHOICE, ids=lambda v: str(v).replace(" ", ""))
+def test_either_engine_against_oracle(O, L, N, kw):
+    p = params(L, N, **kw)
+    op = oparams(O, p)
+    fl = synth.gen_flmn(p, N)
+    f_ref = O.inverse(fl, op)
+    assert rel_err(so3.inverse(fl, p), f_ref) < TOL
+    assert rel_err(so3.forward(f_ref, p), O.forward(f_ref, op)) < TOL
