@@ -79,26 +79,26 @@ int launch_build_dl_trapani(double* table, int L0cap, int Lcap, cudaStream_t s) 
 }
 
 // ---------------------------------------------------------------- Risbo
-// Work layout: two (Lcap+6)^2 layers, index (u+3)*S + (v+3) for u, v >= -3.
-// Layer A holds integer degree l on the eighth plus margin; layer H holds the
-// half degree l+1/2 with H(xp, yp) = d_{xp-1/2, yp-1/2}.
-__global__ void __launch_bounds__(1024) dl_risbo_sweep(double* __restrict__ T, int Lcap, double* __restrict__ work) {
+// Work layout: nine (Lcap+6)^2 layers, index (u+3)*S + (v+3) for u, v >= -3.
+// Layer l % 8 holds integer degree l on the eighth plus margin; the last one the
+// half degree l+1/2 with H(xp, yp) = d_{xp-1/2, yp-1/2}.  One CTA computes 8
+// degrees (from el0, a multiple of 8), then dl_risbo_pack puts them into their
+// blocks of the table with the whole device: the sweep's own 8-byte stores 64
+// bytes apart took as long as its arithmetic (Lcap = 512: 111 ms in all, 88 into
+// row-major planes).
+__global__ void __launch_bounds__(1024) dl_risbo_sweep(double* __restrict__ work, int Lcap, int el0) {
   const int S = Lcap + 6;
-  double* A = work;
-  double* H = work + (size_t)S * S;
+  double* A = nullptr;
+  double* H = work + 8 * (size_t)S * S;
 #define RA(u, v) A[((u) + 3) * S + ((v) + 3)]
 #define RH(u, v) H[((u) + 3) * S + ((v) + 3)]
   const int tid = threadIdx.x, nt = blockDim.x;
   const double c = 0.70710678118654752440084436210484903928;  // cos(pi/4) = sin(pi/4)
-  for (int i = tid; i < 2 * S * S; i += nt) work[i] = 0.0;
+  if (el0 == 0 && tid == 0) work[3 * S + 3] = 1.0;
   __syncthreads();
-  if (tid == 0) {
-    RA(0, 0) = 1.0;
-    T[0] = 1.0;
-  }
-  __syncthreads();
-  for (int el = 1; el < Lcap; el++) {
+  for (int el = max(el0, 1); el < el0 + 8; el++) {
     const int l = el - 1;
+    A = work + (l & 7) * (size_t)S * S;
     // margin of degree l
     for (int i = tid; i < 2 * (l + 1); i += nt) {
       const int u = i >> 1, v = u + 1 + (i & 1);
@@ -133,6 +133,7 @@ __global__ void __launch_bounds__(1024) dl_risbo_sweep(double* __restrict__ T, i
     }
     __syncthreads();
     // integer degree el on the eighth
+    A = work + (el & 7) * (size_t)S * S;
     {
       const int tJ = 2 * el;
       const double inv = 1.0 / tJ;
@@ -149,24 +150,35 @@ __global__ void __launch_bounds__(1024) dl_risbo_sweep(double* __restrict__ T, i
       }
     }
     __syncthreads();
-    // quarter plane el into the table
-    {
-      const int ld = el + 1;
-      for (int i = tid; i < ld * ld; i += nt) {
-        const int u = i / ld, v = i - u * ld;
-        T[dl_index(el, u, v)] = v <= u ? RA(u, v) : sgn(v - u) * RA(v, u);
-      }
-    }
-    __syncthreads();
   }
 #undef RA
 #undef RH
 }
 
+// Degrees 8 lc .. 8 lc + 7 from their layers into the table, one thread per entry.
+__global__ void dl_risbo_pack(double* __restrict__ T, const double* __restrict__ work, int Lcap, int lc) {
+  const int S = Lcap + 6, cols = 8 * (lc + 1), i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= 64 * cols * (lc + 1)) return;
+  const int at = i & 63, mu = (i >> 6) % cols, mp = 8 * ((i >> 6) / cols) + (at >> 3);
+  const int el = 8 * lc + ((at & 7) ^ (((mp >> 1) & 1) * 4));  // dl_slot
+  const double* A = work + (el & 7) * (size_t)S * S;
+  double v = 0.0;
+  if (mp <= el && mu <= el)
+    v = mu <= mp ? A[(mp + 3) * S + mu + 3] : sgn(mu - mp) * A[(mu + 3) * S + mp + 3];
+  T[dl_base(lc) + i] = v;
+}
+
+size_t risbo_work_bytes(int Lcap) { return 9 * (size_t)(Lcap + 6) * (Lcap + 6) * sizeof(double); }
+
+// Lcap: a multiple of 8; work: risbo_work_bytes(Lcap).
 int launch_build_dl_risbo(double* table, int Lcap, double* work, cudaStream_t s) {
-  SO3G_CUDA(cudaMemsetAsync(table, 0, (size_t)dl_entries(Lcap) * sizeof(double), s));
-  dl_risbo_sweep<<<1, 1024, 0, s>>>(table, Lcap, work);
-  SO3G_LAUNCHED();
+  SO3G_CUDA(cudaMemsetAsync(work, 0, risbo_work_bytes(Lcap), s));
+  for (int lc = 0; lc < Lcap / 8; lc++) {
+    dl_risbo_sweep<<<1, 1024, 0, s>>>(work, Lcap, 8 * lc);
+    SO3G_LAUNCHED();
+    dl_risbo_pack<<<2 * (lc + 1) * (lc + 1), 256, 0, s>>>(table, work, Lcap, lc);
+    SO3G_LAUNCHED();
+  }
   SO3G_CUDA(cudaGetLastError());
   return kOk;
 }

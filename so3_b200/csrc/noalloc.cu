@@ -6,8 +6,8 @@
 // cudaMalloc, cudaFree or any allocating routine: the transform scratch, the
 // Wigner Delta(pi/2) tables, the FFT tables and the block-offset table live
 // in the file-scope device arrays below, which every GPU that loads the
-// library holds until the process exits: kStaticBytes = 35,329,592 bytes
-// (33.7 MiB), of which 32 MiB are scratch.
+// library holds until the process exits: kStaticBytes = 35,251,192 bytes
+// (33.6 MiB), of which 32 MiB are scratch.
 //
 // Limits: complex, non-steerable signals only (reality != 0 or steerable !=
 // 0: status 3, before any device work -- a real signal's buffers are sized
@@ -50,25 +50,22 @@ constexpr size_t kScratchBytes = 32u << 20;
 constexpr int kMaxL = 64;
 constexpr int kMaxN = 64;
 constexpr int kDlEntries = 512 * (kMaxL / 8) * (kMaxL / 8 + 1) * (2 * (kMaxL / 8) + 1) / 6;  // dl_entries(kMaxL)
-constexpr int kRisboWork = 2 * (kMaxL + 6) * (kMaxL + 6);
 constexpr int kFftSlot = 2 * 256 + 2 * 128;  // Bluestein m + n + m, then n half-step roots, for n <= 128
 constexpr int kMaxPlanes = 2 * kMaxN - 1;
 
 static __device__ __align__(256) double2 g_scratch[kScratchBytes / sizeof(double2)];
 static __device__ __align__(256) double g_dl[2][kDlEntries];
-static __device__ __align__(256) double g_risbo_work[kRisboWork];
 static __device__ __align__(256) double2 g_fft[2][kFftSlot];
 static __device__ __align__(256) long long g_bases[kMaxPlanes];
-constexpr size_t kStaticBytes = kScratchBytes + sizeof(double) * (2 * (size_t)kDlEntries + kRisboWork) +
+constexpr size_t kStaticBytes = kScratchBytes + sizeof(double) * 2 * (size_t)kDlEntries +
                                 sizeof(double2) * 2 * kFftSlot + sizeof(long long) * kMaxPlanes;
-static_assert(kStaticBytes == 35329592, "the documented size of the static arrays");
+static_assert(kStaticBytes == 35251192, "the documented size of the static arrays");
 
 struct NoAllocDevice {
   bool ready = false;
   unsigned long long ctx_id = 0;  // context the set-up ran in
   double2* scratch = nullptr;
   double* dl[2] = {nullptr, nullptr};
-  double* risbo_work = nullptr;
   double2* fft = nullptr;
   long long* bases = nullptr;
   FftPlan plan[2]{};
@@ -214,10 +211,10 @@ int setup_device(NoAllocDevice& S, cudaStream_t s) {
   SO3G_CUDA(cudaGetSymbolAddress((void**)&S.scratch, g_scratch));
   SO3G_CUDA(cudaGetSymbolAddress((void**)&S.dl[0], g_dl));
   S.dl[1] = S.dl[0] + kDlEntries;
-  SO3G_CUDA(cudaGetSymbolAddress((void**)&S.risbo_work, g_risbo_work));
   SO3G_CUDA(cudaGetSymbolAddress((void**)&S.fft, g_fft));
   SO3G_CUDA(cudaGetSymbolAddress((void**)&S.bases, g_bases));
-  if (int rc = launch_build_dl_risbo(S.dl[SSHT_DL_RISBO], kMaxL, S.risbo_work, s)) return rc;
+  // the transform's scratch is free until the first call's own launches
+  if (int rc = launch_build_dl_risbo(S.dl[SSHT_DL_RISBO], kMaxL, reinterpret_cast<double*>(S.scratch), s)) return rc;
   if (int rc = launch_build_dl_trapani(S.dl[SSHT_DL_TRAPANI], 0, kMaxL, s)) return rc;
   SO3G_CUDA(cudaStreamSynchronize(s));
   S.ctx_id = id;

@@ -225,6 +225,7 @@ size_t resident_bytes(Device* D);
 
 // ---------------------------------------------------------------- launches
 int launch_build_dl_trapani(double* table, int L0cap, int Lcap, cudaStream_t s);
+size_t risbo_work_bytes(int Lcap);
 int launch_build_dl_risbo(double* table, int Lcap, double* work, cudaStream_t s);
 
 struct ModeInfo {

@@ -296,8 +296,7 @@ int ensure_dl(Device* D, int L, int method, cudaStream_t s, const double** out) 
     rc = launch_build_dl_trapani(d, 0, Lcap, s);
   } else {
     double* work = nullptr;
-    size_t wb = 2 * (size_t)(Lcap + 6) * (Lcap + 6) * sizeof(double);
-    e = cudaMalloc(&work, wb);
+    e = cudaMalloc(&work, risbo_work_bytes(Lcap));
     if (e != cudaSuccess) {
       cudaFree(d);
       return fail(kOutOfMemory, "Risbo work allocation failed");
