@@ -164,7 +164,9 @@ struct Angles {
   int P;
   __device__ __forceinline__ double2 at(long long j) const {  // (cos, sin)(pi j / P)
     j %= 2 * P;
-    if (j < 0) j += 2 * P;
+    return on_circle((int)(j < 0 ? j + 2 * P : j));
+  }
+  __device__ __forceinline__ double2 on_circle(int j) const {  // 0 <= j < 2 P
     const double2 e = half[j < P ? j : j - P];
     return j < P ? make_double2(e.x, -e.y) : make_double2(-e.x, e.y);
   }
@@ -187,8 +189,11 @@ __device__ double analysis_entry(const Angles& t, int L, int mw, int sc, int mp,
     if (self) return mp == L - 1 ? -2.0 * pi * pi * t.at((long long)(L - 2) * (2 * b + mw)).x / t.P : 0.0;
   }
   double acc = 0.0, low = 0.0;  // compensated: the terms cancel
-  for (int m = -(L - 1) + ((L - 1 + mp) & 1); m <= L - 1; m += 2) {
-    const double2 e = t.at((long long)m * (2 * b + mw));
+  const int first = -(L - 1) + ((L - 1 + mp) & 1), turn = 2 * t.P, step = 2 * (2 * b + mw) % turn;
+  int j = (int)((long long)first * (2 * b + mw) % turn);
+  if (j < 0) j += turn;
+  for (int m = first; m <= L - 1; m += 2, j = j + step < turn ? j + step : j + step - turn) {
+    const double2 e = t.on_circle(j);
     const double p = mp - m;
     const double term = (sc ? -2.0 * e.y : (self ? e.x : 2.0 * e.x)) * (2.0 / (1.0 - p * p));
     const double sum = acc + term, z = sum - acc;

@@ -27,7 +27,11 @@ static int acquire(Device* D, const Workspace* wk, const so3_parameters_t& p, in
   std::lock_guard<std::mutex> lk(D->mu);
   if (int rc = ensure_dl(D, p.L, p.dl_method, s, &r->dl)) return rc;
   if (int rc = ensure_fft(D, r->g.P, &r->pP)) return rc;
+  if (!mm_pays(r->pP))
+    if (int rc = ensure_fft_scalar(D, r->g.P, &r->pP)) return rc;
   if (int rc = ensure_fft(D, r->g.ng, &r->pg)) return rc;
+  if (!mm_gamma_ok(r->g, r->pg))
+    if (int rc = ensure_fft_scalar(D, r->g.ng, &r->pg)) return rc;
   if (int rc = ensure_bases(D, p, real, &r->bases)) return rc;
   // the inverse's matrix also for forward calls: either may be followed by a
   // captured inverse of the same parameters
@@ -36,7 +40,7 @@ static int acquire(Device* D, const Workspace* wk, const so3_parameters_t& p, in
   if (conv && beta_matrix_pays(r->g, kBetaForward)) {
     if (int rc = ensure_beta_matrix(D, r->g, kBetaForward, r->pP, s, &r->g.beta_mat[kBetaForward])) return rc;
   } else if (conv) {
-    if (int rc = ensure_fft(D, r->g.Pc, &r->pc)) return rc;
+    if (int rc = ensure_fft_scalar(D, r->g.Pc, &r->pc)) return rc;
     if (int rc = ensure_conv_kernel(D, r->g, &r->wr)) return rc;
   }
   return kOk;
@@ -80,7 +84,7 @@ static int ensure_tuned(Device* D, const so3_parameters_t& p, int real, Resource
       if (beta_matrix_pays(g, kBetaForward)) {
         if (int rc = ensure_beta_matrix(D, g, kBetaForward, r->pP, s, &mat)) return rc;
       } else {
-        if (int rc = ensure_fft(D, g.Pc, &pc)) return rc;
+        if (int rc = ensure_fft_scalar(D, g.Pc, &pc)) return rc;
         if (int rc = ensure_conv_kernel(D, g, &wr)) return rc;
       }
     }

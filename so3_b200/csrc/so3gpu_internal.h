@@ -120,8 +120,9 @@ __host__ __device__ inline long long dl_entries(int Lcap) { return dl_base((Lcap
 
 struct DevPlan {
   FftPlan plan{};
-  double2* mem = nullptr;     // owns roots/mroots/chirp/kern/half
-  double2* mm_mem = nullptr;  // own the tensor-core plan's tables
+  double2* mem = nullptr;         // owns half
+  double2* scalar_mem = nullptr;  // owns roots/mroots/chirp/kern
+  double2* mm_mem = nullptr;      // own the tensor-core plan's tables
   int* mm_imem = nullptr;
   size_t mm_bytes = 0;
 };
@@ -205,6 +206,8 @@ Device* device_state(int device);  // lazily created per CUDA device
 
 int ensure_dl(Device* D, int L, int method, cudaStream_t s, const double** out);
 int ensure_fft(Device* D, int n, FftPlan* out);
+// The same with the tables of the scalar engines, which few lengths need (mm_pays, mm_gamma_ok).
+int ensure_fft_scalar(Device* D, int n, FftPlan* out);
 // Tensor-core plan of length n into F->mm and F->l1 (dft_plan.cpp); the caller
 // owns *mem and *imem (device memory, *bytes in total).
 int build_mm_plan(int n, FftPlan* F, double2** mem, int** imem, size_t* bytes);
@@ -276,6 +279,7 @@ int launch_fwd_beta_conv(const Geometry& g, const FftPlan& pP, const FftPlan& pc
 // build_mm_plan covered.
 bool mm_gamma_ok(const Geometry& g, const FftPlan& p);
 bool mm_ok(const FftPlan& p);
+bool mm_pays(const FftPlan& p);  // alpha and inverse beta
 int launch_mm_inv_gamma(const Geometry& g, const FftPlan& p, const double2* W, void* f, cudaStream_t s, int row_lo,
                         int row_hi, const Batch& bt);
 int launch_mm_fwd_gamma(const Geometry& g, const FftPlan& p, const void* f, double2* W, cudaStream_t s, int row_lo,

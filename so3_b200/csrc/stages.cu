@@ -724,7 +724,7 @@ static int each(const Batch& bt, const F& run) {
 // Where the tensor-core DFT replaces the scalar engines below: every length
 // but the 1023 of the compile-time plan (us per 31-plane transform at L = 512,
 // inverse beta / inverse alpha: 276 / 191 against 225 / 175).
-static bool mm_pays(const FftPlan& p) { return mm_ok(p) && pick(p) != Eng::k1023; }
+bool mm_pays(const FftPlan& p) { return mm_ok(p) && pick(p) != Eng::k1023; }
 
 int launch_inv_beta(const Geometry& g, const FftPlan& p, double2* W, cudaStream_t s, const Batch& bt) {
   if (g.beta_mat[kBetaInverse]) return launch_beta_matrix(g, kBetaInverse, g.beta_mat[kBetaInverse], W, s, bt);

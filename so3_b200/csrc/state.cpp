@@ -159,7 +159,11 @@ size_t resident_bytes(Device* D) {
     g.nb = g.mw ? g.L : g.L + 1;
     b += beta_matrix_bytes(g, kv.first % kBetaKinds);
   }
-  for (const auto& kv : D->ffts) b += (size_t)4 * (kv.first + 256) * sizeof(double2) + kv.second->mm_bytes;
+  for (const auto& kv : D->ffts) {
+    const FftPlan& P = kv.second->plan;
+    const size_t scalar = kv.second->scalar_mem ? (P.blue ? 2 * P.m + P.n : P.n) : 0;
+    b += (P.n + scalar) * sizeof(double2) + kv.second->mm_bytes;
+  }
   for (const auto& kv : D->bases) b += 4096 * sizeof(long long);
   return b;
 }
@@ -375,16 +379,10 @@ int ensure_fft(Device* D, int n, FftPlan* out) {
   auto dp = std::make_unique<DevPlan>();
   FftPlan& P = dp->plan;
   P.n = n;
-  int np = factor_stockham(n, P.rad);
-  std::vector<double2> host;
+  const int np = factor_stockham(n, P.rad);
   if (np >= 0) {
     P.npass = np;
     P.blue = 0;
-    host.resize(n);
-    for (int k = 0; k < n; k++) {
-      cld r = root_l(k, n);
-      host[k] = make_double2((double)r.real(), (double)r.imag());
-    }
   } else {
     int m = 1;
     while (m < 2 * n - 1) m <<= 1;
@@ -392,6 +390,37 @@ int ensure_fft(Device* D, int n, FftPlan* out) {
     P.m = m;
     P.npass = 0;
     P.mpass = factor_stockham(m, P.mrad);
+  }
+  std::vector<double2> host(n);
+  for (int k = 0; k < n; k++) {
+    cld r = root_l(k, 2LL * n);  // e^{-i pi k/n}
+    host[k] = make_double2((double)r.real(), (double)r.imag());
+  }
+  cudaError_t e = cudaMalloc(&dp->mem, host.size() * sizeof(double2));
+  if (e != cudaSuccess) return fail(kOutOfMemory, "FFT table allocation failed");
+  e = upload(dp->mem, host.data(), host.size() * sizeof(double2));
+  if (e != cudaSuccess) return fail(kCudaError, std::string("FFT table upload: ") + cudaGetErrorString(e));
+  P.half = dp->mem;
+  if (int rc = build_mm_plan(n, &P, &dp->mm_mem, &dp->mm_imem, &dp->mm_bytes)) return rc;
+  *out = P;
+  D->ffts[key] = std::move(dp);
+  return kOk;
+}
+
+int ensure_fft_scalar(Device* D, int n, FftPlan* out) {
+  if (int rc = ensure_fft(D, n, out)) return rc;
+  DevPlan* dp = D->ffts[n].get();
+  FftPlan& P = dp->plan;
+  if (dp->scalar_mem) return kOk;
+  std::vector<double2> host;
+  if (!P.blue) {
+    host.resize(n);
+    for (int k = 0; k < n; k++) {
+      cld r = root_l(k, n);
+      host[k] = make_double2((double)r.real(), (double)r.imag());
+    }
+  } else {
+    const int m = P.m;
     host.resize((size_t)m + n + m);
     for (int k = 0; k < m; k++) {
       cld r = root_l(k, m);
@@ -412,27 +441,23 @@ int ensure_fft(Device* D, int n, FftPlan* out) {
       host[(size_t)m + n + k] = make_double2((double)v.real(), (double)v.imag());
     }
   }
-  const size_t half_at = host.size();
-  host.resize(half_at + n);
-  for (int k = 0; k < n; k++) {
-    cld r = root_l(k, 2LL * n);  // e^{-i pi k/n}
-    host[half_at + k] = make_double2((double)r.real(), (double)r.imag());
-  }
-  cudaError_t e = cudaMalloc(&dp->mem, host.size() * sizeof(double2));
+  double2* d = nullptr;
+  cudaError_t e = cudaMalloc(&d, host.size() * sizeof(double2));
   if (e != cudaSuccess) return fail(kOutOfMemory, "FFT table allocation failed");
-  e = upload(dp->mem, host.data(), host.size() * sizeof(double2));
-  if (e != cudaSuccess) return fail(kCudaError, std::string("FFT table upload: ") + cudaGetErrorString(e));
-  P.half = dp->mem + half_at;
-  if (!P.blue) {
-    P.roots = dp->mem;
-  } else {
-    P.mroots = dp->mem;
-    P.chirp = dp->mem + P.m;
-    P.kern = dp->mem + P.m + n;
+  e = upload(d, host.data(), host.size() * sizeof(double2));
+  if (e != cudaSuccess) {
+    cudaFree(d);
+    return fail(kCudaError, std::string("FFT table upload: ") + cudaGetErrorString(e));
   }
-  if (int rc = build_mm_plan(n, &P, &dp->mm_mem, &dp->mm_imem, &dp->mm_bytes)) return rc;
+  dp->scalar_mem = d;
+  if (!P.blue) {
+    P.roots = d;
+  } else {
+    P.mroots = d;
+    P.chirp = d + P.m;
+    P.kern = d + P.m + n;
+  }
   *out = P;
-  D->ffts[key] = std::move(dp);
   return kOk;
 }
 
