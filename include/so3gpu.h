@@ -132,7 +132,7 @@ int so3gpu_set_stage_variants(int device, const so3_parameters_t *p, const int *
  * implicit device synchronisation) after start-up.  f and flmn are device
  * pointers; stream is a cudaStream_t (NULL: legacy default stream).  Its
  * scratch, Wigner tables and FFT tables are file-scope device arrays of
- * 35,251,192 bytes in total (32 MiB of them scratch), held by every GPU that
+ * 35,509,240 bytes in total (32 MiB of them scratch), held by every GPU that
  * loads the library until exit.  Complex, non-steerable signals only:
  * reality != 0 or steerable != 0 return status 3 before any device work.
  * L > 64, N > 64 or more than 32 MiB of scratch return status 3 (MW and MWSS

@@ -139,38 +139,34 @@ unsigned magic(int d) { return d < 2 ? 0u : (unsigned)((0x100000000ULL + d - 1) 
 // primes; Bluestein's over the cheapest m in [2n-1, 2.3n]).  A convolution
 // runs two transforms of length m and touches its points about five more
 // times; measured against one level, primes change over near 320.
-int build_mm_plan(int n, FftPlan* F, double2** mem, int** imem, size_t* bytes) {
+void mm_plan_host(int n, bool with_mm, bool with_l1, FftPlan* F, MmTables* T) {
   MmPlan P{};
-  *mem = nullptr;
-  *imem = nullptr;
-  *bytes = 0;
+  MmLevel one{};
+  std::vector<double2>& host = T->host;
+  std::vector<int>& perm = T->perm;
+  if (with_l1 && n <= kMaxLevel) level_shape(n, false, &one);  // the real gamma kernels take q = 0 from the tiles
+  if (one.p) level_table(one, &host);
   int a = n, b = 1;
-  double best = n <= kMaxLevel ? level_cost(n) : 1e30;
-  P.kind = n <= kMaxLevel ? 1 : 0;
-  {
+  if (with_mm) {
+    double best = n <= kMaxLevel ? level_cost(n) : 1e30;
+    P.kind = n <= kMaxLevel ? 1 : 0;
     int ta = 0, tb = 0;
     const double c = two_level_cost(n, &ta, &tb);
     if (c < best) best = c, P.kind = 2, a = ta, b = tb;
+    if (n > 64) {
+      int m = 0, ca = 0, cb = 0;
+      bool rader = false;
+      double conv = 1e30;
+      auto consider = [&](int len, bool r) {
+        int ta = 0, tb = 0;
+        const double c = (2.0 * two_level_cost(len, &ta, &tb) + 40.0) * len / n;
+        if (c < conv) conv = c, m = len, ca = ta, cb = tb, rader = r;
+      };
+      if (is_prime(n)) consider(n - 1, true);
+      for (int len = 2 * n - 1; len <= 2 * n + 3 * n / 10; len++) consider(len, false);
+      if (conv < best) best = conv, P.kind = 3, P.rader = rader, P.m = m, a = ca, b = cb;
+    }
   }
-  if (n > 64) {
-    int m = 0, ca = 0, cb = 0;
-    bool rader = false;
-    double conv = 1e30;
-    auto consider = [&](int len, bool r) {
-      int ta = 0, tb = 0;
-      const double c = (2.0 * two_level_cost(len, &ta, &tb) + 40.0) * len / n;
-      if (c < conv) conv = c, m = len, ca = ta, cb = tb, rader = r;
-    };
-    if (is_prime(n)) consider(n - 1, true);
-    for (int len = 2 * n - 1; len <= 2 * n + 3 * n / 10; len++) consider(len, false);
-    if (conv < best) best = conv, P.kind = 3, P.rader = rader, P.m = m, a = ca, b = cb;
-  }
-  MmLevel one{};
-  if (n <= kMaxLevel) level_shape(n, false, &one);  // the real gamma kernels take q = 0 from the tiles
-  std::vector<double2> host;
-  std::vector<int> perm;
-  size_t at_one = 0, at_a = 0, at_b = 0, at_tw = 0, at_chirp = 0, at_kern = 0;
-  if (one.p) level_table(one, &host);
   if (P.kind) {
     P.n = n;
     P.a = a;
@@ -180,7 +176,7 @@ int build_mm_plan(int n, FftPlan* F, double2** mem, int** imem, size_t* bytes) {
     P.mdiv_a = magic(a);
     P.mdiv_b = magic(b);
     if (P.kind == 1) {
-      at_a = host.size();
+      T->at_a = host.size();
       level_table(P.la, &host);
       P.ts = n;
       while (P.ts % 8 != 4) P.ts++;
@@ -192,11 +188,11 @@ int build_mm_plan(int n, FftPlan* F, double2** mem, int** imem, size_t* bytes) {
       // a sequence buffer also holds the n outputs, and the two columns (n + 1 entries) of
       // an inverse beta pair; a Rader plan transforms only n - 1
       if (P.ts < n + 1) P.ts = n + 1;
-      at_a = host.size();
+      T->at_a = host.size();
       level_table(P.la, &host);
-      at_b = host.size();
+      T->at_b = host.size();
       level_table(P.lb, &host);
-      at_tw = host.size();
+      T->at_tw = host.size();
       std::vector<cld> w(P.m);
       for (int k = 0; k < P.m; k++) w[k] = root_l(k, P.m);
       for (int n2 = 0; n2 < b; n2++)
@@ -213,7 +209,7 @@ int build_mm_plan(int n, FftPlan* F, double2** mem, int** imem, size_t* bytes) {
         for (int j = 0; j < P.m; j++) perm.push_back(pw[(P.m - j) % P.m]);
         for (int j = 0; j < P.m; j++) v[j] = root_l(perm[P.m + j], n);
       } else {
-        at_chirp = host.size();
+        T->at_chirp = host.size();
         for (int k = 0; k < n; k++) {
           const cld c = root_l((long long)k * k % (2LL * n), 2LL * n);
           host.push_back(to_d2(c));
@@ -221,26 +217,40 @@ int build_mm_plan(int n, FftPlan* F, double2** mem, int** imem, size_t* bytes) {
           if (k) v[P.m - k] = std::conj(c);
         }
       }
-      at_kern = host.size();
+      T->at_kern = host.size();
       for (const cld& x : dft_host(v, a, b)) host.push_back(to_d2(x / (long double)P.m));
     }
   }
-  if (host.empty()) {  // length 1: no entries to multiply
-    F->mm = P;
-    F->l1 = one;
-    return kOk;
-  }
-  *bytes = host.size() * sizeof(double2) + perm.size() * sizeof(int);
-  cudaError_t e = cudaMalloc(mem, host.size() * sizeof(double2));
-  if (e == cudaSuccess && !perm.empty()) e = cudaMalloc(imem, perm.size() * sizeof(int));
+  F->mm = P;
+  F->l1 = one;
+}
+
+void mm_plan_device(const MmTables& T, const double2* mem, const int* imem, FftPlan* F) {
+  F->l1.tab = mem;
+  F->mm.la.tab = mem + T.at_a;
+  F->mm.lb.tab = mem + T.at_b;
+  F->mm.tw = mem + T.at_tw;
+  F->mm.chirp = mem + T.at_chirp;
+  F->mm.kern = mem + T.at_kern;
+  F->mm.perm = imem;
+}
+
+int build_mm_plan(int n, FftPlan* F, double2** mem, int** imem, size_t* bytes) {
+  MmTables T;
+  mm_plan_host(n, true, true, F, &T);
+  *mem = nullptr;
+  *imem = nullptr;
+  *bytes = T.host.size() * sizeof(double2) + T.perm.size() * sizeof(int);
+  if (T.host.empty()) return kOk;  // length 1: no entries to multiply
+  cudaError_t e = cudaMalloc(mem, T.host.size() * sizeof(double2));
+  if (e == cudaSuccess && !T.perm.empty()) e = cudaMalloc(imem, T.perm.size() * sizeof(int));
   if (e != cudaSuccess) {
     cudaFree(*mem);
     *mem = nullptr;
     return fail(kOutOfMemory, "DFT table allocation failed");
   }
-  e = upload(*mem, host.data(), host.size() * sizeof(double2));
-  if (e == cudaSuccess && !perm.empty())
-    e = upload(*imem, perm.data(), perm.size() * sizeof(int));
+  e = upload(*mem, T.host.data(), T.host.size() * sizeof(double2));
+  if (e == cudaSuccess && !T.perm.empty()) e = upload(*imem, T.perm.data(), T.perm.size() * sizeof(int));
   if (e != cudaSuccess) {
     cudaFree(*mem);
     cudaFree(*imem);
@@ -248,15 +258,7 @@ int build_mm_plan(int n, FftPlan* F, double2** mem, int** imem, size_t* bytes) {
     *imem = nullptr;
     return fail(kCudaError, std::string("DFT table upload: ") + cudaGetErrorString(e));
   }
-  one.tab = *mem + at_one;
-  P.la.tab = *mem + at_a;
-  P.lb.tab = *mem + at_b;
-  P.tw = *mem + at_tw;
-  P.chirp = *mem + at_chirp;
-  P.kern = *mem + at_kern;
-  P.perm = *imem;
-  F->mm = P;
-  F->l1 = one;
+  mm_plan_device(T, *mem, *imem, F);
   return kOk;
 }
 

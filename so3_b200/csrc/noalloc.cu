@@ -4,10 +4,10 @@
 // device, under an allocator or memory cap owned by someone else, or in a
 // real-time loop that forbids allocation after start-up).  It never calls
 // cudaMalloc, cudaFree or any allocating routine: the transform scratch, the
-// Wigner Delta(pi/2) tables, the FFT tables and the block-offset table live
+// Wigner Delta(pi/2) tables, the DFT and beta tables and the block-offset table live
 // in the file-scope device arrays below, which every GPU that loads the
-// library holds until the process exits: kStaticBytes = 35,251,192 bytes
-// (33.6 MiB), of which 32 MiB are scratch.
+// library holds until the process exits: kStaticBytes = 35,509,240 bytes
+// (33.9 MiB), of which 32 MiB are scratch.
 //
 // Limits: complex, non-steerable signals only (reality != 0 or steerable !=
 // 0: status 3, before any device work -- a real signal's buffers are sized
@@ -23,7 +23,7 @@
 // is keyed by the context's unique id, so a call from a new context (after
 // cudaDeviceReset, or a context made with the driver API) sets up again.  A
 // later call whose band limits, storage or n-order differ from the previous
-// call's uploads new FFT and offset tables from host memory with
+// call's uploads new DFT and offset tables from host memory with
 // cudaMemcpyAsync; make such calls outside capture too (a captured region may
 // only repeat the configuration of the call before it).
 //
@@ -31,6 +31,7 @@
 // each call writes every scratch entry before it reads it, so nothing needs
 // clearing.  Calls whose GPU work overlaps (different streams, or different
 // host threads) race on the shared arrays: serialise them.
+#include <algorithm>
 #include <cmath>
 #include <complex>
 #include <cstdio>
@@ -50,16 +51,22 @@ constexpr size_t kScratchBytes = 32u << 20;
 constexpr int kMaxL = 64;
 constexpr int kMaxN = 64;
 constexpr int kDlEntries = 512 * (kMaxL / 8) * (kMaxL / 8 + 1) * (2 * (kMaxL / 8) + 1) / 6;  // dl_entries(kMaxL)
-constexpr int kFftSlot = 2 * 256 + 2 * 128;  // Bluestein m + n + m, then n half-step roots, for n <= 128
+// DFT tables of lengths up to 128: scalar or half-step roots, then the matrix plan's
+// (one level, at most 9 row tiles x 16 steps x 32 entries; two levels and their
+// twiddles are shorter, and no such length takes a convolution).
+constexpr int kRoots = 128;
+constexpr int kFftSlot = kRoots + 9 * 16 * 32;
+constexpr int kBetaMat = 2 * 16 * 16 * 32;  // beta_matrix_bytes(kBetaInverse) at L = 64, 16 row tiles x 16 steps
 constexpr int kMaxPlanes = 2 * kMaxN - 1;
 
 static __device__ __align__(256) double2 g_scratch[kScratchBytes / sizeof(double2)];
 static __device__ __align__(256) double g_dl[2][kDlEntries];
 static __device__ __align__(256) double2 g_fft[2][kFftSlot];
+static __device__ __align__(256) double g_beta[kBetaMat];
 static __device__ __align__(256) long long g_bases[kMaxPlanes];
-constexpr size_t kStaticBytes = kScratchBytes + sizeof(double) * 2 * (size_t)kDlEntries +
+constexpr size_t kStaticBytes = kScratchBytes + sizeof(double) * (2 * (size_t)kDlEntries + kBetaMat) +
                                 sizeof(double2) * 2 * kFftSlot + sizeof(long long) * kMaxPlanes;
-static_assert(kStaticBytes == 35251192, "the documented size of the static arrays");
+static_assert(kStaticBytes == 35509240, "the documented size of the static arrays");
 
 struct NoAllocDevice {
   bool ready = false;
@@ -67,6 +74,7 @@ struct NoAllocDevice {
   double2* scratch = nullptr;
   double* dl[2] = {nullptr, nullptr};
   double2* fft = nullptr;
+  double* beta = nullptr;
   long long* bases = nullptr;
   FftPlan plan[2]{};
   int plan_n[2] = {0, 0};
@@ -101,76 +109,27 @@ int factor_small(int n, int* rad) {  // same radix order as the allocating plann
   return n == 1 ? np : -1;
 }
 
-// radix-2 FFT in long double on a fixed-size host array (m <= 256)
-void fft_ld_fixed(cld* x, int n, int sign) {
-  for (int i = 1, j = 0; i < n; i++) {
-    int bit = n >> 1;
-    for (; j & bit; bit >>= 1) j ^= bit;
-    j ^= bit;
-    if (i < j) std::swap(x[i], x[j]);
-  }
-  for (int len = 2; len <= n; len <<= 1)
-    for (int i = 0; i < n; i += len)
-      for (int k = 0; k < len / 2; k++) {
-        cld w = root_l(k, len);
-        if (sign > 0) w = std::conj(w);
-        const cld u = x[i + k], v = x[i + k + len / 2] * w;
-        x[i + k] = u + v;
-        x[i + k + len / 2] = u - v;
-      }
-}
-
-// Half-step roots e^{-i pi k/n} of a plan, at slot offset `at`.
-void half_table(int n, FftPlan* P, double2* h, const double2* dev, int at) {
-  for (int k = 0; k < n; k++) {
-    const cld r = root_l(k, 2LL * n);
-    h[at + k] = make_double2((double)r.real(), (double)r.imag());
-  }
-  P->half = dev + at;
-}
-
-// Fills plan tables for length n into host slot h; device pointers point at dev.
-void plan_tables(int n, FftPlan* P, double2* h, const double2* dev) {
+// Plan of length n with its tables in host slot h (device: dev): the alpha stage's
+// (half-step roots, as the beta matrix takes them, and matrix tables), or the gamma
+// stage's (one-level tables, and the scalar engines' roots for lengths that mm_gamma_ok refuses).
+int plan_tables(int n, bool gamma, FftPlan* P, double2* h, const double2* dev) {
   *P = FftPlan{};
   P->n = n;
   const int np = factor_small(n, P->rad);
-  if (np >= 0) {
-    P->npass = np;
-    for (int k = 0; k < n; k++) {
-      const cld r = root_l(k, n);
-      h[k] = make_double2((double)r.real(), (double)r.imag());
-    }
-    P->roots = dev;
-    half_table(n, P, h, dev, n);
-    return;
-  }
-  int m = 1;
-  while (m < 2 * n - 1) m <<= 1;
-  P->blue = 1;
-  P->m = m;
-  P->mpass = factor_small(m, P->mrad);
-  for (int k = 0; k < m; k++) {
-    const cld r = root_l(k, m);
+  P->blue = np < 0;  // such gamma lengths run on the matrix
+  P->npass = np < 0 ? 0 : np;
+  for (int k = 0; k < n; k++) {
+    const cld r = root_l(k, gamma ? n : 2LL * n);
     h[k] = make_double2((double)r.real(), (double)r.imag());
   }
-  cld ch[128];
-  cld ker[256];
-  for (int k = 0; k < n; k++) {
-    ch[k] = root_l(((long long)k * k) % (2LL * n), 2LL * n);
-    h[m + k] = make_double2((double)ch[k].real(), (double)ch[k].imag());
-  }
-  for (int k = 0; k < m; k++) ker[k] = cld(0, 0);
-  ker[0] = std::conj(ch[0]);
-  for (int k = 1; k < n; k++) ker[k] = ker[m - k] = std::conj(ch[k]);
-  fft_ld_fixed(ker, m, -1);
-  for (int k = 0; k < m; k++) {
-    const cld v = ker[k] / (long double)m;
-    h[m + n + k] = make_double2((double)v.real(), (double)v.imag());
-  }
-  P->mroots = dev;
-  P->chirp = dev + m;
-  P->kern = dev + m + n;
-  half_table(n, P, h, dev, 2 * m + n);
+  (gamma ? P->roots : P->half) = dev;
+  MmTables T;
+  mm_plan_host(n, !gamma, gamma, P, &T);
+  if (T.host.size() > kFftSlot - kRoots || !T.perm.empty())
+    return fail(kUnsupported, "so3gpu_inverse_noalloc: DFT tables exceed their static array");
+  std::copy(T.host.begin(), T.host.end(), h + kRoots);
+  mm_plan_device(T, dev + kRoots, nullptr, P);
+  return kOk;
 }
 
 // Unique id of the calling thread's current CUDA context, through the driver
@@ -212,6 +171,7 @@ int setup_device(NoAllocDevice& S, cudaStream_t s) {
   SO3G_CUDA(cudaGetSymbolAddress((void**)&S.dl[0], g_dl));
   S.dl[1] = S.dl[0] + kDlEntries;
   SO3G_CUDA(cudaGetSymbolAddress((void**)&S.fft, g_fft));
+  SO3G_CUDA(cudaGetSymbolAddress((void**)&S.beta, g_beta));
   SO3G_CUDA(cudaGetSymbolAddress((void**)&S.bases, g_bases));
   // the transform's scratch is free until the first call's own launches
   if (int rc = launch_build_dl_risbo(S.dl[SSHT_DL_RISBO], kMaxL, reinterpret_cast<double*>(S.scratch), s)) return rc;
@@ -239,14 +199,19 @@ int run(void* f, const void* flmn, const so3_parameters_t* p, cudaStream_t s) {
   std::lock_guard<std::mutex> lk(g_mu);
   NoAllocDevice& S = g_state[dev];
   if (int rc = setup_device(S, s)) return rc;
-  const Geometry g = make_geometry(*p, 0);
+  Geometry g = make_geometry(*p, 0);
+  if (beta_matrix_bytes(g, kBetaInverse) > kBetaMat * sizeof(double))
+    return fail(kUnsupported, "so3gpu_inverse_noalloc: beta matrix exceeds its static array");
   const int lens[2] = {g.P, g.ng};
+  bool uploaded = false;
   for (int i = 0; i < 2; i++) {
     if (S.plan_n[i] != lens[i]) {
       double2* dev_slot = S.fft + (size_t)i * kFftSlot;
-      plan_tables(lens[i], &S.plan[i], S.host_fft[i], dev_slot);
+      S.plan_n[i] = 0;
+      if (int rc = plan_tables(lens[i], i == 1, &S.plan[i], S.host_fft[i], dev_slot)) return rc;
       SO3G_CUDA(cudaMemcpyAsync(dev_slot, S.host_fft[i], sizeof(double2) * kFftSlot, cudaMemcpyHostToDevice, s));
       S.plan_n[i] = lens[i];
+      uploaded = true;
     }
   }
   char key[64];
@@ -256,7 +221,16 @@ int run(void* f, const void* flmn, const so3_parameters_t* p, cudaStream_t s) {
     for (size_t i = 0; i < b.size(); i++) S.host_bases[i] = b[i];
     SO3G_CUDA(cudaMemcpyAsync(S.bases, S.host_bases, sizeof(long long) * b.size(), cudaMemcpyHostToDevice, s));
     strcpy(S.bases_key, key);
+    uploaded = true;
   }
+  // Also after uploads that leave the matrix as it is: the transform's kernels read
+  // tables before they wait for the kernel before them, which comes after the copies.
+  if (uploaded)
+    if (int rc = launch_beta_matrix_table(g, kBetaInverse, S.plan[0], S.beta, s)) {
+      S.plan_n[0] = 0;
+      return rc;
+    }
+  g.beta_mat[kBetaInverse] = S.beta;
   double2* W = S.scratch;
   const double* dl = S.dl[p->dl_method];
   if (int rc = launch_inverse_contract(g, p->n_mode, static_cast<const double2*>(flmn), S.bases, dl, W, 0, s))

@@ -211,6 +211,15 @@ int ensure_fft_scalar(Device* D, int n, FftPlan* out);
 // Tensor-core plan of length n into F->mm and F->l1 (dft_plan.cpp); the caller
 // owns *mem and *imem (device memory, *bytes in total).
 int build_mm_plan(int n, FftPlan* F, double2** mem, int** imem, size_t* bytes);
+// The same in two steps, for tables that live elsewhere: the plan and its tables
+// on the host (F->mm, F->l1 as asked), then the plan's pointers into their copy.
+struct MmTables {
+  std::vector<double2> host;
+  std::vector<int> perm;
+  size_t at_a = 0, at_b = 0, at_tw = 0, at_chirp = 0, at_kern = 0;  // the one-level tables come first
+};
+void mm_plan_host(int n, bool with_mm, bool with_l1, FftPlan* F, MmTables* T);
+void mm_plan_device(const MmTables& T, const double2* mem, const int* imem, FftPlan* F);
 int ensure_conv_kernel(Device* D, const Geometry& g, const double2** out);
 int ensure_beta_matrix(Device* D, const Geometry& g, int kind, const FftPlan& pP, cudaStream_t s, const double** out);
 int ensure_bases(Device* D, const so3_parameters_t& p, int real, const long long** out);
