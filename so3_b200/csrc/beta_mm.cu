@@ -15,8 +15,8 @@
 //
 // The product costs 2 L multiply-adds per point and reads and writes the
 // planes once; the DFT chain of the forward stage is three to four transforms
-// of 2L or 4L points, so the matrix wins up to a few hundred (see
-// beta_matrix_ok).  A CTA takes 8 MT WR rows x 8 NP WC columns: a warp holds
+// of 2L or 4L points, so the matrix wins wherever those have no compile-time plan
+// (see beta_matrix_pays).  A CTA takes 8 MT WR rows x 8 NP WC columns: a warp holds
 // MT row tiles of NP column tiles of either parity (4 complex columns each),
 // so the two 16-byte values that a lane holds of columns 2c, 2c+1 complete
 // each other's sectors.  Matrix fragments are stored in MMA lane order; both
@@ -246,7 +246,7 @@ int go(const Geometry& g, const BetaMmArgs& a, int nsig, cudaStream_t s) {
 // The adjoints have no other path.
 bool beta_matrix_pays(const Geometry& g, int kind) {
   if (kind == kBetaInverse) return g.L <= 96;
-  if (kind == kBetaForward) return !(g.L == 512 && g.mw);
+  if (kind == kBetaForward) return !conv_chain(g);
   return true;
 }
 

@@ -135,9 +135,9 @@ __device__ __forceinline__ void task(const double2* __restrict__ src, int rp, co
   }
 }
 
-// One level over ncols columns, tasks (up to MTMAX row tiles) dealt to the
+// One level over ncols columns, tasks (up to two row tiles) dealt to the
 // warps of the CTA.
-template <int MTMAX, bool INV, class Off, class Out>
+template <bool INV, class Off, class Out>
 __device__ __forceinline__ void level(const double2* __restrict__ src, int rp, const MmLevel& lv, int ncols,
                                       const Off& off, const Out& out) {
   const int warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
@@ -149,12 +149,8 @@ __device__ __forceinline__ void level(const double2* __restrict__ src, int rp, c
     const int mt = min(lv.MT, lv.QT - qt0);
     if (mt == 1)
       task<1, INV>(src, rp, lv, qt0, j0, ncols, off, out);
-    else if (mt == 2 || MTMAX == 2)
-      task<2, INV>(src, rp, lv, qt0, j0, ncols, off, out);
-    else if (mt == 3)
-      task<3, INV>(src, rp, lv, qt0, j0, ncols, off, out);
     else
-      task<MTMAX, INV>(src, rp, lv, qt0, j0, ncols, off, out);
+      task<2, INV>(src, rp, lv, qt0, j0, ncols, off, out);
     jc += nwarps;
     while (jc >= nc) jc -= nc, gi++;
   }
@@ -227,7 +223,7 @@ __device__ __forceinline__ void first_level(const MmPlan& P, const double2* A, d
     const int t = fastdiv(j, db);
     return t * ts + (j - t * b);
   };
-  level<2, INV>(A, ldb, FLIP ? P.lb : P.la, T * b, off,
+  level<INV>(A, ldb, FLIP ? P.lb : P.la, T * b, off,
                 TwiddleOut<INV>{Z, P.tw, b, lda, ts, FLIP ? 1 : a, FLIP ? b : 1, db});
 }
 template <bool INV, bool FLIP, class Out>
@@ -238,7 +234,7 @@ __device__ __forceinline__ void second_level(const MmPlan& P, const double2* Z, 
     const int t = fastdiv(j, da);
     return t * ts + (j - t * a);
   };
-  level<2, INV>(Z, lda, FLIP ? P.la : P.lb, T * a, off, SplitOut<Out>{out, a, da});
+  level<INV>(Z, lda, FLIP ? P.la : P.lb, T * a, off, SplitOut<Out>{out, a, da});
 }
 
 // Stages entry n (0 <= n < P.n) of a sequence: x(n) returns it.  Convolution
@@ -312,7 +308,7 @@ template <bool INV, class Out>
 __device__ __forceinline__ void run(const MmPlan& P, double2* A, double2* Z, int T, double2* x0, const Out& out) {
   if (P.kind == 1) {
     const int ts = P.ts;
-    level<2, INV>(A, 1, P.la, T, [&](int j) { return j * ts; }, PlainOut<Out>{out});
+    level<INV>(A, 1, P.la, T, [&](int j) { return j * ts; }, PlainOut<Out>{out});
   } else if (P.kind == 2) {
     first_level<INV, false>(P, A, Z, T);
     __syncthreads();

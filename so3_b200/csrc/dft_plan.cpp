@@ -88,8 +88,7 @@ void level_shape(int p, bool sum_apart, MmLevel* v) {
   v->KS = (v->H + 3) / 4;
   v->q0 = sum_apart && v->H > 0 && v->H % 8 == 0;
   v->QT = v->q0 ? v->H / 8 : v->H / 8 + 1;
-  v->QG = (v->QT + 3) / 4;
-  v->MT = (v->QT + v->QG - 1) / v->QG;
+  v->MT = v->QT < 2 ? v->QT : 2;
   v->QG = (v->QT + v->MT - 1) / v->MT;
 }
 

@@ -88,7 +88,7 @@ static int ensure_tuned(Device* D, const so3_parameters_t& p, int real, Resource
         if (int rc = ensure_conv_kernel(D, g, &wr)) return rc;
       }
     }
-    if (int rc = autotune_stages(&g, r->pP, r->pg, pc, wr, W, s, 3)) return rc;
+    if (int rc = autotune_stages(&g, r->pP, pc, wr, W, s, 3)) return rc;
   }
   std::lock_guard<std::mutex> lk(D->mu);
   D->tuned[key] = std::vector<signed char>(g.var, g.var + 8);

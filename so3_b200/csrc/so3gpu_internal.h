@@ -151,7 +151,7 @@ struct Device {
   std::map<std::string, std::vector<signed char>> tuned;  // stage variants by geometry key
   DlTable dl[2];                                 // per dl_method
   std::map<int, std::unique_ptr<DevPlan>> ffts;  // by length
-  std::map<int, double2*> conv_kernels;          // forward-beta weight tables by 2L + (MW)
+  std::map<int, double2*> conv_kernels;          // forward-beta weight tables by L
   std::map<int, double*> beta_matrices;          // by (2L + (MW)) * kBetaKinds + kind
   std::map<std::string, long long*> bases;       // block bases by parameter key
   std::vector<std::unique_ptr<DigitTable>> digit_tables;
@@ -288,7 +288,8 @@ int launch_fwd_beta_conv(const Geometry& g, const FftPlan& pP, const FftPlan& pc
 // build_mm_plan covered.
 bool mm_gamma_ok(const Geometry& g, const FftPlan& p);
 bool mm_ok(const FftPlan& p);
-bool mm_pays(const FftPlan& p);  // alpha and inverse beta
+bool mm_pays(const FftPlan& p);      // alpha and inverse beta
+bool conv_chain(const Geometry& g);  // forward beta through DFT and weight convolution
 int launch_mm_inv_gamma(const Geometry& g, const FftPlan& p, const double2* W, void* f, cudaStream_t s, int row_lo,
                         int row_hi, const Batch& bt);
 int launch_mm_fwd_gamma(const Geometry& g, const FftPlan& p, const void* f, double2* W, cudaStream_t s, int row_lo,
@@ -316,10 +317,10 @@ int launch_zero(void* p, size_t bytes, cudaStream_t s);
 // the workspace W (its contents are scratch; results are discarded) and
 // writes the fastest into g->var.  Synchronises stream s: never call it while
 // s is being captured.  reps timed launches per variant after one warm-up.
-int autotune_stages(Geometry* g, const FftPlan& pP, const FftPlan& pg, const FftPlan& pc, const double2* wr,
-                    double2* W, cudaStream_t s, int reps);
+int autotune_stages(Geometry* g, const FftPlan& pP, const FftPlan& pc, const double2* wr, double2* W, cudaStream_t s,
+                    int reps);
 // Number of kernel variants the tuner can choose from for a stage.
-int stage_variants(const Geometry& g, const FftPlan& pP, const FftPlan& pg, const FftPlan& pc, int stage);
+int stage_variants(const Geometry& g, const FftPlan& pP, int stage);
 
 // Split-precision (int8 tensor-core) contractions of a batch of complex
 // signals sharing one parameter set.  flmn_dev / W: per-signal coefficient

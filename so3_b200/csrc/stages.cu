@@ -61,15 +61,8 @@ template <bool BIG>
 struct Gen {
   static constexpr bool fixed = false;
   static constexpr int NT = kThreads, MINB = BIG ? 1 : 2, T = 0, LD = 0, nP = 0;
-  static constexpr bool has_out = false;
-  template <class Out>
-  static __device__ __forceinline__ void runPOut(double2*, double2*, const FftPlan&, const Out&) {}
   static __device__ __forceinline__ int at(int k) { return k; }
-  static __device__ __forceinline__ int atC(int k) { return k; }
   static __device__ __forceinline__ double2* runP(double2* a, double2* b, int T_, int ld, const FftPlan& P) {
-    return fft_fwd_smem<BIG>(a, b, T_, ld, P);
-  }
-  static __device__ __forceinline__ double2* runC(double2* a, double2* b, int T_, int ld, const FftPlan& P) {
     return fft_fwd_smem<BIG>(a, b, T_, ld, P);
   }
 };
@@ -80,11 +73,10 @@ struct Fix {
   static constexpr int NT = NT_, MINB = MINB_, T = T_;
   static constexpr int ldP = PP<1, 1, 1>::ld, ldC = PC<1, 1, 1>::ld;
   static constexpr int nP = PP<1, 1, 1>::n;  // runP length
-  // the runP plan's last pass can store through a callable (1023 = 31*11*3)
-  static constexpr bool has_out = nP == 1023;
+  // the last pass of the 1023 = 31*11*3 plan can store through a callable
   template <class Out>
   static __device__ __forceinline__ void runPOut(double2* a, double2* b, const FftPlan& P, const Out& out) {
-    if constexpr (has_out) PP<T_, LD, NT_>::run_out(a, b, P, out);
+    if constexpr (nP == 1023) PP<T_, LD, NT_>::run_out(a, b, P, out);
   }
   static constexpr int ldmax = ldP > ldC ? ldP : ldC;
   // pitch = 8/T (mod 8) 16-byte slots: the T sequences of one index, which
@@ -473,10 +465,11 @@ __global__ void __launch_bounds__(E::NT, E::MINB) fwd_alpha_pf_kernel(Geometry g
   }
 }
 
-// Forward beta stage, two columns per pipeline.  Per column (plane n,
+// Forward beta stage of MW signals at the compile-time lengths (conv_chain), two
+// columns per pipeline.  Per column (plane n,
 // order m, s = (-1)^{m+n}): extend the beta samples onto the circle with
-// x(mirror(b)) = s x(b) (mirror(b) = 2L-2-b for MW, 2L-b for MWSS), DFT,
-// divide by P, MW phase e^{-i m'' pi/P}, convolve with the quadrature weights
+// x(2L-2-b) = s x(b), DFT,
+// divide by P, phase e^{-i m'' pi/P}, convolve with the quadrature weights
 // w (so3_sampling.c:32-51) through a power-of-two oversampled product and
 // fold G(m') + s G(-m') onto m' >= 0.  The spectrum v of an s = +1 column is
 // even in m'', that of an s = -1 column odd, and w = w_e + w_o with w_e the
@@ -485,26 +478,24 @@ __global__ void __launch_bounds__(E::NT, E::MINB) fwd_alpha_pf_kernel(Geometry g
 //   out_A(m') = G(m') + G(-m')   (m' >= 1),   out_A(0) = G(0)
 //   out_B(m') = G(m') - G(-m')   (m' >= 1),   out_B(0) = i pi^2 (v(1) - v(-1))
 // (the terms of w_o cancel in both folds except in out_B(0)).  This holds for
-// the antisymmetric part of B; B's samples at its self-mirror rows (MW: row
-// L-1; MWSS: rows 0 and L), which the unpaired extension keeps as they are,
-// are taken out of the pipeline and added back through the stage's response
-// to a unit sample there (the vectors h of the weight table).  Sequence t of
+// the antisymmetric part of B; B's sample at its self-mirror row L-1, which the
+// unpaired extension keeps as it is, is taken out of the pipeline and added back
+// through the stage's response to a unit sample there (the vector h of the weight
+// table).  Sequence t of
 // a CTA is column pair q = blockIdx.x * T + t (columns 2q, 2q+1).
 template <class E>
 __global__ void __launch_bounds__(E::NT, E::MINB) fwd_beta_conv_kernel(Geometry g, FftPlan P, FftPlan Pc,
                                                                   const double2* __restrict__ wr,
-                                                                  double2* __restrict__ W, int T_, int ld_) {
+                                                                  double2* __restrict__ W) {
   extern __shared__ double2 sm[];
-  constexpr int TS = E::fixed ? E::T : 8;
-  __shared__ double2 selfB[TS][2];  // B's samples at its self-mirror rows
-  __shared__ double2 b0[TS];        // out_B(0)
-  const int T = E::fixed ? E::T : T_, ld = E::fixed ? E::LD : ld_;
+  constexpr int T = E::T, ld = E::LD;
+  __shared__ double2 selfB[T];  // B's sample at its self-mirror row
+  __shared__ double2 b0[T];     // out_B(0)
   double2* a = sm;
   double2* b = sm + (size_t)T * ld;
   const int plane = blockIdx.y, n = plane - g.plane0;
   const int q0 = blockIdx.x * T, L = g.L, ncols = 2 * L - 1, Pn = g.P, pc = g.Pc;
   const bool first_is_a = ((L - 1 + n) & 1) == 0;  // column 2q has m + n even
-  const int sm0 = g.mw ? L - 1 : 0, sm1 = g.mw ? -1 : L;
   const double2* base = W + (long long)plane * g.PS;
   auto fetch = [&](int t, int row, double2& v0, double2& v1) {
     const int c = 2 * (q0 + t);
@@ -514,36 +505,26 @@ __global__ void __launch_bounds__(E::NT, E::MINB) fwd_beta_conv_kernel(Geometry 
   auto put = [&](int t, int row, double2 v0, double2 v1) {
     const double2 A = first_is_a ? v0 : v1;
     double2 B = first_is_a ? v1 : v0;
-    if (row == sm0 || row == sm1) {
-      selfB[t][row == sm0 ? 0 : 1] = B;
+    if (row == L - 1) {
+      selfB[t] = B;
       B = make_double2(0.0, 0.0);
     }
     a[t * ld + E::at(row)] = cadd(A, B);
-    const int mr = g.mw ? 2 * L - 2 - row : 2 * L - row;  // mirror row on the extended circle
+    const int mr = 2 * L - 2 - row;  // mirror row on the extended circle
     if (mr >= g.nb && mr < Pn) a[t * ld + E::at(mr)] = csub(A, B);
   };
-  constexpr int LC = E::fixed ? (E::nP + 1) / 2 : 0;  // nb of the MW circle of an odd fixed plan
-  if (E::fixed && g.nb == LC) {  // all loads of a sequence before its first shared-memory store
-    constexpr int NI = E::fixed ? (LC + E::NT - 1) / E::NT : 1;
-    for (int t = 0; t < T; t++) {
-      double2 v0[NI], v1[NI];
+  constexpr int LC = (E::nP + 1) / 2, NI = (LC + E::NT - 1) / E::NT;  // rows of the circle
+  for (int t = 0; t < T; t++) {  // all loads of a sequence before its first shared-memory store
+    double2 v0[NI], v1[NI];
 #pragma unroll
-      for (int i = 0; i < NI; i++) {
-        const int row = threadIdx.x + i * E::NT;
-        if (row < LC) fetch(t, row, v0[i], v1[i]);
-      }
-#pragma unroll
-      for (int i = 0; i < NI; i++) {
-        const int row = threadIdx.x + i * E::NT;
-        if (row < LC) put(t, row, v0[i], v1[i]);
-      }
+    for (int i = 0; i < NI; i++) {
+      const int row = threadIdx.x + i * E::NT;
+      if (row < LC) fetch(t, row, v0[i], v1[i]);
     }
-  } else {
-    for (int idx = threadIdx.x; idx < g.nb * T; idx += E::NT) {
-      const int t = idx % T, row = idx / T;
-      double2 v0, v1;
-      fetch(t, row, v0, v1);
-      put(t, row, v0, v1);
+#pragma unroll
+    for (int i = 0; i < NI; i++) {
+      const int row = threadIdx.x + i * E::NT;
+      if (row < LC) put(t, row, v0[i], v1[i]);
     }
   }
   __syncthreads();
@@ -558,11 +539,8 @@ __global__ void __launch_bounds__(E::NT, E::MINB) fwd_beta_conv_kernel(Geometry 
   __syncthreads();
   for (int idx = threadIdx.x; idx < T * (2 * L - 1); idx += E::NT) {
     const int t = idx / (2 * L - 1), mpp = idx - t * (2 * L - 1) - (L - 1);
-    double2 v = cscale(r[t * ld + E::at(wrapi(mpp, Pn))], invP);
-    if (g.mw) {  // e^{-i pi m''/(2L-1)}
-      const double2 e = __ldg(P.half + (mpp < 0 ? -mpp : mpp));
-      v = cmul(v, mpp < 0 ? cconj(e) : e);
-    }
+    const double2 e = __ldg(P.half + (mpp < 0 ? -mpp : mpp));  // e^{-i pi m''/(2L-1)}
+    const double2 v = cmul(cscale(r[t * ld + E::at(wrapi(mpp, Pn))], invP), mpp < 0 ? cconj(e) : e);
     o[t * ld + E::atC(wrapi(mpp, pc))] = cconj(v);
   }
   __syncthreads();
@@ -584,8 +562,7 @@ __global__ void __launch_bounds__(E::NT, E::MINB) fwd_beta_conv_kernel(Geometry 
   double2* q2 = (q == a) ? b : a;
   double2* G = E::runC(q, q2, T, ld, Pc);
   double2* cbase = W + g.QOFF + (long long)plane * g.QS;  // column-major output
-  const double2* h0 = wr + pc;
-  const double2* h1 = wr + pc + L;
+  const double2* h = wr + pc;
   for (int idx = threadIdx.x; idx < L * T; idx += E::NT) {
     const int mp = idx % L, t = idx / L, c = 2 * (q0 + t);  // m' fastest: whole columns written contiguously
     if (c >= ncols) continue;
@@ -596,8 +573,7 @@ __global__ void __launch_bounds__(E::NT, E::MINB) fwd_beta_conv_kernel(Geometry 
       oa = cadd(gp, gm);
       ob = csub(gp, gm);
     }
-    ob = cadd(ob, cmul(selfB[t][0], __ldg(h0 + mp)));
-    if (!g.mw) ob = cadd(ob, cmul(selfB[t][1], __ldg(h1 + mp)));
+    ob = cadd(ob, cmul(selfB[t], __ldg(h + mp)));
     const int ca = first_is_a ? c : c + 1, cb = first_is_a ? c + 1 : c;
     if (ca < ncols) cbase[(long long)ca * g.CS + mp] = oa;
     if (cb < ncols) cbase[(long long)cb * g.CS + mp] = ob;
@@ -697,11 +673,9 @@ int fwd_alpha(const Geometry& g, const FftPlan& p, double2* W, cudaStream_t s) {
 template <class E>
 int fwd_beta_conv(const Geometry& g, const FftPlan& p, const FftPlan& pc, const double2* wr, double2* W,
                   cudaStream_t s) {
-  const int ld = p.ld() > pc.ld() ? p.ld() : pc.ld();
-  const Sizing z = sizing<E>(ld, 8);
-  dim3 grid((g.L + z.T - 1) / z.T, g.nplanes);  // L column pairs per plane
-  if (int rc = set_smem(fwd_beta_conv_kernel<E>, z.smem)) return rc;
-  fwd_beta_conv_kernel<E><<<grid, E::NT, z.smem, s>>>(g, p, pc, wr, W, z.T, ld);
+  dim3 grid((g.L + E::T - 1) / E::T, g.nplanes);  // L column pairs per plane
+  if (int rc = set_smem(fwd_beta_conv_kernel<E>, E::smem())) return rc;
+  fwd_beta_conv_kernel<E><<<grid, E::NT, E::smem(), s>>>(g, p, pc, wr, W);
   return kOk;
 }
 
@@ -819,44 +793,39 @@ int launch_fwd_alpha(const Geometry& g, const FftPlan& p, double2* W, cudaStream
   return rc ? rc : launched();
 }
 
-namespace {
-bool conv_fixed(const FftPlan& p, const FftPlan& pc) { return pick(p) == Eng::k1023 && !pc.blue && pc.n == 2048; }
-}  // namespace
+// The lengths that the chain of DFT and weight convolution has compile-time plans for.
+bool conv_chain(const Geometry& g) { return g.P == 1023 && g.Pc == 2048; }
 
 int launch_fwd_beta_conv(const Geometry& g, const FftPlan& p, const FftPlan& pc, const double2* wr, double2* W,
                          cudaStream_t s, const Batch& bt) {
   if (g.beta_mat[kBetaForward]) return launch_beta_matrix(g, kBetaForward, g.beta_mat[kBetaForward], W, s, bt);
   if (bt.n) return each(bt, [&](int b) { return launch_fwd_beta_conv(g, p, pc, wr, W + b * bt.wstride, s); });
-  int rc;
-  if (conv_fixed(p, pc))
-    rc = g.var[kStFwdBetaConv] == 1 ? fwd_beta_conv<EConv1023b>(g, p, pc, wr, W, s)
-                                    : fwd_beta_conv<EConv1023a>(g, p, pc, wr, W, s);
-  else
-    return fail(kUnsupported, "forward beta stage: no plan for this length");
+  const int rc = g.var[kStFwdBetaConv] == 1 ? fwd_beta_conv<EConv1023b>(g, p, pc, wr, W, s)
+                                            : fwd_beta_conv<EConv1023a>(g, p, pc, wr, W, s);
   return rc ? rc : launched();
 }
 
 // ------------------------------------------------------------------ autotuner
-int stage_variants(const Geometry& g, const FftPlan& pP, const FftPlan& pg, const FftPlan& pc, int stage) {
+int stage_variants(const Geometry& g, const FftPlan& pP, int stage) {
   switch (stage) {
     case kStInvBeta:
     case kStInvAlpha:
     case kStFwdAlpha:
       return pick(pP) == Eng::k1023 ? 4 : 1;
-    case kStFwdBetaConv: return conv_fixed(pP, pc) ? 2 : 1;
+    case kStFwdBetaConv: return conv_chain(g) ? 2 : 1;
     default: return 1;
   }
 }
 
-int autotune_stages(Geometry* g, const FftPlan& pP, const FftPlan& pg, const FftPlan& pc, const double2* wr,
-                    double2* W, cudaStream_t s, int reps) {
-  const int stages[] = {kStInvBeta, kStInvAlpha, kStInvGamma, kStFwdGamma, kStFwdAlpha, kStFwdBetaConv};
+int autotune_stages(Geometry* g, const FftPlan& pP, const FftPlan& pc, const double2* wr, double2* W, cudaStream_t s,
+                    int reps) {
+  const int stages[] = {kStInvBeta, kStInvAlpha, kStFwdAlpha, kStFwdBetaConv};
   cudaEvent_t e0, e1;
   SO3G_CUDA(cudaEventCreate(&e0));
   SO3G_CUDA(cudaEventCreate(&e1));
   int rc = kOk;
   for (int st : stages) {
-    const int nv = stage_variants(*g, pP, pg, pc, st);
+    const int nv = stage_variants(*g, pP, st);
     if (nv <= 1) {
       g->var[st] = 0;
       continue;
@@ -869,8 +838,6 @@ int autotune_stages(Geometry* g, const FftPlan& pP, const FftPlan& pg, const Fft
         switch (st) {
           case kStInvBeta: return launch_inv_beta(*g, pP, W, s);
           case kStInvAlpha: return launch_inv_alpha(*g, pP, W, s);
-          case kStInvGamma: return launch_inv_gamma(*g, pg, W, W, s);  // samples written over the scratch
-          case kStFwdGamma: return launch_fwd_gamma(*g, pg, W, W, s);
           case kStFwdAlpha: return launch_fwd_alpha(*g, pP, W, s);
           default: return launch_fwd_beta_conv(*g, pP, pc, wr, W, s);
         }

@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(kGT, 6) inv_gamma_mm_kernel(Geometry g, MmLeve
   dep_launch();
   const long long plane_sz = (long long)g.nb * g.na;
   double2* dst = f + (long long)row * g.na + a0;
-  mm::level<2, true>(sm, rp, lv, nc, [](int j) { return j; }, InvGammaOut{dst, plane_sz, g.nf});
+  mm::level<true>(sm, rp, lv, nc, [](int j) { return j; }, InvGammaOut{dst, plane_sz, g.nf});
 }
 
 // Complex forward; steerable: samples N..2N-1 of the circle are zero and only
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(kGT, 6) fwd_gamma_mm_kernel(Geometry g, MmLeve
   dep_launch();
   const double scale = 2.0 * 3.141592653589793238462643383279502884 / g.nf;
   double2* dst = W + (long long)row * g.RS + a0;
-  mm::level<2, false>(sm, rp, lv, nc, [](int j) { return j; },
+  mm::level<false>(sm, rp, lv, nc, [](int j) { return j; },
             FwdGammaOut{dst, g.PS, scale, g.N, ng, g.plane0, g.steer});
 }
 
@@ -491,15 +491,10 @@ Shape shape_for(const MmPlan& P0, int nseq, int bufs) {
   return z;
 }
 
-// Gamma kernels: two row tiles per warp task (80 registers, 24 warps per SM;
-// four tiles at 128 registers and 16 warps: 766 against 697 us at L = 512, N = 64,
-// 277 / 241 at N = 32, 255 / 177 at L = 1024, N = 8).
-MmLevel gamma_level(const FftPlan& p) {
-  MmLevel lv = p.l1;
-  lv.MT = std::min(2, lv.QT);
-  lv.QG = (lv.QT + lv.MT - 1) / lv.MT;
-  return lv;
-}
+// Gamma kernels: two row tiles per warp task, as level_shape sets them (80 registers,
+// 24 warps per SM; four tiles at 128 registers and 16 warps: 766 against 697 us at
+// L = 512, N = 64, 277 / 241 at N = 32, 255 / 177 at L = 1024, N = 8).
+//
 // log2 of the alpha samples per CTA: the planes of six CTAs fit in shared memory
 // and a CTA has four tasks or more (L = 1024, N = 2: 16 samples 224 us, 256: 78; N = 8:
 // 16: 292, 64: 177; L = 512, N = 32: 16: 241, 32: 253), fewer where the device would not fill.
@@ -536,7 +531,7 @@ bool mm_ok(const FftPlan& p) { return p.mm.n == p.n && seq_smem(p.mm, 1, 2) <= k
 int launch_mm_inv_gamma(const Geometry& g, const FftPlan& p, const double2* W, void* f, cudaStream_t s, int row_lo,
                         int row_hi, const Batch& bt) {
   int sh = gamma_shift(g.ng, g.na, (row_hi - row_lo) * count(bt));
-  const MmLevel lv = gamma_level(p);
+  const MmLevel& lv = p.l1;
   const int rows = g.real ? g.nplanes : g.ng;
   while (sh > 4 && (size_t)rows * ((1 << sh) + 2) * sizeof(double2) > kSmemMax / 4) sh--;
   const size_t smem = (size_t)rows * ((1 << sh) + 2) * sizeof(double2);
@@ -551,7 +546,7 @@ int launch_mm_inv_gamma(const Geometry& g, const FftPlan& p, const double2* W, v
 int launch_mm_fwd_gamma(const Geometry& g, const FftPlan& p, const void* f, double2* W, cudaStream_t s, int row_lo,
                         int row_hi, const Batch& bt) {
   int sh = gamma_shift(g.ng, g.na, (row_hi - row_lo) * count(bt));
-  const MmLevel lv = gamma_level(p);
+  const MmLevel& lv = p.l1;
   while (sh > 4 && (size_t)g.ng * ((1 << sh) + 4) * (g.real ? 8 : 16) > kSmemMax / 4) sh--;
   const size_t smem = (size_t)g.ng * (g.real ? ((1 << sh) + 4) * 8 : ((1 << sh) + 2) * 16);
   const dim3 grid((g.na + (1 << sh) - 1) >> sh, row_hi - row_lo, count(bt));

@@ -151,7 +151,7 @@ size_t resident_bytes(Device* D) {
     if (t.d) b += (size_t)dl_entries(t.Lcap) * sizeof(double);
   for (const auto& t : D->digit_tables) b += t->bytes + (size_t)t->L * t->N * sizeof(long long);
   for (const auto& t : D->beta_tables) b += t->bytes;
-  for (const auto& kv : D->conv_kernels) b += (size_t)(8 * (kv.first / 2) + 2 * (kv.first / 2)) * sizeof(double2);  // Pc <= 8L, plus 2L
+  for (const auto& kv : D->conv_kernels) b += (size_t)(8 * kv.first + kv.first) * sizeof(double2);  // Pc <= 8L, plus L
   for (const auto& kv : D->beta_matrices) {
     Geometry g{};
     g.L = kv.first / kBetaKinds / 2;
@@ -464,20 +464,17 @@ int ensure_fft_scalar(Device* D, int n, FftPlan* out) {
 // Weight-convolution kernel: wr[r] = (2 pi / Pc) sum_p w(p) e^{+2 pi i p r / Pc},
 // w(p) = int_0^pi e^{-i p theta} sin(theta) d theta (reference
 // src/c/so3_sampling.c:32-51), |p| <= 2(L-1).
-// Tables of the forward beta stage (stages.cu), per (L, sampling), Pc + 2L
-// complex entries:
+// Tables of the forward beta chain (stages.cu; MW), per L, Pc + L complex entries:
 //  [0, Pc)        2 pi / Pc * DFT(w_e): the spectrum of the even part of the
 //                 quadrature weights w_e(p) = 2 / (1 - p^2) (even p, |p| <=
 //                 2(L-1)) that the paired columns are convolved with (real);
-//  [Pc, Pc + L)   h_0(m'): the stage's output for the odd (s = -1) column of
-//                 a unit sample at its first self-mirror beta row (MW: row
-//                 L-1 at beta = pi; MWSS: row 0 at beta = 0), with the full
-//                 weights w (so3_sampling.c:32-51);
-//  [Pc + L, Pc + 2L) h_1(m'): the same for MWSS row L (beta = pi); zero for MW.
+//  [Pc, Pc + L)   h(m'): the stage's output for the odd (s = -1) column of a
+//                 unit sample at its self-mirror beta row L-1 (beta = pi), with
+//                 the full weights w (so3_sampling.c:32-51);
 // h(m') = G(m') - G(-m') (m' >= 1), G(0), with G = 2 pi v * w and v(m'') =
 // e^{-i m'' beta} / P, m'' in [-(L-1), L-1].
 int ensure_conv_kernel(Device* D, const Geometry& g, const double2** out) {
-  const int key = 2 * g.L + (g.mw ? 1 : 0);
+  const int key = g.L;
   auto it = D->conv_kernels.find(key);
   if (it != D->conv_kernels.end()) {
     *out = it->second;
@@ -494,28 +491,22 @@ int ensure_conv_kernel(Device* D, const Geometry& g, const double2** out) {
   std::vector<cld> w(Pc, cld(0, 0));
   for (int p = -2 * (L - 1); p <= 2 * (L - 1); p += 2) w[((p % Pc) + Pc) % Pc] += weight(p);
   fft_ld(w, +1);
-  std::vector<double2> host((size_t)Pc + 2 * (size_t)L, make_double2(0.0, 0.0));
+  std::vector<double2> host((size_t)Pc + (size_t)L, make_double2(0.0, 0.0));
   for (int r = 0; r < Pc; r++) {
     // w_e is real and even: its spectrum is real
     const long double v = w[r].real() * (2.0L * kPiL / (long double)Pc);
     host[r] = make_double2((double)v, 0.0);
   }
-  // correction vectors: v(m'') = (+1 or (-1)^{m''}) / P
-  for (int which = 0; which < (g.mw ? 1 : 2); which++) {
-    const bool alternating = g.mw || which == 1;  // beta = pi
-    std::vector<cld> G(2 * (size_t)L - 1);
-    for (int mp = -(L - 1); mp <= L - 1; mp++) {
-      cld acc(0, 0);
-      for (int mpp = -(L - 1); mpp <= L - 1; mpp++) {
-        const long double v = ((alternating && (mpp & 1)) ? -1.0L : 1.0L) / (long double)P;
-        acc += v * weight((long long)mp - mpp);
-      }
-      G[mp + L - 1] = acc * (2.0L * kPiL);
-    }
-    for (int mp = 0; mp < L; mp++) {
-      const cld h = mp == 0 ? G[L - 1] : G[mp + L - 1] - G[L - 1 - mp];
-      host[(size_t)Pc + (size_t)which * L + mp] = make_double2((double)h.real(), (double)h.imag());
-    }
+  // correction vector: v(m'') = (-1)^{m''} / P
+  std::vector<cld> G(2 * (size_t)L - 1);
+  for (int mp = -(L - 1); mp <= L - 1; mp++) {
+    cld acc(0, 0);
+    for (int mpp = -(L - 1); mpp <= L - 1; mpp++) acc += ((mpp & 1) ? -1.0L : 1.0L) / (long double)P * weight((long long)mp - mpp);
+    G[mp + L - 1] = acc * (2.0L * kPiL);
+  }
+  for (int mp = 0; mp < L; mp++) {
+    const cld h = mp == 0 ? G[L - 1] : G[mp + L - 1] - G[L - 1 - mp];
+    host[(size_t)Pc + mp] = make_double2((double)h.real(), (double)h.imag());
   }
   double2* d = nullptr;
   if (cudaMalloc(&d, host.size() * sizeof(double2)) != cudaSuccess)
