@@ -9,22 +9,22 @@
 //   f_lmn = i^{m-n} sum_{m'=0}^{l} Delta^l_{m'm} Delta^l_{m'n} G[n][m'][m].
 //
 // Both are three-operand contractions (every pair of the free indices shares
-// an operand), so no plain GEMM exists for one signal; the kernels are built
-// for the FP64 pipe:
-//  * Negative m, n use Delta^l_{m',-k} = (-1)^{l+m'} Delta^l_{m'k}: one product
-//    w = Delta_{m'|m|} Delta_{m'|n|} feeds the four sign combinations (+m,+n),
-//    (-m,+n), (+m,-n), (-m,-n) (9 FP64 instructions per 4 complex MACs).  The
-//    (-1)^{l+m'} of combinations with one negative index is split between the
-//    operand that carries l and the one that carries m'.
+// an operand), so no plain GEMM exists for one signal.  Negative m, n use
+// Delta^l_{m',-k} = (-1)^{l+m'} Delta^l_{m'k}: one product w = Delta_{m'|m|}
+// Delta_{m'|n|} feeds the four sign combinations (+m,+n), (-m,+n), (+m,-n),
+// (-m,-n), and the (-1)^{l+m'} of combinations with one negative index is split
+// between the operand that carries l and the one that carries m'.
+//
+// contract_mma_kernel (below, on the FP64 tensor cores) runs every transform.
+// The two kernels before it, on the FP64 FMA pipe, are an independent
+// implementation that the tests compare with (SO3GPU_FP64_MMA=0):
 //  * CTA tile: 32 output rows (m' for the inverse, l for the forward) x 32 |m|
 //    x 2 |n|.  The reduction index (l, resp. m') is walked in chunks of 4,
 //    staged in shared memory with cp.async, double buffered.
 //  * Lanes form an 8 (rows) x 4 (|m|) grid, warps step |m| by 4: a warp reads
 //    32 distinct Delta_{m'|m|} (2 wavefronts with the 36-double row pitch),
 //    8 distinct Delta_{m'|n|} pairs and 4 distinct coefficient quadruples
-//    (1 wavefront each), for 72 FP64 instructions per lane.
-//  * Grid order |n|-pair fastest, then rows, then |m|: CTAs resident at the
-//    same time share one Delta tile column and one coefficient slice in L2.
+//    (1 wavefront each), for 72 FP64 instructions per lane (9 per 4 complex MACs).
 #include <cstdlib>
 #include <type_traits>
 
