@@ -147,8 +147,11 @@ int drain(DropIn* X, int rc) {
   const cudaError_t a = cudaStreamSynchronize(X->cin);
   const cudaError_t b = cudaStreamSynchronize(X->stream);
   const cudaError_t c = cudaStreamSynchronize(X->cout);
-  const int fault = so3g::take_fault(&X->wk);
-  if (rc || fault) return rc ? rc : fault;
+  if (rc) {
+    so3g::clear_fault(&X->wk);  // this call's, not the next one's
+    return rc;
+  }
+  if (int fault = so3g::take_fault(&X->wk)) return fault;
   const cudaError_t e = a != cudaSuccess ? a : (b != cudaSuccess ? b : c);
   if (e != cudaSuccess) return so3g::fail(so3g::kCudaError, std::string("staged transform: ") + cudaGetErrorString(e));
   return so3g::kOk;
@@ -221,6 +224,7 @@ int dropin_adjoint(void* out, const void* in, const so3_parameters_t* p, bool in
                          : so3g::run_adjoint_forward(D, &X->wk, *p, din, dout, X->stream);
   if (rc) {
     cudaStreamSynchronize(X->stream);
+    so3g::clear_fault(&X->wk);
     return rc;
   }
   return download(X, out, dout, inverse ? lb : fb, sout);

@@ -227,6 +227,7 @@ int ensure_ws(Workspace* W, size_t bytes, void** out);
 int open_fault(Workspace* W);
 // kOk, or an error (and the word cleared) if a wait gave up; after the work has ended.
 int take_fault(Workspace* W);
+void clear_fault(Workspace* W);
 // Scratch of up to *n signals of `bytes` each (a multiple of 256), after an
 // ensure_ws for one: *n becomes the number that *out holds, one where no more can be had.
 void chunk_ws(Workspace* W, size_t bytes, cudaStream_t s, int* n, void** out);

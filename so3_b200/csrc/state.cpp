@@ -243,9 +243,12 @@ int open_fault(Workspace* W) {
   *W->fault = 0;
   return kOk;
 }
+void clear_fault(Workspace* W) {
+  if (W->fault) *static_cast<volatile int*>(W->fault) = 0;
+}
 int take_fault(Workspace* W) {
   if (!W->fault || *static_cast<volatile int*>(W->fault) == 0) return kOk;
-  *W->fault = 0;
+  clear_fault(W);
   return fail(kCudaError, "a kernel waited too long for a copy: the results are not valid");
 }
 

@@ -38,3 +38,15 @@ def test_dropin_calls_report_a_wait_that_gave_up(lib, call):
     with pytest.raises(so3.SO3Error, match="status 2"):
         getattr(so3, call)(x, p)
     assert np.array_equal(getattr(so3, call)(x, p), good)  # reported once
+
+
+def test_a_failed_call_leaves_no_report_to_the_next(lib):
+    p, bad = params(12, 3), params(12, 3, sampling=1)
+    f = so3.inverse(synth.gen_flmn(p, 2), p)
+    good = so3.adjoint_inverse(f, p)
+    word = lib.so3g_dropin_fault_word
+    word.restype, word.argtypes = ctypes.POINTER(ctypes.c_int), [ctypes.c_int]
+    word(0)[0] = 4
+    with pytest.raises(so3.SO3Error, match="status 3"):  # adjoints are MW only
+        so3.adjoint_inverse(np.zeros(so3.f_size(bad), np.complex128), bad)
+    assert np.array_equal(so3.adjoint_inverse(f, p), good)
