@@ -573,7 +573,7 @@ int run_inverse_batch(Device* D, Workspace* wk, const so3_parameters_t& p, int r
   int rc;
   const long long wstride = (long long)(bl.wbytes / sizeof(double2));
   const DigitTable* tab = nullptr;
-  if ((rc = ensure_digit_table(D, r.g, p.dl_method, r.dl, s, &tab))) return rc;
+  if ((rc = ensure_digit_table(D, r.g, p.dl_method, r.dl, wk->table_room, s, &tab))) return rc;
   timer_begin(T, s, &ev);
   rc = launch_mixed_inverse(r.g, p.n_mode, reinterpret_cast<const double2* const*>(base + bl.table_off), nsplit, r.bases,
                             r.dl, tab, W, wstride, base + bl.scratch_off, s);
@@ -625,7 +625,7 @@ int run_forward_batch(Device* D, Workspace* wk, const so3_parameters_t& p, int r
       return rc;
   if (nsplit == 0) return kOk;
   const DigitTable* tab = nullptr;
-  if ((rc = ensure_digit_table(D, r.g, p.dl_method, r.dl, s, &tab))) return rc;
+  if ((rc = ensure_digit_table(D, r.g, p.dl_method, r.dl, wk->table_room, s, &tab))) return rc;
   timer_begin(T, s, &ev);
   rc = launch_mixed_forward(r.g, p.n_mode, W, wstride, nsplit, r.bases, r.dl, tab,
                             reinterpret_cast<double2* const*>(base + bl.table_off), p.storage == SO3_STORAGE_COMPACT,
@@ -680,7 +680,7 @@ int run_conv_inverse_batch(Device* D, Workspace* wk, const so3_parameters_t& p, 
   cudaEvent_t ev;
   const long long wstride = (long long)(bl.wbytes / sizeof(double2));
   const DigitTable* tab = nullptr;
-  if ((rc = ensure_digit_table(D, r.g, p.dl_method, r.dl, s, &tab))) return rc;
+  if ((rc = ensure_digit_table(D, r.g, p.dl_method, r.dl, wk->table_room, s, &tab))) return rc;
   timer_begin(T, s, &ev);
   rc = launch_mixed_inverse(r.g, p.n_mode, nullptr, nsig, r.bases, r.dl, tab, W, wstride, base + bl.scratch_off, s,
                             static_cast<const double2*>(flm_d),
@@ -840,7 +840,7 @@ int run_inverse_ragged(Device* D, Workspace* wk, const so3_parameters_t* ps, int
     }
     int Lm = 0, Nm = 0;
     for (const RaggedSig& r : rs[m]) Lm = std::max(Lm, r.g.L), Nm = std::max(Nm, r.g.N);
-    const DigitTable* tab = covering_digit_table(D, Lm, Nm, m, dl, true, s);
+    const DigitTable* tab = covering_digit_table(D, Lm, Nm, m, dl, wk->table_room, s);
     timer_begin(T, s, &ev);
     if ((rc = launch_mixed_ragged(false, rs[m], dl, tab, wsb + sig_end, s))) return rc;
     timer_end(T, s, kStMixInv, ev);
@@ -920,7 +920,7 @@ int run_forward_ragged(Device* D, Workspace* wk, const so3_parameters_t* ps, int
     }
     int Lm = 0, Nm = 0;
     for (const RaggedSig& r : rs[m]) Lm = std::max(Lm, r.g.L), Nm = std::max(Nm, r.g.N);
-    const DigitTable* tab = covering_digit_table(D, Lm, Nm, m, dl, true, s);
+    const DigitTable* tab = covering_digit_table(D, Lm, Nm, m, dl, wk->table_room, s);
     timer_begin(T, s, &ev);
     if ((rc = launch_mixed_ragged(true, rs[m], dl, tab, wsb + sig_end, s))) return rc;
     timer_end(T, s, kStMixFwd, ev);

@@ -1916,7 +1916,7 @@ size_t digit_table_bytes(int L, int N) {
 // use).  Tables are kept until the process exits, so streams that use one
 // never see it change.  Without a table the kernels generate the digits from
 // Delta.
-int ensure_digit_table(Device* D, const Geometry& g, int method, const double* dl, cudaStream_t s,
+int ensure_digit_table(Device* D, const Geometry& g, int method, const double* dl, size_t room, cudaStream_t s,
                        const DigitTable** out, bool force) {
   *out = nullptr;
   const char* env = getenv("SO3GPU_DIGIT_TABLE");
@@ -1937,7 +1937,7 @@ int ensure_digit_table(Device* D, const Geometry& g, int method, const double* d
   for (const auto& t : D->digit_tables) used += t->bytes;
   size_t freeb = 0, total = 0;
   SO3G_CUDA(cudaMemGetInfo(&freeb, &total));
-  if (used + bytes > total / 4 || freeb < bytes + (size_t(4) << 30)) return kOk;  // generate instead
+  if (bytes > room || used + bytes > total / 4 || freeb < bytes + (size_t(4) << 30)) return kOk;  // generate instead
   const int nc = (g.L + kKC - 1) / kKC;
   std::vector<long long> off((size_t)g.L * g.N);
   long long acc = 0;
@@ -1966,10 +1966,10 @@ int ensure_digit_table(Device* D, const Geometry& g, int method, const double* d
 }
 
 // A resident digit table whose (L, N) cover (L, N) for this recursion, for
-// the ragged contractions (digits do not depend on the band limits); with
-// build, the L = 512, N = 64 table is built when none covers and (L, N) fit
+// the ragged contractions (digits do not depend on the band limits); the
+// L = 512, N = 64 table is built when none covers and (L, N) fit
 // it (same memory rule as ensure_digit_table).  Null: generate from Delta.
-const DigitTable* covering_digit_table(Device* D, int L, int N, int method, const double* dl, bool build,
+const DigitTable* covering_digit_table(Device* D, int L, int N, int method, const double* dl, size_t room,
                                        cudaStream_t s) {
   {
     std::lock_guard<std::mutex> lk(D->mu);
@@ -1977,7 +1977,7 @@ const DigitTable* covering_digit_table(Device* D, int L, int N, int method, cons
       if (t->method == method && t->L >= L && t->N >= N) return t.get();
   }
   const char* env = getenv("SO3GPU_DIGIT_TABLE");
-  if (!build || L > 512 || N > 64 || (env && env[0] == '0')) return nullptr;
+  if (L > 512 || N > 64 || (env && env[0] == '0')) return nullptr;
   Geometry g{};
   g.L = 512, g.N = 64;
   const DigitTable* t = nullptr;
@@ -1985,7 +1985,7 @@ const DigitTable* covering_digit_table(Device* D, int L, int N, int method, cons
   // would: the ragged path has no per-geometry history.  The build needs the
   // Delta planes up to l = 511; with a smaller resident Delta table
   // (ensure_digit_table checks) the products generate A from Delta instead.
-  const int rc = ensure_digit_table(D, g, method, dl, s, &t, true);
+  const int rc = ensure_digit_table(D, g, method, dl, room, s, &t, true);
   return rc == kOk ? t : nullptr;
 }
 

@@ -11,7 +11,9 @@
 //    and the callers' input and output buffers of those units.  Scratch comes
 //    from the stream-ordered allocator (cudaMallocAsync / cudaFreeAsync on
 //    the slot's stream), so admitting and retiring work never synchronises
-//    the device.  A request that cannot fit beside the resident tables
+//    the device.  A unit builds a digit table only where the budget holds it
+//    beside everything in flight; without one the split products generate the
+//    digits.  A request that cannot fit beside the resident tables
 //    fails with status 4.
 //  * Batching: queued complex split-precision requests of one direction are
 //    admitted together (up to max_batch) whatever their parameters: the unit
@@ -449,6 +451,8 @@ class Server {
         free_slot->busy = true;
         free_slot->finished.store(false);
         inflight_bytes_ += need;
+        // a table beyond this would leave later requests no room
+        free_slot->wk.table_room = room - inflight_bytes_;
         if (inflight_bytes_ + resident > peak_bytes_) peak_bytes_ = inflight_bytes_ + resident;
         busy_++;
         units_++;

@@ -197,6 +197,9 @@ struct Workspace {
   // holds pointers into ws, which a batch must not free.  Never used by a capture.
   void* chunk = nullptr;
   size_t chunk_bytes = 0;
+  // Largest resident digit table that a call may build (the request server: what
+  // its budget leaves); the split products generate the digits instead.
+  size_t table_room = SIZE_MAX;
   // Host word that a kernel sets when one of its bounded waits gave up and its
   // results are void, for owners that report the end of their calls (null: none).
   int* fault = nullptr;
@@ -329,8 +332,8 @@ int stage_variants(const Geometry& g, const FftPlan& pP, int stage);
 // W + b * wstride); scratch: mixed_scratch_bytes bytes.
 // nsig signals in the contractions, nbeta (forward batches) in the beta stage
 size_t mixed_scratch_bytes(const Geometry& g, int nsig, int nbeta);
-// force: build now instead of on the geometry's second call.
-int ensure_digit_table(Device* D, const Geometry& g, int method, const double* dl, cudaStream_t s,
+// room: see Workspace::table_room; force: build now instead of on the geometry's second call.
+int ensure_digit_table(Device* D, const Geometry& g, int method, const double* dl, size_t room, cudaStream_t s,
                        const DigitTable** out, bool force = false);
 size_t digit_table_bytes(int L, int N);
 // Forward beta stage of a split-precision batch as an int8 tensor-core
@@ -368,8 +371,8 @@ size_t ragged_scratch_bytes(const std::vector<RaggedSig>& sigs, bool fwd);
 int launch_mixed_ragged(bool fwd, const std::vector<RaggedSig>& sigs, const double* dl, const DigitTable* tab,
                         void* scratch, cudaStream_t s);
 // Resident digit table covering (L, N) for a recursion (see mixed.cu), built
-// at L = 512, N = 64 when `build` and none covers; null: digits generated.
-const DigitTable* covering_digit_table(Device* D, int L, int N, int method, const double* dl, bool build,
+// at L = 512, N = 64 when none covers and it fits `room`; null: digits generated.
+const DigitTable* covering_digit_table(Device* D, int L, int N, int method, const double* dl, size_t room,
                                        cudaStream_t s);
 // Reads and clears the flag the tensor-core kernels set when a bounded wait
 // gave up (0: none; synchronous).
